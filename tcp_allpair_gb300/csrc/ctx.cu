@@ -393,6 +393,7 @@ int tcp_destroy(tcp_ctx *c) {
     cudaFree(c->vdf);
     cudaFree(c->rdf_edges);
     cudaFree(c->n3_chunks);
+    cudaFree(c->f64tab);
     cudaFree(c->d_stage);
     cudaFree(c->kvec);
     cudaFree(c->ksum);

@@ -672,6 +672,8 @@ int pair_setup(tcp_ctx *c) {
     c->n_upart = std::max(g.nblk * js, fp64 ? n3_f64_grid(c) : n3_grid(c));
     if (!fp64 && c->pc.cubic)
         if (int rc = n3_prepare_chunks(c)) return rc;
+    if (fp64)
+        if (int rc = n3_f64_prepare(c)) return rc;
     TCP_CUDA(cudaMalloc(&c->fpart, sizeof(double) * 3 * (size_t)c->n * js));
     TCP_CUDA(cudaMalloc(&c->upart, sizeof(double) * (size_t)c->n_upart));
     TCP_CUDA(cudaMemsetAsync(c->upart, 0, sizeof(double) * (size_t)c->n_upart, c->stream));

@@ -1,5 +1,6 @@
-// pair_n3.cuh -- the Newton-3 item schedule shared by the compensated-FP32
-// (pair_n3.cu) and the FP64 (pair_n3_f64.cu) real-space kernels.
+// pair_n3.cuh -- the Newton-3 item schedule of the compensated-FP32 real-space
+// kernels (pair_n3.cu) and the derivative kernels (adjoint.cu), and the
+// arguments they share with the FP64 kernel (pair_n3_f64.cu).
 //
 // Particles are split per species into i-tiles of TILE particles and
 // j-subtiles of kN3Sub (tiles never straddle the e/i boundary).  An item is
@@ -35,8 +36,7 @@ struct N3Args {
     const int4 *xq;                // fixed-point positions (FP32C kernels)
     const double4_32a *xd;         // FP64 positions
     const longlong4_32a *xl;       // 64-bit fixed-point positions (FP64 kernel)
-    long long total;      // items (all systems)
-    long long nstatic;    // FP64: items [0, nstatic) split statically (0: all from the counter)
+    long long total;      // items (all systems; FP32C kernels)
     int ntot;             // stride of facc
     double *facc;         // [3][ntot], zeroed before the launch
     double *upart;        // [gridDim.x] (single system)

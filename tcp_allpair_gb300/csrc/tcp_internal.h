@@ -138,6 +138,9 @@ struct tcp_ctx {
     int4 *xq = nullptr;        // fixed-point positions for the FP32 pair kernel
     double4_32a *xd = nullptr;     // FP64 positions for the FP64 pair kernel
     longlong4_32a *xl = nullptr;   // 64-bit fixed-point positions (2^64 per box length) for the FP64 Newton-3 kernel
+    // radial tables of the FP64 Newton-3 kernel (pair_n3_f64.cu): Ewald and e-i segments
+    void *f64tab = nullptr;
+    int f64_ew_seg = 0, f64_ei_seg = 0;
     // pair-kernel partials
     int jsplit = 1;
     int fpart_splits = 1;      // splits written by the last pair launch
@@ -267,6 +270,7 @@ int launch_force_finalize(tcp_ctx *c, bool add_rec);
 bool n3_applicable(const tcp_ctx *c);
 bool n3_f64_applicable(const tcp_ctx *c);
 int n3_f64_grid(const tcp_ctx *c);
+int n3_f64_prepare(tcp_ctx *c);
 int launch_pair_n3_f64(tcp_ctx *c, bool energy, bool rdf);
 int n3_grid(const tcp_ctx *c);
 int n3_variant_count();
