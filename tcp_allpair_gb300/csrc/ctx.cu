@@ -395,8 +395,7 @@ int tcp_destroy(tcp_ctx *c) {
     cudaFree(c->n3_chunks);
     cudaFree(c->f64tab);
     cudaFree(c->d_stage);
-    cudaFree(c->kvec);
-    cudaFree(c->ksum);
+    ewald_free(c);
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->h_scal) cudaFreeHost(c->h_scal);
     for (auto &e : c->ev)

@@ -449,51 +449,178 @@ __global__ void sum_partials_kernel(const double *__restrict__ part, int np, dou
 }
 
 // ---- plain Ewald k-sum ------------------------------------------------------
-// S(m) = sum_j q_j exp(2 pi i m.x_j) per k-vector (one CTA per vector)
-__global__ void ewald_sfac_kernel(const double *__restrict__ x, int nel, int n, double q0, double q1,
-                                  const double *__restrict__ kvec, double *__restrict__ ksum,
-                                  double *__restrict__ epart) {
-    __shared__ double red[32];
-    const double mx = kvec[4 * blockIdx.x], my = kvec[4 * blockIdx.x + 1], mz = kvec[4 * blockIdx.x + 2];
-    double sr = 0.0, si = 0.0;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        const double q = j < nel ? q0 : q1;
-        const double ph = 2.0 * kPi * (mx * x[j] + my * x[(size_t)n + j] + mz * x[2 * (size_t)n + j]);
-        double s, c;
-        sincos(ph, &s, &c);
-        sr += q * c;
-        si += q * s;
+// S(m) = sum_j q_j exp(2 pi i m.x_j) and the forces, by the product form
+// exp(2 pi i m.x) = ex[n1] ey[n2] ez[n3] of one phase factor per particle, axis
+// and index instead of a sine and cosine per particle and k-vector, and over
+// the half space n1 >= 0 (S(-m) is the conjugate; n1 > 0 counts twice).  Bound:
+// the FP64 pipe, about 5 operations per (k, j) for S and 7 per (k, i) for the
+// forces, one complex factor ey ez serving all n1 of a column (n2, n3).  N =
+// 1,024, |n|^2 <= 64 (2,108 vectors): 74 us for the whole sum, 2,922 us with
+// sincos per term and the force kernel on N/128 CTAs.
+//
+// Items: a column (n2, n3) with up to kEwN1 consecutive n1, columns with the
+// longest n1 range first, so that the lanes of a warp run equally far.
+constexpr int kEwN1 = 9;
+constexpr int kEwThreads = 256;
+constexpr int kEwPart = 8;        // particles whose phases a CTA holds at a time
+
+struct EwArgs {
+    const double *x;
+    int nel, n;
+    double q0, q1;
+    double iL[3];
+    int nm;               // largest index
+    int nitem;
+    const int4 *item;     // n2, n3, first n1, n1 count
+    const double *th;     // [kEwN1][nitem]: theta(m), doubled for n1 > 0, 0 outside the sphere
+    double2 *part;        // [CTA][kEwN1][nitem] partial S
+    double2 *Z;           // [kEwN1][nitem]: th conj(S)
+    double *epart;
+    int nblk, per;        // CTAs of the S kernel, particles per CTA
+};
+
+// exp(2 pi i n u) with n u reduced to the nearest integer first (exact for the
+// leading part of the product, so the phase error does not grow with n)
+__device__ __forceinline__ double2 ew_phase(int n, double u) {
+    const double p = n * u, e = fma((double)n, u, -p);
+    const double f = (p - rint(p)) + e;
+    double s, c;
+    sincospi(2.0 * f, &s, &c);
+    return make_double2(c, s);
+}
+
+// partial S over the particles of this CTA, one item per thread (grid.y groups of items)
+__global__ void __launch_bounds__(kEwThreads) ewald_sfac_kernel(const EwArgs a) {
+    extern __shared__ double2 ph[];               // [3][nm + 1][kEwPart]
+    __shared__ double sq[kEwPart];
+    const int np = a.nm + 1;
+    const int it = blockIdx.y * kEwThreads + threadIdx.x;
+    const int4 im = it < a.nitem ? a.item[it] : make_int4(0, 0, 0, 0);
+    const int i2 = abs(im.x), i3 = abs(im.y);
+    const double s2 = im.x < 0 ? -1.0 : 1.0, s3 = im.y < 0 ? -1.0 : 1.0;
+    const int cnt = __reduce_max_sync(0xffffffffu, im.w);
+    double2 S[kEwN1];
+#pragma unroll
+    for (int k = 0; k < kEwN1; ++k) S[k] = make_double2(0.0, 0.0);
+    const int j0 = blockIdx.x * a.per, j1 = min(a.n, j0 + a.per);
+    for (int jb = j0; jb < j1; jb += kEwPart) {
+        const int nj = min(kEwPart, j1 - jb);
+        __syncthreads();
+        for (int k = threadIdx.x; k < 3 * np * nj; k += kEwThreads) {
+            const int j = k % nj, r = k / nj, n = r % np, d = r / np;
+            ph[(d * np + n) * kEwPart + j] = ew_phase(n, a.x[(size_t)d * a.n + jb + j] * a.iL[d]);
+        }
+        if (threadIdx.x < nj) sq[threadIdx.x] = jb + (int)threadIdx.x < a.nel ? a.q0 : a.q1;
+        __syncthreads();
+        for (int j = 0; j < nj; ++j) {
+            const double2 ey = ph[(np + i2) * kEwPart + j], ez = ph[(2 * np + i3) * kEwPart + j];
+            const double q = sq[j], yr = q * ey.x, yi = (q * s2) * ey.y, zi = s3 * ez.y;
+            const double er = fma(yr, ez.x, -yi * zi), ei = fma(yr, zi, yi * ez.x);
+            const double2 *ex = ph + im.z * kEwPart + j;
+#pragma unroll
+            for (int k = 0; k < kEwN1; ++k)
+                if (k < cnt) {
+                    const double2 e = ex[min(k, np - 1 - im.z) * kEwPart];
+                    S[k].x = fma(er, e.x, fma(-ei, e.y, S[k].x));
+                    S[k].y = fma(er, e.y, fma(ei, e.x, S[k].y));
+                }
+        }
     }
-    sr = block_sum(sr, red);
-    si = block_sum(si, red);
-    if (threadIdx.x == 0) {
-        ksum[2 * blockIdx.x] = sr;
-        ksum[2 * blockIdx.x + 1] = si;
-        epart[blockIdx.x] = kvec[4 * blockIdx.x + 3] * (sr * sr + si * si);
+    if (it < a.nitem) {
+        double2 *o = a.part + (size_t)blockIdx.x * kEwN1 * a.nitem + it;
+#pragma unroll
+        for (int k = 0; k < kEwN1; ++k) o[(size_t)k * a.nitem] = S[k];
     }
 }
 
-// F_i = (2 eps q_i / V) sum_m theta m Im(conj(S) e^{i phase})
-__global__ void ewald_force_kernel(const double *__restrict__ x, int nel, int n, double q0, double q1,
-                                   const double *__restrict__ kvec, const double *__restrict__ ksum, int nk,
-                                   double coef, double *__restrict__ frec) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double q = i < nel ? q0 : q1;
-    const double xi = x[i], yi = x[(size_t)n + i], zi = x[2 * (size_t)n + i];
-    double fx = 0.0, fy = 0.0, fz = 0.0;
-    for (int k = 0; k < nk; ++k) {
-        const double mx = kvec[4 * k], my = kvec[4 * k + 1], mz = kvec[4 * k + 2], th = kvec[4 * k + 3];
-        double s, c;
-        sincos(2.0 * kPi * (mx * xi + my * yi + mz * zi), &s, &c);
-        const double im = (ksum[2 * k] * s - ksum[2 * k + 1] * c) * th;
-        fx += im * mx;
-        fy += im * my;
-        fz += im * mz;
+// Z = th conj(S), S the sum of the partials (a warp per eight vectors: lanes
+// over the CTAs' partials would stride by whole arrays), and the energy
+// partials sum th |S|^2 per CTA
+__global__ void __launch_bounds__(kEwThreads) ewald_sum_kernel(const EwArgs a) {
+    __shared__ double2 sm[kEwThreads];
+    __shared__ double red[32];
+    const int total = kEwN1 * a.nitem;
+    const int v = threadIdx.x & 31, w = threadIdx.x >> 5, k = blockIdx.x * 32 + v;   // 32 vectors, 8 slices
+    double sr = 0.0, si = 0.0;
+    if (k < total)
+        for (int b = w; b < a.nblk; b += kEwThreads / 32) {
+            const double2 z = a.part[(size_t)b * total + k];
+            sr += z.x;
+            si += z.y;
+        }
+    sm[threadIdx.x] = make_double2(sr, si);
+    __syncthreads();
+    double e = 0.0;
+    if (w == 0 && k < total) {
+        sr = si = 0.0;
+        for (int b = 0; b < kEwThreads / 32; ++b) {
+            sr += sm[b * 32 + v].x;
+            si += sm[b * 32 + v].y;
+        }
+        const double t = a.th[k];
+        a.Z[k] = make_double2(t * sr, -t * si);
+        e = t * fma(sr, sr, si * si);
     }
-    frec[i] = coef * q * fx;
-    frec[(size_t)n + i] = coef * q * fy;
-    frec[2 * (size_t)n + i] = coef * q * fz;
+    e = block_sum(e, red);
+    if (threadIdx.x == 0) a.epart[blockIdx.x] = e;
+}
+
+// F_i = (2 eps q_i / V) sum_m theta m Im(conj(S) e^{i phase}); a warp per
+// particle, lanes over the items, so every particle count fills the SMs and
+// the sum over k-vectors ends in one warp reduction.  The last CTA adds up the
+// energy partials.
+__global__ void __launch_bounds__(kEwThreads) ewald_force_kernel(const EwArgs a, double coef,
+                                                                 double *__restrict__ frec, int npart, double escale,
+                                                                 double *__restrict__ um) {
+    extern __shared__ double2 ph[];               // [warps][3][nm + 1]
+    __shared__ double red[32];
+    if (blockIdx.x == gridDim.x - 1) {
+        double e = 0.0;
+        for (int k = threadIdx.x; um && k < npart; k += kEwThreads) e += a.epart[k];
+        e = block_sum(e, red);
+        if (um && threadIdx.x == 0) *um = e * escale;
+        return;
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, np = a.nm + 1;
+    const int i = blockIdx.x * (kEwThreads / 32) + warp;
+    if (i >= a.n) return;                         // warp-uniform
+    double2 *p = ph + (size_t)warp * 3 * np;
+    for (int k = lane; k < 3 * np; k += 32) p[k] = ew_phase(k % np, a.x[(size_t)(k / np) * a.n + i] * a.iL[k / np]);
+    __syncwarp();
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    for (int it = lane; it < a.nitem; it += 32) {
+        const int4 im = a.item[it];
+        double tr = 0.0, ti = 0.0, xr = 0.0, xi = 0.0;   // sum t_k, sum k t_k (as the sum of the suffix sums)
+        for (int k = im.w - 1; k >= 0; --k) {
+            const double2 z = a.Z[(size_t)k * a.nitem + it], e = p[im.z + k];
+            tr = fma(z.x, e.x, fma(-z.y, e.y, tr));
+            ti = fma(z.x, e.y, fma(z.y, e.x, ti));
+            if (k > 0) {
+                xr += tr;
+                xi += ti;
+            }
+        }
+        if (im.z) {
+            xr = fma((double)im.z, tr, xr);
+            xi = fma((double)im.z, ti, xi);
+        }
+        const double2 ey = p[np + abs(im.x)], ez = p[2 * np + abs(im.y)];
+        const double yi = im.x < 0 ? -ey.y : ey.y, zi = im.y < 0 ? -ez.y : ez.y;
+        const double er = fma(ey.x, ez.x, -yi * zi), ei = fma(ey.x, zi, yi * ez.x);
+        const double im_t = fma(er, ti, ei * tr);
+        fx = fma(er, xi, fma(ei, xr, fx));
+        fy = fma((double)im.x, im_t, fy);
+        fz = fma((double)im.y, im_t, fz);
+    }
+    fx = warp_sum(fx);
+    fy = warp_sum(fy);
+    fz = warp_sum(fz);
+    if (lane == 0) {
+        const double q = coef * (i < a.nel ? a.q0 : a.q1);
+        frec[i] = q * a.iL[0] * fx;
+        frec[(size_t)a.n + i] = q * a.iL[1] * fy;
+        frec[2 * (size_t)a.n + i] = q * a.iL[2] * fz;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -836,6 +963,15 @@ int launch_spme(tcp_ctx *c, bool energy) {
     return TCP_OK;
 }
 
+void ewald_free(tcp_ctx *c) {
+    void **bufs[] = {(void **)&c->kvec, (void **)&c->kS4, (void **)&c->ew_item, (void **)&c->ew_th,
+                     (void **)&c->ew_part, (void **)&c->ew_z};
+    for (void **b : bufs) {
+        cudaFree(*b);
+        *b = nullptr;
+    }
+}
+
 int ewald_setup(tcp_ctx *c) {
     const tcp_params &p = c->p;
     const int nmax2 = p.ewald_nmax2;
@@ -856,16 +992,50 @@ int ewald_setup(tcp_ctx *c) {
     c->nk = (int)(kv.size() / 4);
     if (c->nk > c->red_cap - 7 * kick_blocks(c->n))
         return set_error(TCP_ERR_BAD_PARAM, "ewald_nmax2 too large: more k-vectors than the energy buffer holds");
-    cudaFree(c->kvec);
-    cudaFree(c->ksum);
-    cudaFree(c->kS4);
-    c->kvec = nullptr;
-    c->ksum = nullptr;
-    c->kS4 = nullptr;
+    ewald_free(c);
     if (c->nk == 0) return TCP_OK;
     TCP_CUDA(cudaMalloc(&c->kvec, sizeof(double) * kv.size()));
-    TCP_CUDA(cudaMalloc(&c->ksum, sizeof(double) * 2 * (size_t)c->nk));
     TCP_CUDA(cudaMemcpyAsync(c->kvec, kv.data(), sizeof(double) * kv.size(), cudaMemcpyHostToDevice, c->stream));
+    // items of the half space n1 >= 0, the longest columns first
+    std::vector<int4> items;
+    for (int base = 0; base <= nm; base += kEwN1)
+        for (int n3 = -nm; n3 <= nm; ++n3)
+            for (int n2 = -nm; n2 <= nm; ++n2) {
+                const int rest = nmax2 - n2 * n2 - n3 * n3;
+                int top = -1;
+                while (top < nm && (top + 1) * (top + 1) <= rest) ++top;
+                if (top >= base) items.push_back(make_int4(n2, n3, base, std::min(kEwN1, top - base + 1)));
+            }
+    std::stable_sort(items.begin(), items.end(), [](const int4 &p, const int4 &q) { return p.w > q.w; });
+    const int ni = (int)items.size();
+    std::vector<double> th((size_t)kEwN1 * ni, 0.0);
+    for (int it = 0; it < ni; ++it)
+        for (int k = 0; k < items[it].w; ++k) {
+            const int n1 = items[it].z + k;
+            if (n1 == 0 && items[it].x == 0 && items[it].y == 0) continue;
+            const double m[3] = {n1 / p.box[0], items[it].x / p.box[1], items[it].y / p.box[2]};
+            const double m2 = m[0] * m[0] + m[1] * m[1] + m[2] * m[2];
+            th[(size_t)k * ni + it] = (n1 > 0 ? 2.0 : 1.0) * std::exp(-m2 * kPi * kPi / (c->alpha * c->alpha)) / m2;
+        }
+    // CTAs of the S kernel: one per SM and group of items, fewer where their
+    // partial sums would take more than 64 MB
+    const size_t per_cta = sizeof(double2) * kEwN1 * (size_t)ni;
+    int blocks = std::min((c->n + kEwPart - 1) / kEwPart, c->num_sms);
+    blocks = std::max(1, std::min<int>(blocks, (int)((64u << 20) / per_cta)));
+    const int per = (((c->n + blocks - 1) / blocks) + kEwPart - 1) / kEwPart * kEwPart;
+    c->ew_nblk = (c->n + per - 1) / per;
+    c->ew_per = per;
+    c->ew_nitem = ni;
+    c->ew_nm = nm;
+    if (cudaMalloc(&c->ew_item, sizeof(int4) * (size_t)ni) != cudaSuccess ||
+        cudaMalloc(&c->ew_th, sizeof(double) * th.size()) != cudaSuccess ||
+        cudaMalloc(&c->ew_part, per_cta * c->ew_nblk) != cudaSuccess || cudaMalloc(&c->ew_z, per_cta) != cudaSuccess)
+        return set_error(TCP_ERR_NOMEM, "Ewald sum: device allocation failed");
+    TCP_CUDA(cudaMemcpyAsync(c->ew_item, items.data(), sizeof(int4) * (size_t)ni, cudaMemcpyHostToDevice, c->stream));
+    TCP_CUDA(cudaMemcpyAsync(c->ew_th, th.data(), sizeof(double) * th.size(), cudaMemcpyHostToDevice, c->stream));
+    const int smem = (int)(sizeof(double2) * 3 * (size_t)(nm + 1) * std::max(kEwPart, kEwThreads / 32));
+    TCP_CUDA(cudaFuncSetAttribute(ewald_sfac_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    TCP_CUDA(cudaFuncSetAttribute(ewald_force_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     TCP_CUDA(cudaStreamSynchronize(c->stream));
     return TCP_OK;
 }
@@ -876,16 +1046,30 @@ int launch_ewald(tcp_ctx *c, bool energy) {
         TCP_CUDA(cudaMemsetAsync(c->scal + kScalUm, 0, sizeof(double), c->rstream));
         return TCP_OK;
     }
-    const double q0 = c->p.charge_scale * c->p.q[0], q1 = c->p.charge_scale * c->p.q[1];
-    double *epart = recip_epart(c);
-    ewald_sfac_kernel<<<c->nk, 256, 0, c->rstream>>>(c->x, c->nel, c->n, q0, q1, c->kvec, c->ksum, epart);
-    ewald_force_kernel<<<(c->n + 127) / 128, 128, 0, c->rstream>>>(c->x, c->nel, c->n, q0, q1, c->kvec, c->ksum,
-                                                                  c->nk, 2.0 * kEps / c->V, c->frec);
-    c->launches += 2;
-    if (energy) {
-        sum_partials_kernel<<<1, 1024, 0, c->rstream>>>(epart, c->nk, kEps / (2.0 * kPi * c->V), c->scal + kScalUm);
-        c->launches++;
-    }
+    EwArgs a;
+    a.x = c->x;
+    a.nel = c->nel;
+    a.n = c->n;
+    a.q0 = c->p.charge_scale * c->p.q[0];
+    a.q1 = c->p.charge_scale * c->p.q[1];
+    for (int d = 0; d < 3; ++d) a.iL[d] = 1.0 / c->p.box[d];
+    a.nm = c->ew_nm;
+    a.nitem = c->ew_nitem;
+    a.item = c->ew_item;
+    a.th = c->ew_th;
+    a.part = c->ew_part;
+    a.Z = c->ew_z;
+    a.epart = recip_epart(c);
+    a.nblk = c->ew_nblk;
+    a.per = c->ew_per;
+    const size_t phases = sizeof(double2) * 3 * (size_t)(a.nm + 1);
+    const dim3 sgrid(a.nblk, (a.nitem + kEwThreads - 1) / kEwThreads);
+    const int nsum = (kEwN1 * a.nitem + 31) / 32, wpb = kEwThreads / 32;
+    ewald_sfac_kernel<<<sgrid, kEwThreads, phases * kEwPart, c->rstream>>>(a);
+    ewald_sum_kernel<<<nsum, kEwThreads, 0, c->rstream>>>(a);
+    ewald_force_kernel<<<(c->n + wpb - 1) / wpb + 1, kEwThreads, phases * wpb, c->rstream>>>(
+        a, 2.0 * kEps / c->V, c->frec, nsum, kEps / (2.0 * kPi * c->V), energy ? c->scal + kScalUm : nullptr);
+    c->launches += 3;
     TCP_CUDA(cudaGetLastError());
     return TCP_OK;
 }

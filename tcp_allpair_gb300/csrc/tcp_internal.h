@@ -199,7 +199,10 @@ struct tcp_ctx {
     // plain Ewald
     int nk = 0;
     double *kvec = nullptr;             // [nk][4]: m_x, m_y, m_z, theta
-    double *ksum = nullptr;             // [nk][2]: S re, im
+    int ew_nm = 0, ew_nitem = 0, ew_nblk = 0, ew_per = 0;   // items of the half space, CTAs and particles per CTA of the S kernel
+    int4 *ew_item = nullptr;
+    double *ew_th = nullptr;            // [kEwN1][ew_nitem] weights
+    double2 *ew_part = nullptr, *ew_z = nullptr;   // partial S, weighted conj(S)
     // graph of one md step
     cudaGraphExec_t graph = nullptr;
     double graph_dt = 0.0;
@@ -306,6 +309,7 @@ std::vector<double> bspline_moduli(int order, int K);
 int spme_free(tcp_ctx *c);
 int launch_spme(tcp_ctx *c, bool energy);
 int ewald_setup(tcp_ctx *c);
+void ewald_free(tcp_ctx *c);
 int launch_ewald(tcp_ctx *c, bool energy);
 // integrate.cu
 double *fsum_part(tcp_ctx *c);
