@@ -23,7 +23,7 @@
 #include <vector>
 
 #include "device_util.cuh"
-#include "spme_math.cuh"
+#include "spme_chain.cuh"
 #include "tcp_internal.h"
 
 namespace tcp {
@@ -36,7 +36,7 @@ struct BRep {
     double ixm[2];           // 1/xm
     int K[3], Kh;
     long long mesh_off, half_off;
-    int bin_off, grp_off;    // first spreading bin (K2 K3 per replica) and first 8-row group
+    int bin_off, plane_off;  // first spreading bin (K2 K3 per replica) and mesh plane
     double V;
     double Te, Ti, tau;
     int thermo;
@@ -70,22 +70,53 @@ struct BParticles {
     int ntot;
 };
 
-// VVerletNotemp1 (vverlet.f90:148-167) per replica
-__global__ void b_vverlet1_kernel(const BParticles a, double dt) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.ntot) return;
-    const BRep &R = a.reps[a.rep_of[i]];
-    const double ixm = (i - R.off) < R.nel ? R.ixm[0] : R.ixm[1];
-    int q[3];
-    for (int k = 0; k < 3; ++k) {
-        const size_t o = (size_t)k * a.ntot + i;
+// bins of one CTA's particles (sb, sa: base indexes and spline arguments per component)
+__device__ __forceinline__ void b_bin_store(const BParticles &a, const ChainArgs &c, const SpmeGeom &g, int i, int k,
+                                            int (*sb)[kPartBlock], double (*sa)[kPartBlock]) {
+    const double arg[3] = {sa[0][k], sa[1][k], sa[2][k]};
+    bin_store<float>(c.b, i, a.ntot, arg, i - g.off < g.nel ? g.q[0] : g.q[1], sb[0][k], sb[1][k], sb[2][k], g.K[1],
+                     g.bin_off);
+}
+
+// VVerletNotemp1 (vverlet.f90:148-167) per replica, a thread per component,
+// with the binning of the SPME chains and the clearing of the pair accumulators
+__global__ void __launch_bounds__(kPartThreads) b_vverlet1_kernel(const BParticles a, double dt, const ChainArgs c,
+                                                                  unsigned *counter, double *acc, int nacc) {
+    __shared__ int sb[3][kPartBlock];
+    __shared__ double sa[3][kPartBlock];
+    const int k = threadIdx.x % kPartBlock, d = threadIdx.x / kPartBlock, i = blockIdx.x * kPartBlock + k;
+    const int r = i < a.ntot ? a.rep_of[i] : 0;
+    const BRep &R = a.reps[r];
+    const SpmeGeom &g = c.many[r];
+    if (i < a.ntot) {
+        const double ixm = (i - R.off) < R.nel ? R.ixm[0] : R.ixm[1];
+        const size_t o = (size_t)d * a.ntot + i;
         const double vk = a.v[o] + 0.5 * dt * a.f[o] * ixm;
         a.v[o] = vk;
-        const double y = wrap_box(a.x[o] + dt * vk, R.L[k], R.iL[k]);
+        const double y = wrap_fast(a.x[o] + dt * vk, R.L[d], R.iL[d]);
         a.x[o] = y;
-        q[k] = fixed_coord(y, R.iL[k]);
+        reinterpret_cast<int *>(a.xq + i)[d] = fixed_coord(y, R.iL[d]);
+        a.facc[o] = 0.0;
+        sb[d][k] = bin_axis(y, g.hL[d], g.KL[d], g.K[d], c.P, sa[d][k]);
     }
-    a.xq[i] = make_int4(q[0], q[1], q[2], 0);
+    const int t = blockIdx.x * kPartThreads + threadIdx.x;
+    for (int u = t; u < nacc; u += gridDim.x * kPartThreads) acc[u] = 0.0;
+    if (t == 0) *counter = 0u;
+    __syncthreads();
+    if (i < a.ntot && d == 0) b_bin_store(a, c, g, i, k, sb, sa);
+    if (c.nbins <= kScanTail && last_block(c.ticket)) scan_bins(c.b, c.nbins);
+}
+
+// the binning alone (a force call without a step)
+__global__ void __launch_bounds__(kPartThreads) b_bin_kernel(const BParticles a, const ChainArgs c) {
+    __shared__ int sb[3][kPartBlock];
+    __shared__ double sa[3][kPartBlock];
+    const int k = threadIdx.x % kPartBlock, d = threadIdx.x / kPartBlock, i = blockIdx.x * kPartBlock + k;
+    const SpmeGeom &g = c.many[i < a.ntot ? a.rep_of[i] : 0];
+    if (i < a.ntot) sb[d][k] = bin_axis(a.x[(size_t)d * a.ntot + i], g.hL[d], g.KL[d], g.K[d], c.P, sa[d][k]);
+    __syncthreads();
+    if (i < a.ntot && d == 0) b_bin_store(a, c, g, i, k, sb, sa);
+    if (c.nbins <= kScanTail && last_block(c.ticket)) scan_bins(c.b, c.nbins);
 }
 
 __global__ void b_refresh_kernel(const BParticles a) {
@@ -94,149 +125,6 @@ __global__ void b_refresh_kernel(const BParticles a) {
     const BRep &R = a.reps[a.rep_of[i]];
     a.xq[i] = make_int4(fixed_coord(a.x[i], R.iL[0]), fixed_coord(a.x[(size_t)a.ntot + i], R.iL[1]),
                         fixed_coord(a.x[2 * (size_t)a.ntot + i], R.iL[2]), 0);
-}
-
-// ---- atomic-free spreading, cell-sorted per replica ------------------------------
-// The single-system scheme of spme.cu over all replicas: particles are binned by
-// the (y, z) mesh column of their spline base (replica r owns bins
-// [bin_off, bin_off + K2 K3)), the bins are index-ordered, and a warp gathers 8
-// mesh rows of one replica from the bins that reach them, summing in
-// compensated two-float FP32 (no atomics; the same order on every call).
-constexpr int kBRows = 8;
-constexpr int kBRowWarps = 4;
-
-template <int P>
-__global__ void b_bin_count_kernel(const BParticles a, SpreadBins bins) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.ntot) return;
-    const BRep &R = a.reps[a.rep_of[i]];
-    int base[3];
-#pragma unroll
-    for (int d = 1; d < 3; ++d) {
-        const double u = (a.x[(size_t)d * a.ntot + i] + R.L[d] * .5) * R.KL[d];
-        base[d] = wrapi((int)trunc(u) - (P - 3), R.K[d]);
-    }
-    const int bin = R.bin_off + base[1] + R.K[1] * base[2];
-    bins.rank[i] = atomicAdd(&bins.count[bin], 1);
-    bins.ebx[i] = bin;
-}
-
-template <int P>
-__global__ void b_bin_weights_kernel(const BParticles a, SpreadBins bins) {
-    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pos >= a.ntot) return;
-    const int i = bins.list[pos];
-    const BRep &R = a.reps[a.rep_of[i]];
-    float *w = static_cast<float *>(bins.ew) + (size_t)pos * 3 * P;
-    float W[P], dW[P];
-    int base[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const double u = (a.x[(size_t)d * a.ntot + i] + R.L[d] * .5) * R.KL[d];
-        spline_w<P, float>(u, W, dW);
-#pragma unroll
-        for (int j = 0; j < P; ++j) w[d * P + j] = W[j];
-        base[d] = wrapi((int)trunc(u) - (P - 3), R.K[d]);
-    }
-    bins.ebx[pos] = base[0];
-    bins.eby[pos] = base[1];
-    static_cast<float *>(bins.eq)[pos] = (float)((i - R.off) < R.nel ? R.q[0] : R.q[1]);
-}
-
-__host__ __device__ constexpr size_t b_row_warp_bytes(int P, int k1max) {
-    return (size_t)kBRows * k1max * 8 + 32 * (8 + (1 + 3 * P) * 4);
-}
-
-template <int P>
-__global__ void __launch_bounds__(32 * kBRowWarps) b_row_spread_kernel(const BParticles a, const SpreadBins bins,
-                                                                       int nrep, int ngroups, int k1max,
-                                                                       float *__restrict__ Qf) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = blockIdx.x * (blockDim.x >> 5) + warp;
-    if (g >= ngroups) return;                                     // warp-uniform
-    int lo = 0, hi_ = nrep - 1;
-    while (lo < hi_) {
-        const int mid = (lo + hi_ + 1) >> 1;
-        if (a.reps[mid].grp_off <= g) lo = mid; else hi_ = mid - 1;
-    }
-    const BRep &R = a.reps[lo];
-    const int K1 = R.K[0], K2 = R.K[1], K3 = R.K[2];
-    const int ngy = (K2 + kBRows - 1) / kBRows, lg = g - R.grp_off;
-    const int y0 = (lg % ngy) * kBRows, z = lg / ngy;
-    const int nrow = min(kBRows, K2 - y0);
-    unsigned char *base = smem + (size_t)warp * b_row_warp_bytes(P, k1max);
-    float *hi = reinterpret_cast<float *>(base);                    // [kBRows][K1]
-    float *lo_ = hi + (size_t)kBRows * k1max;
-    float *sw = lo_ + (size_t)kBRows * k1max;                       // [32][3P]
-    float *sq = sw + 32 * 3 * P;
-    int *sbx = reinterpret_cast<int *>(sq + 32), *sby = sbx + 32;
-    for (int k = lane; k < kBRows * K1; k += 32) {
-        hi[k] = 0.f;
-        lo_[k] = 0.f;
-    }
-    __syncwarp();
-    const float *ew = static_cast<const float *>(bins.ew);
-    const float *eq = static_cast<const float *>(bins.eq);
-    const int nb = nrow + P - 1;
-    for (int jz = 0; jz < P; ++jz) {
-        int bz = z - jz;
-        bz += bz < 0 ? K3 : 0;
-        int by0 = y0 - P + 1, len0 = nb, len1 = 0;
-        if (by0 < 0) {
-            by0 += K2;
-            len0 = min(nb, K2 - by0);
-            len1 = nb - len0;
-        }
-        if (nb >= K2) {
-            by0 = 0;
-            len0 = K2;
-            len1 = 0;
-        }
-        for (int piece = 0; piece < 2; ++piece) {
-            const int blo = R.bin_off + (piece == 0 ? by0 : 0) + K2 * bz, len = piece == 0 ? len0 : len1;
-            if (len <= 0) continue;
-            const int p0 = bins.start[blo], p1 = bins.start[blo + len];
-            for (int c0 = p0; c0 < p1; c0 += 32) {
-                const int ne = min(32, p1 - c0);
-                if (lane < ne) {
-                    const int pos = c0 + lane;
-#pragma unroll
-                    for (int j = 0; j < 3 * P; ++j) sw[lane * 3 * P + j] = ew[(size_t)pos * 3 * P + j];
-                    sq[lane] = eq[pos];
-                    sbx[lane] = bins.ebx[pos];
-                    sby[lane] = bins.eby[pos];
-                }
-                __syncwarp();
-                for (int e = 0; e < ne; ++e) {
-                    const float *w = sw + e * 3 * P;
-                    const float qz = sq[e] * w[2 * P + jz];
-                    const int bx = sbx[e], by = sby[e];
-                    for (int l = lane; l < P * P; l += 32) {
-                        const int jy = l / P, jx = l - jy * P;
-                        int rl = by + jy - y0;
-                        rl += rl < 0 ? K2 : 0;
-                        rl -= rl >= K2 ? K2 : 0;
-                        if (rl < nrow) {
-                            int x = bx + jx;
-                            x -= x >= K1 ? K1 : 0;
-                            const float v = qz * w[P + jy] * w[jx];
-                            const int k = rl * K1 + x;
-                            const float sum = hi[k] + v, bp = sum - hi[k];
-                            lo_[k] += (hi[k] - (sum - bp)) + (v - bp);
-                            hi[k] = sum;
-                        }
-                    }
-                    __syncwarp();
-                }
-            }
-        }
-    }
-    float *mesh = Qf + R.mesh_off;
-    for (int k = lane; k < nrow * K1; k += 32) {
-        const int rl = k / K1, x = k - rl * K1;
-        mesh[(size_t)K1 * ((y0 + rl) + (size_t)K2 * z) + x] = hi[k] + lo_[k];
-    }
 }
 
 // influence multiply; blocks [blk0[r], blk0[r+1]) belong to replica r
@@ -272,53 +160,6 @@ __global__ void b_influence_kernel(cufftComplex *__restrict__ Qk, const float *_
     }
     const double t = block_sum((double)e, red);
     if (threadIdx.x == 0) atomicAdd(&um[lo], t * kEps / (2.0 * kPi * R.V));
-}
-
-// Particles in the cell-sort order of the spread (order[t]): the lanes of a
-// warp share replicas and mesh columns; mesh indices wrap by comparison.
-template <int P>
-__global__ void b_gather_kernel(const BParticles a, const float *__restrict__ phi, const int *__restrict__ order) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= a.ntot) return;
-    const int i = order[t];
-    const BRep &R = a.reps[a.rep_of[i]];
-    const double q = (i - R.off) < R.nel ? R.q[0] : R.q[1];
-    float W[3][P], dW[3][P];
-    int base[3];
-    for (int d = 0; d < 3; ++d) {
-        const double u = (a.x[(size_t)d * a.ntot + i] + R.L[d] * .5) * R.KL[d];
-        spline_w<P, float>(u, W[d], dW[d]);
-        base[d] = wrapi((int)trunc(u) - (P - 3), R.K[d]);
-    }
-    const float *mesh = phi + R.mesh_off;
-    float gx = 0.f, gy = 0.f, gz = 0.f;
-    int iz = base[2];
-#pragma unroll 1
-    for (int k = 0; k < P; ++k) {
-        int iy = base[1];
-#pragma unroll 1
-        for (int j = 0; j < P; ++j) {
-            const float *row = mesh + (size_t)R.K[0] * (iy + (size_t)R.K[1] * iz);
-            float sx = 0.f, sd = 0.f;
-            int ix = base[0];
-#pragma unroll
-            for (int ii = 0; ii < P; ++ii) {
-                const float ph = row[ix];
-                sx += dW[0][ii] * ph;
-                sd += W[0][ii] * ph;
-                ix = ix + 1 == R.K[0] ? 0 : ix + 1;
-            }
-            gx += sx * W[1][j] * W[2][k];
-            gy += sd * dW[1][j] * W[2][k];
-            gz += sd * W[1][j] * dW[2][k];
-            iy = iy + 1 == R.K[1] ? 0 : iy + 1;
-        }
-        iz = iz + 1 == R.K[2] ? 0 : iz + 1;
-    }
-    const double coef = kEps / (kPi * R.V);
-    a.frec[i] = -coef * q * (double)gx * R.KL[0];
-    a.frec[(size_t)a.ntot + i] = -coef * q * (double)gy * R.KL[1];
-    a.frec[2 * (size_t)a.ntot + i] = -coef * q * (double)gz * R.KL[2];
 }
 
 // f = real-space + reciprocal (SPME_SUM); per-replica sum f (REMOVE_RIGIDMTN)
@@ -430,11 +271,10 @@ struct tcp_batch {
     unsigned *status = nullptr, *counter = nullptr;
     // SPME
     float *Qf = nullptr, *infl = nullptr;
-    // cell-sorted spreading
-    int *bin_count = nullptr, *bin_start = nullptr, *bin_bsum = nullptr, *bin_rank = nullptr;
-    int *bin_list = nullptr, *bin_ebx = nullptr, *bin_eby = nullptr;
-    float *bin_ew = nullptr, *bin_eq = nullptr;
-    int nbins = 0, ngroups = 0, k1max = 0;
+    tcp::SpreadBins bins{};             // cell sort of the spread over all replicas (spme_chain.cu)
+    tcp::SpmeGeom *geo = nullptr;       // device table of the replicas' meshes
+    unsigned *ticket = nullptr;
+    int nbins = 0, k1max = 0, k2max = 0, planes = 0;
     cufftComplex *Qk = nullptr;
     long long mesh_total = 0, half_total = 0;
     int *blk0 = nullptr;
@@ -483,62 +323,23 @@ static BParticles parts(tcp_batch *b) {
     return a;
 }
 
-static SpreadBins b_bins(tcp_batch *b) {
-    SpreadBins s;
-    s.count = b->bin_count;
-    s.start = b->bin_start;
-    s.bsum = b->bin_bsum;
-    s.rank = b->bin_rank;
-    s.list = b->bin_list;
-    s.ebx = b->bin_ebx;
-    s.eby = b->bin_eby;
-    s.ew = b->bin_ew;
-    s.eq = b->bin_eq;
-    return s;
-}
-
-template <int P>
-static void b_spme_launch(tcp_batch *b, bool gather, cudaStream_t st) {
-    const int blocks = (b->ntot + 127) / 128;
-    if (gather) {
-        b_gather_kernel<P><<<blocks, 128, 0, st>>>(parts(b), b->Qf, b->bin_list);   // sorted by the spread
-        return;
-    }
-    const SpreadBins bins = b_bins(b);
-    cudaMemsetAsync(b->bin_count, 0, sizeof(int) * (size_t)b->nbins, st);
-    b_bin_count_kernel<P><<<blocks, 128, 0, st>>>(parts(b), bins);
-    b->launches += launch_bin_sort(st, b->ntot, b->nbins, bins) - 5;   // the step's count assumes five
-    b_bin_weights_kernel<P><<<blocks, 128, 0, st>>>(parts(b), bins);
-    const size_t sm = kBRowWarps * b_row_warp_bytes(P, b->k1max);   // attribute set at tcp_batch_create
-    b_row_spread_kernel<P><<<(b->ngroups + kBRowWarps - 1) / kBRowWarps, 32 * kBRowWarps, sm, st>>>(
-        parts(b), bins, b->nrep, b->ngroups, b->k1max, b->Qf);
-}
-
-template <int P>
-static int b_prepare_spread_p(tcp_batch *b) {
-    TCP_CUDA(cudaFuncSetAttribute(b_row_spread_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(kBRowWarps * b_row_warp_bytes(P, b->k1max))));
-    return TCP_OK;
-}
-
-static int b_prepare_spread(tcp_batch *b) {
-    switch (b->order) {
-        case 4: return b_prepare_spread_p<4>(b);
-        case 5: return b_prepare_spread_p<5>(b);
-        case 6: return b_prepare_spread_p<6>(b);
-        case 7: return b_prepare_spread_p<7>(b);
-        default: return b_prepare_spread_p<8>(b);
-    }
-}
-
-static void b_spme(tcp_batch *b, bool gather, cudaStream_t st) {
-    switch (b->order) {
-        case 4: b_spme_launch<4>(b, gather, st); break;
-        case 5: b_spme_launch<5>(b, gather, st); break;
-        case 6: b_spme_launch<6>(b, gather, st); break;
-        case 7: b_spme_launch<7>(b, gather, st); break;
-        default: b_spme_launch<8>(b, gather, st); break;
-    }
+static ChainArgs b_chain(tcp_batch *b) {
+    ChainArgs c;
+    c.n = b->ntot;
+    c.nbins = b->nbins;
+    c.P = b->order;
+    c.fp64 = 0;
+    c.k1max = b->k1max;
+    c.k2max = b->k2max;
+    c.planes = b->planes;
+    c.nsys = b->nrep;
+    c.b = b->bins;
+    c.one = SpmeGeom();
+    c.many = b->geo;
+    c.sys_of = b->rep_of;
+    c.mesh = b->Qf;
+    c.ticket = b->ticket;
+    return c;
 }
 
 // The batched R2C (dir 0) or C2R (dir 1) of every mesh-size group.  The groups
@@ -575,14 +376,20 @@ static int b_fft_groups(tcp_batch *b, int dir) {
 // influence multiply + energy, C2R, gather into frec), forked onto stream2
 // after the work queued on the main stream, so that it runs beside the
 // real-space launch; b_recip_join makes the main stream wait for it.
-static int b_recip_fork(tcp_batch *b, const BAcc &A) {
+static int b_recip_fork(tcp_batch *b, const BAcc &A, bool binned) {
     TCP_CUDA(cudaEventRecord(b->ev_fork, b->stream));
     TCP_CUDA(cudaStreamWaitEvent(b->stream2, b->ev_fork, 0));
-    b_spme(b, false, b->stream2);                       // atomic-free, every mesh point written
+    const ChainArgs chain = b_chain(b);
+    if (!binned) {
+        b_bin_kernel<<<part_blocks(b->ntot), kPartThreads, 0, b->stream2>>>(parts(b), chain);
+        b->launches++;
+    }
+    b->launches += chain_spread(chain, b->stream2);     // atomic-free, every mesh point written
     if (int rc = b_fft_groups(b, 0)) return rc;
     b_influence_kernel<<<b->infl_blocks, 256, 0, b->stream2>>>(b->Qk, b->infl, b->reps, b->blk0, b->nrep, A.um);
     if (int rc = b_fft_groups(b, 1)) return rc;
-    b_spme(b, true, b->stream2);
+    b->launches += 1 + chain_gather(chain, b->frec, nullptr, 0, 0.0, nullptr, b->stream2);
+    TCP_CUDA(cudaGetLastError());
     return TCP_OK;
 }
 
@@ -615,21 +422,21 @@ static int b_step(tcp_batch *b, double dt) {
     const int nb = (b->ntot + kBThreads - 1) / kBThreads;
     int rc;
     if ((rc = b_mark(b, 0, b->stream))) return rc;
-    TCP_CUDA(cudaMemsetAsync(A.um, 0, sizeof(double) * 8 * (size_t)b->nrep, b->stream));   // um, mv0, mv1, fsum
-    b_vverlet1_kernel<<<nb, kBThreads, 0, b->stream>>>(parts(b), dt);
+    b_vverlet1_kernel<<<part_blocks(b->ntot), kPartThreads, 0, b->stream>>>(parts(b), dt, b_chain(b), b->counter, b->acc,
+                                                                           9 * b->nrep);
     if ((rc = b_mark(b, 1, b->stream))) return rc;
-    rc = b_recip_fork(b, A);
+    rc = b_recip_fork(b, A, true);
     if (!rc)
         rc = launch_pair_n3_batch(b->stream, b->xq, b->ntot, b->facc, b->n3reps, b->nrep, b->n3_items, b->n3_chunks, b->n3_nchunks, A.ur,
                                   b->status, b->counter, b->num_sms, true, b->pair_variant, b->pair_reserve,
-                                  &b->rejoin, b->ev_ready);
+                                  &b->rejoin, b->ev_ready, true);
     if (!rc) rc = b_mark(b, 3, b->stream);
     if (int jrc = b_recip_join(b)) return jrc;
     if (rc) return rc;
     b_finalize_kernel<<<nb, kBThreads, 0, b->stream>>>(parts(b), A.fsum);
     b_kick2_kernel<<<nb, kBThreads, 0, b->stream>>>(parts(b), dt, A.fsum, A.mv0);
     b_rescale_kernel<<<nb, kBThreads, 0, b->stream>>>(parts(b), dt, A.mv0, A.mv1);
-    b->launches += 15;
+    b->launches += 5;
     TCP_CUDA(cudaGetLastError());
     return b_mark(b, 4, b->stream);
 }
@@ -674,7 +481,7 @@ static int b_choose_reserve(tcp_batch *b) {
     double best = 1e300;
     const long long before = b->launches;
     auto once = [&]() -> int {
-        int r = b_recip_fork(b, A);
+        int r = b_recip_fork(b, A, false);
         if (!r)
             r = launch_pair_n3_batch(b->stream, b->xq, b->ntot, b->facc, b->n3reps, b->nrep, b->n3_items, b->n3_chunks,
                                      b->n3_nchunks, A.ur, b->status, b->counter, b->num_sms, true, b->pair_variant,
@@ -818,10 +625,9 @@ int tcp_batch_destroy(tcp_batch *b) {
     for (void *ptr : {(void *)b->x, (void *)b->v, (void *)b->f, (void *)b->frec, (void *)b->facc, (void *)b->xq,
                       (void *)b->rep_of, (void *)b->reps, b->n3reps, (void *)b->n3_chunks, (void *)b->acc, (void *)b->status,
                       (void *)b->counter, (void *)b->Qf, (void *)b->infl, (void *)b->Qk, (void *)b->blk0,
-                      (void *)b->bin_count, (void *)b->bin_start, (void *)b->bin_bsum, (void *)b->bin_rank,
-                      (void *)b->bin_list, (void *)b->bin_ebx, (void *)b->bin_eby, (void *)b->bin_ew,
-                      (void *)b->bin_eq})
+                      (void *)b->geo, (void *)b->ticket})
         cudaFree(ptr);
+    chain_free(b->bins);
     if (b->h_acc) cudaFreeHost(b->h_acc);
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
     if (b->ev_join) cudaEventDestroy(b->ev_join);
@@ -976,25 +782,21 @@ int tcp_batch_create(const tcp_params *params, const int *nel, const int *nion, 
         if (cudaEventCreateWithFlags(&b->ev_fft[d], cudaEventDisableTiming) != cudaSuccess)
             return fail(cuda_check(cudaGetLastError(), "cudaEventCreate"));
     TCP_BALLOC(b->Qf, sizeof(float) * (size_t)b->mesh_total);
-    // spreading bins (K2 K3 per replica) and 8-row groups (ceil(K2/8) K3 per replica)
+    // spreading bins (K2 K3 per replica: its mesh rows)
     for (int r = 0; r < nrep; ++r) {
         BRep &R = b->h_reps[r];
         R.bin_off = b->nbins;
-        R.grp_off = b->ngroups;
+        R.plane_off = b->planes;
+        b->planes += b->p[r].K[2];
+        b->k2max = std::max(b->k2max, b->p[r].K[1]);
         b->nbins += b->p[r].K[1] * b->p[r].K[2];
-        b->ngroups += ((b->p[r].K[1] + kBRows - 1) / kBRows) * b->p[r].K[2];
         b->k1max = std::max(b->k1max, b->p[r].K[0]);
     }
-    TCP_BALLOC(b->bin_count, sizeof(int) * ((size_t)b->nbins + 1));
-    TCP_BALLOC(b->bin_start, sizeof(int) * ((size_t)b->nbins + 1));
-    TCP_BALLOC(b->bin_bsum, sizeof(int) * (size_t)((b->nbins + bin_scan_block() - 1) / bin_scan_block()));
-    TCP_BALLOC(b->bin_rank, sizeof(int) * (size_t)b->ntot);
-    TCP_BALLOC(b->bin_list, sizeof(int) * (size_t)b->ntot);
-    TCP_BALLOC(b->bin_ebx, sizeof(int) * (size_t)b->ntot);
-    TCP_BALLOC(b->bin_eby, sizeof(int) * (size_t)b->ntot);
-    TCP_BALLOC(b->bin_ew, sizeof(float) * 3 * kMaxOrder * (size_t)b->ntot);
-    TCP_BALLOC(b->bin_eq, sizeof(float) * (size_t)b->ntot);
-    if (b_prepare_spread(b)) return fail(TCP_ERR_CUDA);
+    if (int rc = chain_alloc(b->bins, b->ntot, b->nbins, b->order)) return fail(rc);
+    TCP_BALLOC(b->geo, sizeof(SpmeGeom) * nrep);
+    TCP_BALLOC(b->ticket, sizeof(unsigned));
+    cudaMemsetAsync(b->ticket, 0, sizeof(unsigned), b->stream);
+    if (int rc = chain_prepare(b_chain(b))) return fail(rc);
     TCP_BALLOC(b->infl, sizeof(float) * (size_t)b->half_total);
     TCP_BALLOC(b->Qk, sizeof(cufftComplex) * (size_t)b->half_total);
     TCP_BALLOC(b->blk0, sizeof(int) * (nrep + 1));
@@ -1082,6 +884,25 @@ int tcp_batch_ewald_self(tcp_batch *b, double *Uo) {
     b->tuned = false;
     int frc = b_fill_n3(b, b->pair_variant);
     if (frc) return frc;
+    std::vector<SpmeGeom> geo(nrep);
+    for (int r = 0; r < nrep; ++r) {
+        const BRep &R = b->h_reps[r];
+        SpmeGeom &g = geo[r];
+        g.off = R.off;
+        g.nel = R.nel;
+        g.bin_off = R.bin_off;
+        g.plane_off = R.plane_off;
+        g.mesh_off = R.mesh_off;
+        for (int d = 0; d < 3; ++d) {
+            g.K[d] = R.K[d];
+            g.hL[d] = R.L[d] * .5;
+            g.KL[d] = R.KL[d];
+        }
+        g.q[0] = R.q[0];
+        g.q[1] = R.q[1];
+        g.coef = kEps / (kPi * R.V);
+    }
+    TCP_CUDA(cudaMemcpyAsync(b->geo, geo.data(), sizeof(SpmeGeom) * nrep, cudaMemcpyHostToDevice, b->stream));
     TCP_CUDA(cudaMemcpyAsync(b->reps, b->h_reps.data(), sizeof(BRep) * nrep, cudaMemcpyHostToDevice, b->stream));
     TCP_CUDA(cudaMemcpyAsync(b->blk0, blk0.data(), sizeof(int) * (nrep + 1), cudaMemcpyHostToDevice, b->stream));
     TCP_CUDA(cudaMemcpyAsync(b->infl, infl.data(), sizeof(float) * infl.size(), cudaMemcpyHostToDevice, b->stream));
@@ -1148,7 +969,7 @@ int tcp_batch_force(tcp_batch *b, tcp_energies *e) {
     const int nb = (b->ntot + kBThreads - 1) / kBThreads;
     b_refresh_kernel<<<nb, kBThreads, 0, b->stream>>>(parts(b));
     TCP_CUDA(cudaMemsetAsync(A.um, 0, sizeof(double) * 8 * (size_t)b->nrep, b->stream));
-    int rc = b_recip_fork(b, A);
+    int rc = b_recip_fork(b, A, false);
     if (!rc)
         rc = launch_pair_n3_batch(b->stream, b->xq, b->ntot, b->facc, b->n3reps, b->nrep, b->n3_items, b->n3_chunks, b->n3_nchunks, A.ur,
                                   b->status, b->counter, b->num_sms, true, b->pair_variant, b->pair_reserve,
@@ -1232,7 +1053,7 @@ int tcp_batch_time_component(tcp_batch *b, int which, int reps, double *ms_per_l
                                         b->n3_chunks, b->n3_nchunks, A.ur, b->status, b->counter, b->num_sms, true,
                                         b->pair_variant);
         TCP_CUDA(cudaMemsetAsync(A.um, 0, sizeof(double) * (size_t)b->nrep, b->stream));
-        if (int r = b_recip_fork(b, A)) return r;
+        if (int r = b_recip_fork(b, A, false)) return r;
         return b_recip_join(b);
     };
     rc = one();   // warm-up

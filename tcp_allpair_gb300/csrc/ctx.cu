@@ -179,9 +179,8 @@ static int force_chain(tcp_ctx *c, bool remove_net) {
     rc = launch_pair(c, energy_on(c), (c->flags & TCP_FLAG_RDF) != 0);
     if (int jrc = recip_join(c)) return jrc;
     if (rc) return rc;
-    if ((rc = launch_force_finalize(c, c->p.reciprocal != TCP_RECIP_NONE))) return rc;
+    if ((rc = launch_force_finalize(c, c->p.reciprocal != TCP_RECIP_NONE, energy_on(c)))) return rc;
     if (remove_net && (rc = launch_remove_rigid(c))) return rc;
-    if (energy_on(c) && (rc = launch_reduce(c, kRedUr, 0))) return rc;
     return TCP_OK;
 }
 
@@ -197,7 +196,7 @@ static bool thermostat_due(const tcp_ctx *c) {
     return ((c->step_index + 1) % c->p.thermo_period) == 0;
 }
 
-// One MD step (main.f90:81-153) on the stream; *pass = kinetic partial set.
+// One MD step (main.f90:81-153) on the stream.
 // Phase mark k: an event-record node when the stream is being captured, a
 // plain record otherwise (the External flag is only valid during capture).
 static int mark_on(tcp_ctx *c, int k, cudaStream_t s) {
@@ -217,10 +216,10 @@ static int mark(tcp_ctx *c, int k) { return mark_on(c, k, c->stream); }
 // with the pair kernel), 3 end of the pair launch on the main stream (the
 // reserved CTAs that rejoin it after the chain drain the same chunk counter,
 // so they end within a chunk of it), 4 step end.
-static int step_chain(tcp_ctx *c, double dt, bool apply, int *pass) {
+static int step_launch(tcp_ctx *c, double dt, bool apply) {
     int rc;
     if ((rc = mark(c, 0))) return rc;
-    if ((rc = launch_vverlet1(c, dt, 0.0))) return rc;
+    if ((rc = launch_vverlet1(c, dt, true))) return rc;
     if ((rc = mark(c, 1))) return rc;
     if ((rc = recip_fork(c))) return rc;
     if (c->p.reciprocal != TCP_RECIP_NONE) {
@@ -231,11 +230,16 @@ static int step_chain(tcp_ctx *c, double dt, bool apply, int *pass) {
     if ((rc = launch_pair(c, energy_on(c), (c->flags & TCP_FLAG_RDF) != 0))) return rc;
     if ((rc = mark(c, 3))) return rc;
     if ((rc = recip_join(c))) return rc;
-    if ((rc = launch_force_finalize(c, c->p.reciprocal != TCP_RECIP_NONE))) return rc;
-    if ((rc = launch_kick2(c, dt, true, apply, (c->flags & TCP_FLAG_VDF) != 0, pass))) return rc;
-    if ((rc = launch_reduce(c, (energy_on(c) ? kRedUr : 0) | kRedMv2, *pass))) return rc;
+    if ((rc = launch_force_finalize(c, c->p.reciprocal != TCP_RECIP_NONE, energy_on(c)))) return rc;
+    if ((rc = launch_kick2(c, dt, true, apply, (c->flags & TCP_FLAG_VDF) != 0))) return rc;
     if ((rc = mark(c, 4))) return rc;
     return TCP_OK;
+}
+
+static int step_chain(tcp_ctx *c, double dt, bool apply) {
+    const int rc = step_launch(c, dt, apply);
+    c->cleared = c->binned = false;   // of this step only, also where it failed half-way
+    return rc;
 }
 
 // ---- composition used by the derivative routines (adjoint.cu) ----------------
@@ -347,6 +351,7 @@ int tcp_create(const tcp_params *p_in, int nel, int nion, int device, tcp_ctx **
     TCP_ALLOC(c->scal, sizeof(double) * kScalCount);
     TCP_ALLOC(c->status, sizeof(unsigned));
     TCP_ALLOC(c->counter, sizeof(unsigned));
+    TCP_ALLOC(c->tickets, sizeof(unsigned) * 8);
     TCP_ALLOC(c->rdf, sizeof(unsigned long long) * 3 * kNbin);
     TCP_ALLOC(c->vdf, sizeof(unsigned long long) * 2 * kNbin);
     TCP_ALLOC(c->rdf_edges, sizeof(RdfEdges));
@@ -359,6 +364,7 @@ int tcp_create(const tcp_params *p_in, int nel, int nion, int device, tcp_ctx **
     cudaMemsetAsync(c->frec, 0, sizeof(double) * 3 * n, c->stream);
     cudaMemsetAsync(c->scal, 0, sizeof(double) * kScalCount, c->stream);
     cudaMemsetAsync(c->status, 0, sizeof(unsigned), c->stream);
+    cudaMemsetAsync(c->tickets, 0, sizeof(unsigned) * 8, c->stream);
     cudaMemsetAsync(c->rdf, 0, sizeof(unsigned long long) * 3 * kNbin, c->stream);
     cudaMemsetAsync(c->vdf, 0, sizeof(unsigned long long) * 2 * kNbin, c->stream);
     if ((rc = launch_refresh_positions(c))) return fail(rc);
@@ -389,6 +395,7 @@ int tcp_destroy(tcp_ctx *c) {
     cudaFree(c->scal);
     cudaFree(c->status);
     cudaFree(c->counter);
+    cudaFree(c->tickets);
     cudaFree(c->rdf);
     cudaFree(c->vdf);
     cudaFree(c->rdf_edges);
@@ -663,8 +670,7 @@ int tcp_force_direct(tcp_ctx *c, double *Ur) {
     int rc;
     if ((rc = autotune_pair(c))) return rc;
     if ((rc = launch_pair(c, energy_on(c), (c->flags & TCP_FLAG_RDF) != 0))) return rc;
-    if ((rc = launch_force_finalize(c, false))) return rc;
-    if (energy_on(c) && (rc = launch_reduce(c, kRedUr, 0))) return rc;
+    if ((rc = launch_force_finalize(c, false, energy_on(c)))) return rc;
     if ((rc = sync_scalars(c))) return rc;
     if (Ur) *Ur = energy_on(c) ? c->h_scal[kScalUr] : 0.0;
     return TCP_OK;
@@ -719,7 +725,7 @@ int tcp_vverlet1(tcp_ctx *c, double dt) {
     TCP_TRACE("tcp_vverlet1");
     TCP_REQUIRE_READY(c);
     int rc;
-    if ((rc = launch_vverlet1(c, dt, 0.0))) return rc;
+    if ((rc = launch_vverlet1(c, dt, false))) return rc;
     TCP_CUDA(cudaStreamSynchronize(c->stream));
     return TCP_OK;
 }
@@ -727,9 +733,8 @@ int tcp_vverlet1(tcp_ctx *c, double dt) {
 int tcp_vverlet2(tcp_ctx *c, double dt, double *mv2el, double *mv2ion) {
     TCP_TRACE("tcp_vverlet2");
     TCP_REQUIRE_READY(c);
-    int rc, pass = 0;
-    if ((rc = launch_kick2(c, dt, false, thermostat_due(c), (c->flags & TCP_FLAG_VDF) != 0, &pass))) return rc;
-    if ((rc = launch_reduce(c, kRedMv2, pass))) return rc;
+    int rc;
+    if ((rc = launch_kick2(c, dt, false, thermostat_due(c), (c->flags & TCP_FLAG_VDF) != 0))) return rc;
     if ((rc = sync_scalars(c))) return rc;
     c->step_index++;
     c->last.mv2el = c->h_scal[kScalMv2e];
@@ -756,8 +761,7 @@ static int build_graph(tcp_ctx *c, double dt, bool apply, cudaGraphExec_t *out, 
     cudaGraph_t g;
     const long long before = c->launches;
     TCP_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    int pass = 0;
-    int rc = step_chain(c, dt, apply, &pass);
+    int rc = step_chain(c, dt, apply);
     cudaError_t ce = cudaStreamEndCapture(c->stream, &g);
     if (rc) return rc;
     if (ce != cudaSuccess) return cuda_check(ce, "cudaStreamEndCapture");
@@ -789,8 +793,7 @@ static int launch_step(tcp_ctx *c, double dt) {
     const bool has_thermo = c->p.thermo == TCP_THERMO_ISOKIN || c->p.thermo == TCP_THERMO_BEREND;
     int rc;
     if (has_thermo && thermostat_due(c)) {
-        int pass = 0;
-        if ((rc = step_chain(c, dt, true, &pass))) return rc;
+        if ((rc = step_chain(c, dt, true))) return rc;
     } else {
         TCP_CUDA(cudaGraphLaunch(c->graph, c->stream));
         c->launches += c->graph_kernels;

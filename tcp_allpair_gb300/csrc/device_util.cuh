@@ -93,7 +93,20 @@ __device__ __forceinline__ double wrap_box(double x, double L, double iL) {
     return x - L * round(q);
 }
 
+// x - L DNINT(x/L); positions inside the box, where DNINT gives 0, are told
+// apart by their leading bits and need no arithmetic
+__device__ __forceinline__ double wrap_fast(double x, double L, double iL) {
+    const int inside = __double2hiint(L) - 0x100000;      // leading bits of L/2
+    if ((__double2hiint(x) & 0x7fffffff) < inside) return x;
+    return wrap_box(x, L, iL);
+}
+
+// One FMA puts round(2^32 (x/L + 1/2)) into the low mantissa bits of a number
+// between 2^52 and 2^53; positions too many boxes away for that take the
+// general form.
 __device__ __forceinline__ int fixed_coord(double x, double iL) {
+    const double s = fma(x, iL * 4294967296.0, 6755399441055744.0 + 2147483648.0);   // 1.5 2^52 + 2^31
+    if ((__double2hiint(s) >> 20) == 0x433) return __double2loint(s);
     double t = fma(x, iL, 0.5);
     t -= floor(t);
     const unsigned long long u = (unsigned long long)llrint(t * 4294967296.0);

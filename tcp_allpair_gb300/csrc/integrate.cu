@@ -9,6 +9,7 @@
 #include <cmath>
 
 #include "device_util.cuh"
+#include "spme_chain.cuh"
 #include "tcp_internal.h"
 
 namespace tcp {
@@ -72,25 +73,71 @@ __global__ void shift_kernel(const IntArgs a, double sdt) {
     store_pos(a, i, y[0], y[1], y[2]);
 }
 
-// VVerletNotemp1 (vverlet.f90:148-167) / VVerletStoch1 (vverlet.f90:34-55)
-__global__ void vverlet1_kernel(const IntArgs a, double dt, double hdm0, double hdm1, double alpha_lgv, int stoch) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    const double hdm = i < a.nel ? hdm0 : hdm1;        // dt/(2m), divided on the host
-    const double damp = 1.0 - alpha_lgv * hdm;
-    const double L[3] = {a.L0, a.L1, a.L2}, iL[3] = {a.iL0, a.iL1, a.iL2};
-    double y[3];
-    for (int k = 0; k < 3; ++k) {
-        const size_t o = (size_t)k * a.n + i;
-        double vk = a.v[o];
+// component d of particle i
+__device__ __forceinline__ void store_comp(const IntArgs &a, int d, int i, double x, double iL) {
+    a.x[(size_t)d * a.n + i] = x;
+    if (a.copies & kCopyXq) reinterpret_cast<int *>(a.xq + i)[d] = fixed_coord(x, iL);
+    if (a.copies & kCopyXd) reinterpret_cast<double *>(a.xd + i)[d] = x;
+    if (a.copies & kCopyXl) reinterpret_cast<long long *>(a.xl + i)[d] = fixed_coord64(x, iL);
+}
+
+// What the half kick of a step does besides: the accumulators of the pair
+// launch and the bins of the SPME chain (their own launches otherwise).
+struct StepPrep {
+    double *fpart;           // [3][n], cleared; null: not this kernel's job
+    double *upart;
+    int nupart;
+    unsigned *counter;
+    int bin;                 // bin the positions for the chain
+    ChainArgs chain;
+};
+
+// VVerletNotemp1 (vverlet.f90:148-167) / VVerletStoch1 (vverlet.f90:34-55).
+// A thread per component: the FP64 chain of a particle (its three components
+// one after the other took 45 dependent operations of 34 ns) is a third as
+// long and a small system spreads over three times the warps.
+template <bool BIN>
+__global__ void __launch_bounds__(kPartThreads) vverlet1_kernel(const IntArgs a, double dt, double hdm0, double hdm1,
+                                                                double alpha_lgv, int stoch, const StepPrep s) {
+    __shared__ int sb[BIN ? 3 : 1][kPartBlock];
+    __shared__ double sa[BIN ? 3 : 1][kPartBlock];
+    const int k = threadIdx.x % kPartBlock, d = threadIdx.x / kPartBlock, i = blockIdx.x * kPartBlock + k;
+    const bool live = i < a.n;
+    if (live) {
+        const double L = d == 0 ? a.L0 : (d == 1 ? a.L1 : a.L2), iL = d == 0 ? a.iL0 : (d == 1 ? a.iL1 : a.iL2);
+        const double hdm = i < a.nel ? hdm0 : hdm1;    // dt/(2m), divided on the host
+        const size_t o = (size_t)d * a.n + i;
+        double v = a.v[o];
         if (stoch)
-            vk = vk * damp + hdm * a.f[o];             // vverlet.f90:37-38
+            v = v * (1.0 - alpha_lgv * hdm) + hdm * a.f[o];   // vverlet.f90:37-38
         else
-            vk = vk + hdm * a.f[o];                    // vverlet.f90:151
-        a.v[o] = vk;
-        y[k] = wrap(a.x[o] + dt * vk, L[k], iL[k]);    // vverlet.f90:152-153
+            v = v + hdm * a.f[o];                      // vverlet.f90:151
+        a.v[o] = v;
+        const double y = wrap_fast(a.x[o] + dt * v, L, iL);   // vverlet.f90:152-153
+        store_comp(a, d, i, y, iL);
+        if (s.fpart) s.fpart[o] = 0.0;
+        if (BIN) {
+            const SpmeGeom &g = s.chain.one;
+            sb[d][k] = bin_axis(y, g.hL[d], g.KL[d], g.K[d], s.chain.P, sa[d][k]);
+        }
     }
-    store_pos(a, i, y[0], y[1], y[2]);
+    const int t = blockIdx.x * kPartThreads + threadIdx.x;
+    if (s.fpart) {
+        for (int u = t; u < s.nupart; u += gridDim.x * kPartThreads) s.upart[u] = 0.0;
+        if (t == 0) *s.counter = 0u;
+    }
+    if (BIN) {
+        __syncthreads();
+        if (live && d == 0) {
+            const ChainArgs &c = s.chain;
+            const double arg[3] = {sa[0][k], sa[1][k], sa[2][k]}, q = i < a.nel ? c.one.q[0] : c.one.q[1];
+            if (c.fp64)
+                bin_store<double>(c.b, i, a.n, arg, q, sb[0][k], sb[1][k], sb[2][k], c.one.K[1], 0);
+            else
+                bin_store<float>(c.b, i, a.n, arg, q, sb[0][k], sb[1][k], sb[2][k], c.one.K[1], 0);
+        }
+        if (s.chain.nbins <= kScanTail && last_block(s.chain.ticket)) scan_bins(s.chain.b, s.chain.nbins);
+    }
 }
 
 // ---- Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11) ---------------------
@@ -128,167 +175,212 @@ struct KickArgs {
     double hdm0, hdm1;       // dt/(2m) per species (host-divided: the same correctly rounded value)
     int thermo;              // TCP_THERMO_*
     int remove_net;          // subtract sum(f)/n first (REMOVE_RIGIDMTN fused)
-    const double *fsum_part; // [3][nbf]
-    int nbf;
     double *mv_part;         // [2][nb] output partials (species)
-    const double *mv_in;     // [2][nb] partials of the first pass (rescale pass)
-    int nb;
     int vdf;
     unsigned long long *vdf_counts;
     double dv0, dv1;
     double T0, T1, tau, alpha_lgv;
     uint64_t seed;
-    const double *step;      // device step counter (advanced by the reduction kernel)
-    int rescale;             // 0 kick pass, 1 rescale pass
+    double *scal;            // kScal*: mean force in, sums of m v^2 in (rescale) and out, the step counter
+    int last_pass;           // this pass ends the step's second half
+    unsigned *ticket;
 };
-
-__device__ __forceinline__ double sum_strided(const double *p, int np) {
-    double s = 0.0;
-    for (int k = 0; k < np; ++k) s += p[k];
-    return s;
-}
 
 __device__ __forceinline__ void vdf_add(const KickArgs &k, int s, double mv2) {
     const double t = mv2 / 3.0 / (s == 0 ? k.dv0 : k.dv1);   // vverlet.f90:201
     if (t < (double)kNbin) atomicAdd(&k.vdf_counts[s * kNbin + (int)t], 1ull);
 }
 
-// Second half kick (vverlet.f90:194-219 NOTEMP, :250-255 BEREND/ISOKIN first
-// loop, :91-123 STOCH); per-species sum m v^2 partials; VDF when final.
-__global__ void kick2_kernel(const KickArgs k) {
-    __shared__ double red[32];
-    __shared__ double fbar[3];
-    const IntArgs &a = k.a;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k.remove_net) {
-        if (threadIdx.x < 3) fbar[threadIdx.x] = sum_strided(k.fsum_part + threadIdx.x * k.nbf, k.nbf) / (double)a.n;
+// Sum over a CTA of kPartThreads threads; valid in thread 0.
+__device__ __forceinline__ double part_sum(double v, double *sh) {
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double r = 0.0;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < kPartThreads / 32; ++w) r += sh[w];
+    __syncthreads();
+    return r;
+}
+
+// The end of a kinetic pass: the CTA's sums of m v^2 per species, and in the
+// last CTA the totals (in a fixed order) and the VDF of the final velocities.
+__device__ __forceinline__ void kick_end(const KickArgs &k, double mv2, bool live, int s) {
+    __shared__ double red[8];
+    __shared__ double smv[3][kPartBlock];
+    if (k.vdf) {
+        const int p = threadIdx.x % kPartBlock, d = threadIdx.x / kPartBlock;
+        smv[d][p] = mv2;
         __syncthreads();
+        if (d == 0 && live) vdf_add(k, s, smv[0][p] + smv[1][p] + smv[2][p]);
     }
-    double mv_e = 0.0, mv_i = 0.0;
-    if (i < a.n) {
-        const int s = i < a.nel ? 0 : 1;
-        const double xm = s == 0 ? a.xm0 : a.xm1;
-        const double hdm = s == 0 ? k.hdm0 : k.hdm1;      // dt/(2m)
-        const double idamp = k.thermo == TCP_THERMO_STOCH ? 1.0 / (1.0 + k.alpha_lgv * hdm) : 1.0;
-        double vv[3];
-        double eta[3] = {0.0, 0.0, 0.0};
-        if (k.thermo == TCP_THERMO_STOCH) gauss3(k.seed, (long long)*k.step, i, eta);
-        const double beta = k.thermo == TCP_THERMO_STOCH ? sqrt(2.0 * k.alpha_lgv * (s == 0 ? k.T0 : k.T1) / k.dt) : 0.0;
-        for (int d = 0; d < 3; ++d) {
-            const size_t o = (size_t)d * a.n + i;
-            double fd = a.f[o];
-            if (k.remove_net) fd -= fbar[d];                                 // force.f90:999-1004
-            if (k.thermo == TCP_THERMO_STOCH) {
-                fd = fd + eta[d] * beta;                                     // vverlet.f90:95
-                vv[d] = (a.v[o] + hdm * fd) * idamp;                          // vverlet.f90:96-97
-            } else {
-                vv[d] = a.v[o] + hdm * fd;                                   // vverlet.f90:197
-            }
-            if (k.remove_net || k.thermo == TCP_THERMO_STOCH) a.f[o] = fd;
-            a.v[o] = vv[d];
+    // one species per CTA but for the one where the ions begin
+    const int nb = gridDim.x, i0 = blockIdx.x * kPartBlock;
+    const bool mixed = i0 < k.a.nel && i0 + kPartBlock > k.a.nel;
+    double te, ti;
+    if (mixed) {
+        te = part_sum(s == 0 ? mv2 : 0.0, red);
+        ti = part_sum(s == 0 ? 0.0 : mv2, red);
+    } else {
+        te = part_sum(mv2, red);
+        ti = 0.0;
+        if (i0 >= k.a.nel) {
+            ti = te;
+            te = 0.0;
         }
-        const double mv2 = (vv[0] * vv[0] + vv[1] * vv[1] + vv[2] * vv[2]) * xm;   // vverlet.f90:199
-        if (s == 0) mv_e = mv2; else mv_i = mv2;
-        if (k.vdf) vdf_add(k, s, mv2);
     }
-    const double te = block_sum(mv_e, red);
-    const double ti = block_sum(mv_i, red);
     if (threadIdx.x == 0) {
         k.mv_part[blockIdx.x] = te;
-        k.mv_part[k.nb + blockIdx.x] = ti;
+        k.mv_part[nb + blockIdx.x] = ti;
     }
+    if (last_block(k.ticket)) {
+        double e = 0.0, n = 0.0;
+        for (int b = threadIdx.x; b < nb; b += kPartThreads) {
+            e += __ldcg(k.mv_part + b);
+            n += __ldcg(k.mv_part + nb + b);
+        }
+        e = part_sum(e, red);
+        n = part_sum(n, red);
+        if (threadIdx.x == 0) {
+            k.scal[kScalMv2e] = e;
+            k.scal[kScalMv2i] = n;
+            if (k.last_pass) k.scal[kScalStep] += 1.0;   // one second half-kick per MD step
+        }
+    }
+}
+
+// Second half kick (vverlet.f90:194-219 NOTEMP, :250-255 BEREND/ISOKIN first
+// loop, :91-123 STOCH), a thread per component; per-species sums of m v^2 and
+// the VDF when no rescale follows.  The sums of the CTAs are added by the last
+// one to finish (a launch of their own took 10 us, and 3 threads adding the
+// force partials in every CTA as much again).
+__global__ void __launch_bounds__(kPartThreads) kick2_kernel(const KickArgs k) {
+    const IntArgs &a = k.a;
+    const int p = threadIdx.x % kPartBlock, d = threadIdx.x / kPartBlock, i = blockIdx.x * kPartBlock + p;
+    const bool live = i < a.n, stoch = k.thermo == TCP_THERMO_STOCH;
+    const int s = i < a.nel ? 0 : 1;
+    __shared__ double eta[3][kPartBlock];
+    if (stoch) {
+        if (live && d == 0) {
+            double g[3];
+            gauss3(k.seed, (long long)k.scal[kScalStep], i, g);
+            for (int q = 0; q < 3; ++q) eta[q][p] = g[q];
+        }
+        __syncthreads();
+    }
+    double mv2 = 0.0;
+    if (live) {
+        const double xm = s == 0 ? a.xm0 : a.xm1;
+        const double hdm = s == 0 ? k.hdm0 : k.hdm1;      // dt/(2m)
+        const size_t o = (size_t)d * a.n + i;
+        double fd = a.f[o], vv;
+        if (k.remove_net) fd -= k.scal[kScalFx + d];                         // force.f90:999-1004
+        if (stoch) {
+            const double beta = sqrt(2.0 * k.alpha_lgv * (s == 0 ? k.T0 : k.T1) / k.dt);
+            fd = fd + eta[d][p] * beta;                                      // vverlet.f90:95
+            vv = (a.v[o] + hdm * fd) * (1.0 / (1.0 + k.alpha_lgv * hdm));    // vverlet.f90:96-97
+        } else {
+            vv = a.v[o] + hdm * fd;                                          // vverlet.f90:197
+        }
+        if (k.remove_net || stoch) a.f[o] = fd;
+        a.v[o] = vv;
+        mv2 = vv * vv * xm;                                                  // vverlet.f90:199
+    }
+    kick_end(k, mv2, live, s);
 }
 
 // Rescale pass of VVerletIsokin2 / VVerletBerend2 (vverlet.f90:331-344,
 // 257-270): lambda per species from the first-pass sums, v *= lambda,
 // sum m v^2 and VDF.
-__global__ void rescale_kernel(const KickArgs k) {
-    __shared__ double red[32];
-    __shared__ double lam[2];
+__global__ void __launch_bounds__(kPartThreads) rescale_kernel(const KickArgs k) {
     const IntArgs &a = k.a;
-    if (threadIdx.x < 2) {
-        const int s = threadIdx.x;
-        const double mv2 = sum_strided(k.mv_in + s * k.nb, k.nb);
+    const int p = threadIdx.x % kPartBlock, d = threadIdx.x / kPartBlock, i = blockIdx.x * kPartBlock + p;
+    const bool live = i < a.n;
+    const int s = i < a.nel ? 0 : 1;
+    double mv2 = 0.0;
+    if (live) {
         const int cnt = s == 0 ? a.nel : a.n - a.nel;
-        const double T0 = mv2 / (double)(3 * cnt);
+        const double T0 = k.scal[s == 0 ? kScalMv2e : kScalMv2i] / (double)(3 * cnt);
         const double T = s == 0 ? k.T0 : k.T1;
-        lam[s] = k.thermo == TCP_THERMO_ISOKIN ? sqrt(T / T0) : sqrt(1.0 + k.dt * (T / T0 - 1.0) / k.tau);
+        const double lam = k.thermo == TCP_THERMO_ISOKIN ? sqrt(T / T0) : sqrt(1.0 + k.dt * (T / T0 - 1.0) / k.tau);
+        const size_t o = (size_t)d * a.n + i;
+        const double vv = a.v[o] * lam;
+        a.v[o] = vv;
+        mv2 = vv * vv * (s == 0 ? a.xm0 : a.xm1);
     }
+    kick_end(k, mv2, live, s);
+}
+
+// The end of a pass over the forces: sum(f)/n into fbar by the last CTA, with
+// the pair energy when upart is given.
+__device__ __forceinline__ void force_end(double f, double *part, int n, double *scal, const double *upart, int nu,
+                                          unsigned *ticket) {
+    __shared__ double red[8];
+    const int d = threadIdx.x / kPartBlock, w = threadIdx.x >> 5, nb = gridDim.x;
+    f = warp_sum(f);
+    if ((threadIdx.x & 31) == 0) red[w] = f;
     __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double mv_e = 0.0, mv_i = 0.0;
-    if (i < a.n) {
-        const int s = i < a.nel ? 0 : 1;
-        const double xm = s == 0 ? a.xm0 : a.xm1;
-        double vv[3];
-        for (int d = 0; d < 3; ++d) {
-            const size_t o = (size_t)d * a.n + i;
-            vv[d] = a.v[o] * lam[s];
-            a.v[o] = vv[d];
-        }
-        const double mv2 = (vv[0] * vv[0] + vv[1] * vv[1] + vv[2] * vv[2]) * xm;
-        if (s == 0) mv_e = mv2; else mv_i = mv2;
-        if (k.vdf) vdf_add(k, s, mv2);
-    }
-    const double te = block_sum(mv_e, red);
-    const double ti = block_sum(mv_i, red);
-    if (threadIdx.x == 0) {
-        k.mv_part[blockIdx.x] = te;
-        k.mv_part[k.nb + blockIdx.x] = ti;
+    if (threadIdx.x < 3) part[threadIdx.x * nb + blockIdx.x] = red[2 * threadIdx.x] + red[2 * threadIdx.x + 1];
+    if (!last_block(ticket)) return;
+    double s = 0.0;
+    for (int b = threadIdx.x % kPartBlock; b < nb; b += kPartBlock) s += __ldcg(part + d * nb + b);
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) red[w] = s;
+    __syncthreads();
+    if (threadIdx.x < 3) scal[kScalFx + threadIdx.x] = (red[2 * threadIdx.x] + red[2 * threadIdx.x + 1]) / (double)n;
+    if (upart) {
+        __syncthreads();
+        double u = 0.0;
+        for (int k = threadIdx.x; k < nu; k += kPartThreads) u += upart[k];
+        u = part_sum(u, red);
+        if (threadIdx.x == 0) scal[kScalUr] = u;
     }
 }
 
-// f += frec (SPME_SUM, force.f90:953-964) with sum(f) partials
-__global__ void add_rec_kernel(double *__restrict__ f, const double *__restrict__ frec, int n,
-                               double *__restrict__ fsum_part) {
-    __shared__ double red[32];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double s[3] = {0.0, 0.0, 0.0};
-    if (i < n)
-        for (int d = 0; d < 3; ++d) {
-            const size_t o = (size_t)d * n + i;
-            if (frec) f[o] += frec[o];
-            s[d] = f[o];
-        }
-    for (int d = 0; d < 3; ++d) {
-        const double t = block_sum(s[d], red);
-        if (threadIdx.x == 0) fsum_part[d * gridDim.x + blockIdx.x] = t;
+// f = sum over splits of fpart (+ frec: the SPME_SUM add of force.f90:953-964
+// fused), the mean force for REMOVE_RIGIDMTN (force.f90:986-993) and the pair
+// energy.  When a tile wait of the pair kernel ran out (status), some partials
+// were never written: f is then left as it was and the caller reports the error.
+__global__ void __launch_bounds__(kPartThreads) force_finalize_kernel(const double *__restrict__ fpart, int nsplit,
+                                                                      const double *__restrict__ frec,
+                                                                      double *__restrict__ f, int n,
+                                                                      double *__restrict__ fsum_part,
+                                                                      const unsigned *__restrict__ status,
+                                                                      double *__restrict__ scal,
+                                                                      const double *__restrict__ upart, int nu,
+                                                                      unsigned *ticket) {
+    const int k = threadIdx.x % kPartBlock, d = threadIdx.x / kPartBlock, i = blockIdx.x * kPartBlock + k;
+    const bool write = !(*status & kStatusTmaTimeout);
+    double acc = 0.0;
+    if (i < n) {
+        for (int sp = 0; sp < nsplit; ++sp) acc += fpart[((size_t)sp * 3 + d) * n + i];
+        if (frec) acc += frec[(size_t)d * n + i];
+        if (write) f[(size_t)d * n + i] = acc;
     }
+    force_end(acc, fsum_part, n, scal, upart, nu, ticket);
+}
+
+// f += frec (SPME_SUM, force.f90:953-964; null: f as it is) and the mean force
+__global__ void __launch_bounds__(kPartThreads) add_rec_kernel(double *__restrict__ f, const double *__restrict__ frec,
+                                                               int n, double *__restrict__ fsum_part,
+                                                               double *__restrict__ scal, unsigned *ticket) {
+    const int k = threadIdx.x % kPartBlock, d = threadIdx.x / kPartBlock, i = blockIdx.x * kPartBlock + k;
+    double v = 0.0;
+    if (i < n) {
+        const size_t o = (size_t)d * n + i;
+        v = f[o];
+        if (frec) {
+            v += frec[o];
+            f[o] = v;
+        }
+    }
+    force_end(v, fsum_part, n, scal, nullptr, 0, ticket);
 }
 
 // f -= sum(f)/n (REMOVE_RIGIDMTN, force.f90:996-1004)
-__global__ void remove_net_kernel(double *__restrict__ f, int n, const double *__restrict__ fsum_part, int nbf) {
-    __shared__ double fbar[3];
-    if (threadIdx.x < 3) fbar[threadIdx.x] = sum_strided(fsum_part + threadIdx.x * nbf, nbf) / (double)n;
-    __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    for (int d = 0; d < 3; ++d) f[(size_t)d * n + i] -= fbar[d];
-}
-
-__global__ void reduce_scalars_kernel(const double *__restrict__ upart, int nu, const double *__restrict__ mv,
-                                      int nb, double *__restrict__ scal, int mask) {
-    __shared__ double red[32];
-    if (mask & kRedUr) {
-        double s = 0.0;
-        for (int k = threadIdx.x; k < nu; k += blockDim.x) s += upart[k];
-        s = block_sum(s, red);
-        if (threadIdx.x == 0) scal[kScalUr] = s;
-    }
-    if (mask & kRedMv2) {
-        double se = 0.0, si = 0.0;
-        for (int k = threadIdx.x; k < nb; k += blockDim.x) {
-            se += mv[k];
-            si += mv[nb + k];
-        }
-        se = block_sum(se, red);
-        si = block_sum(si, red);
-        if (threadIdx.x == 0) {
-            scal[kScalMv2e] = se;
-            scal[kScalMv2i] = si;
-            scal[kScalStep] += 1.0;   // one second half-kick per MD step
-        }
-    }
+__global__ void remove_net_kernel(double *__restrict__ f, int n, const double *__restrict__ scal) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < 3 * n) f[t] -= scal[kScalFx + t / n];
 }
 
 // ---- host records <-> SoA ------------------------------------------------
@@ -449,11 +541,11 @@ static IntArgs int_args(tcp_ctx *c) {
 static int nblocks(int n) { return (n + kIntThreads - 1) / kIntThreads; }
 
 // red[] layout: [3][nb] force sums | [2][nb] kinetic pass 0 | [2][nb] pass 1 | recip energy
+int part_blocks(int n) { return (n + kPartBlock - 1) / kPartBlock; }
 double *fsum_part(tcp_ctx *c) { return c->red; }
-double *mv_part(tcp_ctx *c, int pass) { return c->red + 3 * (size_t)nblocks(c->n) + (size_t)pass * 2 * nblocks(c->n); }
-double *recip_epart(tcp_ctx *c) { return c->red + 7 * (size_t)nblocks(c->n); }
-int red_capacity(int n, int extra) { return 7 * nblocks(n) + extra; }
-int kick_blocks(int n) { return nblocks(n); }
+double *mv_part(tcp_ctx *c, int pass) { return c->red + 3 * (size_t)part_blocks(c->n) + (size_t)pass * 2 * part_blocks(c->n); }
+double *recip_epart(tcp_ctx *c) { return c->red + 7 * (size_t)part_blocks(c->n); }
+int red_capacity(int n, int extra) { return 7 * part_blocks(n) + extra; }
 
 int launch_refresh_positions(tcp_ctx *c) {
     refresh_kernel<<<nblocks(c->n), kIntThreads, 0, c->stream>>>(int_args(c));
@@ -469,38 +561,67 @@ int launch_shift(tcp_ctx *c, double sdt) {
     return TCP_OK;
 }
 
-int launch_vverlet1(tcp_ctx *c, double dt, double) {
-    vverlet1_kernel<<<nblocks(c->n), kIntThreads, 0, c->stream>>>(int_args(c), dt, 0.5 * dt / c->p.xm[0],
-                                                                  0.5 * dt / c->p.xm[1], c->p.alpha_lgv,
-                                                                  c->p.thermo == TCP_THERMO_STOCH);
+int launch_vverlet1(tcp_ctx *c, double dt, bool prepare) {
+    StepPrep s;
+    s.fpart = nullptr;
+    s.bin = 0;
+    if (prepare) {
+        s.fpart = c->fpart;
+        s.upart = c->upart;
+        s.nupart = c->n_upart;
+        s.counter = c->counter;
+        s.bin = c->p.reciprocal == TCP_RECIP_SPME;
+        if (s.bin) {
+            s.chain = spme_chain_args(c);
+            s.chain.ticket = c->tickets + kTickStep;
+        }
+    }
+    const double h0 = 0.5 * dt / c->p.xm[0], h1 = 0.5 * dt / c->p.xm[1];
+    const int stoch = c->p.thermo == TCP_THERMO_STOCH, nb = part_blocks(c->n);
+    if (s.bin)
+        vverlet1_kernel<true><<<nb, kPartThreads, 0, c->stream>>>(int_args(c), dt, h0, h1, c->p.alpha_lgv, stoch, s);
+    else
+        vverlet1_kernel<false><<<nb, kPartThreads, 0, c->stream>>>(int_args(c), dt, h0, h1, c->p.alpha_lgv, stoch, s);
+    c->cleared = prepare;
+    c->binned = s.bin != 0;
+    c->launches++;
+    TCP_CUDA(cudaGetLastError());
+    return TCP_OK;
+}
+
+int launch_force_finalize(tcp_ctx *c, bool add_rec, bool energy) {
+    force_finalize_kernel<<<part_blocks(c->n), kPartThreads, 0, c->stream>>>(
+        c->fpart, c->fpart_splits, add_rec ? c->frec : nullptr, c->f, c->n, fsum_part(c), c->status, c->scal,
+        energy ? c->upart : nullptr, c->n_upart_used, c->tickets + kTickForce);
     c->launches++;
     TCP_CUDA(cudaGetLastError());
     return TCP_OK;
 }
 
 int launch_spme_sum(tcp_ctx *c) {
-    add_rec_kernel<<<nblocks(c->n), kIntThreads, 0, c->stream>>>(c->f, c->frec, c->n, fsum_part(c));
+    add_rec_kernel<<<part_blocks(c->n), kPartThreads, 0, c->stream>>>(c->f, c->frec, c->n, fsum_part(c), c->scal,
+                                                                      c->tickets + kTickAdd);
     c->launches++;
     TCP_CUDA(cudaGetLastError());
     return TCP_OK;
 }
 
 int launch_fsum(tcp_ctx *c) {
-    add_rec_kernel<<<nblocks(c->n), kIntThreads, 0, c->stream>>>(c->f, nullptr, c->n, fsum_part(c));
+    add_rec_kernel<<<part_blocks(c->n), kPartThreads, 0, c->stream>>>(c->f, nullptr, c->n, fsum_part(c), c->scal,
+                                                                      c->tickets + kTickAdd);
     c->launches++;
     TCP_CUDA(cudaGetLastError());
     return TCP_OK;
 }
 
 int launch_remove_rigid(tcp_ctx *c) {
-    remove_net_kernel<<<nblocks(c->n), kIntThreads, 0, c->stream>>>(c->f, c->n, fsum_part(c), nblocks(c->n));
+    remove_net_kernel<<<nblocks(3 * c->n), kIntThreads, 0, c->stream>>>(c->f, c->n, c->scal);
     c->launches++;
     TCP_CUDA(cudaGetLastError());
     return TCP_OK;
 }
 
-// Returns the kinetic pass whose partials hold the final sum m v^2.
-int launch_kick2(tcp_ctx *c, double dt, bool remove_net, bool apply_thermo, bool vdf, int *final_pass) {
+int launch_kick2(tcp_ctx *c, double dt, bool remove_net, bool apply_thermo, bool vdf) {
     KickArgs k;
     k.a = int_args(c);
     k.dt = dt;
@@ -510,11 +631,7 @@ int launch_kick2(tcp_ctx *c, double dt, bool remove_net, bool apply_thermo, bool
     const bool rescale = apply_thermo && (c->p.thermo == TCP_THERMO_ISOKIN || c->p.thermo == TCP_THERMO_BEREND);
     if (!apply_thermo && k.thermo != TCP_THERMO_STOCH) k.thermo = TCP_THERMO_NOTEMP;
     k.remove_net = remove_net;
-    k.fsum_part = fsum_part(c);
-    k.nbf = nblocks(c->n);
-    k.nb = nblocks(c->n);
     k.mv_part = mv_part(c, 0);
-    k.mv_in = nullptr;
     k.vdf = vdf && !rescale;
     k.vdf_counts = c->vdf;
     k.dv0 = c->p.dv_e;
@@ -524,30 +641,22 @@ int launch_kick2(tcp_ctx *c, double dt, bool remove_net, bool apply_thermo, bool
     k.tau = c->p.tau;
     k.alpha_lgv = c->p.alpha_lgv;
     k.seed = c->p.seed;
-    k.step = c->scal + kScalStep;
-    k.rescale = 0;
-    kick2_kernel<<<k.nb, kIntThreads, 0, c->stream>>>(k);
+    k.scal = c->scal;
+    k.last_pass = !rescale;
+    k.ticket = c->tickets + kTickKick;
+    const int nb = part_blocks(c->n);
+    kick2_kernel<<<nb, kPartThreads, 0, c->stream>>>(k);
     c->launches++;
-    *final_pass = 0;
     if (rescale) {
         k.thermo = c->p.thermo;
         k.remove_net = 0;
-        k.mv_in = mv_part(c, 0);
         k.mv_part = mv_part(c, 1);
         k.vdf = vdf;
-        k.rescale = 1;
-        rescale_kernel<<<k.nb, kIntThreads, 0, c->stream>>>(k);
+        k.last_pass = 1;
+        k.ticket = c->tickets + kTickScale;
+        rescale_kernel<<<nb, kPartThreads, 0, c->stream>>>(k);
         c->launches++;
-        *final_pass = 1;
     }
-    TCP_CUDA(cudaGetLastError());
-    return TCP_OK;
-}
-
-int launch_reduce(tcp_ctx *c, int mask, int pass) {
-    reduce_scalars_kernel<<<1, 1024, 0, c->stream>>>(c->upart, c->n_upart, mv_part(c, pass), nblocks(c->n), c->scal,
-                                                     mask);
-    c->launches++;
     TCP_CUDA(cudaGetLastError());
     return TCP_OK;
 }

@@ -482,33 +482,6 @@ __global__ void __launch_bounds__(kPairThreads) pair_fp64_kernel(const PairArgs 
 }
 
 // ---------------------------------------------------------------------------
-// f = sum over splits of fpart (+ frec: the SPME_SUM add of force.f90:953-964
-// fused); per-block partial sums of f for REMOVE_RIGIDMTN (force.f90:986-993).
-// When a tile wait of the pair kernel ran out (status), some partials were
-// never written: f is then left as it was and the caller reports the error.
-__global__ void force_finalize_kernel(const double *__restrict__ fpart, int nsplit,
-                                      const double *__restrict__ frec, double *__restrict__ f, int n,
-                                      double *__restrict__ fsum_part, const unsigned *__restrict__ status) {
-    __shared__ double red[32];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool write = !(status && (*status & kStatusTmaTimeout));
-    double s[3] = {0.0, 0.0, 0.0};
-    if (i < n) {
-        for (int k = 0; k < 3; ++k) {
-            double acc = 0.0;
-            for (int sp = 0; sp < nsplit; ++sp) acc += fpart[((size_t)sp * 3 + k) * n + i];
-            if (frec) acc += frec[(size_t)k * n + i];
-            if (write) f[(size_t)k * n + i] = acc;
-            s[k] = acc;
-        }
-    }
-    for (int k = 0; k < 3; ++k) {
-        const double t = block_sum(s[k], red);
-        if (threadIdx.x == 0) fsum_part[k * gridDim.x + blockIdx.x] = t;
-    }
-}
-
-// ---------------------------------------------------------------------------
 // host side
 void make_pair_consts(tcp_ctx *c) {
     PairConsts &k = c->pc;
@@ -676,19 +649,20 @@ int pair_setup(tcp_ctx *c) {
         if (int rc = n3_f64_prepare(c)) return rc;
     TCP_CUDA(cudaMalloc(&c->fpart, sizeof(double) * 3 * (size_t)c->n * js));
     TCP_CUDA(cudaMalloc(&c->upart, sizeof(double) * (size_t)c->n_upart));
-    TCP_CUDA(cudaMemsetAsync(c->upart, 0, sizeof(double) * (size_t)c->n_upart, c->stream));
     return TCP_OK;
 }
 
 int launch_pair(tcp_ctx *c, bool energy, bool rdf) {
     const bool fp64 = c->p.precision == TCP_PREC_FP64;
+    const bool cleared = c->cleared;   // by the half kick of the running step
+    c->cleared = false;
     if (n3_applicable(c)) {
         c->fpart_splits = 1;
-        return launch_pair_n3(c, energy, rdf);
+        return launch_pair_n3(c, energy, rdf, cleared);
     }
     if (n3_f64_applicable(c)) {
         c->fpart_splits = 1;
-        return launch_pair_n3_f64(c, energy, rdf);
+        return launch_pair_n3_f64(c, energy, rdf, cleared);
     }
     c->fpart_splits = c->jsplit;
     Geometry g = geometry(c, fp64);
@@ -711,11 +685,7 @@ int launch_pair(tcp_ctx *c, bool energy, bool rdf) {
     a.status = c->status;
     a.c = c->pc;
     dim3 grid(g.nblk, c->jsplit);
-    // the energy reduction sums all n_upart partials: clear the ones this grid
-    // does not write (an earlier Newton-3 launch may have used more CTAs)
-    if (energy && (size_t)g.nblk * c->jsplit < (size_t)c->n_upart)
-        TCP_CUDA(cudaMemsetAsync(c->upart + (size_t)g.nblk * c->jsplit, 0,
-                                 sizeof(double) * ((size_t)c->n_upart - (size_t)g.nblk * c->jsplit), c->stream));
+    c->n_upart_used = g.nblk * c->jsplit;
     const int ei = c->p.ei_model == TCP_EI_DEUTSCH ? 1 : (c->p.ei_model == TCP_EI_KELBG ? 2 : 0);
 #define TCP_PAIR_DISPATCH(KERNEL, ...)                                                                   \
     do {                                                                                                 \
@@ -743,16 +713,6 @@ int launch_pair(tcp_ctx *c, bool energy, bool rdf) {
     else
         TCP_PAIR_DISPATCH(pair_fp32c_kernel, , false);
 #undef TCP_PAIR_DISPATCH
-    c->launches++;
-    TCP_CUDA(cudaGetLastError());
-    return TCP_OK;
-}
-
-int launch_force_finalize(tcp_ctx *c, bool add_rec) {
-    const int threads = 256;
-    const int blocks = ceil_div(c->n, threads);
-    force_finalize_kernel<<<blocks, threads, 0, c->stream>>>(c->fpart, c->fpart_splits, add_rec ? c->frec : nullptr,
-                                                             c->f, c->n, c->red, c->status);
     c->launches++;
     TCP_CUDA(cudaGetLastError());
     return TCP_OK;
@@ -797,6 +757,16 @@ __global__ void noalloc_positions_kernel(const double *__restrict__ x, int n, do
     const double y0 = x[i], y1 = x[(size_t)n + i], y2 = x[2 * (size_t)n + i];
     if (xq) xq[i] = make_int4(fixed_coord(y0, iL0), fixed_coord(y1, iL1), fixed_coord(y2, iL2), 0);
     if (xd) xd[i] = make_double4_32a(y0, y1, y2, 0.0);
+}
+
+// f = sum over splits of fpart; left as it was when a tile wait ran out
+__global__ void noalloc_finalize_kernel(const double *__restrict__ fpart, int nsplit, double *__restrict__ f, int n,
+                                        const unsigned *__restrict__ status) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 3 * n || (*status & kStatusTmaTimeout)) return;
+    double acc = 0.0;
+    for (int sp = 0; sp < nsplit; ++sp) acc += fpart[(size_t)sp * 3 * n + t];
+    f[t] = acc;
 }
 
 __global__ void noalloc_sum_kernel(const double *__restrict__ part, int np, double *out) {
@@ -922,7 +892,7 @@ extern "C" int tcp_force_direct_noalloc(const tcp_params *p, int nel, int nion, 
             else pair_fp32c_kernel<2, true, false, false><<<grid, kPairThreads, 0, st>>>(a);
         }
     }
-    force_finalize_kernel<<<nbf, 256, 0, st>>>(fpart, js, nullptr, f, tmp.n, fsum, status);
+    noalloc_finalize_kernel<<<ceil_div(3 * tmp.n, 256), 256, 0, st>>>(fpart, js, f, tmp.n, status);
     noalloc_sum_kernel<<<1, 1024, 0, st>>>(upart, g.nblk * js, fsum);   // Ur into fsum[0]
     TCP_CUDA(cudaGetLastError());
     double ur = 0.0;

@@ -853,7 +853,7 @@ static void n3_rejoin_set(N3Rejoin &r, const N3Args &a, int grid, int threads, c
     r.fn = fn;
 }
 
-int launch_pair_n3(tcp_ctx *c, bool energy, bool rdf) {
+int launch_pair_n3(tcp_ctx *c, bool energy, bool rdf, bool cleared) {
     int rv = c->pc.erfc5_ok ? 0 : 1;   // the 2-warp forms: the fastest RDF steps measured
     if (const char *forced = getenv("TCP_RDF_VARIANT")) rv = std::min(std::max(atoi(forced), 0), kN3RdfVariants - 1);
     if (kRdfVariants[rv].erfc5 && !c->pc.erfc5_ok) rv = 1;
@@ -891,9 +891,11 @@ int launch_pair_n3(tcp_ctx *c, bool energy, bool rdf) {
     const int rejoin = (int)std::min<long long>(full - grid, total - grid);
     if (grid + std::max(rejoin, 0) > c->n_upart)
         return set_error(TCP_ERR_STATE, "energy partial buffer smaller than the Newton-3 grid");
-    TCP_CUDA(cudaMemsetAsync(c->fpart, 0, sizeof(double) * 3 * (size_t)c->n, c->stream));
-    TCP_CUDA(cudaMemsetAsync(c->counter, 0, sizeof(unsigned), c->stream));
-    if (energy) TCP_CUDA(cudaMemsetAsync(c->upart, 0, sizeof(double) * (size_t)c->n_upart, c->stream));
+    c->n_upart_used = grid + std::max(rejoin, 0);
+    if (!cleared) {
+        TCP_CUDA(cudaMemsetAsync(c->fpart, 0, sizeof(double) * 3 * (size_t)c->n, c->stream));
+        TCP_CUDA(cudaMemsetAsync(c->counter, 0, sizeof(unsigned), c->stream));
+    }
     if (rejoin > 0) {
         TCP_CUDA(cudaEventRecord(c->ev_pair_ready, c->stream));
         N3Args r = a;
@@ -1005,7 +1007,7 @@ int n3_batch_ctas(int num_sms, int v) { return n3_batch_grid(num_sms, std::min(s
 int launch_pair_n3_batch(cudaStream_t st, const int4 *xq, int ntot, double *facc, const void *reps_dev, int nrep,
                          long long total, const long long *chunks, unsigned nchunks, double *ur_rep, unsigned *status,
                          unsigned *counter, int num_sms, bool energy, int variant, int reserve, N3Rejoin *rejoin,
-                         cudaEvent_t ready) {
+                         cudaEvent_t ready, bool cleared) {
     const int v = std::min(std::max(variant, 0), kN3BatchVariants - 1);
     N3Args a;
     std::memset(&a, 0, sizeof a);
@@ -1026,9 +1028,11 @@ int launch_pair_n3_batch(cudaStream_t st, const int4 *xq, int ntot, double *facc
     const int grid = (int)std::min<long long>(std::max(1, full - res), total);
     const int extra = (int)std::min<long long>(full - grid, total - grid);   // rejoin CTAs
     const int nt = 32 * kBatchVariants[v].W;
-    TCP_CUDA(cudaMemsetAsync(facc, 0, sizeof(double) * 3 * (size_t)ntot, st));
-    TCP_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned), st));
-    if (energy) TCP_CUDA(cudaMemsetAsync(ur_rep, 0, sizeof(double) * (size_t)nrep, st));
+    if (!cleared) {
+        TCP_CUDA(cudaMemsetAsync(facc, 0, sizeof(double) * 3 * (size_t)ntot, st));
+        TCP_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned), st));
+        if (energy) TCP_CUDA(cudaMemsetAsync(ur_rep, 0, sizeof(double) * (size_t)nrep, st));
+    }
     if (res > 0 && extra > 0) {   // the batched kernels add Ur per replica by atomics
         TCP_CUDA(cudaEventRecord(ready, st));
         n3_rejoin_set(*rejoin, a, extra, nt,

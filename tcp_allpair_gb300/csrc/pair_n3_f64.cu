@@ -564,7 +564,7 @@ int n3_f64_prepare(tcp_ctx *c) {
     return TCP_OK;
 }
 
-int launch_pair_n3_f64(tcp_ctx *c, bool energy, bool rdf) {
+int launch_pair_n3_f64(tcp_ctx *c, bool energy, bool rdf, bool cleared) {
     if (!c->f64tab) return set_error(TCP_ERR_STATE, "no FP64 pair tables");
     N3Args a;
     std::memset(&a, 0, sizeof a);
@@ -624,9 +624,11 @@ int launch_pair_n3_f64(tcp_ctx *c, bool energy, bool rdf) {
     p.total = (long long)p.group * p.ng * (p.ng + 1) / 2 * p.split;
     const int grid = (int)std::min<long long>(n3_f64_grid(c), (p.total + kF64Warps - 1) / kF64Warps);
     if (grid > c->n_upart) return set_error(TCP_ERR_STATE, "energy partial buffer smaller than the Newton-3 grid");
-    TCP_CUDA(cudaMemsetAsync(c->fpart, 0, sizeof(double) * 3 * (size_t)c->n, c->stream));
-    TCP_CUDA(cudaMemsetAsync(c->counter, 0, sizeof(unsigned), c->stream));
-    if (energy) TCP_CUDA(cudaMemsetAsync(c->upart, 0, sizeof(double) * (size_t)c->n_upart, c->stream));
+    c->n_upart_used = grid;
+    if (!cleared) {
+        TCP_CUDA(cudaMemsetAsync(c->fpart, 0, sizeof(double) * 3 * (size_t)c->n, c->stream));
+        TCP_CUDA(cudaMemsetAsync(c->counter, 0, sizeof(unsigned), c->stream));
+    }
     f64_kernel(c, energy, rdf)<<<grid, kF64Threads, f64_smem(p.ew_seg, p.ei_seg), c->stream>>>(a, p);
     c->launches++;
     TCP_CUDA(cudaGetLastError());

@@ -23,7 +23,7 @@
 #include <vector>
 
 #include "device_util.cuh"
-#include "spme_math.cuh"
+#include "spme_chain.cuh"
 #include "tcp_internal.h"
 
 namespace tcp {
@@ -36,301 +36,6 @@ struct SpmeArgs {
     double kl0, kl1, kl2;   // K/L: the step's kernels multiply (GB300's FP64 division is slow)
     int K1, K2, K3;
 };
-
-// ---- atomic-free charge spreading (cell-sorted) --------------------------------
-// A particle's support is the P^3 mesh points from its base index
-// b = INT(u)-(P-3) (force.f90:742-744).  Particles are counting-sorted by the
-// (y, z) mesh column of their base (bin = by + K2 bz); each bin is put in
-// particle-index order and the B-spline weights of every particle are stored
-// once, in sorted order.  The spread is then a gather by mesh rows: a warp
-// owns ROWS consecutive rows (y0 .. y0 + ROWS - 1, z) in shared memory (ROWS
-// = 8, or 4 / 2 on small meshes) and visits, for jz < P, the bins
-// (y0 - P + 1 .. y0 + ROWS - 1, z - jz) -- a
-// contiguous (or wrapped) range of the sorted list, staged 32 particles at a
-// time.  For one particle its lanes cover the P x P points (jy, jx) of plane
-// z, so no two lanes and no two warps touch the same point: no atomics, and
-// every mesh point is summed in the same order (jz, bins, particle index) on
-// every call.  The bin counts and slots come from integer atomics; the sum
-// does not depend on them.  FP64 mode adds FP64 products in FP64; FP32C mode
-// adds FP32 products in compensated two-float FP32 (TwoSum hi/lo) and writes
-// the FP32 mesh read by the FP32 transforms (GB300's FP64 rate is 1/64 of
-// FP32).
-constexpr int kRows = 8;                 // mesh rows per warp (fewer for small meshes: spread_rows)
-constexpr int kRowWarps = 4;             // warps per CTA (fewer when the rows of a large mesh need the space)
-constexpr int kScanBlock = 1024;         // bins per block of the prefix sum
-constexpr int kSortReg = 8;              // bins up to this size are sorted in registers
-
-
-template <int P>
-__global__ void spme_bin_count_kernel(const SpmeArgs a, SpreadBins b) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= a.n) return;
-    const double L[3] = {a.box0, a.box1, a.box2};
-    const double KL[3] = {a.kl0, a.kl1, a.kl2};
-    const int K[3] = {a.K1, a.K2, a.K3};
-    int base[3];
-#pragma unroll
-    for (int d = 1; d < 3; ++d) {
-        const double u = (a.x[(size_t)d * a.n + m] + L[d] * .5) * KL[d];   // force.f90:700-702, K/L precomputed
-        base[d] = wrapi((int)trunc(u) - (P - 3), K[d]);
-    }
-    const int bin = base[1] + a.K2 * base[2];
-    b.rank[m] = atomicAdd(&b.count[bin], 1);
-    b.ebx[m] = bin;                      // the bin of particle m (read back by the scatter)
-}
-
-// exclusive prefix sum of count[0..nbins) into start[0..nbins], in three steps
-__global__ void scan_block_kernel(const int *__restrict__ count, int nbins, int *__restrict__ start,
-                                  int *__restrict__ bsum) {
-    __shared__ int ws[32];
-    const int i = blockIdx.x * kScanBlock + threadIdx.x;
-    const int v = i < nbins ? count[i] : 0;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) ws[w] = x;
-    __syncthreads();
-    if (w == 0) {
-        int t = ws[lane];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, t, o);
-            if (lane >= o) t += y;
-        }
-        ws[lane] = t;
-    }
-    __syncthreads();
-    const int incl = x + (w > 0 ? ws[w - 1] : 0);
-    if (i < nbins) start[i] = incl - v;
-    if (threadIdx.x == kScanBlock - 1) bsum[blockIdx.x] = incl;
-}
-
-// One CTA for up to kScanBlock * kScanPer bins: each thread sums its run of
-// consecutive bins, the CTA scans the run sums, and each thread writes its
-// run's exclusive prefix; start[nbins] = total.  Above 8,192 bins the runs
-// are long enough that the three-launch scan is faster (16,384 bins: 17.7
-// against 8.4 us under ncu).
-constexpr int kScanPer = 8;
-__global__ void __launch_bounds__(kScanBlock) scan_single_kernel(const int *__restrict__ count, int nbins,
-                                                                 int *__restrict__ start, int total) {
-    __shared__ int ws[32];
-    const int per = (nbins + kScanBlock - 1) / kScanBlock;
-    const int b0 = min(nbins, (int)threadIdx.x * per), b1 = min(nbins, b0 + per);
-    int v = 0;
-    for (int k = b0; k < b1; ++k) v += count[k];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) ws[w] = x;
-    __syncthreads();
-    if (w == 0) {
-        int t = ws[lane];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, t, o);
-            if (lane >= o) t += y;
-        }
-        ws[lane] = t;
-    }
-    __syncthreads();
-    int run = x - v + (w > 0 ? ws[w - 1] : 0);
-    for (int k = b0; k < b1; ++k) {
-        const int t = count[k];
-        start[k] = run;
-        run += t;
-    }
-    if (threadIdx.x == 0) start[nbins] = total;
-}
-
-__global__ void scan_sums_kernel(int *__restrict__ bsum, int nblocks) {
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int k = 0; k < nblocks; ++k) {
-            const int t = bsum[k];
-            bsum[k] = acc;
-            acc += t;
-        }
-    }
-}
-
-__global__ void scan_add_kernel(int *__restrict__ start, int nbins, const int *__restrict__ bsum, int total) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nbins) start[i] += bsum[i / kScanBlock];
-    if (i == 0) start[nbins] = total;
-}
-
-__global__ void spme_bin_scatter_kernel(int n, SpreadBins b) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= n) return;
-    b.list[b.start[b.ebx[m]] + b.rank[m]] = m;
-}
-
-// each bin in particle-index order: small bins by a register sorting pass,
-// larger ones by insertion sort in place
-__global__ void spme_bin_sort_kernel(SpreadBins b, int nbins) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nbins) return;
-    const int s = b.start[k], e = b.start[k + 1], cnt = e - s;
-    if (cnt <= 1) return;
-    if (cnt <= kSortReg) {
-        int v[kSortReg];
-#pragma unroll
-        for (int i = 0; i < kSortReg; ++i) v[i] = i < cnt ? b.list[s + i] : 0x7fffffff;
-#pragma unroll
-        for (int i = 0; i < kSortReg; ++i)            // odd-even transposition sort
-#pragma unroll
-            for (int j = i & 1; j + 1 < kSortReg; j += 2)
-                if (v[j] > v[j + 1]) {
-                    const int t = v[j];
-                    v[j] = v[j + 1];
-                    v[j + 1] = t;
-                }
-#pragma unroll
-        for (int i = 0; i < kSortReg; ++i)
-            if (i < cnt) b.list[s + i] = v[i];
-        return;
-    }
-    for (int i = s + 1; i < e; ++i) {
-        const int v = b.list[i];
-        int j = i - 1;
-        while (j >= s && b.list[j] > v) {
-            b.list[j + 1] = b.list[j];
-            --j;
-        }
-        b.list[j + 1] = v;
-    }
-}
-
-template <int P, typename T>
-__global__ void spme_bin_weights_kernel(const SpmeArgs a, SpreadBins b) {
-    const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pos >= a.n) return;
-    const int m = b.list[pos];
-    const double L[3] = {a.box0, a.box1, a.box2};
-    const double KL[3] = {a.kl0, a.kl1, a.kl2};
-    const int K[3] = {a.K1, a.K2, a.K3};
-    T *w = static_cast<T *>(b.ew) + (size_t)pos * 3 * P;
-    T W[P], dW[P];
-    int base[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const double u = (a.x[(size_t)d * a.n + m] + L[d] * .5) * KL[d];
-        spline_w<P, T>(u, W, dW);
-#pragma unroll
-        for (int j = 0; j < P; ++j) w[d * P + j] = W[j];
-        base[d] = wrapi((int)trunc(u) - (P - 3), K[d]);
-    }
-    b.ebx[pos] = base[0];
-    b.eby[pos] = base[1];
-    static_cast<T *>(b.eq)[pos] = (T)(m < a.nel ? a.q0 : a.q1);
-}
-
-// Shared memory of one warp: ROWS rows of hi (T) [and lo (float)] of K1
-// points, then 32 staged particles (bx, by, q, weights).
-template <int P, typename T, int ROWS = kRows>
-__host__ __device__ constexpr size_t row_warp_bytes(int K1) {
-    return (size_t)ROWS * K1 * (sizeof(T) + (sizeof(T) == 4 ? 4 : 0)) + 32 * (2 * sizeof(int) + (1 + 3 * P) * sizeof(T));
-}
-
-template <int P, typename T, int ROWS>
-__global__ void __launch_bounds__(32 * kRowWarps) spme_row_spread_kernel(const SpmeArgs a, const SpreadBins b,
-                                                                         double *__restrict__ Q,
-                                                                         float *__restrict__ Qf) {
-    constexpr bool F32 = sizeof(T) == 4;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int ngy = (a.K2 + ROWS - 1) / ROWS;
-    const long grp = (long)blockIdx.x * (blockDim.x >> 5) + warp;  // (row group, z)
-    if (grp >= (long)ngy * a.K3) return;                          // warp-uniform
-    const int y0 = (int)(grp % ngy) * ROWS, z = (int)(grp / ngy);
-    const int nrow = min(ROWS, a.K2 - y0);
-    unsigned char *base = smem + (size_t)warp * row_warp_bytes<P, T, ROWS>(a.K1);
-    T *hi = reinterpret_cast<T *>(base);                            // [ROWS][K1]
-    float *lo = reinterpret_cast<float *>(base + (size_t)ROWS * a.K1 * sizeof(T));
-    unsigned char *st = base + (size_t)ROWS * a.K1 * (sizeof(T) + (F32 ? 4 : 0));
-    T *sw = reinterpret_cast<T *>(st);                              // [32][3P]
-    T *sq = sw + 32 * 3 * P;                                        // [32]
-    int *sbx = reinterpret_cast<int *>(sq + 32), *sby = sbx + 32;   // [32], [32]
-    for (int k = lane; k < ROWS * a.K1; k += 32) {
-        hi[k] = (T)0;
-        if (F32) lo[k] = 0.f;
-    }
-    __syncwarp();
-    const int nb = nrow + P - 1;                                    // bins by = y0-P+1 .. y0+nrow-1
-    for (int jz = 0; jz < P; ++jz) {
-        int bz = z - jz;
-        bz += bz < 0 ? a.K3 : 0;
-        // the by range as at most two contiguous pieces of the sorted list
-        int by0 = y0 - P + 1, len0 = nb, len1 = 0;
-        if (by0 < 0) {
-            by0 += a.K2;
-            len0 = min(nb, a.K2 - by0);
-            len1 = nb - len0;
-        }
-        if (nb >= a.K2) {                                           // the range covers every bin
-            by0 = 0;
-            len0 = a.K2;
-            len1 = 0;
-        }
-        for (int piece = 0; piece < 2; ++piece) {
-            const int blo = (piece == 0 ? by0 : 0) + a.K2 * bz, len = piece == 0 ? len0 : len1;
-            if (len <= 0) continue;
-            const int p0 = b.start[blo], p1 = b.start[blo + len];
-            for (int c0 = p0; c0 < p1; c0 += 32) {
-                const int ne = min(32, p1 - c0);
-                if (lane < ne) {
-                    const int pos = c0 + lane;
-                    const T *w = static_cast<const T *>(b.ew) + (size_t)pos * 3 * P;
-#pragma unroll
-                    for (int j = 0; j < 3 * P; ++j) sw[lane * 3 * P + j] = w[j];
-                    sq[lane] = static_cast<const T *>(b.eq)[pos];
-                    sbx[lane] = b.ebx[pos];
-                    sby[lane] = b.eby[pos];
-                }
-                __syncwarp();
-                for (int e = 0; e < ne; ++e) {
-                    const T *w = sw + e * 3 * P;
-                    const T qz = sq[e] * w[2 * P + jz];
-                    const int bx = sbx[e], by = sby[e];
-                    for (int l = lane; l < P * P; l += 32) {
-                        const int jy = l / P, jx = l - jy * P;
-                        int rl = by + jy - y0;                      // owned row of point (jy, jx)
-                        rl += rl < 0 ? a.K2 : 0;
-                        rl -= rl >= a.K2 ? a.K2 : 0;
-                        if (rl < nrow) {
-                            int x = bx + jx;
-                            x -= x >= a.K1 ? a.K1 : 0;
-                            const T v = qz * w[P + jy] * w[jx];
-                            const int k = rl * a.K1 + x;
-                            if (F32) {
-                                const T s = hi[k] + v, bp = s - hi[k];
-                                lo[k] += (hi[k] - (s - bp)) + (v - bp);
-                                hi[k] = s;
-                            } else {
-                                hi[k] += v;
-                            }
-                        }
-                    }
-                    __syncwarp();
-                }
-            }
-        }
-    }
-    for (int k = lane; k < nrow * a.K1; k += 32) {
-        const int rl = k / a.K1, x = k - rl * a.K1;
-        const size_t g = (size_t)a.K1 * ((y0 + rl) + (size_t)a.K2 * z) + x;
-        if (F32) Qf[g] = (float)(hi[k] + lo[k]);
-        else Q[g] = (double)hi[k];
-    }
-}
 
 // Qk *= theta B; energy partial sum_m w_m theta B |Qk|^2 (w = 2 for the
 // kx columns that stand for a conjugate pair in the half spectrum).
@@ -354,58 +59,6 @@ __global__ void spme_influence_kernel(cufftDoubleComplex *__restrict__ Qk, const
         const double t = block_sum(e, red);
         if (threadIdx.x == 0) epart[blockIdx.x] = t;
     }
-}
-
-// force gather, force.f90:868-919.  T = double (FP64 mode) or float (FP32C
-// mode: FP32 mesh and weights, the per-particle sum in FP32, force in FP64).
-template <int P, typename T>
-__global__ void spme_gather_kernel(const SpmeArgs a, const T *__restrict__ phi, double coef,
-                                   double *__restrict__ frec, const int *__restrict__ order) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= a.n) return;
-    // particles in the cell-sort order of the spread: the lanes of a warp share
-    // their (y, z) mesh columns, so their mesh rows are read together
-    const int m = order ? order[t] : t;
-    const double q = m < a.nel ? a.q0 : a.q1;
-    const double L[3] = {a.box0, a.box1, a.box2};
-    const double KL[3] = {a.kl0, a.kl1, a.kl2};
-    const int K[3] = {a.K1, a.K2, a.K3};
-    T W[3][P], dW[3][P];
-    int base[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const double u = (a.x[(size_t)d * a.n + m] + L[d] * .5) * KL[d];
-        spline_w<P, T>(u, W[d], dW[d]);
-        base[d] = wrapi((int)trunc(u) - (P - 3), K[d]);    // first mesh index, wrapped once
-    }
-    T gx = 0, gy = 0, gz = 0;
-    int iz = base[2];
-#pragma unroll 1
-    for (int k = 0; k < P; ++k) {
-        int iy = base[1];
-#pragma unroll 1
-        for (int j = 0; j < P; ++j) {
-            const T *row = phi + (size_t)a.K1 * (iy + (size_t)a.K2 * iz);
-            T sx = 0, sd = 0;
-            int ix = base[0];
-#pragma unroll
-            for (int i = 0; i < P; ++i) {
-                const T ph = row[ix];
-                sx += dW[0][i] * ph;
-                sd += W[0][i] * ph;
-                ix = ix + 1 == a.K1 ? 0 : ix + 1;
-            }
-            gx += sx * W[1][j] * W[2][k];
-            gy += sd * dW[1][j] * W[2][k];
-            gz += sd * W[1][j] * dW[2][k];
-            iy = iy + 1 == a.K2 ? 0 : iy + 1;
-        }
-        iz = iz + 1 == a.K3 ? 0 : iz + 1;
-    }
-    // F = -eps/(pi V) q (K_d/L_d) sum dW W W phi
-    frec[m] = -coef * q * (double)gx * a.kl0;
-    frec[(size_t)a.n + m] = -coef * q * (double)gy * a.kl1;
-    frec[2 * (size_t)a.n + m] = -coef * q * (double)gz * a.kl2;
 }
 
 // FP32C influence multiply.  Energy terms are summed in FP32 per thread (a
@@ -437,15 +90,6 @@ __global__ void spme_influence_f_kernel(cufftComplex *__restrict__ Qk, const flo
         const double t = block_sum((double)e, red);
         if (threadIdx.x == 0) epart[blockIdx.x] = t;
     }
-}
-
-__global__ void sum_partials_kernel(const double *__restrict__ part, int np, double scale,
-                                    double *__restrict__ out) {
-    __shared__ double red[32];
-    double s = 0.0;
-    for (int i = threadIdx.x; i < np; i += blockDim.x) s += part[i];
-    s = block_sum(s, red);
-    if (threadIdx.x == 0) *out = s * scale;
 }
 
 // ---- plain Ewald k-sum ------------------------------------------------------
@@ -660,14 +304,7 @@ int spme_free(tcp_ctx *c) {
         cufftDestroy(c->plan_b);
         c->plans = false;
     }
-    int **ib[] = {&c->bin_count, &c->bin_start, &c->bin_bsum, &c->bin_rank, &c->bin_list, &c->bin_ebx, &c->bin_eby};
-    for (int **q : ib) {
-        cudaFree(*q);
-        *q = nullptr;
-    }
-    cudaFree(c->bin_ew);
-    cudaFree(c->bin_eq);
-    c->bin_ew = c->bin_eq = nullptr;
+    chain_free(c->bins);
     cudaFree(c->Q);
     cudaFree(c->Qk);
     cudaFree(c->infl);
@@ -690,8 +327,6 @@ static int spme_energy_blocks(const tcp_ctx *c) {
     return (int)std::max<long>(1, std::min<long>((total + 1023) / 1024, 4096));
 }
 
-static int prepare_cell_spread(tcp_ctx *c);
-
 int spme_setup(tcp_ctx *c) {
     const tcp_params &p = c->p;
     c->K1 = p.K[0];
@@ -702,17 +337,8 @@ int spme_setup(tcp_ctx *c) {
     const size_t nhalf = (size_t)c->Kh * c->K2 * c->K3;
     c->spme_fp32 = c->p.precision == TCP_PREC_FP32C && !c->recip_fp64;
     if (!c->Q) {
-        const size_t nbins = (size_t)c->K2 * c->K3;
-        if (cudaMalloc(&c->bin_count, sizeof(int) * (nbins + 1)) != cudaSuccess ||
-            cudaMalloc(&c->bin_start, sizeof(int) * (nbins + 1)) != cudaSuccess ||
-            cudaMalloc(&c->bin_bsum, sizeof(int) * ((nbins + kScanBlock - 1) / kScanBlock)) != cudaSuccess ||
-            cudaMalloc(&c->bin_rank, sizeof(int) * (size_t)c->n) != cudaSuccess ||
-            cudaMalloc(&c->bin_list, sizeof(int) * (size_t)c->n) != cudaSuccess ||
-            cudaMalloc(&c->bin_ebx, sizeof(int) * (size_t)c->n) != cudaSuccess ||
-            cudaMalloc(&c->bin_eby, sizeof(int) * (size_t)c->n) != cudaSuccess ||
-            cudaMalloc(&c->bin_ew, sizeof(double) * 3 * kMaxOrder * (size_t)c->n) != cudaSuccess ||
-            cudaMalloc(&c->bin_eq, sizeof(double) * (size_t)c->n) != cudaSuccess ||
-            cudaMalloc(&c->Q, sizeof(double) * nreal) != cudaSuccess ||
+        if (int rc = chain_alloc(c->bins, c->n, c->K2 * c->K3, p.order)) return rc;
+        if (cudaMalloc(&c->Q, sizeof(double) * nreal) != cudaSuccess ||
             cudaMalloc(&c->Qk, sizeof(cufftDoubleComplex) * nhalf) != cudaSuccess ||
             cudaMalloc(&c->infl, sizeof(double) * nhalf) != cudaSuccess)
             return set_error(TCP_ERR_NOMEM, "SPME mesh allocation failed");
@@ -735,7 +361,7 @@ int spme_setup(tcp_ctx *c) {
         cufftSetStream(c->plan_b, c->stream);
         c->plans = true;
     }
-    if (int rc = prepare_cell_spread(c)) return rc;
+    if (int rc = chain_prepare(spme_chain_args(c))) return rc;
     // theta(m) = exp(-pi^2 m^2/a^2)/m^2 (EWALD_SELF, force.f90:27-42) times
     // the B-spline moduli, on the half spectrum; theta(0) = 0.
     std::vector<double> bx = bspline_moduli(p.order, c->K1), by = bspline_moduli(p.order, c->K2),
@@ -788,155 +414,45 @@ static SpmeArgs spme_args(const tcp_ctx *c) {
     return a;
 }
 
-// prefix sum of the bin counts, placement by the counting-sort slots, and
-// each bin in particle-index order (shared by the single-system and batched paths)
-int launch_bin_sort(cudaStream_t st, int n, int nbins, const SpreadBins &b) {
-    const int threads = 256;
-    const int sblocks = (nbins + kScanBlock - 1) / kScanBlock;
-    const bool single = nbins <= kScanBlock * kScanPer;   // up to 8,192 (y, z) columns: one launch
-    if (single) {
-        scan_single_kernel<<<1, kScanBlock, 0, st>>>(b.count, nbins, b.start, n);
-    } else {
-        scan_block_kernel<<<sblocks, kScanBlock, 0, st>>>(b.count, nbins, b.start, b.bsum);
-        scan_sums_kernel<<<1, 32, 0, st>>>(b.bsum, sblocks);
-        scan_add_kernel<<<(nbins + threads - 1) / threads, threads, 0, st>>>(b.start, nbins, b.bsum, n);
+ChainArgs spme_chain_args(tcp_ctx *c) {
+    ChainArgs a;
+    a.n = c->n;
+    a.nbins = c->K2 * c->K3;
+    a.P = c->p.order;
+    a.fp64 = !c->spme_fp32;
+    a.k1max = c->K1;
+    a.k2max = c->K2;
+    a.planes = c->K3;
+    a.nsys = 1;
+    a.b = c->bins;
+    const int K[3] = {c->K1, c->K2, c->K3};
+    a.one.off = 0;
+    a.one.nel = c->nel;
+    a.one.bin_off = 0;
+    a.one.plane_off = 0;
+    a.one.mesh_off = 0;
+    for (int d = 0; d < 3; ++d) {
+        a.one.K[d] = K[d];
+        a.one.hL[d] = c->p.box[d] * .5;
+        a.one.KL[d] = (double)K[d] / c->p.box[d];
     }
-    spme_bin_scatter_kernel<<<(n + threads - 1) / threads, threads, 0, st>>>(n, b);
-    spme_bin_sort_kernel<<<(nbins + threads - 1) / threads, threads, 0, st>>>(b, nbins);
-    return single ? 3 : 5;
-}
-
-int bin_scan_block() { return kScanBlock; }
-
-// atomic-free spread into Q (FP64) or straight into Qf (FP32C mode)
-static SpreadBins spread_bins(tcp_ctx *c) {
-    SpreadBins b;
-    b.count = c->bin_count;
-    b.start = c->bin_start;
-    b.bsum = c->bin_bsum;
-    b.rank = c->bin_rank;
-    b.list = c->bin_list;
-    b.ebx = c->bin_ebx;
-    b.eby = c->bin_eby;
-    b.ew = c->bin_ew;
-    b.eq = c->bin_eq;
-    return b;
-}
-
-// Mesh rows per warp of the spread: 8, or 4 / 2 on meshes of fewer (y, z)
-// columns, so that the kernel keeps about 2,048 warps (13 per SM) where a
-// small mesh would leave a few warps per SM with long serial loops.  A warp
-// visits the particles of ROWS + P - 1 bin rows for ROWS mesh rows.
-static int spread_rows(const tcp_ctx *c) {
-    const long cols = (long)c->K2 * c->K3;
-    return cols >= 16384 ? kRows : (cols >= 8192 ? 4 : 2);
-}
-
-template <int P, typename T, int ROWS>
-static void launch_row_spread(tcp_ctx *c, const SpmeArgs &a, const SpreadBins &b, double *Q, float *Qf) {
-    const long groups = (long)((c->K2 + ROWS - 1) / ROWS) * c->K3;
-    const size_t per_warp = row_warp_bytes<P, T, ROWS>(c->K1);
-    const int warps = (int)std::max<size_t>(1, std::min<size_t>(kRowWarps, (200u << 10) / per_warp));
-    const size_t sm = warps * per_warp;
-    const int rblocks = (int)((groups + warps - 1) / warps);
-    spme_row_spread_kernel<P, T, ROWS><<<rblocks, 32 * warps, sm, c->rstream>>>(a, b, Q, Qf);
-}
-
-template <int P>
-static int launch_cell_spread(tcp_ctx *c, const SpmeArgs &a, double *Q, float *Qf) {
-    const SpreadBins b = spread_bins(c);
-    const int threads = 256, pblocks = (c->n + threads - 1) / threads;
-    const int nbins = c->K2 * c->K3;
-    TCP_CUDA(cudaMemsetAsync(c->bin_count, 0, sizeof(int) * (size_t)nbins, c->rstream));
-    spme_bin_count_kernel<P><<<pblocks, threads, 0, c->rstream>>>(a, b);
-    const int sort_kernels = launch_bin_sort(c->rstream, c->n, nbins, b);
-    if (Qf) {
-        spme_bin_weights_kernel<P, float><<<pblocks, threads, 0, c->rstream>>>(a, b);
-        switch (spread_rows(c)) {
-            case 2: launch_row_spread<P, float, 2>(c, a, b, nullptr, Qf); break;
-            case 4: launch_row_spread<P, float, 4>(c, a, b, nullptr, Qf); break;
-            default: launch_row_spread<P, float, kRows>(c, a, b, nullptr, Qf); break;
-        }
-    } else {
-        spme_bin_weights_kernel<P, double><<<pblocks, threads, 0, c->rstream>>>(a, b);
-        switch (spread_rows(c)) {
-            case 2: launch_row_spread<P, double, 2>(c, a, b, Q, nullptr); break;
-            case 4: launch_row_spread<P, double, 4>(c, a, b, Q, nullptr); break;
-            default: launch_row_spread<P, double, kRows>(c, a, b, Q, nullptr); break;
-        }
-    }
-    c->launches += 3 + sort_kernels;
-    TCP_CUDA(cudaGetLastError());
-    return TCP_OK;
-}
-
-// shared-memory limits of the spread kernels for this mesh (set once, outside
-// any stream capture; a launch uses at most kRowWarps warps' worth)
-template <int P, typename T, int ROWS>
-static int prepare_row_spread(tcp_ctx *c) {
-    const size_t s = std::min<size_t>(kRowWarps * row_warp_bytes<P, T, ROWS>(c->K1), 200u << 10);
-    TCP_CUDA(cudaFuncSetAttribute(spme_row_spread_kernel<P, T, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)std::max(s, row_warp_bytes<P, T, ROWS>(c->K1))));
-    return TCP_OK;
-}
-
-template <int P>
-static int prepare_cell_spread_p(tcp_ctx *c) {
-    for (int rc : {prepare_row_spread<P, float, 2>(c), prepare_row_spread<P, float, 4>(c),
-                   prepare_row_spread<P, float, kRows>(c), prepare_row_spread<P, double, 2>(c),
-                   prepare_row_spread<P, double, 4>(c), prepare_row_spread<P, double, kRows>(c)})
-        if (rc) return rc;
-    return TCP_OK;
-}
-
-static int prepare_cell_spread(tcp_ctx *c) {
-    switch (c->p.order) {
-        case 4: return prepare_cell_spread_p<4>(c);
-        case 5: return prepare_cell_spread_p<5>(c);
-        case 6: return prepare_cell_spread_p<6>(c);
-        case 7: return prepare_cell_spread_p<7>(c);
-        default: return prepare_cell_spread_p<8>(c);
-    }
-}
-
-static int cell_spread(tcp_ctx *c, const SpmeArgs &a, double *Q, float *Qf) {
-    switch (c->p.order) {
-        case 4: return launch_cell_spread<4>(c, a, Q, Qf);
-        case 5: return launch_cell_spread<5>(c, a, Q, Qf);
-        case 6: return launch_cell_spread<6>(c, a, Q, Qf);
-        case 7: return launch_cell_spread<7>(c, a, Q, Qf);
-        default: return launch_cell_spread<8>(c, a, Q, Qf);
-    }
-}
-
-template <int P>
-static void launch_gather(tcp_ctx *c, const SpmeArgs &a, double coef) {
-    const int threads = 128, blocks = (c->n + threads - 1) / threads;
-    const int *order = c->bin_list;      // the spread of this chain sorted the particles
-    if (c->spme_fp32)
-        spme_gather_kernel<P, float><<<blocks, threads, 0, c->rstream>>>(a, c->Qf, coef, c->frec, order);
-    else
-        spme_gather_kernel<P, double><<<blocks, threads, 0, c->rstream>>>(a, c->Q, coef, c->frec, order);
-}
-
-static void gather(tcp_ctx *c, const SpmeArgs &a, double coef) {
-    switch (c->p.order) {
-        case 4: launch_gather<4>(c, a, coef); break;
-        case 5: launch_gather<5>(c, a, coef); break;
-        case 6: launch_gather<6>(c, a, coef); break;
-        case 7: launch_gather<7>(c, a, coef); break;
-        default: launch_gather<8>(c, a, coef); break;
-    }
+    for (int t = 0; t < 2; ++t) a.one.q[t] = c->p.charge_scale * c->p.q[t];
+    a.one.coef = kEps / (kPi * c->V);
+    a.many = nullptr;
+    a.sys_of = nullptr;
+    a.mesh = c->spme_fp32 ? (void *)c->Qf : (void *)c->Q;
+    a.ticket = c->tickets + kTickBin;
+    return a;
 }
 
 // the red[] region after the force and kinetic partials holds the energy partials
 double *recip_epart(tcp_ctx *c);
 
 int launch_spme(tcp_ctx *c, bool energy) {
-    const SpmeArgs a = spme_args(c);
-    // charge accumulation, atomic-free (every mesh point is written)
-    int rcs = cell_spread(c, a, c->spme_fp32 ? nullptr : c->Q, c->spme_fp32 ? c->Qf : nullptr);
-    if (rcs) return rcs;
+    const ChainArgs chain = spme_chain_args(c);
+    if (!c->binned) c->launches += chain_bin(chain, c->x, c->rstream);
+    c->binned = false;
+    c->launches += chain_spread(chain, c->rstream);
     const long total = (long)c->K3 * c->K2 * c->Kh;
     const int eb = spme_energy_blocks(c);
     double *epart = recip_epart(c);
@@ -953,12 +469,8 @@ int launch_spme(tcp_ctx *c, bool energy) {
         c->launches++;
         if (cufftExecZ2D(c->plan_b, c->Qk, c->Q) != CUFFT_SUCCESS) return set_error(TCP_ERR_CUFFT, "cufftExecZ2D failed");
     }
-    gather(c, a, kEps / (kPi * c->V));
-    c->launches++;
-    if (energy) {
-        sum_partials_kernel<<<1, 1024, 0, c->rstream>>>(epart, eb, kEps / (2.0 * kPi * c->V), c->scal + kScalUm);
-        c->launches++;
-    }
+    c->launches += chain_gather(chain, c->frec, epart, eb, kEps / (2.0 * kPi * c->V),
+                                energy ? c->scal + kScalUm : nullptr, c->rstream);
     TCP_CUDA(cudaGetLastError());
     return TCP_OK;
 }
@@ -990,7 +502,7 @@ int ewald_setup(tcp_ctx *c) {
                 kv.push_back(std::exp(-m2 * kPi * kPi / (c->alpha * c->alpha)) / m2);
             }
     c->nk = (int)(kv.size() / 4);
-    if (c->nk > c->red_cap - 7 * kick_blocks(c->n))
+    if (c->nk > c->red_cap - 7 * part_blocks(c->n))
         return set_error(TCP_ERR_BAD_PARAM, "ewald_nmax2 too large: more k-vectors than the energy buffer holds");
     ewald_free(c);
     if (c->nk == 0) return TCP_OK;
@@ -1177,8 +689,7 @@ __global__ void spme_gather_hvp_kernel(const SpmeArgs a, const double *__restric
 template <int P>
 static void launch_hvp_kernels(tcp_ctx *c, const SpmeArgs &a, const double *w, double *hw, int which) {
     const int threads = 128, blocks = (c->n + threads - 1) / threads;
-    if (which == 0) (void)launch_cell_spread<P>(c, a, c->hQ, nullptr);
-    else if (which == 1) spme_spread_dipole_kernel<P><<<blocks, threads, 0, c->stream>>>(a, w, c->hdQ);
+    if (which == 1) spme_spread_dipole_kernel<P><<<blocks, threads, 0, c->stream>>>(a, w, c->hdQ);
     else spme_gather_hvp_kernel<P><<<blocks, threads, 0, c->stream>>>(a, c->hQ, c->hdQ, w, kEps / (kPi * c->V), hw);
 }
 
@@ -1231,9 +742,14 @@ int launch_spme_hvp(tcp_ctx *c, const double *w, double *hw) {
     const long total = (long)nhalf;
     const int eb = spme_energy_blocks(c);
     double *mesh[2] = {c->hQ, c->hdQ};
+    ChainArgs chain = spme_chain_args(c);
+    chain.fp64 = 1;
+    chain.mesh = c->hQ;
+    c->launches += chain_bin(chain, c->x, c->stream);
+    c->launches += chain_spread(chain, c->stream);
     for (int pass = 0; pass < 2; ++pass) {    // phi = A Q, then dphi = A dQ
         if (pass == 1) TCP_CUDA(cudaMemsetAsync(mesh[pass], 0, sizeof(double) * nreal, c->stream));
-        hvp_kernels(c, a, w, hw, pass);
+        if (pass == 1) hvp_kernels(c, a, w, hw, pass);
         if (cufftExecD2Z(c->hplan_f, mesh[pass], c->hQk) != CUFFT_SUCCESS) return set_error(TCP_ERR_CUFFT, "cufftExecD2Z failed");
         spme_influence_kernel<<<eb, 256, 0, c->stream>>>(c->hQk, c->infl, total, c->Kh, c->K1, nullptr, false);
         if (cufftExecZ2D(c->hplan_b, c->hQk, mesh[pass]) != CUFFT_SUCCESS) return set_error(TCP_ERR_CUFFT, "cufftExecZ2D failed");

@@ -6,28 +6,9 @@
 
 namespace tcp {
 
-// B-spline weights W[j] = M_P(w + P-1-j) and dW[j] = dM_P/du on the grid
-// points INT(u) + j - (P-3).  Order 4 uses the reference's explicit cubics
-// (force.f90:703-738); other orders the Cox-de Boor recursion run upward on
-// the P nonzero values.
+// Cox-de Boor recursion run upward on the P nonzero values at fraction w.
 template <int P, typename T>
-__device__ __forceinline__ void spline_w(double u, T *W, T *dW) {
-    if (P == 4) {
-        T z = (T)(trunc(u) - u + 1.0);
-        W[0] = z * z * z / (T)6;
-        dW[0] = (T)-3. * z * z / (T)6;
-        z += (T)1;
-        W[1] = ((T)-3. * z * z * z + (T)12. * z * z - (T)12. * z + (T)4.) / (T)6;
-        dW[1] = ((T)9. * z * z - (T)24. * z + (T)12.) / (T)6;
-        z += (T)1;
-        W[2] = ((T)3. * z * z * z - (T)24. * z * z + (T)60. * z - (T)44.) / (T)6;
-        dW[2] = ((T)-9. * z * z + (T)48. * z - (T)60.) / (T)6;
-        z += (T)1;
-        W[3] = (-z * z * z + (T)12. * z * z - (T)48. * z + (T)64.) / (T)6;
-        dW[3] = ((T)3. * z * z - (T)24. * z + (T)48.) / (T)6;
-        return;
-    }
-    const T w = (T)(u - trunc(u));
+__device__ __forceinline__ void spline_rec(T w, T *W, T *dW) {
     T a[P];
     a[0] = (T)1;
 #pragma unroll
@@ -49,6 +30,54 @@ __device__ __forceinline__ void spline_w(double u, T *W, T *dW) {
     }
 #pragma unroll
     for (int j = 0; j < P; ++j) W[j] = a[j];
+}
+
+// B-spline weights W[j] = M_P(w + P-1-j) and dW[j] = dM_P/du on the grid
+// points INT(u) + j - (P-3).  Order 4 uses the reference's explicit cubics
+// (force.f90:703-738); other orders the Cox-de Boor recursion run upward on
+// the P nonzero values.
+template <int P, typename T>
+__device__ __forceinline__ void spline_w(double u, T *W, T *dW) {
+    if (P == 4) {
+        T z = (T)(trunc(u) - u + 1.0);
+        W[0] = z * z * z / (T)6;
+        dW[0] = (T)-3. * z * z / (T)6;
+        z += (T)1;
+        W[1] = ((T)-3. * z * z * z + (T)12. * z * z - (T)12. * z + (T)4.) / (T)6;
+        dW[1] = ((T)9. * z * z - (T)24. * z + (T)12.) / (T)6;
+        z += (T)1;
+        W[2] = ((T)3. * z * z * z - (T)24. * z * z + (T)60. * z - (T)44.) / (T)6;
+        dW[2] = ((T)-9. * z * z + (T)48. * z - (T)60.) / (T)6;
+        z += (T)1;
+        W[3] = (-z * z * z + (T)12. * z * z - (T)48. * z + (T)64.) / (T)6;
+        dW[3] = ((T)3. * z * z - (T)24. * z + (T)48.) / (T)6;
+        return;
+    }
+    spline_rec<P, T>((T)(u - trunc(u)), W, dW);
+}
+
+// The same values from the argument that the binning stores (bin_axis): z =
+// INT(u) - u + 1 for order 4, the fraction of u otherwise.  The cubics' sixth
+// is a multiplication (a division by 6 is a subroutine in either precision).
+template <int P, typename T>
+__device__ __forceinline__ void spline_at(T arg, T *W, T *dW) {
+    if (P == 4) {
+        constexpr T c6 = (T)(1.0 / 6.0);
+        T z = arg;
+        W[0] = z * z * z * c6;
+        dW[0] = (T)-0.5 * z * z;
+        z += (T)1;
+        W[1] = ((T)-3 * z * z * z + (T)12 * z * z - (T)12 * z + (T)4) * c6;
+        dW[1] = ((T)9 * z * z - (T)24 * z + (T)12) * c6;
+        z += (T)1;
+        W[2] = ((T)3 * z * z * z - (T)24 * z * z + (T)60 * z - (T)44) * c6;
+        dW[2] = ((T)-9 * z * z + (T)48 * z - (T)60) * c6;
+        z += (T)1;
+        W[3] = (-z * z * z + (T)12 * z * z - (T)48 * z + (T)64) * c6;
+        dW[3] = ((T)3 * z * z - (T)24 * z + (T)48) * c6;
+        return;
+    }
+    spline_rec<P, T>(arg, W, dW);
 }
 
 // Weights with first and second derivatives (d/du, d^2/du^2) for every order

@@ -117,6 +117,33 @@ struct N3Rejoin {
 
 }  // namespace tcp
 
+namespace tcp {
+// Particles sorted by the (y, z) mesh column of their spline base.  "m" arrays
+// are by particle, the others by place in the sorted order.
+struct SpreadBins {
+    int *count, *start, *bsum;   // per bin; count is zero between binnings
+    int *rank, *bin, *base_m;    // slot in the bin, bin, packed base indexes (10 bits each)
+    int *list, *order, *base;    // particles by bin, the same in particle order inside each bin
+    void *arg, *q_m, *q, *ew;    // [3][n] spline arguments, charges, [n][3][2 P] weights and derivatives
+};
+// One system's mesh and charges as the chain kernels need them.
+struct SpmeGeom {
+    int off, nel, K[3], bin_off, plane_off;   // first particle, electrons, mesh, first bin and (x, y) plane
+    long long mesh_off;
+    double q[2], hL[3], KL[3];   // charges, L/2, K/L
+    double coef;                 // eps/(pi V)
+};
+struct ChainArgs {
+    int n, nbins, P, fp64, k1max, k2max, planes, nsys;   // planes: of all systems
+    SpreadBins b;
+    SpmeGeom one;                // single system
+    const SpmeGeom *many;        // batch: every system, and the system of each particle
+    const int *sys_of;
+    void *mesh;                  // double (fp64) or float
+    unsigned *ticket;
+};
+}  // namespace tcp
+
 struct tcp_ctx {
     tcp_params p;
     int nel = 0, nion = 0, n = 0;
@@ -160,6 +187,7 @@ struct tcp_ctx {
     double *fpart = nullptr;   // [jsplit][3][n]
     double *upart = nullptr;   // energy partial per pair block
     int n_upart = 0;
+    int n_upart_used = 0;      // entries the last pair launch writes
     // reductions
     double *red = nullptr;     // block partials (size red_cap)
     int red_cap = 0;
@@ -182,10 +210,10 @@ struct tcp_ctx {
     bool host_direct = false;
     // SPME
     int K1 = 0, K2 = 0, K3 = 0, Kh = 0; // Kh = K1/2+1
-    // cell-sorted spreading: counting sort by the (y, z) mesh column of the spline base
-    int *bin_count = nullptr, *bin_start = nullptr, *bin_bsum = nullptr;   // [K2 K3 (+1)], block sums
-    int *bin_rank = nullptr, *bin_list = nullptr, *bin_ebx = nullptr, *bin_eby = nullptr;   // [n]
-    void *bin_ew = nullptr, *bin_eq = nullptr;                               // weights [n][3][P], charges [n]
+    tcp::SpreadBins bins{};             // cell sort of the atomic-free spread (spme_chain.cu)
+    bool binned = false;                // the half kick of the running step has binned the positions
+    bool cleared = false;               // ... and cleared the pair accumulators
+    unsigned *tickets = nullptr;        // [8] arrival counters of the kernels whose last CTA finishes a reduction
     double *Q = nullptr;                // real mesh [K3][K2][K1]
     cufftDoubleComplex *Qk = nullptr;   // [K3][K2][Kh]
     double *infl = nullptr;             // theta * |b|^-2 on the half mesh
@@ -268,20 +296,20 @@ int cuda_check(cudaError_t e, const char *what);
 void make_pair_consts(tcp_ctx *c);                 // c->pc from c->p, c->alpha, c->rc2
 int pair_setup(tcp_ctx *c);                        // constants, jsplit, partial buffers
 int launch_pair(tcp_ctx *c, bool energy, bool rdf);
-int launch_force_finalize(tcp_ctx *c, bool add_rec);
+int launch_force_finalize(tcp_ctx *c, bool add_rec, bool energy);   // energy: Ur from the pair partials
 // pair_n3.cu
 bool n3_applicable(const tcp_ctx *c);
 bool n3_f64_applicable(const tcp_ctx *c);
 int n3_f64_grid(const tcp_ctx *c);
 int n3_f64_prepare(tcp_ctx *c);
-int launch_pair_n3_f64(tcp_ctx *c, bool energy, bool rdf);
+int launch_pair_n3_f64(tcp_ctx *c, bool energy, bool rdf, bool cleared);
 int n3_grid(const tcp_ctx *c);
 int n3_variant_count();
 const char *n3_variant_name(int v);
 bool n3_variant_usable(const tcp_ctx *c, int v);
 int autotune_pair(tcp_ctx *c);
 int time_pair_with_recip(tcp_ctx *c, int reps, double *ms);   // ctx.cu
-int launch_pair_n3(tcp_ctx *c, bool energy, bool rdf);
+int launch_pair_n3(tcp_ctx *c, bool energy, bool rdf, bool cleared);   // cleared: fpart and counter are zero
 int launch_pair_n3_rejoin(tcp_ctx *c, cudaStream_t st);   // on stream2, after the reciprocal chain
 void n3_free(tcp_ctx *c);
 int n3_rejoin_launch(N3Rejoin &r, cudaStream_t st, cudaEvent_t ready, long long *launches);
@@ -299,7 +327,7 @@ long long n3_batch_fill(void *reps_host, int nrep, const int *off, const int *ne
 int launch_pair_n3_batch(cudaStream_t st, const int4 *xq, int ntot, double *facc, const void *reps_dev, int nrep,
                          long long total, const long long *chunks, unsigned nchunks, double *ur_rep, unsigned *status,
                          unsigned *counter, int num_sms, bool energy, int variant, int reserve = 0,
-                         N3Rejoin *rejoin = nullptr, cudaEvent_t ready = nullptr);
+                         N3Rejoin *rejoin = nullptr, cudaEvent_t ready = nullptr, bool cleared = false);
 int n3_batch_ctas(int num_sms, int v);
 void n3_chunk_table(long long total, int ctas, std::vector<long long> &starts);
 int n3_prepare_chunks(tcp_ctx *c);
@@ -316,15 +344,14 @@ double *fsum_part(tcp_ctx *c);
 double *mv_part(tcp_ctx *c, int pass);
 double *recip_epart(tcp_ctx *c);
 int red_capacity(int n, int extra);
-int kick_blocks(int n);
+int part_blocks(int n);
 int launch_refresh_positions(tcp_ctx *c);
 int launch_shift(tcp_ctx *c, double sdt);
-int launch_vverlet1(tcp_ctx *c, double dt, double unused);
+int launch_vverlet1(tcp_ctx *c, double dt, bool prepare);   // prepare: also clear and bin for the forces of this step
 int launch_spme_sum(tcp_ctx *c);
 int launch_fsum(tcp_ctx *c);
 int launch_remove_rigid(tcp_ctx *c);
-int launch_kick2(tcp_ctx *c, double dt, bool remove_net, bool apply_thermo, bool vdf, int *final_pass);
-int launch_reduce(tcp_ctx *c, int mask, int pass);
+int launch_kick2(tcp_ctx *c, double dt, bool remove_net, bool apply_thermo, bool vdf);
 int launch_extract(tcp_ctx *c, const unsigned char *src, int first, int count, long stride, long off_x, long off_v,
                    long off_f, cudaStream_t st = nullptr);   // st: c->stream when null
 int launch_scatter(tcp_ctx *c, unsigned char *dst, int first, int count, long stride, long off_x, long off_v,
@@ -332,15 +359,16 @@ int launch_scatter(tcp_ctx *c, unsigned char *dst, int first, int count, long st
 int launch_pack(tcp_ctx *c, int first, int count, bool x, bool v, bool f, bool frec, int *nf);
 int launch_fp32_peak(int device, double *tffma);
 
-// spme.cu: cell sort of the atomic-free spread (single system and batch)
-struct SpreadBins {
-    int *count, *start, *bsum, *rank, *list, *ebx, *eby;
-    void *ew, *eq;                       // [n][3][P] weights, [n] charges (float or double)
-};
-// start = exclusive prefix of count (plus start[nbins] = n), list = particles
-// by bin (ebx[m] holds the bin of particle m on entry), each bin index-ordered
-int launch_bin_sort(cudaStream_t st, int n, int nbins, const SpreadBins &b);   // returns its kernel count
-int bin_scan_block();
+// spme_chain.cu: spread and gather of the SPME chain, one system or a batch
+int chain_alloc(SpreadBins &b, int n, int nbins, int order);
+void chain_free(SpreadBins &b);
+int chain_prepare(const ChainArgs &c);
+// kernel launches; each returns how many
+int chain_bin(const ChainArgs &c, const double *x, cudaStream_t st);   // not after a half kick that binned
+int chain_spread(const ChainArgs &c, cudaStream_t st);                 // place, weights, spread into c.mesh
+int chain_gather(const ChainArgs &c, double *frec, const double *epart, int nepart, double escale, double *um,
+                 cudaStream_t st);
+ChainArgs spme_chain_args(tcp_ctx *c);                                 // spme.cu
 
 // ctx.cu: step and force composition for the derivative routines
 int force_eval(tcp_ctx *c, bool remove_net);        // main.f90:100-141 on the stream
@@ -353,7 +381,7 @@ void spme_hvp_free(tcp_ctx *c);
 // adjoint.cu
 void adjoint_free(tcp_ctx *c);
 
-// reduce targets for launch_reduce
-enum { kRedUr = 1, kRedMv2 = 4 };
+// ctx->tickets
+enum { kTickStep = 0, kTickForce = 1, kTickKick = 2, kTickScale = 3, kTickBin = 4, kTickAdd = 5 };
 
 }  // namespace tcp
