@@ -40,6 +40,7 @@ struct BRep {
     double V;
     double Te, Ti, tau;
     int thermo;
+    int own;                 // transformed by fft_convolve
 };
 
 constexpr int kBThreads = 256;
@@ -283,12 +284,17 @@ struct tcp_batch {
         int K[3];
         long long mesh_off, half_off;
         int count;
+        bool own;                       // fft_convolve, not cuFFT
+        int *list = nullptr;            // device: its replicas
+        void *tw = nullptr;
         cufftHandle fwd, inv;
     };
     std::vector<Group> groups;
     // the transforms of mesh-size group k >= 1 run on gstream[k - 1] beside group 0's on stream2
     std::vector<cudaStream_t> gstream;
     cudaEvent_t ev_fft[2] = {};                 // forks: after the spread, after the influence multiply
+    cudaEvent_t ev_own = nullptr;               // fork of the groups of fft_convolve
+    int cufft_groups = 0;
     std::vector<cudaEvent_t> ev_gdone[2];       // joins of groups 1.. (each direction)
     bool ready = false;
     cudaGraphExec_t graph = nullptr;
@@ -348,6 +354,7 @@ static ChainArgs b_chain(tcp_batch *b) {
 // joined back into it.
 static int b_fft_groups(tcp_batch *b, int dir) {
     const size_t ng = b->groups.size();
+    if (b->cufft_groups == 0) return TCP_OK;
     if (ng > 1) {
         TCP_CUDA(cudaEventRecord(b->ev_fft[dir], b->stream2));
         for (size_t k = 1; k < ng; ++k) TCP_CUDA(cudaStreamWaitEvent(b->gstream[k - 1], b->ev_fft[dir], 0));
@@ -355,6 +362,7 @@ static int b_fft_groups(tcp_batch *b, int dir) {
     for (size_t k = 0; k < ng; ++k) {
         const auto &g = b->groups[k];
         const cudaStream_t st = k ? b->gstream[k - 1] : b->stream2;
+        if (g.own) continue;
         if (dir == 0) {
             cufftSetStream(g.fwd, st);
             if (cufftExecR2C(g.fwd, b->Qf + g.mesh_off, b->Qk + g.half_off) != CUFFT_SUCCESS)
@@ -372,6 +380,34 @@ static int b_fft_groups(tcp_batch *b, int dir) {
     return TCP_OK;
 }
 
+// Spread and convolution of the groups with meshes of spme_fft.cu, group k >= 1
+// on gstream[k - 1] as above.
+static int b_own_groups(tcp_batch *b, const ChainArgs &chain, const BAcc &A) {
+    const size_t ng = b->groups.size();
+    if (ng > 1) {
+        TCP_CUDA(cudaEventRecord(b->ev_own, b->stream2));
+        for (size_t k = 1; k < ng; ++k) TCP_CUDA(cudaStreamWaitEvent(b->gstream[k - 1], b->ev_own, 0));
+    }
+    for (size_t k = 0; k < ng; ++k) {
+        const auto &g = b->groups[k];
+        if (!g.own) continue;
+        FftArgs f;
+        f.half = b->Qk;
+        f.infl = b->infl;
+        f.tw = g.tw;
+        f.list = g.list;
+        f.epart = nullptr;
+        f.um = A.um;
+        f.energy = 1;
+        b->launches += fft_convolve(chain, f, g.K[0], g.count, true, k ? b->gstream[k - 1] : b->stream2);
+    }
+    for (size_t k = 1; k < ng; ++k) {
+        TCP_CUDA(cudaEventRecord(b->ev_gdone[0][k - 1], b->gstream[k - 1]));
+        TCP_CUDA(cudaStreamWaitEvent(b->stream2, b->ev_gdone[0][k - 1], 0));
+    }
+    return TCP_OK;
+}
+
 // The SPME chain of every replica (spread, batched R2C per mesh size,
 // influence multiply + energy, C2R, gather into frec), forked onto stream2
 // after the work queued on the main stream, so that it runs beside the
@@ -384,11 +420,15 @@ static int b_recip_fork(tcp_batch *b, const BAcc &A, bool binned) {
         b_bin_kernel<<<part_blocks(b->ntot), kPartThreads, 0, b->stream2>>>(parts(b), chain);
         b->launches++;
     }
-    b->launches += chain_spread(chain, b->stream2);     // atomic-free, every mesh point written
-    if (int rc = b_fft_groups(b, 0)) return rc;
-    b_influence_kernel<<<b->infl_blocks, 256, 0, b->stream2>>>(b->Qk, b->infl, b->reps, b->blk0, b->nrep, A.um);
-    if (int rc = b_fft_groups(b, 1)) return rc;
-    b->launches += 1 + chain_gather(chain, b->frec, nullptr, 0, 0.0, nullptr, b->stream2);
+    b->launches += chain_sort(chain, b->stream2);
+    if (int rc = b_own_groups(b, chain, A)) return rc;
+    if (b->cufft_groups) {                              // meshes that fft_convolve does not take
+        b->launches += 1 + chain_spread(chain, b->stream2);
+        if (int rc = b_fft_groups(b, 0)) return rc;
+        b_influence_kernel<<<b->infl_blocks, 256, 0, b->stream2>>>(b->Qk, b->infl, b->reps, b->blk0, b->nrep, A.um);
+        if (int rc = b_fft_groups(b, 1)) return rc;
+    }
+    b->launches += chain_gather(chain, b->frec, nullptr, 0, 0.0, nullptr, b->stream2);
     TCP_CUDA(cudaGetLastError());
     return TCP_OK;
 }
@@ -619,9 +659,13 @@ int tcp_batch_destroy(tcp_batch *b) {
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->graph) cudaGraphExecDestroy(b->graph);
     for (auto &g : b->groups) {
+        cudaFree(g.list);
+        cudaFree(g.tw);
+        if (g.own) continue;
         cufftDestroy(g.fwd);
         cufftDestroy(g.inv);
     }
+    if (b->ev_own) cudaEventDestroy(b->ev_own);
     for (void *ptr : {(void *)b->x, (void *)b->v, (void *)b->f, (void *)b->frec, (void *)b->facc, (void *)b->xq,
                       (void *)b->rep_of, (void *)b->reps, b->n3reps, (void *)b->n3_chunks, (void *)b->acc, (void *)b->status,
                       (void *)b->counter, (void *)b->Qf, (void *)b->infl, (void *)b->Qk, (void *)b->blk0,
@@ -747,6 +791,7 @@ int tcp_batch_create(const tcp_params *params, const int *nel, const int *nion, 
         g.mesh_off = b->mesh_total;
         g.half_off = b->half_total;
         g.count = (int)kv.second.size();
+        g.own = fft_own(g.K[0], g.K[1], g.K[2]);
         const long long nreal = (long long)g.K[0] * g.K[1] * g.K[2];
         const long long nhalf = (long long)(g.K[0] / 2 + 1) * g.K[1] * g.K[2];
         for (int k = 0; k < g.count; ++k) {
@@ -756,6 +801,16 @@ int tcp_batch_create(const tcp_params *params, const int *nel, const int *nion, 
         }
         b->mesh_total += nreal * g.count;
         b->half_total += nhalf * g.count;
+        for (int r : kv.second) b->h_reps[r].own = g.own;
+        if (g.own) {
+            if (int rc = fft_twiddles(g.K[0], false, &g.tw)) return fail(rc);
+            b->groups.push_back(g);
+            tcp_batch::Group &h = b->groups.back();
+            TCP_BALLOC(h.list, sizeof(int) * kv.second.size());
+            TCP_CUDA(cudaMemcpy(h.list, kv.second.data(), sizeof(int) * kv.second.size(), cudaMemcpyHostToDevice));
+            continue;
+        }
+        b->cufft_groups++;
         int nfwd[3] = {g.K[2], g.K[1], g.K[0]};
         if (cufftPlanMany(&g.fwd, 3, nfwd, nullptr, 1, (int)nreal, nullptr, 1, (int)nhalf, CUFFT_R2C, g.count) !=
                 CUFFT_SUCCESS ||
@@ -778,6 +833,8 @@ int tcp_batch_create(const tcp_params *params, const int *nel, const int *nion, 
             b->ev_gdone[d].push_back(e);
         }
     }
+    if (cudaEventCreateWithFlags(&b->ev_own, cudaEventDisableTiming) != cudaSuccess)
+        return fail(cuda_check(cudaGetLastError(), "cudaEventCreate"));
     for (int d = 0; d < 2 && b->groups.size() > 1; ++d)
         if (cudaEventCreateWithFlags(&b->ev_fft[d], cudaEventDisableTiming) != cudaSuccess)
             return fail(cuda_check(cudaGetLastError(), "cudaEventCreate"));
@@ -797,6 +854,9 @@ int tcp_batch_create(const tcp_params *params, const int *nel, const int *nion, 
     TCP_BALLOC(b->ticket, sizeof(unsigned));
     cudaMemsetAsync(b->ticket, 0, sizeof(unsigned), b->stream);
     if (int rc = chain_prepare(b_chain(b))) return fail(rc);
+    for (const auto &g : b->groups)
+        if (g.own)
+            if (int rc = fft_prepare(b_chain(b), g.K[0], false)) return fail(rc);
     TCP_BALLOC(b->infl, sizeof(float) * (size_t)b->half_total);
     TCP_BALLOC(b->Qk, sizeof(cufftComplex) * (size_t)b->half_total);
     TCP_BALLOC(b->blk0, sizeof(int) * (nrep + 1));
@@ -874,10 +934,16 @@ int tcp_batch_ewald_self(tcp_batch *b, double *Uo) {
             }
         }
         const long long half = (long long)R.Kh * p.K[1] * p.K[2];
+        if (R.own) {
+            const std::vector<int> order = fft_order(p.K[0]);
+            std::vector<float> t(half);
+            for (long long i = 0; i < half; ++i) t[i] = infl[R.half_off + order[i]];
+            std::copy(t.begin(), t.end(), infl.begin() + R.half_off);
+        }
         // a few blocks per replica: each block adds its energy partial to the
         // replica's Um with one FP64 atomic, and hundreds of atomics on one
         // address serialise (512 blocks a replica: 80 us for the 64 replicas)
-        blk0[r + 1] = blk0[r] + (int)std::max<long long>(1, std::min<long long>((half + 255) / 256, 16));
+        blk0[r + 1] = blk0[r] + (R.own ? 0 : (int)std::max<long long>(1, std::min<long long>((half + 255) / 256, 16)));
     }
     b->infl_blocks = blk0[nrep];
     b->pcs = pcs;
@@ -893,6 +959,8 @@ int tcp_batch_ewald_self(tcp_batch *b, double *Uo) {
         g.bin_off = R.bin_off;
         g.plane_off = R.plane_off;
         g.mesh_off = R.mesh_off;
+        g.half_off = R.half_off;
+        g.own = R.own;
         for (int d = 0; d < 3; ++d) {
             g.K[d] = R.K[d];
             g.hL[d] = R.L[d] * .5;
@@ -901,6 +969,7 @@ int tcp_batch_ewald_self(tcp_batch *b, double *Uo) {
         g.q[0] = R.q[0];
         g.q[1] = R.q[1];
         g.coef = kEps / (kPi * R.V);
+        g.ecoef = kEps / (2.0 * kPi * R.V);
     }
     TCP_CUDA(cudaMemcpyAsync(b->geo, geo.data(), sizeof(SpmeGeom) * nrep, cudaMemcpyHostToDevice, b->stream));
     TCP_CUDA(cudaMemcpyAsync(b->reps, b->h_reps.data(), sizeof(BRep) * nrep, cudaMemcpyHostToDevice, b->stream));

@@ -2,10 +2,11 @@
 // generalised to B-spline order 4..8) and the plain Ewald k-sum.
 //
 // Mesh layout: Q[iz][iy][ix] (ix fastest, the Fortran order of Q(ix,iy,iz)),
-// FP64.  The 3-D FFT is cuFFT D2Z / Z2D on that layout (the only library
-// call of the path); spreading (cell-sorted and atomic-free), the
-// influence-function multiply fused with the energy reduction, and the force
-// gather are kernels of this file.
+// FP64.  Cubic meshes of 32, 48, 64, 96 or 128 points a side are spread and
+// convolved by spme_fft.cu; for the others the 3-D FFT is cuFFT D2Z / Z2D on
+// that layout (the only library call of the path), with the influence multiply
+// and energy reduction of this file between.  Spreading (cell-sorted and
+// atomic-free) and force gather: spme_chain.cu.
 // In the compensated-FP32 mode the charge mesh is summed in two-float FP32
 // and written as FP32 for R2C / C2R transforms, the influence multiply
 // (energy summed in FP64) and the force gather: on GB300 FP64 runs at 1/64 of
@@ -305,6 +306,9 @@ int spme_free(tcp_ctx *c) {
         c->plans = false;
     }
     chain_free(c->bins);
+    cudaFree(c->fft_tw32);
+    cudaFree(c->fft_tw64);
+    c->fft_tw32 = c->fft_tw64 = nullptr;
     cudaFree(c->Q);
     cudaFree(c->Qk);
     cudaFree(c->infl);
@@ -347,7 +351,14 @@ int spme_setup(tcp_ctx *c) {
                              cudaMalloc(&c->infl_f, sizeof(float) * nhalf) != cudaSuccess))
             return set_error(TCP_ERR_NOMEM, "SPME FP32 mesh allocation failed");
     }
-    if (!c->plans) {
+    c->own_fft = fft_own(c->K1, c->K2, c->K3);
+    if (c->own_fft) {
+        for (const bool d : {false, true}) {
+            if (!d && !c->spme_fp32) continue;
+            if (int rc = fft_twiddles(c->K1, d, d ? &c->fft_tw64 : &c->fft_tw32)) return rc;
+            if (int rc = fft_prepare(spme_chain_args(c), c->K1, d)) return rc;
+        }
+    } else if (!c->plans) {
         if (inject_fault("cufft_plan")) return set_error(TCP_ERR_CUFFT, "injected: cufftPlan3d failed");
         const cufftType tf = c->spme_fp32 ? CUFFT_R2C : CUFFT_D2Z;
         const cufftType tb = c->spme_fp32 ? CUFFT_C2R : CUFFT_Z2D;
@@ -384,6 +395,12 @@ int spme_setup(tcp_ctx *c) {
                 h[idx] = std::exp(-m2 * kPi * kPi / a2) / m2 * bx[i] * by[j] * bz[k];
             }
         }
+    }
+    if (c->own_fft) {   // in the order of fft_convolve's transforms
+        const std::vector<int> order = fft_order(c->K1);
+        std::vector<double> t(nhalf);
+        for (size_t i = 0; i < nhalf; ++i) t[i] = h[order[i]];
+        h.swap(t);
     }
     TCP_CUDA(cudaMemcpyAsync(c->infl, h.data(), sizeof(double) * nhalf, cudaMemcpyHostToDevice, c->stream));
     if (c->spme_fp32) {
@@ -437,12 +454,29 @@ ChainArgs spme_chain_args(tcp_ctx *c) {
         a.one.KL[d] = (double)K[d] / c->p.box[d];
     }
     for (int t = 0; t < 2; ++t) a.one.q[t] = c->p.charge_scale * c->p.q[t];
+    a.one.half_off = 0;
+    a.one.own = c->own_fft;
     a.one.coef = kEps / (kPi * c->V);
+    a.one.ecoef = kEps / (2.0 * kPi * c->V);
     a.many = nullptr;
     a.sys_of = nullptr;
     a.mesh = c->spme_fp32 ? (void *)c->Qf : (void *)c->Q;
     a.ticket = c->tickets + kTickBin;
     return a;
+}
+
+// fft_convolve's arrays: the FP64 ones also serve the Hessian-vector products
+// of FP32C contexts
+static FftArgs spme_fft_args(tcp_ctx *c, bool fp64, bool energy) {
+    FftArgs f;
+    f.half = fp64 ? (void *)c->Qk : (void *)c->Qkf;
+    f.infl = fp64 ? (const void *)c->infl : (const void *)c->infl_f;
+    f.tw = fp64 ? c->fft_tw64 : c->fft_tw32;
+    f.list = nullptr;
+    f.epart = recip_epart(c);
+    f.um = nullptr;
+    f.energy = energy;
+    return f;
 }
 
 // the red[] region after the force and kinetic partials holds the energy partials
@@ -452,10 +486,19 @@ int launch_spme(tcp_ctx *c, bool energy) {
     const ChainArgs chain = spme_chain_args(c);
     if (!c->binned) c->launches += chain_bin(chain, c->x, c->rstream);
     c->binned = false;
-    c->launches += chain_spread(chain, c->rstream);
+    c->launches += chain_sort(chain, c->rstream);
     const long total = (long)c->K3 * c->K2 * c->Kh;
-    const int eb = spme_energy_blocks(c);
+    const int eb = c->own_fft ? fft_energy_parts(c->K1) : spme_energy_blocks(c);
     double *epart = recip_epart(c);
+    if (c->own_fft) {
+        const FftArgs f = spme_fft_args(c, !c->spme_fp32, energy);
+        c->launches += fft_convolve(chain, f, c->K1, 1, true, c->rstream);
+        c->launches += chain_gather(chain, c->frec, epart, eb, kEps / (2.0 * kPi * c->V),
+                                    energy ? c->scal + kScalUm : nullptr, c->rstream);
+        TCP_CUDA(cudaGetLastError());
+        return TCP_OK;
+    }
+    c->launches += chain_spread(chain, c->rstream);
     cufftSetStream(c->plan_f, c->rstream);
     cufftSetStream(c->plan_b, c->rstream);
     if (c->spme_fp32) {
@@ -727,7 +770,7 @@ int launch_spme_hvp(tcp_ctx *c, const double *w, double *hw) {
             cudaMalloc(&c->hQk, sizeof(cufftDoubleComplex) * nhalf) != cudaSuccess)
             return set_error(TCP_ERR_NOMEM, "SPME Hessian mesh allocation failed");
     }
-    if (!c->hplans) {
+    if (!c->own_fft && !c->hplans) {
         if (cufftPlan3d(&c->hplan_f, c->K3, c->K2, c->K1, CUFFT_D2Z) != CUFFT_SUCCESS)
             return set_error(TCP_ERR_CUFFT, "cufftPlan3d D2Z failed");
         if (cufftPlan3d(&c->hplan_b, c->K3, c->K2, c->K1, CUFFT_Z2D) != CUFFT_SUCCESS) {
@@ -746,10 +789,19 @@ int launch_spme_hvp(tcp_ctx *c, const double *w, double *hw) {
     chain.fp64 = 1;
     chain.mesh = c->hQ;
     c->launches += chain_bin(chain, c->x, c->stream);
-    c->launches += chain_spread(chain, c->stream);
+    c->launches += chain_sort(chain, c->stream);
+    if (!c->own_fft) c->launches += chain_spread(chain, c->stream);
     for (int pass = 0; pass < 2; ++pass) {    // phi = A Q, then dphi = A dQ
-        if (pass == 1) TCP_CUDA(cudaMemsetAsync(mesh[pass], 0, sizeof(double) * nreal, c->stream));
-        if (pass == 1) hvp_kernels(c, a, w, hw, pass);
+        if (pass == 1) {
+            TCP_CUDA(cudaMemsetAsync(mesh[pass], 0, sizeof(double) * nreal, c->stream));
+            hvp_kernels(c, a, w, hw, pass);
+            c->launches++;
+        }
+        if (c->own_fft) {
+            chain.mesh = mesh[pass];
+            c->launches += fft_convolve(chain, spme_fft_args(c, true, false), c->K1, 1, pass == 0, c->stream);
+            continue;
+        }
         if (cufftExecD2Z(c->hplan_f, mesh[pass], c->hQk) != CUFFT_SUCCESS) return set_error(TCP_ERR_CUFFT, "cufftExecD2Z failed");
         spme_influence_kernel<<<eb, 256, 0, c->stream>>>(c->hQk, c->infl, total, c->Kh, c->K1, nullptr, false);
         if (cufftExecZ2D(c->hplan_b, c->hQk, mesh[pass]) != CUFFT_SUCCESS) return set_error(TCP_ERR_CUFFT, "cufftExecZ2D failed");

@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kSpreadThreads) chain_spread_kernel(const Chai
     const SpmeGeom &g = BATCH ? c.many[s] : c.one;
     const int z = blockIdx.x / per_plane - (BATCH ? g.plane_off : 0), y0 = (blockIdx.x % per_plane) * rows;
     const int nrow = min(rows, g.K[1] - y0), K1 = g.K[0];
-    if (nrow <= 0) return;                       // batch: a smaller mesh than the largest
+    if (nrow <= 0 || (BATCH && g.own)) return;   // batch: a smaller mesh than the largest, or fft_convolve's
     T *h = reinterpret_cast<T *>(smem);
     float *lo = reinterpret_cast<float *>(h + (size_t)rows * c.k1max);
     const StageBuf<T> st = stage_at<T>(smem + (size_t)rows * c.k1max * 8, P);
@@ -260,10 +260,10 @@ static size_t chain_spread_bytes(int P, int k1max) {   // two-float FP32 or FP64
     return (size_t)chain_spread_rows(P, k1max) * k1max * 8 + stage_bytes<double>(P);
 }
 
-template <int P, typename T, bool BATCH>
-static int spread_p(const ChainArgs &c, cudaStream_t st) {
+template <int P, typename T>
+static int sort_p(const ChainArgs &c, cudaStream_t st) {
     const int nb = (c.n + kPartBlock - 1) / kPartBlock;
-    int launches = 3;
+    int launches = 2;
     if (c.nbins > kScanTail) {
         const int sb = (c.nbins + kScanBlock - 1) / kScanBlock;
         scan_block_kernel<<<sb, kScanBlock, 0, st>>>(c.b, c.nbins);
@@ -272,10 +272,15 @@ static int spread_p(const ChainArgs &c, cudaStream_t st) {
     }
     chain_place_kernel<<<(c.n + 127) / 128, 128, 0, st>>>(c.n, c.b);
     chain_weights_kernel<P, T><<<nb, kPartThreads, 0, st>>>(c.n, c.b);
+    return launches;
+}
+
+template <int P, typename T, bool BATCH>
+static int spread_p(const ChainArgs &c, cudaStream_t st) {
     const int rows = chain_spread_rows(P, c.k1max), per_plane = (c.k2max + rows - 1) / rows;
     chain_spread_kernel<P, T, BATCH><<<c.planes * per_plane, kSpreadThreads, chain_spread_bytes(P, c.k1max), st>>>(c, rows,
                                                                                                               per_plane);
-    return launches;
+    return 1;
 }
 
 #define TCP_CHAIN_ORDER(CALL)           \
@@ -286,6 +291,14 @@ static int spread_p(const ChainArgs &c, cudaStream_t st) {
         case 7: CALL(7); break;         \
         default: CALL(8); break;        \
     }
+
+int chain_sort(const ChainArgs &c, cudaStream_t st) {
+    int n = 0;
+#define TCP_CALL(P) n = c.fp64 ? sort_p<P, double>(c, st) : sort_p<P, float>(c, st)
+    TCP_CHAIN_ORDER(TCP_CALL)
+#undef TCP_CALL
+    return n;
+}
 
 int chain_spread(const ChainArgs &c, cudaStream_t st) {
     int n = 0;

@@ -129,9 +129,10 @@ struct SpreadBins {
 // One system's mesh and charges as the chain kernels need them.
 struct SpmeGeom {
     int off, nel, K[3], bin_off, plane_off;   // first particle, electrons, mesh, first bin and (x, y) plane
-    long long mesh_off;
+    long long mesh_off, half_off;
     double q[2], hL[3], KL[3];   // charges, L/2, K/L
-    double coef;                 // eps/(pi V)
+    double coef, ecoef;          // eps/(pi V), eps/(2 pi V)
+    int own;                     // transformed by spme_fft.cu, not cuFFT
 };
 struct ChainArgs {
     int n, nbins, P, fp64, k1max, k2max, planes, nsys;   // planes: of all systems
@@ -217,6 +218,8 @@ struct tcp_ctx {
     double *Q = nullptr;                // real mesh [K3][K2][K1]
     cufftDoubleComplex *Qk = nullptr;   // [K3][K2][Kh]
     double *infl = nullptr;             // theta * |b|^-2 on the half mesh
+    bool own_fft = false;               // the mesh is transformed by spme_fft.cu
+    void *fft_tw32 = nullptr, *fft_tw64 = nullptr;
     bool spme_fp32 = false;             // FP32C mode: FP32 transforms, influence and gather
     bool recip_fp64 = false;            // TCP_PREC_FP32C_R64: p.precision is FP32C, the reciprocal chain FP64
     float *Qf = nullptr;                // FP32 real mesh [K3][K2][K1]
@@ -363,9 +366,26 @@ int launch_fp32_peak(int device, double *tffma);
 int chain_alloc(SpreadBins &b, int n, int nbins, int order);
 void chain_free(SpreadBins &b);
 int chain_prepare(const ChainArgs &c);
+// spme_fft.cu: spread + convolution on cubic meshes of 32, 48, 64, 96, 128
+struct FftArgs {
+    void *half;            // [system][z][N/2 + 1 columns][N] complex
+    const void *infl;      // influence function in the same order (fft_order), of the precision
+    const void *tw;        // fft_twiddles
+    const int *list;       // batch: the systems of this mesh size
+    double *epart;         // single: one energy partial per CTA of the z kernel (fft_energy_parts)
+    double *um;            // batch: Um per system (zeroed before)
+    int energy;
+};
+bool fft_own(int K1, int K2, int K3);
+std::vector<int> fft_order(int N);   // element of the transform order -> index in [kz][ky][kx <= N/2]
+int fft_twiddles(int N, bool fp64, void **tw);
+int fft_energy_parts(int N);
+int fft_prepare(const ChainArgs &c, int N, bool fp64);
+int fft_convolve(const ChainArgs &c, const FftArgs &f, int N, int systems, bool spread, cudaStream_t st);
 // kernel launches; each returns how many
 int chain_bin(const ChainArgs &c, const double *x, cudaStream_t st);   // not after a half kick that binned
-int chain_spread(const ChainArgs &c, cudaStream_t st);                 // place, weights, spread into c.mesh
+int chain_sort(const ChainArgs &c, cudaStream_t st);                   // the binned particles' order and spline values
+int chain_spread(const ChainArgs &c, cudaStream_t st);                 // sorted particles -> c.mesh
 int chain_gather(const ChainArgs &c, double *frec, const double *epart, int nepart, double escale, double *um,
                  cudaStream_t st);
 ChainArgs spme_chain_args(tcp_ctx *c);                                 // spme.cu
