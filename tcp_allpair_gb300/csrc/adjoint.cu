@@ -20,9 +20,9 @@
 // 1/r^3), G2 -= y (3/(rs r^2) + 3/r^3 + 1/(rs^2 r))/r^2, dl = -y/rs^2,
 // gl = -y/(rs^3 r), y = exp(-r/rs).
 //
-// The default real-space kernel (adj_n3_kernel) visits every unique pair once
-// on the Newton-3 item schedule of the force kernels and adds +t to row i and
-// -t to row j.  With TCP_FLAG_DETERMINISTIC the ordered-pair kernel visits
+// The default real-space kernels visit every unique pair once and add +t to
+// row i and -t to row j: adj_f64_kernel on the tiles and tables of the FP64
+// force kernel, adj_n3_kernel (FP32C) on the Newton-3 item schedule.  With TCP_FLAG_DETERMINISTIC the ordered-pair kernel visits
 // every ordered pair (i, j) once: thread i sums
 // (H w)_i = sum_j qq (-G1 dw + G2 (u.dw) u), dw = w_i - w_j, and the scalars
 // dE/dlambda = 1/2 sum qq dl and dF/dlambda . w = sum qq gl (u.w_i).  The
@@ -35,7 +35,10 @@
 #include <type_traits>
 #include <vector>
 
+#include <cstring>
+
 #include "device_util.cuh"
+#include "pair_f64.cuh"
 #include "pair_math.cuh"
 #include "pair_n3.cuh"
 #include "tcp_internal.h"
@@ -426,6 +429,216 @@ __global__ void __launch_bounds__(kAdjN3Threads) adj_n3_kernel(const AdjArgs a, 
     }
 }
 
+// ---- FP64 tile form --------------------------------------------------------------
+// The unique-pair sums in FP64 on the tiles and radial tables of the FP64 force
+// kernel (pair_f64.cuh; bound: the FP64 pipe).  Per pair of a Hessian-vector
+// product 32 FP64 operations (r^2 3, table argument 1, G1 and G2 4 each, dw 3,
+// u.dw 3, weight 2, the six components of +t and -t 12), about 100 with the
+// radial functions of radial_f64: N = 4,096 Kelbg takes 617 us for the real-space part (2,150 us then).  dE/dlambda
+// (hw null) needs the e-i chunks only, and of those the pairs within the e-i
+// table.
+struct AdjFast {
+    F64Fast p;
+    const double *w;      // [3][n] or null
+    double *hw;
+    double c2, ia5;       // G2 of the e-i term in units of a^5; 1/a^5
+    double hq[3];         // H.w per unit t and pair type
+    double kgl, kdl;      // gl and dl per unit of their tables
+    double qgl, qdl;      // their sums to dF/dlambda . w and dE/dlambda
+};
+
+template <int KIND>
+__device__ __noinline__ void radial_general(const AdjArgs &a, const F64Tab &tb, double r2, double *g) {
+    radial_f64<KIND>(a, tb, r2, g[0], g[1], g[2], g[3]);
+}
+
+// minimum-image separation of two particles in units of the box (A where it is not cubic)
+template <bool CUBIC>
+__device__ __forceinline__ void f64_separation(const PairConsts &c, const long long (&xi)[3], const long long (&xj)[3],
+                                               double (&u)[3]) {
+    long long d[3];
+    bool small = false;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        d[k] = (long long)((unsigned long long)xi[k] - (unsigned long long)xj[k]);
+        u[k] = box_diff(d[k], small);
+    }
+    if (__any_sync(0xffffffffu, small))
+#pragma unroll
+        for (int k = 0; k < 3; ++k) u[k] = (double)d[k] * 5.421010862427522e-20;   // 2^-64
+    if (!CUBIC)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) u[k] *= c.box[k];
+}
+
+template <int KIND, bool HVP, bool MASKED, bool CUBIC>
+__device__ __forceinline__ void adj_tile_f64(const AdjArgs &a, const AdjFast &f, const uint4 *ew, const uint4 *ei,
+                                             const F64Tab &tb, int pt, bool diag, int icnt, const long long (&xi)[3],
+                                             const double (&wi)[3], int jstart, int jcnt, int s0, int s1,
+                                             double (&ti)[3], double &sum) {
+    constexpr int NEI = HVP ? 3 : 1;
+    const F64Fast &p = f.p;
+    const int lane = threadIdx.x & 31, src = (lane + 1) & 31;
+    const int j0 = jstart + min((lane + s0) & 31, jcnt - 1);
+    const longlong4_32a t = a.xl[j0];
+    long long xj[3] = {t.x, t.y, t.z};
+    double wj[3] = {0.0, 0.0, 0.0}, hj[3] = {0.0, 0.0, 0.0};
+    if (HVP)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) wj[k] = f.w[(size_t)k * a.n + j0];
+#pragma unroll 1
+    for (int s = s0; s < s1; ++s) {
+        double u[3];
+        f64_separation<CUBIC>(a.c, xi, xj, u);
+        const double r2 = fma(u[0], u[0], fma(u[1], u[1], u[2] * u[2]));
+        const long long rb = __double_as_longlong(r2);
+        bool ok = rb > 0 && rb < __double_as_longlong(p.rc2);
+        if (MASKED) {
+            ok = ok && lane < icnt && ((lane + s) & 31) < jcnt;
+            if (diag) ok = ok && s >= 1 && (s < 16 || (s == 16 && lane < 16));
+        }
+        const float r2f = narrow(r2);
+        const unsigned xb = __float_as_uint(r2f * p.kxf), yb = __float_as_uint(r2f * p.kyf);
+        const bool near = KIND != 0 && ok && yb < p.ei_hi;
+        const bool any_near = KIND != 0 && __any_sync(0xffffffffu, near);
+        bool need = (HVP && ok && xb < kTabLowBits) || (near && yb < kTabLowBits);
+        double g1 = 0.0, g2 = 0.0, gl = 0.0;     // units of a^3, a^5; gl (HVP) or dl
+        F64At y;
+        if (any_near) y = f64_at<kEiBits>(ei, yb, p.ei_hi, r2, p.ky, r2f, p.kyf);
+        if (HVP) {
+            const bool in = ok && xb < p.ew_hi;
+            const F64At x = f64_at<kEwBits>(ew, xb, p.ew_hi, r2, p.kx, r2f, p.kxf);
+            g1 = ew_poly(x, p.ew_seg, 0);
+            g2 = ew_poly(x, p.ew_seg, 1);
+            g1 = in ? g1 : 0.0;
+            g2 = in ? g2 : 0.0;
+            if (any_near) {
+                g1 = fma(near ? p.cf : 0.0, ei_poly<true>(y, p.ei_seg, 0, NEI), g1);
+                g2 = fma(near ? f.c2 : 0.0, ei_poly<true>(y, p.ei_seg, 1, NEI), g2);
+            }
+        }
+        if (any_near) {
+            gl = ei_poly<true>(y, p.ei_seg, NEI - 1, NEI);
+            gl = near ? gl : 0.0;
+        }
+        if (__any_sync(0xffffffffu, need)) {
+            if (need) {
+                double g[4];
+                radial_general<KIND>(a, tb, r2 * p.to_a2, g);
+                g1 = g[0] * p.ia3;
+                g2 = g[1] * f.ia5;
+                gl = KIND == 0 ? 0.0 : (HVP ? g[3] / f.kgl : g[2] / f.kdl);
+            }
+        }
+        if (HVP) {
+            double dw[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) dw[k] = wi[k] - wj[k];
+            const double ud = fma(u[0], dw[0], fma(u[1], dw[1], u[2] * dw[2]));
+            const double a2 = (p.kx * g2) * ud;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                ti[k] = fma(a2, u[k], fma(-g1, dw[k], ti[k]));
+                hj[k] = fma(-a2, u[k], fma(g1, dw[k], hj[k]));
+            }
+            if (any_near) sum = fma(gl, ud, sum);
+        } else if (any_near) {
+            sum += gl;
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            xj[k] = __shfl_sync(0xffffffffu, xj[k], src);
+            if (HVP) {
+                wj[k] = __shfl_sync(0xffffffffu, wj[k], src);
+                hj[k] = __shfl_sync(0xffffffffu, hj[k], src);
+            }
+        }
+    }
+    const int jl = (lane + s1) & 31;
+    if (HVP && jl < jcnt)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) atomicAdd(f.hw + (size_t)k * a.n + jstart + jl, f.hq[pt] * hj[k]);
+}
+
+template <int EI, bool HVP, bool CUBIC>
+__global__ void __launch_bounds__(kF64Threads, 1) adj_f64_kernel(const AdjArgs a, const AdjFast f, unsigned *counter,
+                                                                 unsigned *status) {
+    extern __shared__ __align__(128) uint4 tabs[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ double red[32];
+    __shared__ F64Tab tab;
+    constexpr int NEI = HVP ? 3 : 1;
+    const F64Fast &p = f.p;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const uint32_t b0 = (uint32_t)p.ew_seg * ew_vec(2) * 16u, b1 = (uint32_t)p.ei_seg * ei_vec(NEI) * 16u;
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        fence_mbar_init();
+        mbar_arrive_expect_tx(&bar, b0 + b1);
+        if (b0) bulk_g2s(tabs, p.tab, b0, &bar);
+        if (b1) bulk_g2s(reinterpret_cast<unsigned char *>(tabs) + b0, reinterpret_cast<const unsigned char *>(p.tab) + b0, b1, &bar);
+    }
+    load_f64_tab(tab);
+    __syncthreads();
+    const bool got = mbar_wait_bounded(&bar, 0u, kWaitLimitCycles);
+    if (__syncthreads_or(!got)) {
+        if (tid == 0) atomicOr(status, kStatusTmaTimeout);
+        return;
+    }
+    const uint4 *ew = tabs, *ei = reinterpret_cast<const uint4 *>(reinterpret_cast<unsigned char *>(tabs) + b0);
+    N3Geom g;
+    g.nel = a.nel;
+    g.n = a.n;
+    double total = 0.0;
+    for (;;) {
+        unsigned nx = 0;
+        if (lane == 0) nx = atomicAdd(counter, 1u);
+        const long long it = __shfl_sync(0xffffffffu, nx, 0);
+        if (it >= p.total) break;
+        int ca, grp, part, istart, icnt, isp;
+        f64_item(p, it, ca, grp, part);
+        if (ca >= p.nc) continue;
+        const int b1c = min(p.nc, (grp + 1) * p.group);
+        int b = max(ca, grp * p.group);
+        if (!HVP) {                              // e-i chunks only
+            if (ca >= p.nce) continue;
+            b = max(b, p.nce);
+            if (b >= b1c) continue;
+        }
+        f64_chunk(p, g, ca, istart, icnt, isp);
+        const int s0 = part * 32 / p.split, s1 = (part + 1) * 32 / p.split, i = istart + min(lane, icnt - 1);
+        const longlong4_32a t = a.xl[i];
+        const long long xi[3] = {t.x, t.y, t.z};
+        double wi[3] = {0.0, 0.0, 0.0}, hi[3] = {0.0, 0.0, 0.0};
+        if (HVP)
+            for (int k = 0; k < 3; ++k) wi[k] = f.w[(size_t)k * a.n + i];
+        for (; b < b1c; ++b) {
+            int jstart, jcnt, jsp;
+            f64_chunk(p, g, b, jstart, jcnt, jsp);
+            const int pt = isp + jsp;
+            const bool diag = b == ca, masked = diag || icnt < 32 || jcnt < 32;
+            double ti[3] = {0.0, 0.0, 0.0}, sum = 0.0;
+#define TCP_ADJ_TILE(KIND, MASKED) \
+    adj_tile_f64<KIND, HVP, MASKED, CUBIC>(a, f, ew, ei, tab, pt, diag, icnt, xi, wi, jstart, jcnt, s0, s1, ti, sum)
+            if (EI != 0 && pt == 1) {
+                if (masked) TCP_ADJ_TILE(EI, true);
+                else TCP_ADJ_TILE(EI, false);
+            } else if (HVP) {
+                if (masked) TCP_ADJ_TILE(0, true);
+                else TCP_ADJ_TILE(0, false);
+            }
+#undef TCP_ADJ_TILE
+            if (HVP)
+                for (int k = 0; k < 3; ++k) hi[k] = fma(f.hq[pt], ti[k], hi[k]);
+            total += sum;
+        }
+        if (HVP && lane < icnt)
+            for (int k = 0; k < 3; ++k) atomicAdd(f.hw + (size_t)k * a.n + istart + lane, hi[k]);
+    }
+    total = block_sum(total, red);
+    if (tid == 0) atomicAdd(a.scal + (HVP ? kAdjDFdl : kAdjDEdl), total * (HVP ? f.qgl : f.qdl));
+}
+
 // ---- host-layout transposes ---------------------------------------------------
 __global__ void aos_to_soa_kernel(const double *__restrict__ in, double *__restrict__ out, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -518,6 +731,13 @@ __global__ void rev_accum_kernel(const double *__restrict__ scal, double *__rest
 constexpr int kRevThreads = 256;
 static int rev_blocks(int n) { return (n + kRevThreads - 1) / kRevThreads; }
 
+void adj_tables_free(tcp_ctx *c) {
+    for (auto &t : c->adjtab) {
+        cudaFree(t.dev);
+        t.dev = nullptr;
+    }
+}
+
 void adjoint_free(tcp_ctx *c) {
     double **bufs[] = {&c->adj_w, &c->adj_hw, &c->adj_xb, &c->adj_vb, &c->adj_fb, &c->adj_save,
                        &c->adj_io, &c->adj_scal, &c->adj_part, &c->adj_ck, &c->adj_seg};
@@ -527,6 +747,7 @@ void adjoint_free(tcp_ctx *c) {
     }
     c->adj_ck_cap = 0;
     c->adj_seg_cap = 0;
+    adj_tables_free(c);
 }
 
 static int adj_alloc(tcp_ctx *c) {
@@ -588,6 +809,67 @@ static int launch_adj_n3_t(tcp_ctx *c, const AdjArgs &a) {
     return TCP_OK;
 }
 
+static const int kHvpEw[] = {kFuncF, kFuncG2}, kHvpEi[] = {kFuncF, kFuncG2, kFuncGl}, kDlEi[] = {kFuncDl};
+
+typedef void (*AdjF64Kernel)(const AdjArgs, const AdjFast, unsigned *, unsigned *);
+template <int EI>
+static AdjF64Kernel adj_f64_of(bool hvp, bool cubic) {
+    if (hvp) return cubic ? adj_f64_kernel<EI, true, true> : adj_f64_kernel<EI, true, false>;
+    return cubic ? adj_f64_kernel<EI, false, true> : adj_f64_kernel<EI, false, false>;
+}
+
+// The FP64 tile form; *done = 0 where its tables do not fit in shared memory
+// (Deutsch with alpha rc > 4: the item form below takes it).
+static int launch_adj_f64(tcp_ctx *c, const AdjArgs &a, const double *w, double *hw, int *done) {
+    const bool hvp = w != nullptr;
+    const int k = hvp ? 0 : 1, eim = c->p.ei_model;
+    *done = 1;
+    if (!hvp && eim == TCP_EI_COULOMB) return TCP_OK;   // no term depends on lambda
+    const AdjF64Kernel fn = eim == TCP_EI_DEUTSCH ? adj_f64_of<1>(hvp, c->pc.cubic)
+                            : (eim == TCP_EI_KELBG ? adj_f64_of<2>(hvp, c->pc.cubic) : adj_f64_of<0>(hvp, c->pc.cubic));
+    tcp_ctx::AdjTab &T = c->adjtab[k];
+    if (!T.dev) {
+        std::vector<F64Vec> t;
+        T.ew = T.ei = 0;
+        if (hvp) t = f64_table(TCP_EI_COULOMB, kHvpEw, 2, ewald_octaves(c), &T.ew);
+        if (eim != TCP_EI_COULOMB) {
+            const std::vector<F64Vec> m = f64_table(eim, hvp ? kHvpEi : kDlEi, hvp ? 3 : 1, 0, &T.ei);
+            t.insert(t.end(), m.begin(), m.end());
+        }
+        T.bytes = sizeof(F64Vec) * t.size();
+        T.fits = T.bytes + 10240 <= 232448;             // beside the kernel's own shared memory
+        TCP_CUDA(cudaMalloc(&T.dev, T.bytes));
+        TCP_CUDA(cudaMemcpy(T.dev, t.data(), T.bytes, cudaMemcpyHostToDevice));
+        if (T.fits)
+            TCP_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void *>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)T.bytes));
+    }
+    *done = T.fits;
+    if (!T.fits) return TCP_OK;
+    AdjFast f;
+    std::memset(&f, 0, sizeof f);
+    f.p = f64_args(c, T.ew, T.ei);
+    f.p.tab = static_cast<const uint4 *>(T.dev);
+    f.w = w;
+    f.hw = hw;
+    const PairConsts &pc = c->pc;
+    const double al = pc.alpha, a5 = al * al * al * al * al, L = pc.cubic ? pc.box[0] : 1.0;
+    const double l = eim == TCP_EI_DEUTSCH ? pc.rs : pc.lambda;
+    f.c2 = -1.0 / (l * l * l * l * l * a5);
+    f.ia5 = 1.0 / a5;
+    f.kgl = (eim == TCP_EI_DEUTSCH ? -1.0 : -2.0) / (l * l * l * l);
+    f.kdl = (eim == TCP_EI_DEUTSCH ? -1.0 : -kSqrtPi) / (l * l);
+    for (int t = 0; t < 3; ++t) f.hq[t] = kEps * pc.qq[t] * al * al * al;
+    f.qgl = kEps * pc.qq[1] * f.kgl * L;
+    f.qdl = kEps * pc.qq[1] * f.kdl;
+    const int grid = (int)std::min<long long>(c->num_sms, (f.p.total + kF64Warps - 1) / kF64Warps);
+    TCP_CUDA(cudaMemsetAsync(c->counter, 0, sizeof(unsigned), c->stream));
+    fn<<<grid, kF64Threads, T.bytes, c->stream>>>(a, f, c->counter, c->status);
+    c->launches++;
+    TCP_CUDA(cudaGetLastError());
+    return TCP_OK;
+}
+
 // Real-space part: hw += H_real w (when w), scalars into adj_scal.  The
 // Newton-3 form unless TCP_FLAG_DETERMINISTIC asks for the ordered-pair sums
 // (which add their rows in a fixed pattern).
@@ -596,7 +878,8 @@ static int launch_adj_pair(tcp_ctx *c, const double *w, double *hw) {
     if (!(c->flags & TCP_FLAG_DETERMINISTIC)) {
         const bool f32 = c->p.precision == TCP_PREC_FP32C;
         const int eik = c->p.ei_model == TCP_EI_DEUTSCH ? 1 : (c->p.ei_model == TCP_EI_KELBG ? 2 : 0);
-        int rc;
+        int rc, done = 0;
+        if (!f32 && ((rc = launch_adj_f64(c, a, w, hw, &done)) || done)) return rc;
 #define ADJ_N3(F, E, H) rc = launch_adj_n3_t<F, E, H>(c, a)
         if (w) {
             if (f32) {
@@ -669,8 +952,14 @@ static int hvp_device(tcp_ctx *c, const double *w, double *hw) {
 }
 
 static int read_adj(tcp_ctx *c, double *out, int count) {
+    unsigned st = 0;
     TCP_CUDA(cudaMemcpyAsync(out, c->adj_scal, sizeof(double) * count, cudaMemcpyDeviceToHost, c->stream));
+    TCP_CUDA(cudaMemcpyAsync(&st, c->status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
     TCP_CUDA(cudaStreamSynchronize(c->stream));
+    if (st & kStatusTmaTimeout) {
+        cudaMemsetAsync(c->status, 0, sizeof(unsigned), c->stream);
+        return set_error(TCP_ERR_TIMEOUT, "a pair-kernel tile wait exceeded its bound");
+    }
     return TCP_OK;
 }
 

@@ -1,0 +1,177 @@
+// pair_f64.cuh -- what the FP64 tile kernels share (the real-space sum,
+// pair_n3_f64.cu, and its derivatives, adjoint.cu): the radial tables and their
+// evaluation, the conversions that stay off the FP64 pipe, and the items.  The
+// reasons stand in pair_n3_f64.cu.
+#pragma once
+
+#include "device_util.cuh"
+#include "pair_n3.cuh"
+
+#include <vector>
+
+namespace tcp {
+
+// Three warps per SM quarter hide the latency of the FP32 and integer work and
+// leave registers and shared memory for the reciprocal chain beside the launch.
+constexpr int kF64Threads = 384;
+constexpr int kF64Warps = kF64Threads / 32;
+
+// ---- tables ---------------------------------------------------------------------
+// Segments of an argument x in [2^-6, 2^top): the leading kEwBits (kEiBits)
+// mantissa bits of x.  Per segment and function the Taylor coefficients c0..c3
+// (Ewald) or c0..c4 (e-i) in FP64 and the magnitudes of the four next ones in
+// FP32, in 16-byte vectors [vector][segment] so that lanes on different
+// segments use different banks.  A table holds several functions:
+//   Ewald   c0 c1 | c2 c3 | t4 .. t7           per function
+//   e-i     c0 c1 | c2 c3 | c4 t5 t6           per function, then t7 t8 of two functions per vector
+constexpr int kEwBits = 7, kEiBits = 5;
+__host__ __device__ constexpr int ew_vec(int nf) { return 3 * nf; }
+__host__ __device__ constexpr int ei_vec(int nf) { return 3 * nf + (nf + 1) / 2; }
+constexpr int kTabLow = -6;              // the tables start at 2^-6
+constexpr unsigned kTabLowBits = (127 + kTabLow) << 23;
+constexpr int kEwTopMax = 6;             // Ewald: erfc(ar) is 0 beyond ar = 8 (1e-29 of the pair's 1/r)
+constexpr int kKelbgTop = 6;             // Kelbg: e^{-64} = 1.6e-28
+constexpr int kDeutschTop = 11;          // Deutsch: e^{-45} = 2.6e-20 of the pair's Coulomb term
+
+// The functions.  Ewald (x = a^2 r^2): the Taylor families of B_n, B_0 =
+// erfc(sqrt x)/sqrt x; Deutsch (z = r^2/rs^2): A_n, A_0 = e^{-s}/s, s = sqrt z;
+// Kelbg (y = r^2/lambda^2).
+enum F64Func {
+    kFuncU,      // energy: B_0, A_0, sqrt(pi) erfc(sqrt y) - e^{-y} y^{-1/2}
+    kFuncF,      // force weight: B_1, A_1, e^{-y} y^{-3/2}
+    kFuncG2,     // -2 dF/d(argument): B_2, A_2
+    kFuncGl,     // lambda derivative of the force weight: A_0, e^{-y} y^{-1/2}
+    kFuncDl      // lambda derivative of the energy: e^{-s}, erfc(sqrt y)
+};
+
+// Host side (pair_n3_f64.cu): the vectors of one table for the functions
+// given, the first `octaves` of it (0: all); *nseg: its segments.
+struct F64Vec {
+    union {
+        double d[2];
+        float f[4];
+    };
+};
+std::vector<F64Vec> f64_table(int model, const int *funcs, int nf, int octaves, int *nseg);
+int ewald_octaves(const tcp_ctx *c);   // octaves of the Ewald table that the cut-off reaches
+
+// What the kernel needs besides PairConsts.  Lengths in units of the box where
+// it is cubic (the fixed-point differences unscaled), in A otherwise.
+struct F64Fast {
+    const uint4 *tab;        // Ewald vectors, then e-i vectors
+    int ew_seg, ei_seg;      // segments per vector
+    unsigned ew_hi, ei_hi;   // float bits of the table ends
+    double kx, ky;           // r^2 -> a^2 r^2, r^2/lambda^2 (or /rs^2)
+    float kxf, kyf;
+    double rc2;              // cut-off^2 (r^2 < rc2)
+    double to_a2;            // r^2 -> A^2 (the general form)
+    double cf, cu;           // weight and energy of the e-i term in units of the Ewald term's a^3 and a
+    double ia3, ia;          // 1/a^3, 1/a
+    double qf[3], qe[3];     // force factor (eV/A per unit weight and separation) and energy factor per pair type
+    float rinv_dx[3];        // RDF: sqrt(r^2) -> r/dx
+    int group, split;        // j-chunks per item; items per tile of rotation steps
+    int nce, nc, ng;         // electron chunks, chunks, groups
+    long long total;
+};
+
+F64Fast f64_args(const tcp_ctx *c, int ew_seg, int ei_seg);   // tab: the caller's
+
+// ---- pair arithmetic --------------------------------------------------------------
+// (double)d 2^-64 for a 64-bit integer d without the FP64 pipe: the magnitude
+// is normalised by its leading zeros, rounded to 53 bits and packed.  Valid
+// for a nonzero upper word of the magnitude; small is set otherwise.
+__device__ __forceinline__ double box_diff(long long d, bool &small) {
+    const long long sg = d >> 63;
+    const unsigned long long mag = (unsigned long long)((d ^ sg) - sg);
+    const unsigned s = (unsigned)sg, ah = (unsigned)(mag >> 32), al = (unsigned)mag;
+    const int z = __clz((int)ah);
+    const unsigned nh = __funnelshift_l(al, ah, z), nl = al << (z & 31);
+    const unsigned hi = (nh >> 11) + ((1021u - (unsigned)z) << 20), lo = __funnelshift_r(nl, nh, 11);
+    const unsigned long long v = (((unsigned long long)hi << 32) | lo) + ((nl >> 10) & 1u);
+    small = small || ah == 0u;
+    return __hiloint2double((int)((unsigned)(v >> 32) | (s & 0x80000000u)), (int)(unsigned)v);
+}
+
+// positive normal float -> double without the FP64 pipe
+__device__ __forceinline__ double widen(float t) {
+    const unsigned b = __float_as_uint(t);
+    return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+}
+
+// the leading 24 bits of a double >= 0 as a float (0 below the normal floats;
+// the separations stay far below their upper end)
+__device__ __forceinline__ float narrow(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x);
+    const unsigned b = __funnelshift_l((unsigned)__double2loint(x), hi, 3) + 0x40000000u;
+    return __uint_as_float(hi < 0x38100000u ? 0u : b);
+}
+
+__device__ __forceinline__ double2 lds2(const uint4 *p) { return *reinterpret_cast<const double2 *>(p); }
+__device__ __forceinline__ float4 lds4(const uint4 *p) { return *reinterpret_cast<const float4 *>(p); }
+
+// Where an argument lies in a table: vector offset of its segment, distance to
+// the centre in FP64 and FP32.  xb: the bits of the FP32 argument.
+struct F64At {
+    const uint4 *t;
+    double h;
+    float hf;
+};
+template <int BITS>
+__device__ __forceinline__ F64At f64_at(const uint4 *tab, unsigned xb, unsigned hi, double r2, double k, float r2f,
+                                        float kf) {
+    const unsigned xi = min(max(xb, kTabLowBits), hi - 1u);
+    const unsigned cb = (xi & ~((1u << (23 - BITS)) - 1u)) | (1u << (22 - BITS));   // segment centre
+    F64At a;
+    a.t = tab + ((xi - kTabLowBits) >> (23 - BITS));
+    a.h = fma(r2, k, -widen(__uint_as_float(cb)));
+    a.hf = fmaf(r2f, kf, -__uint_as_float(cb));
+    return a;
+}
+
+// function f of an Ewald table of n segments
+__device__ __forceinline__ double ew_poly(const F64At &a, int n, int f) {
+    const double2 c01 = lds2(a.t + 3 * f * n), c23 = lds2(a.t + (3 * f + 1) * n);
+    const float4 t4 = lds4(a.t + (3 * f + 2) * n);
+    const double w = fma(a.h, widen(fmaf(fmaf(fmaf(t4.w, a.hf, t4.z), a.hf, t4.y), a.hf, t4.x)), c23.y);
+    return fma(a.h, fma(a.h, fma(a.h, w, c23.x), c01.y), c01.x);
+}
+
+// function f of nf of an e-i table of n segments; NEG: its FP32 part T is
+// negative (k = 5 of a completely monotone function; the Kelbg energy's is
+// positive, U' = F/2)
+template <bool NEG>
+__device__ __forceinline__ double ei_poly(const F64At &a, int n, int f, int nf) {
+    const double2 c01 = lds2(a.t + 3 * f * n), c23 = lds2(a.t + (3 * f + 1) * n), c4 = lds2(a.t + (3 * f + 2) * n);
+    const float2 t78 = reinterpret_cast<const float2 *>(a.t + (3 * nf + f / 2) * n)[f & 1];
+    const float t5 = __int_as_float(__double2loint(c4.y)), t6 = __int_as_float(__double2hiint(c4.y));
+    const float t = fmaf(fmaf(fmaf(t78.y, a.hf, t78.x), a.hf, t6), a.hf, t5);
+    const double v = NEG ? fma(-a.h, widen(-t), c4.x) : fma(a.h, widen(t), c4.x);
+    return fma(a.h, fma(a.h, fma(a.h, fma(a.h, v, c23.y), c23.x), c01.y), c01.x);
+}
+
+// ---- items ----------------------------------------------------------------------
+// Chunks of 32 particles, electrons first (a chunk holds one species).
+__device__ __forceinline__ void f64_chunk(const F64Fast &p, const N3Geom &g, int k, int &start, int &cnt, int &sp) {
+    sp = k < p.nce ? 0 : 1;
+    start = sp ? g.nel + (k - p.nce) * 32 : k * 32;
+    cnt = min(32, (sp ? g.n : g.nel) - start);
+}
+
+// Item -> (chunk a, group of j-chunks, part of the rotation).  Rows come in
+// blocks of `group` chunks: the rows of block A hold the groups A .. ng-1, so
+// block A starts at group (A ng - A (A - 1)/2).
+__device__ __forceinline__ void f64_item(const F64Fast &p, long long it, int &a, int &grp, int &part) {
+    part = (int)(it % p.split);
+    const long long t = it / p.split;
+    auto start = [&](int A) { return (long long)p.group * ((long long)A * p.ng - (long long)A * (A - 1) / 2); };
+    const float b = (float)p.ng + 0.5f;
+    int A = (int)(b - sqrtf(fmaxf(b * b - 2.0f * (float)t / (float)p.group, 0.0f)));
+    A = max(0, min(A, p.ng - 1));
+    while (A > 0 && start(A) > t) --A;
+    while (A + 1 < p.ng && start(A + 1) <= t) ++A;
+    const int o = (int)(t - start(A)), w = p.ng - A;
+    a = A * p.group + o / w;
+    grp = A + o % w;
+}
+
+}  // namespace tcp

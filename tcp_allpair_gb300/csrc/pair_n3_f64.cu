@@ -43,77 +43,82 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
-#include "device_util.cuh"
-#include "pair_n3.cuh"
+#include "pair_f64.cuh"
 
 namespace tcp {
 
-// Three warps per SM quarter hide the latency of the FP32 and integer work and
-// leave registers and shared memory for the reciprocal chain beside the launch.
-constexpr int kF64Threads = 384;
-constexpr int kF64Warps = kF64Threads / 32;
-
-// ---- tables ---------------------------------------------------------------------
-// Segments of an argument x in [2^-6, 2^top): the leading kEwBits (kEiBits)
-// mantissa bits of x.  Per segment and function the coefficients c0..c3 (Ewald)
-// or c0..c4 (e-i) in FP64 and the magnitudes of the four next ones in FP32,
-// in 16-byte vectors [vector][segment] so that lanes on different segments
-// use different banks.
-constexpr int kEwBits = 7, kEwVec = 6;   // F: c0 c1 | c2 c3 | t4..t7, then U the same
-constexpr int kEiBits = 5, kEiVec = 7;   // F: c0 c1 | c2 c3 | c4 t5 t6, U the same, then t7 t8 of F and U
-constexpr int kTabLow = -6;              // the tables start at 2^-6
-constexpr unsigned kTabLowBits = (127 + kTabLow) << 23;
-constexpr int kEwTopMax = 6;             // Ewald: erfc(ar) is 0 beyond ar = 8 (1e-29 of the pair's 1/r)
-constexpr int kKelbgTop = 6;             // Kelbg: e^{-64} = 1.6e-28
-constexpr int kDeutschTop = 11;          // Deutsch: e^{-45} = 2.6e-20 of the pair's Coulomb term
-
-// Taylor coefficients of F and U at xc, k = 0..8, in the working precision of
-// long double (64 bits or more).  All three families obey upward recursions
-// of positive terms for the derivatives with respect to -x/2:
-//  Ewald    B_{n+1} = ((2n+1) B_n + 2^{n+1}/sqrt(pi) e^{-x})/x,  U = B_0, F = B_1
-//  Deutsch  A_{n+1} = (A_{n-1} + (2n+1) A_n)/z,                  U = A_0, F = A_1
-//  Kelbg    F = e^{-y} y^{-3/2} as the product of two series; U' = F/2.
+// Taylor coefficients of function `func` at xc, k = 0..8, in long double (64
+// bits or more).  The families obey upward recursions of positive terms for
+// the derivatives with respect to -x/2:
+//  Ewald    B_{n+1} = ((2n+1) B_n + 2^{n+1}/sqrt(pi) e^{-x})/x
+//  Deutsch  A_{n+1} = (A_{n-1} + (2n+1) A_n)/z
+//  Kelbg    e^{-y} y^{-p} as the product of two series; the energy's derivative is F/2.
 constexpr int kTaylor = 9;
-static void taylor_of(int model, long double xc, long double *F, long double *U) {
-    const long double rt = sqrtl(xc);
+static void gauss_power(long double xc, long double p, long double *out) {   // e^{-x} x^{-p}
+    long double e[kTaylor], s[kTaylor];              // e^{-h}, (1 + h/xc)^{-p}
+    e[0] = s[0] = 1.0L;
+    for (int k = 1; k < kTaylor; ++k) {
+        e[k] = -e[k - 1] / k;
+        s[k] = s[k - 1] * (-p - (k - 1)) / (k * xc);
+    }
+    const long double f0 = expl(-xc) * powl(xc, -p);
+    for (int k = 0; k < kTaylor; ++k) {
+        long double t = 0.0L;
+        for (int q = 0; q <= k; ++q) t += e[q] * s[k - q];
+        out[k] = f0 * t;
+    }
+}
+
+// c0 and the series of the derivative -> the series
+static void integrate_series(long double c0, long double scale, const long double *d, long double *out) {
+    out[0] = c0;
+    for (int k = 1; k < kTaylor; ++k) out[k] = scale * d[k - 1] / k;
+}
+
+static void taylor_of(int model, int func, long double xc, long double *out) {
+    const long double rt = sqrtl(xc), spi = sqrtl(acosl(-1.0L));
     if (model == TCP_EI_KELBG) {
-        const long double spi = sqrtl(acosl(-1.0L));
-        long double e[kTaylor], s[kTaylor];          // e^{-h}, (1 + h/xc)^{-3/2}
-        e[0] = s[0] = 1.0L;
-        for (int k = 1; k < kTaylor; ++k) {
-            e[k] = -e[k - 1] / k;
-            s[k] = s[k - 1] * (-1.5L - (k - 1)) / (k * xc);
+        long double g[kTaylor], f[kTaylor];
+        gauss_power(xc, 0.5L, g);
+        gauss_power(xc, 1.5L, f);
+        if (func == kFuncU) {
+            integrate_series(spi * erfcl(rt) - expl(-xc) / rt, 0.5L, f, out);
+        } else if (func == kFuncDl) {
+            integrate_series(erfcl(rt), -1.0L / spi, g, out);
+        } else if (func == kFuncG2) {                // -2 F' = 2 F + 3 e^{-y} y^{-5/2}
+            gauss_power(xc, 2.5L, g);
+            for (int k = 0; k < kTaylor; ++k) out[k] = 2.0L * f[k] + 3.0L * g[k];
+        } else {
+            std::copy(func == kFuncGl ? g : f, (func == kFuncGl ? g : f) + kTaylor, out);
         }
-        const long double f0 = expl(-xc) / (xc * rt);
-        for (int k = 0; k < kTaylor; ++k) {
-            long double t = 0.0L;
-            for (int q = 0; q <= k; ++q) t += e[q] * s[k - q];
-            F[k] = f0 * t;
-        }
-        U[0] = spi * erfcl(rt) - expl(-xc) / rt;
-        for (int k = 1; k < kTaylor; ++k) U[k] = 0.5L * F[k - 1] / k;
         return;
     }
-    long double d[kTaylor + 1];                      // (-2 d/dx)^n of U
+    constexpr int ND = kTaylor + 2;
+    long double d[ND];                               // (-2 d/dx)^n of U
     if (model == TCP_EI_DEUTSCH) {
         d[0] = expl(-rt) / rt;
         d[1] = d[0] * (1.0L + rt) / xc;
-        for (int n = 1; n < kTaylor; ++n) d[n + 1] = (d[n - 1] + (2 * n + 1) * d[n]) / xc;
+        for (int n = 1; n + 1 < ND; ++n) d[n + 1] = (d[n - 1] + (2 * n + 1) * d[n]) / xc;
     } else {
-        long double g = 2.0L / sqrtl(acosl(-1.0L)) * expl(-xc);
+        long double g = 2.0L / spi * expl(-xc);
         d[0] = erfcl(rt) / rt;
-        for (int n = 0; n < kTaylor; ++n) {
+        for (int n = 0; n + 1 < ND; ++n) {
             d[n + 1] = ((2 * n + 1) * d[n] + g) / xc;
             g *= 2.0L;
         }
     }
+    const int n0 = func == kFuncF ? 1 : (func == kFuncG2 ? 2 : 0);
     long double c = 1.0L;                            // (-1/2)^k / k!
     for (int k = 0; k < kTaylor; ++k) {
-        U[k] = d[k] * c;
-        F[k] = d[k + 1] * c;
+        out[k] = d[k + n0] * c;
         c *= -0.5L / (k + 1);
+    }
+    if (func == kFuncDl) {                           // e^{-s}: derivative -A_0/2
+        const std::vector<long double> a(out, out + kTaylor);
+        integrate_series(expl(-rt), -0.5L, a.data(), out);
     }
 }
 
@@ -122,101 +127,60 @@ static long double segment_centre(int k, int bits) {
     return ldexpl(1.0L + (m + 0.5L) / (1 << bits), oct);
 }
 
-struct F64Vec {
-    union {
-        double d[2];
-        float f[4];
-    };
-};
-
-// Full Ewald table (all octaves), or one e-i table; written once per process.
-static std::vector<F64Vec> build_table(int model) {
+// One function over all its octaves, [vector][segment]: three vectors, and for
+// the e-i families a fourth with t7, t8.  Written once per process.
+static std::vector<F64Vec> build_function(int model, int func) {
     const bool ew = model == TCP_EI_COULOMB;
-    const int bits = ew ? kEwBits : kEiBits, nvec = ew ? kEwVec : kEiVec;
+    const int bits = ew ? kEwBits : kEiBits;
     const int top = ew ? kEwTopMax : (model == TCP_EI_KELBG ? kKelbgTop : kDeutschTop);
-    const int nseg = (top - kTabLow) << bits;
-    std::vector<F64Vec> t((size_t)nvec * nseg);
-    for (int s = 0; s < nseg; ++s) {
-        long double c[2][kTaylor];
-        taylor_of(model, segment_centre(s, bits), c[0], c[1]);
-        for (int q = 0; q < 2; ++q) {
-            double *lo = t[(size_t)(3 * q) * nseg + s].d, *mid = t[(size_t)(3 * q + 1) * nseg + s].d;
-            lo[0] = (double)c[q][0];
-            lo[1] = (double)c[q][1];
-            mid[0] = (double)c[q][2];
-            mid[1] = (double)c[q][3];
-            F64Vec &v = t[(size_t)(3 * q + 2) * nseg + s];
-            if (ew) {
-                for (int k = 0; k < 4; ++k) v.f[k] = (float)c[q][4 + k];
-            } else {   // T = t5 + t6 h + ...: of one sign within a family (F and U alternate)
-                v.d[0] = (double)c[q][4];
-                v.f[2] = (float)c[q][5];
-                v.f[3] = (float)c[q][6];
-                t[(size_t)6 * nseg + s].f[2 * q] = (float)c[q][7];
-                t[(size_t)6 * nseg + s].f[2 * q + 1] = (float)c[q][8];
-            }
+    const int n = (top - kTabLow) << bits;
+    std::vector<F64Vec> t((size_t)4 * n);
+    for (int s = 0; s < n; ++s) {
+        long double c[kTaylor];
+        taylor_of(model, func, segment_centre(s, bits), c);
+        t[s].d[0] = (double)c[0];
+        t[s].d[1] = (double)c[1];
+        t[n + s].d[0] = (double)c[2];
+        t[n + s].d[1] = (double)c[3];
+        F64Vec &v = t[2 * n + s];
+        if (ew) {
+            for (int k = 0; k < 4; ++k) v.f[k] = (float)c[4 + k];
+        } else {
+            v.d[0] = (double)c[4];
+            v.f[2] = (float)c[5];
+            v.f[3] = (float)c[6];
+            t[3 * n + s].f[0] = (float)c[7];
+            t[3 * n + s].f[1] = (float)c[8];
         }
     }
     return t;
 }
 
-static const std::vector<F64Vec> &table_of(int model) {
-    static const std::vector<F64Vec> ew = build_table(TCP_EI_COULOMB), ke = build_table(TCP_EI_KELBG),
-                                     de = build_table(TCP_EI_DEUTSCH);
-    return model == TCP_EI_KELBG ? ke : (model == TCP_EI_DEUTSCH ? de : ew);
+static const std::vector<F64Vec> &function_of(int model, int func) {
+    static std::once_flag once[3][5];
+    static std::vector<F64Vec> tab[3][5];
+    const int m = model == TCP_EI_COULOMB ? 0 : (model == TCP_EI_KELBG ? 1 : 2);
+    std::call_once(once[m][func], [&] { tab[m][func] = build_function(model, func); });
+    return tab[m][func];
 }
 
-// What the kernel needs besides PairConsts.  Lengths in units of the box where
-// it is cubic (the fixed-point differences unscaled), in A otherwise.
-struct F64Fast {
-    const uint4 *tab;        // Ewald vectors, then e-i vectors
-    int ew_seg, ei_seg;      // segments per vector
-    unsigned ew_hi, ei_hi;   // float bits of the table ends
-    double kx, ky;           // r^2 -> a^2 r^2, r^2/lambda^2 (or /rs^2)
-    float kxf, kyf;
-    double rc2;              // cut-off^2 (r^2 < rc2)
-    double to_a2;            // r^2 -> A^2 (the general form)
-    double cf, cu;           // weight and energy of the e-i term in units of the Ewald term's a^3 and a
-    double ia3, ia;          // 1/a^3, 1/a
-    double qf[3], qe[3];     // force factor (eV/A per unit weight and separation) and energy factor per pair type
-    float rinv_dx[3];        // RDF: sqrt(r^2) -> r/dx
-    int group, split;        // j-chunks per item; items per tile of rotation steps
-    int nce, nc, ng;         // electron chunks, chunks, groups
-    long long total;
-};
-
-// ---- pair arithmetic --------------------------------------------------------------
-// (double)d 2^-64 for a 64-bit integer d without the FP64 pipe: the magnitude
-// is normalised by its leading zeros, rounded to 53 bits and packed.  Valid
-// for a nonzero upper word of the magnitude; small is set otherwise.
-__device__ __forceinline__ double box_diff(long long d, bool &small) {
-    const long long sg = d >> 63;
-    const unsigned long long mag = (unsigned long long)((d ^ sg) - sg);
-    const unsigned s = (unsigned)sg, ah = (unsigned)(mag >> 32), al = (unsigned)mag;
-    const int z = __clz((int)ah);
-    const unsigned nh = __funnelshift_l(al, ah, z), nl = al << (z & 31);
-    const unsigned hi = (nh >> 11) + ((1021u - (unsigned)z) << 20), lo = __funnelshift_r(nl, nh, 11);
-    const unsigned long long v = (((unsigned long long)hi << 32) | lo) + ((nl >> 10) & 1u);
-    small = small || ah == 0u;
-    return __hiloint2double((int)((unsigned)(v >> 32) | (s & 0x80000000u)), (int)(unsigned)v);
+std::vector<F64Vec> f64_table(int model, const int *funcs, int nf, int octaves, int *nseg) {
+    const bool ew = model == TCP_EI_COULOMB;
+    const int full = (int)function_of(model, funcs[0]).size() / 4;
+    const int n = octaves > 0 ? std::min(full, octaves << (ew ? kEwBits : kEiBits)) : full;
+    std::vector<F64Vec> t((size_t)(ew ? ew_vec(nf) : ei_vec(nf)) * n);
+    for (int f = 0; f < nf; ++f) {
+        const std::vector<F64Vec> &q = function_of(model, funcs[f]);
+        for (int v = 0; v < 3; ++v)
+            std::copy(q.begin() + (size_t)v * full, q.begin() + (size_t)v * full + n, t.begin() + (size_t)(3 * f + v) * n);
+        if (!ew)
+            for (int s = 0; s < n; ++s)
+                for (int k = 0; k < 2; ++k)
+                    t[(size_t)(3 * nf + f / 2) * n + s].f[2 * (f & 1) + k] = q[(size_t)3 * full + s].f[k];
+    }
+    *nseg = n;
+    return t;
 }
-
-// positive normal float -> double without the FP64 pipe
-__device__ __forceinline__ double widen(float t) {
-    const unsigned b = __float_as_uint(t);
-    return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
-}
-
-// the leading 24 bits of a double >= 0 as a float (0 below the normal floats;
-// the separations stay far below their upper end)
-__device__ __forceinline__ float narrow(double x) {
-    const unsigned hi = (unsigned)__double2hiint(x);
-    const unsigned b = __funnelshift_l((unsigned)__double2loint(x), hi, 3) + 0x40000000u;
-    return __uint_as_float(hi < 0x38100000u ? 0u : b);
-}
-
-__device__ __forceinline__ double2 lds2(const uint4 *p) { return *reinterpret_cast<const double2 *>(p); }
-__device__ __forceinline__ float4 lds4(const uint4 *p) { return *reinterpret_cast<const float4 *>(p); }
 
 // The general form of one pair at squared distance r2 (> 0, A^2): the weight w
 // (force on i = eps qq w d) and the energy term pe, by rsqrt, exp and erfcx.
@@ -256,54 +220,22 @@ __device__ __forceinline__ double n3_pair_f64(const F64Fast &p, const PairConsts
     const float r2f = narrow(r2);
     const unsigned xb = __float_as_uint(r2f * p.kxf);
     bool need = ok && xb < kTabLowBits;                   // below the tables
-    const unsigned xi = min(max(xb, kTabLowBits), p.ew_hi - 1u);
-    const unsigned cb = (xi & ~((1u << (23 - kEwBits)) - 1u)) | (1u << (22 - kEwBits));   // segment centre
-    const uint4 *t = sh.ew + ((xi - kTabLowBits) >> (23 - kEwBits));
-    const double h = fma(r2, p.kx, -widen(__uint_as_float(cb)));
-    const float hf = fmaf(r2f, p.kxf, -__uint_as_float(cb));
-    const int n = p.ew_seg;
-    const double2 f01 = lds2(t), f23 = lds2(t + n);
-    const float4 f4 = lds4(t + 2 * n);
-    double w = fma(h, widen(fmaf(fmaf(fmaf(f4.w, hf, f4.z), hf, f4.y), hf, f4.x)), f23.y);
-    w = fma(h, fma(h, fma(h, w, f23.x), f01.y), f01.x);
-    double u = 0.0;
-    if (ENERGY) {
-        const double2 u01 = lds2(t + 3 * n), u23 = lds2(t + 4 * n);
-        const float4 u4 = lds4(t + 5 * n);
-        u = fma(h, widen(fmaf(fmaf(fmaf(u4.w, hf, u4.z), hf, u4.y), hf, u4.x)), u23.y);
-        u = fma(h, fma(h, fma(h, u, u23.x), u01.y), u01.x);
-    }
     const bool in = ok && xb < p.ew_hi;
+    const F64At x = f64_at<kEwBits>(sh.ew, xb, p.ew_hi, r2, p.kx, r2f, p.kxf);
+    double w = ew_poly(x, p.ew_seg, 0), u = 0.0;
     w = in ? w : 0.0;
-    u = in ? u : 0.0;
+    if (ENERGY) {
+        u = ew_poly(x, p.ew_seg, 1);
+        u = in ? u : 0.0;
+    }
     if (KIND != 0) {
         const unsigned yb = __float_as_uint(r2f * p.kyf);
         const bool near = ok && yb < p.ei_hi;
         if (__any_sync(0xffffffffu, near)) {
             need = need || (near && yb < kTabLowBits);
-            const unsigned yi = min(max(yb, kTabLowBits), p.ei_hi - 1u);
-            const unsigned db = (yi & ~((1u << (23 - kEiBits)) - 1u)) | (1u << (22 - kEiBits));
-            const uint4 *s = sh.ei + ((yi - kTabLowBits) >> (23 - kEiBits));
-            const double g = fma(r2, p.ky, -widen(__uint_as_float(db)));
-            const float gf = fmaf(r2f, p.kyf, -__uint_as_float(db));
-            const int m = p.ei_seg;
-            const float4 t78 = lds4(s + 6 * m);
-            // the FP32 part T has the sign of its leading term: F negative
-            // (k = 5), U negative for Deutsch, positive for Kelbg (U' = F/2)
-            const double2 a01 = lds2(s), a23 = lds2(s + m), a4 = lds2(s + 2 * m);
-            const float a5 = __int_as_float(__double2loint(a4.y)), a6 = __int_as_float(__double2hiint(a4.y));
-            const float tf = fmaf(fmaf(fmaf(t78.y, gf, t78.x), gf, a6), gf, a5);
-            double v = fma(-g, widen(-tf), a4.x);
-            v = fma(g, fma(g, fma(g, fma(g, v, a23.y), a23.x), a01.y), a01.x);
-            w = fma(near ? p.cf : 0.0, v, w);
-            if (ENERGY) {
-                const double2 b01 = lds2(s + 3 * m), b23 = lds2(s + 4 * m), b4 = lds2(s + 5 * m);
-                const float b5 = __int_as_float(__double2loint(b4.y)), b6 = __int_as_float(__double2hiint(b4.y));
-                const float tu = fmaf(fmaf(fmaf(t78.w, gf, t78.z), gf, b6), gf, b5);
-                v = KIND == 2 ? fma(g, widen(tu), b4.x) : fma(-g, widen(-tu), b4.x);
-                v = fma(g, fma(g, fma(g, fma(g, v, b23.y), b23.x), b01.y), b01.x);
-                u = fma(near ? p.cu : 0.0, v, u);
-            }
+            const F64At y = f64_at<kEiBits>(sh.ei, yb, p.ei_hi, r2, p.ky, r2f, p.kyf);
+            w = fma(near ? p.cf : 0.0, ei_poly<true>(y, p.ei_seg, 0, 2), w);
+            if (ENERGY) u = fma(near ? p.cu : 0.0, ei_poly<KIND == 1>(y, p.ei_seg, 1, 2), u);
         }
     }
     if (__any_sync(0xffffffffu, need)) {
@@ -332,31 +264,6 @@ __device__ __forceinline__ void rdf_add_f64(const F64Fast &p, const PairConsts &
         if (edge) bin = (int)(sqrt(r2 * p.to_a2) * c.inv_dxd[pt]);
     }
     if (ok && bin < kNbin) atomicAdd(&hist[bin], 2u);
-}
-
-// ---- items ----------------------------------------------------------------------
-// Chunks of 32 particles, electrons first (a chunk holds one species).
-__device__ __forceinline__ void f64_chunk(const F64Fast &p, const N3Geom &g, int k, int &start, int &cnt, int &sp) {
-    sp = k < p.nce ? 0 : 1;
-    start = sp ? g.nel + (k - p.nce) * 32 : k * 32;
-    cnt = min(32, (sp ? g.n : g.nel) - start);
-}
-
-// Item -> (chunk a, group of j-chunks, part of the rotation).  Rows come in
-// blocks of `group` chunks: the rows of block A hold the groups A .. ng-1, so
-// block A starts at group (A ng - A (A - 1)/2).
-__device__ __forceinline__ void f64_item(const F64Fast &p, long long it, int &a, int &grp, int &part) {
-    part = (int)(it % p.split);
-    const long long t = it / p.split;
-    auto start = [&](int A) { return (long long)p.group * ((long long)A * p.ng - (long long)A * (A - 1) / 2); };
-    const float b = (float)p.ng + 0.5f;
-    int A = (int)(b - sqrtf(fmaxf(b * b - 2.0f * (float)t / (float)p.group, 0.0f)));
-    A = max(0, min(A, p.ng - 1));
-    while (A > 0 && start(A) > t) --A;
-    while (A + 1 < p.ng && start(A + 1) <= t) ++A;
-    const int o = (int)(t - start(A)), w = p.ng - A;
-    a = A * p.group + o / w;
-    grp = A + o % w;
 }
 
 // One tile: the warp's 32 i-particles against chunk b, rotation steps [s0, s1).
@@ -434,10 +341,10 @@ __global__ void __launch_bounds__(kF64Threads, 1) pair_n3_f64_kernel(const N3Arg
         mbar_init(&bar, 1);
         fence_mbar_init();
         if (!(a.inject_skip && blockIdx.x == 0)) {        // test hook: the copy never comes
-            const uint32_t b0 = (uint32_t)p.ew_seg * kEwVec * 16u, b1 = (uint32_t)p.ei_seg * kEiVec * 16u;
+            const uint32_t b0 = (uint32_t)p.ew_seg * ew_vec(2) * 16u, b1 = (uint32_t)p.ei_seg * ei_vec(2) * 16u;
             mbar_arrive_expect_tx(&bar, b0 + b1);
             bulk_g2s(tabs, p.tab, b0, &bar);
-            if (b1) bulk_g2s(tabs + p.ew_seg * kEwVec, p.tab + p.ew_seg * kEwVec, b1, &bar);
+            if (b1) bulk_g2s(tabs + p.ew_seg * ew_vec(2), p.tab + p.ew_seg * ew_vec(2), b1, &bar);
         }
     }
     load_f64_tab(tab);
@@ -449,7 +356,7 @@ __global__ void __launch_bounds__(kF64Threads, 1) pair_n3_f64_kernel(const N3Arg
     }
     F64Shared sh;
     sh.ew = tabs;
-    sh.ei = tabs + p.ew_seg * kEwVec;
+    sh.ei = tabs + p.ew_seg * ew_vec(2);
     sh.tb = &tab;
     sh.hist = nullptr;
     double etot = 0.0;
@@ -529,29 +436,25 @@ bool n3_f64_applicable(const tcp_ctx *c) {
 
 int n3_f64_grid(const tcp_ctx *c) { return std::max(1, c->num_sms); }   // the tables: one CTA per SM
 
-// octaves of the Ewald table that the cut-off reaches
-static int ewald_octaves(const tcp_ctx *c) {
+int ewald_octaves(const tcp_ctx *c) {
     int top = kTabLow + 1;
     while (top < kEwTopMax && std::ldexp(1.0, top) < c->pc.alpha2 * c->rc2) ++top;
     return top - kTabLow;
 }
 
-static size_t f64_smem(int ew_seg, int ei_seg) { return 16 * ((size_t)ew_seg * kEwVec + (size_t)ei_seg * kEiVec); }
+static const int kPairFuncs[] = {kFuncF, kFuncU};
+static size_t f64_smem(int ew_seg, int ei_seg) { return 16 * ((size_t)ew_seg * ew_vec(2) + (size_t)ei_seg * ei_vec(2)); }
 
 // Device tables of an FP64 context for its e-i model and cut-off (rebuilt with
 // the pair constants, outside any stream capture).
 int n3_f64_prepare(tcp_ctx *c) {
-    const int oct = ewald_octaves(c), ew = oct << kEwBits;
-    const std::vector<F64Vec> &full = table_of(TCP_EI_COULOMB);
-    const int nfull = (int)(full.size() / kEwVec);
-    std::vector<F64Vec> t;
-    for (int v = 0; v < kEwVec; ++v) t.insert(t.end(), full.begin() + (size_t)v * nfull, full.begin() + (size_t)v * nfull + ew);
-    int ei = 0;
+    int ew = 0, ei = 0;
+    std::vector<F64Vec> t = f64_table(TCP_EI_COULOMB, kPairFuncs, 2, ewald_octaves(c), &ew);
     if (c->p.ei_model != TCP_EI_COULOMB) {
-        const std::vector<F64Vec> &m = table_of(c->p.ei_model);
-        ei = (int)(m.size() / kEiVec);
+        const std::vector<F64Vec> m = f64_table(c->p.ei_model, kPairFuncs, 2, 0, &ei);
         t.insert(t.end(), m.begin(), m.end());
     }
+    adj_tables_free(c);                  // they follow the same parameters
     cudaFree(c->f64tab);
     c->f64tab = nullptr;
     TCP_CUDA(cudaMalloc(&c->f64tab, sizeof(F64Vec) * t.size()));
@@ -564,29 +467,15 @@ int n3_f64_prepare(tcp_ctx *c) {
     return TCP_OK;
 }
 
-int launch_pair_n3_f64(tcp_ctx *c, bool energy, bool rdf, bool cleared) {
-    if (!c->f64tab) return set_error(TCP_ERR_STATE, "no FP64 pair tables");
-    N3Args a;
-    std::memset(&a, 0, sizeof a);
-    a.g.nel = c->nel;
-    a.g.n = c->n;
-    a.xl = c->xl;
-    a.ntot = c->n;
-    a.facc = c->fpart;
-    a.upart = c->upart;
-    a.status = c->status;
-    a.counter = c->counter;
-    a.c = c->pc;
-    a.inject_skip = inject_fault("tile_wait") ? 1 : 0;
-    a.rdf = c->rdf;
+// Constants and items for tables of ew_seg and ei_seg segments.
+F64Fast f64_args(const tcp_ctx *c, int ew_seg, int ei_seg) {
     const PairConsts &pc = c->pc;
     const double L = pc.cubic ? pc.box[0] : 1.0, l = c->p.ei_model == TCP_EI_DEUTSCH ? pc.rs : pc.lambda;
     const double al = pc.alpha, a3 = al * al * al;
     F64Fast p;
     std::memset(&p, 0, sizeof p);
-    p.tab = reinterpret_cast<const uint4 *>(c->f64tab);
-    p.ew_seg = c->f64_ew_seg;
-    p.ei_seg = c->f64_ei_seg;
+    p.ew_seg = ew_seg;
+    p.ei_seg = ei_seg;
     p.ew_hi = kTabLowBits + ((unsigned)(p.ew_seg >> kEwBits) << 23);
     p.ei_hi = kTabLowBits + ((unsigned)(p.ei_seg >> kEiBits) << 23);
     p.kx = pc.alpha2 * (L * L);
@@ -622,6 +511,26 @@ int launch_pair_n3_f64(tcp_ctx *c, bool energy, bool rdf, bool cleared) {
     p.split = tiles >= 16 * quarters ? 1 : (tiles >= 8 * quarters ? 2 : 4);
     p.ng = (p.nc + p.group - 1) / p.group;
     p.total = (long long)p.group * p.ng * (p.ng + 1) / 2 * p.split;
+    return p;
+}
+
+int launch_pair_n3_f64(tcp_ctx *c, bool energy, bool rdf, bool cleared) {
+    if (!c->f64tab) return set_error(TCP_ERR_STATE, "no FP64 pair tables");
+    N3Args a;
+    std::memset(&a, 0, sizeof a);
+    a.g.nel = c->nel;
+    a.g.n = c->n;
+    a.xl = c->xl;
+    a.ntot = c->n;
+    a.facc = c->fpart;
+    a.upart = c->upart;
+    a.status = c->status;
+    a.counter = c->counter;
+    a.c = c->pc;
+    a.inject_skip = inject_fault("tile_wait") ? 1 : 0;
+    a.rdf = c->rdf;
+    F64Fast p = f64_args(c, c->f64_ew_seg, c->f64_ei_seg);
+    p.tab = reinterpret_cast<const uint4 *>(c->f64tab);
     const int grid = (int)std::min<long long>(n3_f64_grid(c), (p.total + kF64Warps - 1) / kF64Warps);
     if (grid > c->n_upart) return set_error(TCP_ERR_STATE, "energy partial buffer smaller than the Newton-3 grid");
     c->n_upart_used = grid;

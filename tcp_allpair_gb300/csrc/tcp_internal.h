@@ -245,7 +245,14 @@ struct tcp_ctx {
     size_t l2_flush_bytes = 0;
     long long step_index = 0;
     tcp_energies last{};
-    // derivatives (allocated on first use): vectors SoA [3][n]
+    // derivatives (allocated on first use): radial tables of the FP64 Hessian-vector
+    // product and of dE/dlambda, vectors SoA [3][n]
+    struct AdjTab {
+        void *dev = nullptr;
+        int ew = 0, ei = 0;
+        size_t bytes = 0;
+        bool fits = false;
+    } adjtab[2];
     double *adj_w = nullptr, *adj_hw = nullptr;       // Hessian-vector product input / output
     double *adj_xb = nullptr, *adj_vb = nullptr, *adj_fb = nullptr;   // reverse-mode adjoints
     double *adj_save = nullptr;        // [3][3][n] x, v, f after the forward pass
@@ -400,6 +407,7 @@ int launch_ewald_hvp(tcp_ctx *c, const double *w, double *hw);
 void spme_hvp_free(tcp_ctx *c);
 // adjoint.cu
 void adjoint_free(tcp_ctx *c);
+void adj_tables_free(tcp_ctx *c);
 
 // ctx->tickets
 enum { kTickStep = 0, kTickForce = 1, kTickKick = 2, kTickScale = 3, kTickBin = 4, kTickAdd = 5 };
