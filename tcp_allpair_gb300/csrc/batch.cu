@@ -344,6 +344,7 @@ static ChainArgs b_chain(tcp_batch *b) {
     c.many = b->geo;
     c.sys_of = b->rep_of;
     c.mesh = b->Qf;
+    c.dipole = nullptr;
     c.ticket = b->ticket;
     return c;
 }
@@ -399,7 +400,7 @@ static int b_own_groups(tcp_batch *b, const ChainArgs &chain, const BAcc &A) {
         f.epart = nullptr;
         f.um = A.um;
         f.energy = 1;
-        b->launches += fft_convolve(chain, f, g.K[0], g.count, true, k ? b->gstream[k - 1] : b->stream2);
+        b->launches += fft_convolve(chain, f, g.K[0], g.count, k ? b->gstream[k - 1] : b->stream2);
     }
     for (size_t k = 1; k < ng; ++k) {
         TCP_CUDA(cudaEventRecord(b->ev_gdone[0][k - 1], b->gstream[k - 1]));

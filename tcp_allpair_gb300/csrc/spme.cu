@@ -29,15 +29,6 @@
 
 namespace tcp {
 
-struct SpmeArgs {
-    const double *x;     // SoA [3][n]
-    int nel, n;
-    double q0, q1;       // scaled charges per species
-    double box0, box1, box2;
-    double kl0, kl1, kl2;   // K/L: the step's kernels multiply (GB300's FP64 division is slow)
-    int K1, K2, K3;
-};
-
 // Qk *= theta B; energy partial sum_m w_m theta B |Qk|^2 (w = 2 for the
 // kx columns that stand for a conjugate pair in the half spectrum).
 __global__ void spme_influence_kernel(cufftDoubleComplex *__restrict__ Qk, const double *__restrict__ infl,
@@ -412,25 +403,6 @@ int spme_setup(tcp_ctx *c) {
     return TCP_OK;
 }
 
-static SpmeArgs spme_args(const tcp_ctx *c) {
-    SpmeArgs a;
-    a.x = c->x;
-    a.nel = c->nel;
-    a.n = c->n;
-    a.q0 = c->p.charge_scale * c->p.q[0];
-    a.q1 = c->p.charge_scale * c->p.q[1];
-    a.box0 = c->p.box[0];
-    a.box1 = c->p.box[1];
-    a.box2 = c->p.box[2];
-    a.K1 = c->K1;
-    a.K2 = c->K2;
-    a.K3 = c->K3;
-    a.kl0 = (double)c->K1 / c->p.box[0];
-    a.kl1 = (double)c->K2 / c->p.box[1];
-    a.kl2 = (double)c->K3 / c->p.box[2];
-    return a;
-}
-
 ChainArgs spme_chain_args(tcp_ctx *c) {
     ChainArgs a;
     a.n = c->n;
@@ -461,6 +433,7 @@ ChainArgs spme_chain_args(tcp_ctx *c) {
     a.many = nullptr;
     a.sys_of = nullptr;
     a.mesh = c->spme_fp32 ? (void *)c->Qf : (void *)c->Q;
+    a.dipole = nullptr;
     a.ticket = c->tickets + kTickBin;
     return a;
 }
@@ -492,7 +465,7 @@ int launch_spme(tcp_ctx *c, bool energy) {
     double *epart = recip_epart(c);
     if (c->own_fft) {
         const FftArgs f = spme_fft_args(c, !c->spme_fp32, energy);
-        c->launches += fft_convolve(chain, f, c->K1, 1, true, c->rstream);
+        c->launches += fft_convolve(chain, f, c->K1, 1, c->rstream);
         c->launches += chain_gather(chain, c->frec, epart, eb, kEps / (2.0 * kPi * c->V),
                                     energy ? c->scal + kScalUm : nullptr, c->rstream);
         TCP_CUDA(cudaGetLastError());
@@ -637,115 +610,6 @@ int launch_ewald(tcp_ctx *c, bool energy) {
 // Always FP64 (meshes hQ / hdQ, own D2Z / Z2D plans), whatever the precision
 // of the force path.
 
-// dQ(k) += q_j grad W_j(k) . w_j
-template <int P>
-__global__ void spme_spread_dipole_kernel(const SpmeArgs a, const double *__restrict__ w, double *__restrict__ dQ) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= a.n) return;
-    const double q = m < a.nel ? a.q0 : a.q1;
-    const double L[3] = {a.box0, a.box1, a.box2};
-    const int K[3] = {a.K1, a.K2, a.K3};
-    double W[3][P], dW[3][P];
-    int base[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const double u = (double)K[d] * (a.x[(size_t)d * a.n + m] + L[d] * .5) / L[d];
-        spline_w<P, double>(u, W[d], dW[d]);
-        base[d] = (int)trunc(u) - (P - 3);
-    }
-    const double wx = q * w[m] * ((double)a.K1 / a.box0), wy = q * w[(size_t)a.n + m] * ((double)a.K2 / a.box1),
-                 wz = q * w[2 * (size_t)a.n + m] * ((double)a.K3 / a.box2);
-#pragma unroll 1
-    for (int k = 0; k < P; ++k) {
-        const int iz = wrapi(base[2] + k, a.K3);
-#pragma unroll 1
-        for (int j = 0; j < P; ++j) {
-            const int iy = wrapi(base[1] + j, a.K2);
-            const double cx = wx * W[1][j] * W[2][k];
-            const double cyz = wy * dW[1][j] * W[2][k] + wz * W[1][j] * dW[2][k];
-            double *row = dQ + (size_t)a.K1 * (iy + (size_t)a.K2 * iz);
-#pragma unroll
-            for (int i = 0; i < P; ++i) atomicAdd(row + wrapi(base[0] + i, a.K1), cx * dW[0][i] + cyz * W[0][i]);
-        }
-    }
-}
-
-template <int P>
-__global__ void spme_gather_hvp_kernel(const SpmeArgs a, const double *__restrict__ phi,
-                                       const double *__restrict__ dphi, const double *__restrict__ w, double coef,
-                                       double *__restrict__ hw) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= a.n) return;
-    const double q = m < a.nel ? a.q0 : a.q1;
-    const double L[3] = {a.box0, a.box1, a.box2};
-    const int K[3] = {a.K1, a.K2, a.K3};
-    double W[3][P], dW[3][P], d2W[3][P];
-    int base[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const double u = (double)K[d] * (a.x[(size_t)d * a.n + m] + L[d] * .5) / L[d];
-        spline_w2<P>(u, W[d], dW[d], d2W[d]);
-        const double kl = (double)K[d] / L[d];
-#pragma unroll
-        for (int j = 0; j < P; ++j) {
-            dW[d][j] *= kl;
-            d2W[d][j] *= kl * kl;
-        }
-        base[d] = (int)trunc(u) - (P - 3);
-    }
-    const double w0 = w[m], w1 = w[(size_t)a.n + m], w2 = w[2 * (size_t)a.n + m];
-    double h0 = 0.0, h1 = 0.0, h2 = 0.0;
-#pragma unroll 1
-    for (int k = 0; k < P; ++k) {
-        const int iz = wrapi(base[2] + k, a.K3);
-#pragma unroll 1
-        for (int j = 0; j < P; ++j) {
-            const int iy = wrapi(base[1] + j, a.K2);
-            const size_t ro = (size_t)a.K1 * (iy + (size_t)a.K2 * iz);
-            // per row: sums over i of W, dW, d2W times phi and dphi
-            double sp = 0, sdp = 0, sd2p = 0, sq = 0, sdq = 0;
-#pragma unroll
-            for (int i = 0; i < P; ++i) {
-                const size_t idx = ro + wrapi(base[0] + i, a.K1);
-                const double ph = phi[idx], dph = dphi[idx];
-                sp += W[0][i] * ph;
-                sdp += dW[0][i] * ph;
-                sd2p += d2W[0][i] * ph;
-                sq += W[0][i] * dph;
-                sdq += dW[0][i] * dph;
-            }
-            const double Wy = W[1][j], dWy = dW[1][j], d2Wy = d2W[1][j];
-            const double Wz = W[2][k], dWz = dW[2][k], d2Wz = d2W[2][k];
-            // Hessian of W x gradient rows, times w, times phi; gradient times dphi
-            const double hxx = sd2p * Wy * Wz, hyy = sp * d2Wy * Wz, hzz = sp * Wy * d2Wz;
-            const double hxy = sdp * dWy * Wz, hxz = sdp * Wy * dWz, hyz = sp * dWy * dWz;
-            h0 += hxx * w0 + hxy * w1 + hxz * w2 + sdq * Wy * Wz;
-            h1 += hxy * w0 + hyy * w1 + hyz * w2 + sq * dWy * Wz;
-            h2 += hxz * w0 + hyz * w1 + hzz * w2 + sq * Wy * dWz;
-        }
-    }
-    hw[m] += coef * q * h0;
-    hw[(size_t)a.n + m] += coef * q * h1;
-    hw[2 * (size_t)a.n + m] += coef * q * h2;
-}
-
-template <int P>
-static void launch_hvp_kernels(tcp_ctx *c, const SpmeArgs &a, const double *w, double *hw, int which) {
-    const int threads = 128, blocks = (c->n + threads - 1) / threads;
-    if (which == 1) spme_spread_dipole_kernel<P><<<blocks, threads, 0, c->stream>>>(a, w, c->hdQ);
-    else spme_gather_hvp_kernel<P><<<blocks, threads, 0, c->stream>>>(a, c->hQ, c->hdQ, w, kEps / (kPi * c->V), hw);
-}
-
-static void hvp_kernels(tcp_ctx *c, const SpmeArgs &a, const double *w, double *hw, int which) {
-    switch (c->p.order) {
-        case 4: launch_hvp_kernels<4>(c, a, w, hw, which); break;
-        case 5: launch_hvp_kernels<5>(c, a, w, hw, which); break;
-        case 6: launch_hvp_kernels<6>(c, a, w, hw, which); break;
-        case 7: launch_hvp_kernels<7>(c, a, w, hw, which); break;
-        default: launch_hvp_kernels<8>(c, a, w, hw, which); break;
-    }
-}
-
 void spme_hvp_free(tcp_ctx *c) {
     if (c->hplans) {
         cufftDestroy(c->hplan_f);
@@ -781,34 +645,27 @@ int launch_spme_hvp(tcp_ctx *c, const double *w, double *hw) {
         cufftSetStream(c->hplan_b, c->stream);
         c->hplans = true;
     }
-    const SpmeArgs a = spme_args(c);
     const long total = (long)nhalf;
     const int eb = spme_energy_blocks(c);
     double *mesh[2] = {c->hQ, c->hdQ};
     ChainArgs chain = spme_chain_args(c);
     chain.fp64 = 1;
-    chain.mesh = c->hQ;
     c->launches += chain_bin(chain, c->x, c->stream);
     c->launches += chain_sort(chain, c->stream);
-    if (!c->own_fft) c->launches += chain_spread(chain, c->stream);
     for (int pass = 0; pass < 2; ++pass) {    // phi = A Q, then dphi = A dQ
-        if (pass == 1) {
-            TCP_CUDA(cudaMemsetAsync(mesh[pass], 0, sizeof(double) * nreal, c->stream));
-            hvp_kernels(c, a, w, hw, pass);
-            c->launches++;
-        }
+        chain.mesh = mesh[pass];
+        chain.dipole = pass ? w : nullptr;
         if (c->own_fft) {
-            chain.mesh = mesh[pass];
-            c->launches += fft_convolve(chain, spme_fft_args(c, true, false), c->K1, 1, pass == 0, c->stream);
+            c->launches += fft_convolve(chain, spme_fft_args(c, true, false), c->K1, 1, c->stream);
             continue;
         }
+        c->launches += chain_spread(chain, c->stream);
         if (cufftExecD2Z(c->hplan_f, mesh[pass], c->hQk) != CUFFT_SUCCESS) return set_error(TCP_ERR_CUFFT, "cufftExecD2Z failed");
         spme_influence_kernel<<<eb, 256, 0, c->stream>>>(c->hQk, c->infl, total, c->Kh, c->K1, nullptr, false);
         if (cufftExecZ2D(c->hplan_b, c->hQk, mesh[pass]) != CUFFT_SUCCESS) return set_error(TCP_ERR_CUFFT, "cufftExecZ2D failed");
-        c->launches += 2;
+        c->launches++;
     }
-    hvp_kernels(c, a, w, hw, 2);
-    c->launches++;
+    c->launches += chain_gather_hvp(chain, c->hQ, c->hdQ, w, hw, c->stream);
     TCP_CUDA(cudaGetLastError());
     return TCP_OK;
 }

@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kPartThreads) chain_weights_kernel(int n, Spre
 // its lanes executed 3-5 times the instructions, most lanes past the owned
 // rows (whole chain at N = 9,000, 48^3, order 6, FP64: 240 us then, 163 us now).
 constexpr int kSpreadThreads = 128;
-template <int P, typename T, bool BATCH>
+template <int P, typename T, bool BATCH, bool DIP = false>
 __global__ void __launch_bounds__(kSpreadThreads) chain_spread_kernel(const ChainArgs c, int rows, int per_plane) {
     constexpr bool F32 = sizeof(T) == 4;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kSpreadThreads) chain_spread_kernel(const Chai
         h[k] = (T)0;
         if (F32) lo[k] = 0.f;
     }
-    chain_rows<P, T, kSpreadThreads>(c, g, z, y0, nrow, h, lo, K1, st, threadIdx.x, 1, 0, 1);
+    chain_rows<P, T, kSpreadThreads, DIP>(c, g, z, y0, nrow, h, lo, K1, st, threadIdx.x, 1, 0, 1);
     __syncthreads();
     T *mesh = static_cast<T *>(c.mesh) + g.mesh_off + (size_t)K1 * (y0 + (size_t)g.K[1] * z);
     for (int k = threadIdx.x; k < nrow * K1; k += kSpreadThreads) mesh[k] = F32 ? h[k] + (T)lo[k] : h[k];
@@ -241,6 +241,74 @@ __global__ void __launch_bounds__(kGatherThreads) chain_gather_kernel(const Chai
     }
 }
 
+// The reciprocal Hessian-vector product's gather, 8 lanes per particle as
+// above, always FP64: (H w)_i = c q_i [sum_k (hess W_i(k) w_i) phi(k) + sum_k
+// grad W_i(k) dphi(k)].  Bound: the FP64 pipe (about 45 operations a mesh row)
+// and L2 latency; a thread per particle took 45 us at N = 4,096, order 4.
+template <int P>
+__global__ void __launch_bounds__(kGatherThreads) chain_gather_hvp_kernel(const ChainArgs c, const double *__restrict__ phi,
+                                                                          const double *__restrict__ dphi,
+                                                                          const double *__restrict__ w,
+                                                                          double *__restrict__ hw) {
+    constexpr int NP = kGatherThreads / 8;
+    __shared__ double sw[NP][3][3 * P];          // W, W', W'' per axis
+    const int t0 = blockIdx.x * NP, np = min(NP, c.n - t0);
+    const int p = min((int)threadIdx.x >> 3, np - 1), sub = threadIdx.x & 7;   // idle groups repeat the last particle
+    const bool live = (int)threadIdx.x >> 3 < np;
+    const int m = c.b.order[t0 + p];
+    const SpmeGeom &g = c.one;
+    if (live && sub < 3) {
+        double W[P], dW[P], d2W[P];
+        const double arg = static_cast<const double *>(c.b.arg)[(size_t)sub * c.n + m], kl = g.KL[sub];
+        spline_w2<P>(P == 4 ? 1.0 - arg : arg, W, dW, d2W);
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+            sw[p][sub][j] = W[j];
+            sw[p][sub][P + j] = dW[j] * kl;
+            sw[p][sub][2 * P + j] = d2W[j] * (kl * kl);
+        }
+    }
+    __syncthreads();
+    const int pk = c.b.base[t0 + p], K1 = g.K[0], K2 = g.K[1], K3 = g.K[2];
+    const int bx = pk & 1023, by = (pk >> 10) & 1023, bz = pk >> 20;
+    const double *sx = sw[p][0], *sy = sw[p][1], *sz = sw[p][2];
+    const double w0 = w[m], w1 = w[(size_t)c.n + m], w2 = w[2 * (size_t)c.n + m];
+    double h[3] = {0.0, 0.0, 0.0};
+    for (int r = sub; r < P * P; r += 8) {
+        const int k = r / P, j = r - k * P;
+        int iy = by + j, iz = bz + k;
+        iy -= iy >= K2 ? K2 : 0;
+        iz -= iz >= K3 ? K3 : 0;
+        const size_t ro = (size_t)K1 * (iy + (size_t)K2 * iz);
+        double sp = 0, sdp = 0, sd2p = 0, sq = 0, sdq = 0;
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+            const int x = bx + i >= K1 ? bx + i - K1 : bx + i;
+            const double ph = phi[ro + x], dph = dphi[ro + x];
+            sp = fma(sx[i], ph, sp);
+            sdp = fma(sx[P + i], ph, sdp);
+            sd2p = fma(sx[2 * P + i], ph, sd2p);
+            sq = fma(sx[i], dph, sq);
+            sdq = fma(sx[P + i], dph, sdq);
+        }
+        const double Wy = sy[j], dWy = sy[P + j], d2Wy = sy[2 * P + j], Wz = sz[k], dWz = sz[P + k], d2Wz = sz[2 * P + k];
+        // Hessian of W x gradient rows, times w, times phi; gradient times dphi
+        const double yz = Wy * Wz, dyz = dWy * Wz, ydz = Wy * dWz;
+        const double hxy = sdp * dyz, hxz = sdp * ydz, hyz = sp * (dWy * dWz);
+        h[0] += fma(fma(sd2p, w0, sdq), yz, fma(hxy, w1, hxz * w2));
+        h[1] += fma(hxy, w0, fma(fma(sp, d2Wy * w1, sq * dWy), Wz, hyz * w2));
+        h[2] += fma(hxz, w0, fma(hyz, w1, Wy * fma(sp, d2Wz * w2, sq * dWz)));
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) h[d] += __shfl_xor_sync(0xffffffffu, h[d], o);
+    if (live && sub < 3) {
+        const double q = m < g.nel ? g.q[0] : g.q[1];
+        hw[(size_t)sub * c.n + m] += g.coef * q * (sub == 0 ? h[0] : (sub == 1 ? h[1] : h[2]));
+    }
+}
+
 // ---------------------------------------------------------------------------
 int chain_bin(const ChainArgs &c, const double *x, cudaStream_t st) {
     const int blocks = (c.n + kPartBlock - 1) / kPartBlock;
@@ -257,7 +325,7 @@ static int chain_spread_rows(int P, int k1max) {
     return std::max(1, std::min(rows, (int)((150u << 10) / ((size_t)k1max * 8))));
 }
 static size_t chain_spread_bytes(int P, int k1max) {   // two-float FP32 or FP64: 8 bytes a point
-    return (size_t)chain_spread_rows(P, k1max) * k1max * 8 + stage_bytes<double>(P);
+    return (size_t)chain_spread_rows(P, k1max) * k1max * 8 + std::max(stage_bytes<double>(P), stage_bytes<double>(P, true));
 }
 
 template <int P, typename T>
@@ -278,8 +346,11 @@ static int sort_p(const ChainArgs &c, cudaStream_t st) {
 template <int P, typename T, bool BATCH>
 static int spread_p(const ChainArgs &c, cudaStream_t st) {
     const int rows = chain_spread_rows(P, c.k1max), per_plane = (c.k2max + rows - 1) / rows;
-    chain_spread_kernel<P, T, BATCH><<<c.planes * per_plane, kSpreadThreads, chain_spread_bytes(P, c.k1max), st>>>(c, rows,
-                                                                                                              per_plane);
+    const size_t sm = chain_spread_bytes(P, c.k1max);
+    if (!BATCH && sizeof(T) == 8 && c.dipole)
+        chain_spread_kernel<P, double, false, true><<<c.planes * per_plane, kSpreadThreads, sm, st>>>(c, rows, per_plane);
+    else
+        chain_spread_kernel<P, T, BATCH><<<c.planes * per_plane, kSpreadThreads, sm, st>>>(c, rows, per_plane);
     return 1;
 }
 
@@ -300,7 +371,7 @@ int chain_sort(const ChainArgs &c, cudaStream_t st) {
     return n;
 }
 
-int chain_spread(const ChainArgs &c, cudaStream_t st) {
+int chain_spread(const ChainArgs &c, cudaStream_t st) {   // c.dipole: FP64 single systems
     int n = 0;
 #define TCP_CALL(P) \
     n = c.many ? spread_p<P, float, true>(c, st) : (c.fp64 ? spread_p<P, double, false>(c, st) : spread_p<P, float, false>(c, st))
@@ -328,6 +399,15 @@ int chain_gather(const ChainArgs &c, double *frec, const double *epart, int nepa
     return 1;
 }
 
+int chain_gather_hvp(const ChainArgs &c, const double *phi, const double *dphi, const double *w, double *hw,
+                     cudaStream_t st) {
+    constexpr int NP = kGatherThreads / 8;
+#define TCP_CALL(P) chain_gather_hvp_kernel<P><<<(c.n + NP - 1) / NP, kGatherThreads, 0, st>>>(c, phi, dphi, w, hw)
+    TCP_CHAIN_ORDER(TCP_CALL)
+#undef TCP_CALL
+    return 1;
+}
+
 // shared-memory limit of the spread for this mesh (once, outside any capture)
 int chain_prepare(const ChainArgs &c) {
     const int bytes = (int)chain_spread_bytes(c.P, c.k1max);
@@ -337,6 +417,7 @@ int chain_prepare(const ChainArgs &c) {
         TCP_LIMIT((chain_spread_kernel<P, float, true>));    \
         TCP_LIMIT((chain_spread_kernel<P, float, false>));   \
         TCP_LIMIT((chain_spread_kernel<P, double, false>));  \
+        TCP_LIMIT((chain_spread_kernel<P, double, false, true>)); \
     } while (0)
     TCP_CHAIN_ORDER(TCP_CALL)
 #undef TCP_CALL

@@ -101,7 +101,7 @@ __device__ __forceinline__ void bin_store(const SpreadBins &b, int m, int n, con
 // named barrier `bar`; the whole CTA where there is one group).  For each jz =
 // jz0, jz0 + jzs, .. the particles of plane z - jz whose support reaches the
 // rows -- at most two runs of the sorted list -- are staged in shared memory,
-// kStage at a time, with their factors q W_z W_y; then P lanes own one row and
+// kStage (or half that) at a time, with their factors q W_z W_y; then P lanes own one row and
 // walk its particles, lane l adding the point bx + l: no two lanes ever add to
 // one point, and every point is summed in the same order (jz, bin, particle)
 // on every call.  hi, and lo in FP32, hold the rows (cleared by the caller;
@@ -115,20 +115,20 @@ constexpr int kStage = 256;
 constexpr int kStageBins = 136;          // bins that reach one CTA's rows: at most 128 (a plane) or rows + P - 1
 template <typename T>
 struct StageBuf {
-    T *w;                // [kStage][2 P]: W_x, then q W_z W_y
+    T *w;                // [kStage][2 P]: W_x, then q W_z W_y (dipoles: [kStage][4 P], W_x, W_x', then their factors)
     int *bx;             // [kStage] base x and y
     int2 *run;           // [kStageBins] list range of each bin
 };
 template <typename T>
-__host__ __device__ constexpr size_t stage_bytes(int P) {
-    return kStage * (2 * (size_t)P * sizeof(T) + sizeof(int)) + kStageBins * sizeof(int2);
+__host__ __device__ constexpr size_t stage_bytes(int P, bool dipole = false) {
+    return (dipole ? kStage / 2 : kStage) * ((dipole ? 4 : 2) * (size_t)P * sizeof(T) + sizeof(int)) + kStageBins * sizeof(int2);
 }
 template <typename T>
 __device__ __forceinline__ StageBuf<T> stage_at(void *p, int P) {
     StageBuf<T> s;
     s.run = static_cast<int2 *>(p);
     s.w = reinterpret_cast<T *>(s.run + kStageBins);
-    s.bx = reinterpret_cast<int *>(s.w + kStage * 2 * P);
+    s.bx = reinterpret_cast<int *>(s.w + kStage * 2 * P);   // half as many dipoles, twice the factors
     return s;
 }
 
@@ -136,12 +136,14 @@ __device__ __forceinline__ void group_sync(int bar, int threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(threads) : "memory");
 }
 
-template <int P, typename T, int NG>
+// DIP: the mesh dipole grad W . c.dipole of every particle (K/L times the index
+// derivatives) instead of its charge.
+template <int P, typename T, int NG, bool DIP = false>
 __device__ __forceinline__ void chain_rows(const ChainArgs &c, const SpmeGeom &g, int z, int y0, int nrow, T *hi,
                                            float *lo, int stride, const StageBuf<T> &st, int tid, int bar, int jz0,
                                            int jzs) {
     constexpr bool F32 = sizeof(T) == 4;
-    constexpr int RG = 32 / P;
+    constexpr int RG = 32 / P, ST = DIP ? kStage / 2 : kStage;
     const int K1 = g.K[0], K2 = g.K[1], K3 = g.K[2];
     const int lane = tid & 31, grp = lane / P, l = lane - grp * P;
     const unsigned mask = ((1u << P) - 1u) << (grp * P);
@@ -157,17 +159,32 @@ __device__ __forceinline__ void chain_rows(const ChainArgs &c, const SpmeGeom &g
         }
         for (int piece = blo < 0 ? 0 : 1; piece < 2; ++piece) {
             const int q0 = start[piece ? max(blo, 0) : blo + K2], q1 = start[piece ? blo + nb : K2];
-            for (int c0 = q0; c0 < q1; c0 += kStage) {
-                const int cn = min(kStage, q1 - c0);
+            for (int c0 = q0; c0 < q1; c0 += ST) {
+                const int cn = min(ST, q1 - c0);
                 if (c0 != q0 || piece) group_sync(bar, NG);   // the chunk before is read
                 for (int e = tid; e < cn; e += NG) {
                     const T *w = ew + (size_t)(c0 + e) * 6 * P;
-                    const T qz = eq[c0 + e] * w[4 * P + jz];
-                    T *o = st.w + e * 2 * P;
+                    T *o = st.w + e * (DIP ? 4 : 2) * P;
+                    if (DIP) {
+                        const int m = c.b.order[c0 + e];
+                        const T q = eq[c0 + e], wz = w[4 * P + jz], dz = w[5 * P + jz];
+                        const T vx = q * (T)(c.dipole[m] * g.KL[0]) * wz;
+                        const T vy = q * (T)(c.dipole[(size_t)c.n + m] * g.KL[1]) * wz;
+                        const T vz = q * (T)(c.dipole[2 * (size_t)c.n + m] * g.KL[2]) * dz;
 #pragma unroll
-                    for (int j = 0; j < P; ++j) {
-                        o[j] = w[j];
-                        o[P + j] = qz * w[2 * P + j];
+                        for (int j = 0; j < P; ++j) {
+                            o[j] = w[j];
+                            o[P + j] = w[P + j];
+                            o[2 * P + j] = vy * w[3 * P + j] + vz * w[2 * P + j];
+                            o[3 * P + j] = vx * w[2 * P + j];
+                        }
+                    } else {
+                        const T qz = eq[c0 + e] * w[4 * P + jz];
+#pragma unroll
+                        for (int j = 0; j < P; ++j) {
+                            o[j] = w[j];
+                            o[P + j] = qz * w[2 * P + j];
+                        }
                     }
                     st.bx[e] = c.b.base[c0 + e];
                 }
@@ -191,9 +208,11 @@ __device__ __forceinline__ void chain_rows(const ChainArgs &c, const SpmeGeom &g
                                 jy += jy < 0 ? K2 : 0;
                                 int x = (pk & 1023) + l;
                                 x -= x >= K1 ? K1 : 0;
-                                const T *w = st.w + e * 2 * P;
-                                const T v = w[P + jy], wx = w[l];
-                                if (F32) {
+                                const T *w = st.w + e * (DIP ? 4 : 2) * P;
+                                const T v = w[(DIP ? 2 : 1) * P + jy], wx = w[l];
+                                if (DIP) {
+                                    h[x] = fma(v, wx, fma(w[3 * P + jy], w[P + l], h[x]));
+                                } else if (F32) {
                                     const T u = v * wx, a = h[x], s = a + u, bp = s - a;
                                     lw[x] += (float)((a - (s - bp)) + (u - bp));
                                     h[x] = s;

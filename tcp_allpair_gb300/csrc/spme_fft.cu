@@ -149,9 +149,9 @@ __host__ __device__ constexpr int spread_groups() { return N == 32 ? 4 : (N <= 6
 template <int N>
 __host__ __device__ constexpr int plane_stride() { return N + 1; }
 template <int N, typename T>
-__host__ __device__ constexpr size_t plane_bytes(int P) {   // P = 0: no charges are spread
+__host__ __device__ constexpr size_t plane_bytes(int P, bool dipole = false) {   // P = 0: the inverse kernel
     const size_t plane = (size_t)N * plane_stride<N>();
-    return 2 * N * sizeof(T) + (P ? spread_groups<N>() * (plane * 8 + stage_bytes<T>(P)) : plane * sizeof(T));
+    return 2 * N * sizeof(T) + (P ? spread_groups<N>() * (plane * 8 + stage_bytes<T>(P, dipole)) : plane * sizeof(T));
 }
 
 // The two passes over a line whose points are re[n * step], im[n * step]; the
@@ -197,8 +197,8 @@ __device__ __forceinline__ const SpmeGeom &geom_of_block(const ChainArgs &c, con
     return BATCH ? c.many[sys] : c.one;
 }
 
-// SPREAD: gather the plane's charges; otherwise read the plane from c.mesh.
-template <int N, typename T, bool BATCH, bool SPREAD>
+// DIP: the mesh dipoles of c.dipole instead of the charges.
+template <int N, typename T, bool BATCH, bool DIP>
 __global__ void __launch_bounds__(plane_threads<N, T>()) fft_forward_kernel(const ChainArgs c, const FftArgs f) {
     constexpr int NT = plane_threads<N, T>(), S = plane_stride<N>(), R1 = Line<N>::R1, R2 = Line<N>::R2;
     constexpr bool F32 = sizeof(T) == 4;
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(plane_threads<N, T>()) fft_forward_kernel(cons
     int z, sys;
     const SpmeGeom &g = geom_of_block<N, T, BATCH>(c, f, N, z, sys);
     for (int k = tid; k < N; k += NT) tw[k] = static_cast<const C2<T> *>(f.tw)[k];
-    if (SPREAD) {
+    {
         constexpr int G = spread_groups<N>(), NG = NT / G;
         const int q = tid / NG, t = tid - q * NG;
         // group q: its rows (two-float FP32 or FP64, 8 bytes a point) and its stage
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(plane_threads<N, T>()) fft_forward_kernel(cons
         }
 #define TCP_ROWS(P)                                                                                                    \
     case P:                                                                                                            \
-        chain_rows<P, T, NG>(c, g, z, 0, N, h, lo, S, stage_at<T>(stages + q * stage_bytes<T>(P), P), t, 1 + q, q, G); \
+        chain_rows<P, T, NG, DIP>(c, g, z, 0, N, h, lo, S, stage_at<T>(stages + q * stage_bytes<T>(P, DIP), P), t, 1 + q, q, G); \
         break
         switch (c.P) {
             TCP_ROWS(4);
@@ -248,10 +248,6 @@ __global__ void __launch_bounds__(plane_threads<N, T>()) fft_forward_kernel(cons
             }
             hi[k] = F32 ? v + (T)e : v;
         }
-        __syncthreads();
-    } else {
-        const T *mesh = static_cast<const T *>(c.mesh) + g.mesh_off + (size_t)z * N * N;
-        for (int k = tid; k < N * N; k += NT) hi[(k / N) * S + k % N] = mesh[k];
         __syncthreads();
     }
     // x: rows 2j and 2j + 1 as real and imaginary part
@@ -481,12 +477,13 @@ int fft_twiddles(int N, bool fp64, void **tw) {
 }
 
 template <int N, typename T, bool BATCH>
-static int convolve_n(const ChainArgs &c, const FftArgs &f, int systems, bool spread, cudaStream_t st) {
+static int convolve_n(const ChainArgs &c, const FftArgs &f, int systems, cudaStream_t st) {
     constexpr int NT = plane_threads<N, T>();
-    if (spread)
-        fft_forward_kernel<N, T, BATCH, true><<<N * systems, NT, plane_bytes<N, T>(c.P), st>>>(c, f);
+    constexpr bool D = !BATCH && sizeof(T) == 8;
+    if (D && c.dipole)
+        fft_forward_kernel<N, T, BATCH, D><<<N * systems, NT, plane_bytes<N, T>(c.P, true), st>>>(c, f);
     else
-        fft_forward_kernel<N, T, BATCH, false><<<N * systems, NT, plane_bytes<N, T>(0), st>>>(c, f);
+        fft_forward_kernel<N, T, BATCH, false><<<N * systems, NT, plane_bytes<N, T>(c.P), st>>>(c, f);
     fft_z_kernel<N, T, BATCH><<<(N / 2 + 1) * N / kZCols * systems, z_threads<N>(), 0, st>>>(c, f);
     fft_inverse_kernel<N, T, BATCH><<<N * systems, NT, plane_bytes<N, T>(0), st>>>(c, f);
     return 3;
@@ -494,9 +491,10 @@ static int convolve_n(const ChainArgs &c, const FftArgs &f, int systems, bool sp
 
 template <int N, typename T, bool BATCH>
 static int prepare_n(int P) {
-    TCP_CUDA(cudaFuncSetAttribute(fft_forward_kernel<N, T, BATCH, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_bytes<N, T>(P)));
-    if (!BATCH)
-        TCP_CUDA(cudaFuncSetAttribute(fft_forward_kernel<N, T, BATCH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_bytes<N, T>(0)));
+    constexpr bool D = !BATCH && sizeof(T) == 8;
+    TCP_CUDA(cudaFuncSetAttribute(fft_forward_kernel<N, T, BATCH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_bytes<N, T>(P)));
+    if (D)
+        TCP_CUDA(cudaFuncSetAttribute(fft_forward_kernel<N, T, BATCH, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_bytes<N, T>(P, true)));
     TCP_CUDA(cudaFuncSetAttribute(fft_inverse_kernel<N, T, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_bytes<N, T>(0)));
     return TCP_OK;
 }
@@ -514,11 +512,11 @@ int fft_energy_parts(int N) { return (N / 2 + 1) * N / kZCols; }
 
 // Spread, transform, influence multiply and inverse transform of `systems`
 // meshes of N points a side (a batch's in f.list), phi left in c.mesh.
-int fft_convolve(const ChainArgs &c, const FftArgs &f, int N, int systems, bool spread, cudaStream_t st) {
+int fft_convolve(const ChainArgs &c, const FftArgs &f, int N, int systems, cudaStream_t st) {
     int n = 0;
 #define TCP_CALL(N)                                                               \
-    n = c.many ? convolve_n<N, float, true>(c, f, systems, spread, st)            \
-               : (c.fp64 ? convolve_n<N, double, false>(c, f, 1, spread, st) : convolve_n<N, float, false>(c, f, 1, spread, st))
+    n = c.many ? convolve_n<N, float, true>(c, f, systems, st)            \
+               : (c.fp64 ? convolve_n<N, double, false>(c, f, 1, st) : convolve_n<N, float, false>(c, f, 1, st))
     TCP_FFT_SIZE(N, TCP_CALL)
 #undef TCP_CALL
     return n;

@@ -33,32 +33,11 @@ __device__ __forceinline__ void spline_rec(T w, T *W, T *dW) {
 }
 
 // B-spline weights W[j] = M_P(w + P-1-j) and dW[j] = dM_P/du on the grid
-// points INT(u) + j - (P-3).  Order 4 uses the reference's explicit cubics
-// (force.f90:703-738); other orders the Cox-de Boor recursion run upward on
-// the P nonzero values.
-template <int P, typename T>
-__device__ __forceinline__ void spline_w(double u, T *W, T *dW) {
-    if (P == 4) {
-        T z = (T)(trunc(u) - u + 1.0);
-        W[0] = z * z * z / (T)6;
-        dW[0] = (T)-3. * z * z / (T)6;
-        z += (T)1;
-        W[1] = ((T)-3. * z * z * z + (T)12. * z * z - (T)12. * z + (T)4.) / (T)6;
-        dW[1] = ((T)9. * z * z - (T)24. * z + (T)12.) / (T)6;
-        z += (T)1;
-        W[2] = ((T)3. * z * z * z - (T)24. * z * z + (T)60. * z - (T)44.) / (T)6;
-        dW[2] = ((T)-9. * z * z + (T)48. * z - (T)60.) / (T)6;
-        z += (T)1;
-        W[3] = (-z * z * z + (T)12. * z * z - (T)48. * z + (T)64.) / (T)6;
-        dW[3] = ((T)3. * z * z - (T)24. * z + (T)48.) / (T)6;
-        return;
-    }
-    spline_rec<P, T>((T)(u - trunc(u)), W, dW);
-}
-
-// The same values from the argument that the binning stores (bin_axis): z =
-// INT(u) - u + 1 for order 4, the fraction of u otherwise.  The cubics' sixth
-// is a multiplication (a division by 6 is a subroutine in either precision).
+// points INT(u) + j - (P-3), from the argument that the binning stores
+// (bin_axis): z = INT(u) - u + 1 for order 4, in which the reference writes its
+// explicit cubics (force.f90:703-738), the fraction w of u for the others.  The
+// cubics' sixth is a multiplication (a division by 6 is a subroutine in either
+// precision).
 template <int P, typename T>
 __device__ __forceinline__ void spline_at(T arg, T *W, T *dW) {
     if (P == 4) {
@@ -84,9 +63,9 @@ __device__ __forceinline__ void spline_at(T arg, T *W, T *dW) {
 // P >= 4 by the same recursion: the order P-2 values give
 // M_P''(y) = M_{P-2}(y) - 2 M_{P-2}(y-1) + M_{P-2}(y-2), the order P-1 values
 // M_P'(y) = M_{P-1}(y) - M_{P-1}(y-1).
+// At fraction w.
 template <int P>
-__device__ __forceinline__ void spline_w2(double u, double *W, double *dW, double *d2W) {
-    const double w = u - trunc(u);
+__device__ __forceinline__ void spline_w2(double w, double *W, double *dW, double *d2W) {
     double a[P];
     a[0] = 1.0;
 #pragma unroll

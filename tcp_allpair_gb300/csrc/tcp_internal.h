@@ -141,6 +141,7 @@ struct ChainArgs {
     const SpmeGeom *many;        // batch: every system, and the system of each particle
     const int *sys_of;
     void *mesh;                  // double (fp64) or float
+    const double *dipole;        // [3][n]: spread sum_j q_j grad W_j . dipole_j instead (FP64 single systems; null: charges)
     unsigned *ticket;
 };
 }  // namespace tcp
@@ -388,13 +389,15 @@ std::vector<int> fft_order(int N);   // element of the transform order -> index 
 int fft_twiddles(int N, bool fp64, void **tw);
 int fft_energy_parts(int N);
 int fft_prepare(const ChainArgs &c, int N, bool fp64);
-int fft_convolve(const ChainArgs &c, const FftArgs &f, int N, int systems, bool spread, cudaStream_t st);
+int fft_convolve(const ChainArgs &c, const FftArgs &f, int N, int systems, cudaStream_t st);
 // kernel launches; each returns how many
 int chain_bin(const ChainArgs &c, const double *x, cudaStream_t st);   // not after a half kick that binned
 int chain_sort(const ChainArgs &c, cudaStream_t st);                   // the binned particles' order and spline values
 int chain_spread(const ChainArgs &c, cudaStream_t st);                 // sorted particles -> c.mesh
 int chain_gather(const ChainArgs &c, double *frec, const double *epart, int nepart, double escale, double *um,
                  cudaStream_t st);
+int chain_gather_hvp(const ChainArgs &c, const double *phi, const double *dphi, const double *w, double *hw,
+                     cudaStream_t st);
 ChainArgs spme_chain_args(tcp_ctx *c);                                 // spme.cu
 
 // ctx.cu: step and force composition for the derivative routines
