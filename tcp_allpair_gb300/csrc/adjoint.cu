@@ -39,6 +39,7 @@
 
 #include "device_util.cuh"
 #include "pair_f64.cuh"
+#include "spme_chain.cuh"
 #include "pair_math.cuh"
 #include "pair_n3.cuh"
 #include "tcp_internal.h"
@@ -654,9 +655,11 @@ __global__ void soa_to_aos_kernel(const double *__restrict__ in, double *__restr
 
 // ---- reverse-mode step kernels ------------------------------------------------
 struct RevArgs {
-    const double *v;      // v_k [3][n]
+    const double *x, *v;  // x_k, v_k [3][n]
     double *xb, *vb, *fb, *g, *part;
-    const double *hw;
+    double *hw;
+    double *mean;         // mean of g per component
+    unsigned *ticket;
     int nel, n;
     double a0, a1;        // dt/(2 m) per species
     double cj0, cj1;      // 2 m/(3 N K) per species
@@ -664,62 +667,55 @@ struct RevArgs {
 };
 
 // step k >= 1: vb += 2 m v_k/(3NK), g = fb + a vb (the two uses of F_k);
-// k = 0 (initial_only): g = fb.  Per-block sums of g for the mean.
-__global__ void rev_seed_kernel(const RevArgs r, bool initial_only) {
-    __shared__ double red[32];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double s[3] = {0.0, 0.0, 0.0};
+// k = 0 (initial_only): g = fb.  A thread per component; the mean of g by the
+// last CTA.  H w is cleared on the way.
+__global__ void __launch_bounds__(kPartThreads) rev_seed_kernel(const RevArgs r, bool initial_only) {
+    __shared__ double red[8];
+    const int k = threadIdx.x % kPartBlock, d = threadIdx.x / kPartBlock, i = blockIdx.x * kPartBlock + k;
+    const int w = threadIdx.x >> 5, nb = gridDim.x;
+    double s = 0.0;
     if (i < r.n) {
         const bool el = i < r.nel;
-        const double a = el ? r.a0 : r.a1, cj = el ? r.cj0 : r.cj1;
-        for (int d = 0; d < 3; ++d) {
-            const size_t k = (size_t)d * r.n + i;
-            if (initial_only) {
-                s[d] = r.fb[k];
-            } else {
-                const double vb = r.vb[k] + cj * r.v[k];
-                r.vb[k] = vb;
-                s[d] = r.fb[k] + a * vb;
-            }
-            r.g[k] = s[d];
+        const size_t o = (size_t)d * r.n + i;
+        if (initial_only) {
+            s = r.fb[o];
+        } else {
+            const double vb = r.vb[o] + (el ? r.cj0 : r.cj1) * r.v[o];
+            r.vb[o] = vb;
+            s = r.fb[o] + (el ? r.a0 : r.a1) * vb;
         }
+        r.g[o] = s;
+        r.hw[o] = 0.0;
     }
-    for (int d = 0; d < 3; ++d) {
-        const double t = block_sum(s[d], red);
-        if (threadIdx.x == 0) r.part[3 * blockIdx.x + d] = t;
-    }
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) red[w] = s;
+    __syncthreads();
+    if (threadIdx.x < 3) r.part[threadIdx.x * nb + blockIdx.x] = red[2 * threadIdx.x] + red[2 * threadIdx.x + 1];
+    if (!last_block(r.ticket)) return;
+    s = 0.0;
+    for (int b = k; b < nb; b += kPartBlock) s += __ldcg(r.part + d * nb + b);
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) red[w] = s;
+    __syncthreads();
+    if (threadIdx.x < 3) r.mean[threadIdx.x] = (red[2 * threadIdx.x] + red[2 * threadIdx.x + 1]) / (double)r.n;
 }
 
-// g -= mean(g) (REMOVE_RIGIDMTN applied to the adjoint, force.f90:986-1004);
-// every block sums the per-block partials in the same order.
-__global__ void rev_center_kernel(const RevArgs r, int nparts) {
-    __shared__ double mean[3];
-    __shared__ double red[32];
-    for (int d = 0; d < 3; ++d) {
-        double s = 0.0;
-        for (int b = threadIdx.x; b < nparts; b += blockDim.x) s += r.part[3 * b + d];
-        s = block_sum(s, red);
-        if (threadIdx.x == 0) mean[d] = s / (double)r.n;
-    }
-    __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= r.n) return;
-    for (int d = 0; d < 3; ++d) r.g[(size_t)d * r.n + i] -= mean[d];
+// g -= mean(g) (REMOVE_RIGIDMTN applied to the adjoint, force.f90:986-1004)
+__global__ void rev_center_kernel(const RevArgs r) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < 3 * r.n) r.g[t] -= r.mean[t / r.n];
 }
 
 // xb -= H P g;  vb += dt xb;  fb = a vb
 __global__ void rev_update_kernel(const RevArgs r) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= r.n) return;
-    const double a = i < r.nel ? r.a0 : r.a1;
-    for (int d = 0; d < 3; ++d) {
-        const size_t k = (size_t)d * r.n + i;
-        const double xb = r.xb[k] - r.hw[k];
-        const double vb = r.vb[k] + r.dt * xb;
-        r.xb[k] = xb;
-        r.vb[k] = vb;
-        r.fb[k] = a * vb;
-    }
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 3 * r.n) return;
+    const double a = t % r.n < r.nel ? r.a0 : r.a1;
+    const double xb = r.xb[t] - r.hw[t];
+    const double vb = r.vb[t] + r.dt * xb;
+    r.xb[t] = xb;
+    r.vb[t] = vb;
+    r.fb[t] = a * vb;
 }
 
 // J accumulator: scal[kAdjJ] += mv2el + mv2ion of the step just taken
@@ -758,7 +754,7 @@ static int adj_alloc(tcp_ctx *c) {
         cudaMalloc(&c->adj_fb, v3) != cudaSuccess || cudaMalloc(&c->adj_save, 3 * v3) != cudaSuccess ||
         cudaMalloc(&c->adj_io, v3) != cudaSuccess ||
         cudaMalloc(&c->adj_scal, sizeof(double) * kAdjCount) != cudaSuccess ||
-        cudaMalloc(&c->adj_part, sizeof(double) * 3 * (size_t)rev_blocks(c->n)) != cudaSuccess) {
+        cudaMalloc(&c->adj_part, sizeof(double) * (3 * (size_t)part_blocks(c->n) + 3)) != cudaSuccess) {
         adjoint_free(c);
         return set_error(TCP_ERR_NOMEM, "derivative buffers: device allocation failed");
     }
@@ -942,11 +938,11 @@ static int launch_adj_pair(tcp_ctx *c, const double *w, double *hw) {
 }
 
 // hw = H w at the current positions (device SoA), scal[kAdjDFdl] += dF/dl . w
-static int hvp_device(tcp_ctx *c, const double *w, double *hw) {
+static int hvp_device(tcp_ctx *c, const double *w, double *hw, bool cleared = false) {
     int rc;
-    TCP_CUDA(cudaMemsetAsync(hw, 0, sizeof(double) * 3 * (size_t)c->n, c->stream));
+    if (!cleared) TCP_CUDA(cudaMemsetAsync(hw, 0, sizeof(double) * 3 * (size_t)c->n, c->stream));
+    if (c->p.reciprocal == TCP_RECIP_SPME) return launch_spme_hvp(c, w, hw, [&] { return launch_adj_pair(c, w, hw); });
     if ((rc = launch_adj_pair(c, w, hw))) return rc;
-    if (c->p.reciprocal == TCP_RECIP_SPME) return launch_spme_hvp(c, w, hw);
     if (c->p.reciprocal == TCP_RECIP_EWALD) return launch_ewald_hvp(c, w, hw);
     return TCP_OK;
 }
@@ -971,6 +967,8 @@ static RevArgs rev_args(tcp_ctx *c, const double *v, double dt, int K) {
     r.fb = c->adj_fb;
     r.g = c->adj_w;
     r.part = c->adj_part;
+    r.mean = c->adj_part + 3 * (size_t)part_blocks(c->n);
+    r.ticket = c->tickets + kTickRev;
     r.hw = c->adj_hw;
     r.nel = c->nel;
     r.n = c->n;
@@ -984,9 +982,8 @@ static RevArgs rev_args(tcp_ctx *c, const double *v, double dt, int K) {
 
 // g (adj_w) = P (fb + a vb) for a step k >= 1, P fb for k = 0
 static int rev_seed(tcp_ctx *c, const RevArgs &r, bool initial_only) {
-    const int nb = rev_blocks(c->n);
-    rev_seed_kernel<<<nb, kRevThreads, 0, c->stream>>>(r, initial_only);
-    rev_center_kernel<<<nb, kRevThreads, 0, c->stream>>>(r, nb);
+    rev_seed_kernel<<<part_blocks(c->n), kPartThreads, 0, c->stream>>>(r, initial_only);
+    rev_center_kernel<<<rev_blocks(3 * c->n), kRevThreads, 0, c->stream>>>(r);
     c->launches += 2;
     TCP_CUDA(cudaGetLastError());
     return TCP_OK;
@@ -1122,8 +1119,8 @@ int tcp_reverse_md(tcp_ctx *c, double dt, int nsteps, int every, double *J, doub
     TCP_CUDA(cudaMemsetAsync(c->adj_fb, 0, b, c->stream));
     for (int s = nck - 1; s >= 0; --s) {
         const int k0 = s * M, k1 = std::min(k0 + M, K);
-        if ((rc = copy_state(c, c->x, c->v, c->adj_ck + 2 * n3 * s, c->adj_ck + 2 * n3 * s + n3))) return rc;
-        if ((rc = launch_refresh_positions(c))) return rc;
+        if ((rc = copy_state(c, nullptr, c->v, nullptr, c->adj_ck + 2 * n3 * s + n3))) return rc;
+        if ((rc = launch_refresh_positions(c, c->adj_ck + 2 * n3 * s))) return rc;
         if ((rc = force_eval(c, true))) return rc;
         for (int k = k0 + 1; k <= k1; ++k) {
             if ((rc = md_advance(c, dt, 1))) return rc;
@@ -1132,19 +1129,17 @@ int tcp_reverse_md(tcp_ctx *c, double dt, int nsteps, int every, double *J, doub
         }
         for (int k = k1; k > k0; --k) {
             const double *xk = c->adj_seg + 2 * n3 * (k - k0), *vk = xk + n3;
-            if ((rc = copy_state(c, c->x, nullptr, xk, nullptr))) return rc;
-            if ((rc = launch_refresh_positions(c))) return rc;
+            if ((rc = launch_refresh_positions(c, xk))) return rc;
             const RevArgs r = rev_args(c, vk, dt, K);
             if ((rc = rev_seed(c, r, false))) return rc;
-            if ((rc = hvp_device(c, c->adj_w, c->adj_hw))) return rc;   // scal[kAdjDFdl] accumulates dJ/dlambda
-            rev_update_kernel<<<rev_blocks(c->n), kRevThreads, 0, c->stream>>>(r);
+            if ((rc = hvp_device(c, c->adj_w, c->adj_hw, true))) return rc;   // scal[kAdjDFdl] accumulates dJ/dlambda
+            rev_update_kernel<<<rev_blocks(3 * c->n), kRevThreads, 0, c->stream>>>(r);
             c->launches++;
             TCP_CUDA(cudaGetLastError());
         }
     }
     // f_0 = F(x_0; lambda): the lambda term only
-    if ((rc = copy_state(c, c->x, nullptr, c->adj_ck, nullptr))) return rc;
-    if ((rc = launch_refresh_positions(c))) return rc;
+    if ((rc = launch_refresh_positions(c, c->adj_ck))) return rc;
     {
         const RevArgs r = rev_args(c, c->v, dt, K);
         if ((rc = rev_seed(c, r, true))) return rc;

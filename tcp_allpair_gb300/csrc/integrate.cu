@@ -57,11 +57,6 @@ __device__ __forceinline__ void store_pos(const IntArgs &a, int i, double x0, do
 
 __device__ __forceinline__ double wrap(double x, double L, double iL) { return wrap_box(x, L, iL); }
 
-__global__ void refresh_kernel(const IntArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    store_pos(a, i, a.x[i], a.x[(size_t)a.n + i], a.x[2 * (size_t)a.n + i]);
-}
 
 // Finit's step back / forward, init.f90:171-185 and 223-237
 __global__ void shift_kernel(const IntArgs a, double sdt) {
@@ -79,6 +74,13 @@ __device__ __forceinline__ void store_comp(const IntArgs &a, int d, int i, doubl
     if (a.copies & kCopyXq) reinterpret_cast<int *>(a.xq + i)[d] = fixed_coord(x, iL);
     if (a.copies & kCopyXd) reinterpret_cast<double *>(a.xd + i)[d] = x;
     if (a.copies & kCopyXl) reinterpret_cast<long long *>(a.xl + i)[d] = fixed_coord64(x, iL);
+}
+
+__global__ void refresh_kernel(const IntArgs a, const double *__restrict__ x) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 3 * a.n) return;
+    const int d = t / a.n;
+    store_comp(a, d, t - d * a.n, x[t], d == 0 ? a.iL0 : (d == 1 ? a.iL1 : a.iL2));
 }
 
 // What the half kick of a step does besides: the accumulators of the pair
@@ -547,8 +549,8 @@ double *mv_part(tcp_ctx *c, int pass) { return c->red + 3 * (size_t)part_blocks(
 double *recip_epart(tcp_ctx *c) { return c->red + 7 * (size_t)part_blocks(c->n); }
 int red_capacity(int n, int extra) { return 7 * part_blocks(n) + extra; }
 
-int launch_refresh_positions(tcp_ctx *c) {
-    refresh_kernel<<<nblocks(c->n), kIntThreads, 0, c->stream>>>(int_args(c));
+int launch_refresh_positions(tcp_ctx *c, const double *x) {
+    refresh_kernel<<<nblocks(3 * c->n), kIntThreads, 0, c->stream>>>(int_args(c), x ? x : c->x);
     c->launches++;
     TCP_CUDA(cudaGetLastError());
     return TCP_OK;

@@ -6,6 +6,7 @@
 #include <cufft.h>
 #include <stdint.h>
 
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -356,7 +357,7 @@ double *mv_part(tcp_ctx *c, int pass);
 double *recip_epart(tcp_ctx *c);
 int red_capacity(int n, int extra);
 int part_blocks(int n);
-int launch_refresh_positions(tcp_ctx *c);
+int launch_refresh_positions(tcp_ctx *c, const double *x = nullptr);   // from x [3][n] (null: the positions as they are)
 int launch_shift(tcp_ctx *c, double sdt);
 int launch_vverlet1(tcp_ctx *c, double dt, bool prepare);   // prepare: also clear and bin for the forces of this step
 int launch_spme_sum(tcp_ctx *c);
@@ -404,8 +405,9 @@ ChainArgs spme_chain_args(tcp_ctx *c);                                 // spme.c
 int force_eval(tcp_ctx *c, bool remove_net);        // main.f90:100-141 on the stream
 int md_advance(tcp_ctx *c, double dt, int nsteps);  // nsteps MD steps (graph), no host sync
 int md_finish(tcp_ctx *c);                          // sync scalars, fill c->last
-// spme.cu: reciprocal Hessian-vector products, hw += H_rec w (w, hw SoA [3][n])
-int launch_spme_hvp(tcp_ctx *c, const double *w, double *hw);
+// spme.cu: reciprocal Hessian-vector products, hw += H_rec w (w, hw SoA [3][n]);
+// the SPME one queues the real-space part, real(), beside its mesh work
+int launch_spme_hvp(tcp_ctx *c, const double *w, double *hw, const std::function<int()> &real);
 int launch_ewald_hvp(tcp_ctx *c, const double *w, double *hw);
 void spme_hvp_free(tcp_ctx *c);
 // adjoint.cu
@@ -413,6 +415,6 @@ void adjoint_free(tcp_ctx *c);
 void adj_tables_free(tcp_ctx *c);
 
 // ctx->tickets
-enum { kTickStep = 0, kTickForce = 1, kTickKick = 2, kTickScale = 3, kTickBin = 4, kTickAdd = 5 };
+enum { kTickStep = 0, kTickForce = 1, kTickKick = 2, kTickScale = 3, kTickBin = 4, kTickAdd = 5, kTickRev = 6 };
 
 }  // namespace tcp
