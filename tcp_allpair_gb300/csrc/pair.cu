@@ -76,7 +76,7 @@ __device__ __forceinline__ void tile_range(const PairArgs &a, int t, int &j0, in
 // One j-tile for one i-particle (FP32).  KIND: 0 Coulomb erfc (e-e, i-i and
 // TCP_EI_COULOMB), 1 Deutsch e-i, 2 Kelbg e-i.  Accumulates sum_j w dx (the
 // force divided by eps q_i q_j) and sum_j u/r (energy / q_i q_j).
-// FULL: the tile holds kTjF particles (no tail test).  DIAG: the tile may
+// FULL: the tile holds a multiple of 32 particles (no tail test).  DIAG: the tile may
 // contain the i-particle itself (r^2 > 0 test).  CUBIC: all box lengths are
 // equal, so the fixed-point difference is used unscaled (lengths in units of
 // L/2^32) and the scale is folded into the constants and the per-tile factor
@@ -89,7 +89,8 @@ __device__ __forceinline__ void tile_f32(const int4 *__restrict__ tj, int cnt, i
                                          const PairConsts &c, float &px, float &py, float &pz,
                                          float &pe, unsigned *hist, float inv_dx, bool vi = true,
                                          const RdfEdges *E = nullptr, int pt = 0) {
-    const int cnt_up = FULL ? kTjF : (cnt + TPP - 1) / TPP * TPP;   // uniform trip count per warp
+    if (FULL) __builtin_assume(cnt > 0 && (cnt & 31) == 0);
+    const int cnt_up = FULL ? cnt : (cnt + TPP - 1) / TPP * TPP;   // uniform trip count per warp
     // constants in the units of this path
     const float rc2 = CUBIC ? c.u_rc2 : c.rc2f;
     const float p_alpha = CUBIC ? c.u_p_alpha : c.p_alpha;
@@ -185,7 +186,7 @@ __device__ __forceinline__ void tile_f32_any(const int4 *__restrict__ tj, int cn
     if (RDF) {
         tile_f32<KIND, ENERGY, RDF, TPP, false, true, CUBIC>(tj, cnt, sub, xi, c, px, py, pz, pe, hist, inv_dx, vi,
                                                               E, pt);
-    } else if (cnt == kTjF) {
+    } else if ((cnt & 31) == 0) {
         if (diag) tile_f32<KIND, ENERGY, false, TPP, true, true, CUBIC>(tj, cnt, sub, xi, c, px, py, pz, pe, hist, inv_dx);
         else tile_f32<KIND, ENERGY, false, TPP, true, false, CUBIC>(tj, cnt, sub, xi, c, px, py, pz, pe, hist, inv_dx);
     } else {
@@ -571,6 +572,10 @@ static Geometry geometry(const tcp_ctx *c, bool fp64) {
     g.tj = fp64 ? kTjD : kTjF;
     g.nblk_e = ceil_div(c->nel, g.bi);
     g.nblk = g.nblk_e + ceil_div(c->nion, g.bi);
+    // shorter tiles on small systems, so that the j-splits can fill the SMs:
+    // about 16 (i-block, tile) pairs per SM.  FP32C sums at N = 512, 1,024, 4,096:
+    // 20.6, 22, 36.9 us with tiles of 512, now 7.3, 12.4, 34.9
+    while (g.tj > 32 && (long)g.nblk * (ceil_div(c->nel, g.tj) + ceil_div(c->nion, g.tj)) < 16L * c->num_sms) g.tj /= 2;
     g.ntile_e = ceil_div(c->nel, g.tj);
     g.ntile = g.ntile_e + ceil_div(c->nion, g.tj);
     return g;
