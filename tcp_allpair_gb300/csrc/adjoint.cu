@@ -236,8 +236,8 @@ __global__ void __launch_bounds__(kAdjThreads) adj_pair_kernel(const AdjArgs a) 
 
 // ---- Newton-3 form -------------------------------------------------------------
 // The same sums over unique pairs (i < j), on the item schedule of the Newton-3
-// force kernels (pair_n3.cuh: i-tiles of kAdjN3Tile particles x j-subtiles of
-// kN3Sub, every item taken from an atomic counter).  A lane holds one
+// force kernels (pair_n3.cuh: i-tiles of kAdjN3Tile particles x j-units of
+// kN3Unit, every unit taken from an atomic counter).  A lane holds one
 // i-particle; the j position, w_j and the reaction (H w)_j rotate through the
 // warp with shuffles.  Per unique pair with t = qq (-G1 dw + G2 (u.dw) u):
 // (H w)_i += t, (H w)_j -= t; dE/dlambda += qq dl; dF/dlambda . w += qq gl (u.dw)
@@ -273,16 +273,16 @@ template <bool F32, int EIK, bool HVP>
 __global__ void __launch_bounds__(kAdjN3Threads) adj_n3_kernel(const AdjArgs a, const N3Geom g, long long total,
                                                                  unsigned *counter) {
     using T = typename std::conditional<F32, float, double>::type;
-    __shared__ int4 sxq[F32 ? kN3Sub : 1];
-    __shared__ longlong4_32a sxl[F32 ? 1 : kN3Sub];
-    __shared__ double sw[3][HVP ? kN3Sub : 1];
-    __shared__ double sh[HVP ? kN3Sub : 1][3];
+    __shared__ int4 sxq[F32 ? kN3Unit : 1];
+    __shared__ longlong4_32a sxl[F32 ? 1 : kN3Unit];
+    __shared__ double sw[3][HVP ? kN3Unit : 1];
+    __shared__ double sh[HVP ? kN3Unit : 1][3];
     __shared__ double red[32];
     __shared__ long long s_next;
     __shared__ F64Tab tab;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int src = (lane + 1) & 31;
-    for (int k = tid; k < (HVP ? kN3Sub : 1) * 3; k += kAdjN3Threads) (&sh[0][0])[k] = 0.0;
+    for (int k = tid; k < (HVP ? kN3Unit : 1) * 3; k += kAdjN3Threads) (&sh[0][0])[k] = 0.0;
     load_f64_tab(tab);     // ordered before first use by the item loop's barrier
 
     int curI = -1, istart = 0, iend = 0, isp = 0, ifirst = 0, ibase = 0;
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kAdjN3Threads) adj_n3_kernel(const AdjArgs a, 
                 for (int d = 0; d < 3; ++d) wi[d] = (T)a.w[(size_t)d * a.n + ir];
         }
         int jstart, cnt, jsp;
-        n3_sub(g, S, jstart, cnt, jsp);
+        n3_sub(g, S, 1, jstart, cnt, jsp);
         for (int k = tid; k < cnt; k += kAdjN3Threads) {
             if (F32) sxq[k] = a.xq[jstart + k];
             else sxl[k] = a.xl[jstart + k];
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(kAdjN3Threads) adj_n3_kernel(const AdjArgs a, 
                 for (int d = 0; d < 3; ++d) sw[d][k] = a.w[(size_t)d * a.n + jstart + k];
         }
         __syncthreads();
-        const bool masked = (S < ifirst + kAdjN3Tile / kN3Sub && jsp == isp) || cnt < kN3Sub || (iend - istart) < kAdjN3Tile;
+        const bool masked = (S < ifirst + kAdjN3Tile / kN3Unit && jsp == isp) || cnt < kN3Unit || (iend - istart) < kAdjN3Tile;
         const int type = isp + jsp;
         const T qq = F32 ? (T)(a.c.qqf[type] * (float)kEps) : (T)(a.c.qq[type] * kEps);
         T ti0 = 0, ti1 = 0, ti2 = 0, te = 0, tf = 0;   // per-item partials (FP32 in FP32C mode)

@@ -4,19 +4,20 @@
 // triangular loops also evaluate each pair once).
 //
 // Work: particles are split per species into i-tiles of TILE = 32 R W
-// particles (W warps, R i-particles per lane) and j-subtiles of kN3Sub = 128
-// (tiles never straddle the e/i boundary).  An item is (i-tile I, j-subtile
-// S) with S at or after I's first subtile; items are enumerated row by row.
-// A persistent grid claims chunks of consecutive items from an atomic
-// counter, the chunks shorter towards the end of the list (guided
-// self-scheduling): the i-tile stays in registers along the long early
-// chunks, and the single items at the end absorb the cost differences
-// between items (pair types, masked items).
+// particles (W warps, R i-particles per lane) and j-units of 32 (neither
+// straddles the e/i boundary).  A unit of work is (i-tile I, j-unit S) with S at
+// or after I's first unit; units are enumerated row by row.  A persistent grid
+// claims chunks of consecutive units from an atomic counter, the chunks shorter
+// towards the end of the list (guided self-scheduling), and works on up to four
+// units of a row, 128 j-particles, at a time (an item): the i-tile stays in
+// registers along the long early chunks, and the single units at the end absorb
+// the cost differences between items (pair types, masked items).  Pair sums
+// with units of 128 and three items claimed ahead: N = 4,096 45 us, 9,000 94,
+// 16,384 202, 65,536 2,433; with these 33, 85, 191 and 2,373.
 //
-// A lane holds R i-particles (R i-chunks of 32 per warp).  A j-subtile is
-// copied into shared memory by the bulk-copy engine (cp.async.bulk +
-// mbarrier, kN3Stages-deep ring, issued three items ahead).  Each
-// warp takes the subtile in chunks of 32: lane l loads j = l, and for 32
+// A lane holds R i-particles (R i-chunks of 32 per warp).  An item's j-particles
+// are copied into shared memory by the bulk-copy engine (cp.async.bulk +
+// mbarrier, one item ahead).  Each warp takes them in chunks of 32: lane l loads j = l, and for 32
 // steps computes the R pairs (i_r, j) and rotates j's position and reaction
 // accumulator to the next lane with shuffles, so after 32 steps every lane
 // holds the reaction of its own j again (the LDSJ variants read j's position
@@ -446,18 +447,18 @@ __global__ void __launch_bounds__(32 * W, MINB) pair_n3_kernel(const N3Args a) {
     static_assert(W >= 1, "at least one warp per CTA");
     static_assert(!RDF || (MODE >= 1 && !BATCH), "RDF histograms: packed single-system forms");
     static_assert(PD == kErfcH6 || MODE >= 1, "the degree-5 erfc exists in the packed forms");
-    static_assert((32 * R * W) % kN3Sub == 0, "i-tiles hold whole j-subtiles");
+    static_assert((32 * R * W) % kN3Unit == 0, "i-tiles hold whole j-units");
     constexpr int NT = 32 * W;
     constexpr bool X2 = MODE >= 1;
     constexpr bool SACC = MODE >= 1;
     constexpr int TILE = 32 * R * W;
-    constexpr int SPT = TILE / kN3Sub;
+    constexpr int SPT = TILE / kN3Unit;
     __shared__ __align__(128) int4 tiles[kN3Stages][kN3Sub];
     __shared__ __align__(8) uint64_t bars[kN3Stages];
     __shared__ float sjacc[kN3Sub][3];
     __shared__ double red[32];
     // the item of each ring slot, decoded once by thread 0 (s_I < 0: no item)
-    __shared__ int s_rep[kN3Stages], s_I[kN3Stages], s_S[kN3Stages];
+    __shared__ int s_rep[kN3Stages], s_I[kN3Stages], s_S[kN3Stages], s_run[kN3Stages];
     __shared__ unsigned hist[RDF ? kRdfSpare + 32 : 1];
     // per-thread TwoSum (hi, lo) i-force accumulators, touched once per item:
     // in shared memory ([slot][thread], conflict-free) for the packed forms,
@@ -476,12 +477,15 @@ __global__ void __launch_bounds__(32 * W, MINB) pair_n3_kernel(const N3Args a) {
     }
     __syncthreads();
 
-    // Guided self-scheduling: thread 0 claims chunks of consecutive items
+    // Guided self-scheduling: thread 0 claims chunks of consecutive units
     // (a.chunks, shorter towards the end of the list) from the counter, so the
     // CTAs end together whatever their items cost, and the i-tile stays in
     // registers along the long early chunks.  It decodes each item once,
-    // publishes it in the ring slot of its subtile copy and issues the copy
-    // kN3Stages items ahead of the one being processed.
+    // publishes it in the ring slot of its j-particles and issues their copy
+    // while the item before is processed.  Only one item is claimed ahead:
+    // with three, a CTA held three of the last ones back while others idled,
+    // and on mid-size systems (N = 16,384: 3.4 items of 128 x 128 a CTA) nothing
+    // was left to balance.
     long long cur = 0, cend = 0;   // thread 0: the rest of the current chunk
     bool drained = false;          // thread 0: the chunk list is exhausted
     int last_filled = -1;          // thread 0: ring index of the last item with a copy
@@ -501,21 +505,23 @@ __global__ void __launch_bounds__(32 * W, MINB) pair_n3_kernel(const N3Args a) {
             return;
         }
         int rep, I_, S_;
-        n3_locate<TILE, BATCH>(a, cur++, rep, I_, S_);
+        n3_locate<TILE, BATCH>(a, cur, rep, I_, S_);
+        const N3Geom &g = n3_geom<BATCH>(a, rep);
+        const int run = n3_run(g, S_, cend - cur);
+        cur += run;
         s_rep[stage] = rep;
         s_I[stage] = I_;
         s_S[stage] = S_;
+        s_run[stage] = run;
         last_filled = k;
         if (a.inject_skip && blockIdx.x == 0 && k == 0) return;   // test hook: the copy never comes
-        const N3Geom &g = n3_geom<BATCH>(a, rep);
         int js, jc, jsp;
-        n3_sub(g, S_, js, jc, jsp);
+        n3_sub(g, S_, run, js, jc, jsp);
         const uint32_t bytes = (uint32_t)jc * sizeof(int4);
         mbar_arrive_expect_tx(&bars[stage], bytes);
         bulk_g2s(tiles[stage], a.xq + g.off + js, bytes, &bars[stage]);
     };
-    if (tid == 0)
-        for (int k = 0; k < kN3Stages; ++k) fill(k);
+    if (tid == 0) fill(0);
 
     double etot = 0.0;
     int curRep = -1, curI = -1, istart = 0, iend = 0, isp = 0, ifirst = 0, ioff = 0;
@@ -560,9 +566,9 @@ __global__ void __launch_bounds__(32 * W, MINB) pair_n3_kernel(const N3Args a) {
         eh = el = 0.f;
     };
 
-    // process the item (replica rep, row I_, subtile S_) of ring index k;
+    // process the item (replica rep, row I_, j-units S_ ..) of ring index k;
     // false on timeout
-    auto process = [&](int k, int rep, int I_, int S_) -> bool {
+    auto process = [&](int k, int rep, int I_, int S_, int run) -> bool {
         const N3Geom &g = n3_geom<BATCH>(a, rep);
         if (I_ != curI || rep != curRep) {
             flush_i();
@@ -578,9 +584,9 @@ __global__ void __launch_bounds__(32 * W, MINB) pair_n3_kernel(const N3Args a) {
             }
         }
         int jstart, cnt, jsp;
-        n3_sub(g, S_, jstart, cnt, jsp);
+        n3_sub(g, S_, run, jstart, cnt, jsp);
         const int pt = isp + jsp;
-        const bool masked = (S_ < ifirst + SPT && jsp == isp) || cnt < kN3Sub || (iend - istart) < TILE;
+        const bool masked = (S_ < ifirst + SPT && jsp == isp) || (cnt & 31) || (iend - istart) < TILE;
         const int stage = k % kN3Stages;
         const bool ok = mbar_wait_bounded(&bars[stage], (uint32_t)((k / kN3Stages) & 1), kWaitLimitCycles);
         const PairConsts &c = n3_consts<BATCH>(a, rep);
@@ -624,26 +630,15 @@ __global__ void __launch_bounds__(32 * W, MINB) pair_n3_kernel(const N3Args a) {
         if (ENERGY) acc2(eh, el, pe * c.u_qq_energy[pt]);
         // all warps are done with this subtile and its reaction sums
         const bool timeout = __syncthreads_or(!ok);
-        if constexpr (NT >= kN3Sub) {
-            if (!timeout && tid < cnt) {
+        for (int t = tid; t < cnt; t += NT) {
+            if (!timeout) {
                 const double sc = -kEps * (double)qf;
-                const size_t j = (size_t)ioff + jstart + tid;
-                atomicAdd(&a.facc[j], sc * (double)sjacc[tid][0]);
-                atomicAdd(&a.facc[(size_t)a.ntot + j], sc * (double)sjacc[tid][1]);
-                atomicAdd(&a.facc[2 * (size_t)a.ntot + j], sc * (double)sjacc[tid][2]);
+                const size_t j = (size_t)ioff + jstart + t;
+                atomicAdd(&a.facc[j], sc * (double)sjacc[t][0]);
+                atomicAdd(&a.facc[(size_t)a.ntot + j], sc * (double)sjacc[t][1]);
+                atomicAdd(&a.facc[2 * (size_t)a.ntot + j], sc * (double)sjacc[t][2]);
             }
-            if (tid < kN3Sub) sjacc[tid][0] = sjacc[tid][1] = sjacc[tid][2] = 0.f;
-        } else {   // fewer threads than subtile particles: each flushes several
-            for (int t = tid; t < kN3Sub; t += NT) {
-                if (!timeout && t < cnt) {
-                    const double sc = -kEps * (double)qf;
-                    const size_t j = (size_t)ioff + jstart + t;
-                    atomicAdd(&a.facc[j], sc * (double)sjacc[t][0]);
-                    atomicAdd(&a.facc[(size_t)a.ntot + j], sc * (double)sjacc[t][1]);
-                    atomicAdd(&a.facc[2 * (size_t)a.ntot + j], sc * (double)sjacc[t][2]);
-                }
-                sjacc[t][0] = sjacc[t][1] = sjacc[t][2] = 0.f;
-            }
+            sjacc[t][0] = sjacc[t][1] = sjacc[t][2] = 0.f;
         }
         return !timeout;
     };
@@ -655,11 +650,11 @@ __global__ void __launch_bounds__(32 * W, MINB) pair_n3_kernel(const N3Args a) {
         const int stage = k % kN3Stages;
         const int I_ = s_I[stage];
         if (I_ < 0) break;
-        if (!process(k, s_rep[stage], I_, s_S[stage])) {   // ends with a CTA barrier
+        if (tid == 0) fill(k + 1);                         // its slot was item k - 1's
+        if (!process(k, s_rep[stage], I_, s_S[stage], s_run[stage])) {   // ends with a CTA barrier
             good = false;
             break;
         }
-        if (tid == 0) fill(k + kN3Stages);
         __syncthreads();
     }
     if (!good) {
@@ -787,14 +782,14 @@ int n3_grid(const tcp_ctx *c) {
 // Tile geometry of a system of nel + nion particles for i-tiles of `tile`.
 N3Geom n3_geometry(int off, int nel, int nion, int tile, long long item0, long long *items) {
     N3Geom g;
-    const int spt = tile / kN3Sub;
+    const int spt = tile / kN3Unit;
     g.off = off;
     g.nel = nel;
     g.n = nel + nion;
     g.nIe = cdiv(nel, tile);
     g.nI = g.nIe + cdiv(nion, tile);
-    g.nSe = cdiv(nel, kN3Sub);
-    g.nS = g.nSe + cdiv(nion, kN3Sub);
+    g.nSe = cdiv(nel, kN3Unit);
+    g.nS = g.nSe + cdiv(nion, kN3Unit);
     g.item0 = item0;
     long long total = 0;
     for (int I = 0; I < g.nI; ++I) total += g.nS - (I < g.nIe ? I * spt : g.nSe + (I - g.nIe) * spt);

@@ -2,10 +2,11 @@
 // kernels (pair_n3.cu) and the derivative kernels (adjoint.cu), and the
 // arguments they share with the FP64 kernel (pair_n3_f64.cu).
 //
-// Particles are split per species into i-tiles of TILE particles and
-// j-subtiles of kN3Sub (tiles never straddle the e/i boundary).  An item is
-// (i-tile I, j-subtile S) with S at or after I's first subtile; items are
-// enumerated row by row, system by system for a batch.
+// Particles are split per species into i-tiles of TILE particles and j-units
+// of kN3Unit (neither straddles the e/i boundary).  A unit of work is (i-tile I,
+// j-unit S) with S at or after I's first unit; they are enumerated row by row,
+// system by system for a batch.  The pair kernels take up to kN3Sub / kN3Unit
+// consecutive ones of a row and species as one item.
 #pragma once
 
 #include "pair_math.cuh"
@@ -15,16 +16,17 @@ namespace tcp {
 
 constexpr int kN3Warps = 8;
 constexpr int kN3Threads = 32 * kN3Warps;
-constexpr int kN3Sub = 128;                // j-subtile
-constexpr int kN3Stages = 3;
+constexpr int kN3Unit = 32;                // j-particles of a unit of work
+constexpr int kN3Sub = 128;                // most j-particles of an item
+constexpr int kN3Stages = 2;               // items copied ahead, and the one in work
 
 // Tile geometry of one system (a replica of a batch, or the only system).
 struct N3Geom {
     int off;              // first particle in the global arrays
     int nel, n;           // electrons, particles
     int nIe, nI;          // i-tiles, electron tiles first
-    int nSe, nS;          // j-subtiles, electron subtiles first
-    long long item0;      // first item of this system in the global item list
+    int nSe, nS;          // j-units, electron units first
+    long long item0;      // first unit of work of this system in the global list
 };
 
 struct N3Rep {
@@ -56,7 +58,7 @@ struct N3Args {
 
 template <int TILE>
 __device__ __forceinline__ void n3_itile(const N3Geom &a, int I, int &start, int &end, int &sp, int &first) {
-    constexpr int SPT = TILE / kN3Sub;
+    constexpr int SPT = TILE / kN3Unit;
     if (I < a.nIe) {
         sp = 0;
         start = I * TILE;
@@ -70,19 +72,26 @@ __device__ __forceinline__ void n3_itile(const N3Geom &a, int I, int &start, int
     }
 }
 
-__device__ __forceinline__ void n3_sub(const N3Geom &a, int S, int &start, int &cnt, int &sp) {
+// the j-particles of the units S .. S + run - 1 (of one species)
+__device__ __forceinline__ void n3_sub(const N3Geom &a, int S, int run, int &start, int &cnt, int &sp) {
     if (S < a.nSe) {
         sp = 0;
-        start = S * kN3Sub;
-        cnt = min(kN3Sub, a.nel - start);
+        start = S * kN3Unit;
+        cnt = min(run * kN3Unit, a.nel - start);
     } else {
         sp = 1;
-        start = a.nel + (S - a.nSe) * kN3Sub;
-        cnt = min(kN3Sub, a.n - start);
+        start = a.nel + (S - a.nSe) * kN3Unit;
+        cnt = min(run * kN3Unit, a.n - start);
     }
 }
 
-// local item index of one system -> (row I, subtile S), in closed form.
+// how many of up to `most` units from S on belong to S's row and species
+__device__ __forceinline__ int n3_run(const N3Geom &a, int S, long long most) {
+    const int end = S < a.nSe ? a.nSe : a.nS;
+    return (int)min((long long)min(kN3Sub / kN3Unit, end - S), most);
+}
+
+// local unit index of one system -> (row I, unit S), in closed form.
 // Electron row k (k < nIe) holds nS - k SPT items and starts at item
 // k nS - SPT k (k - 1) / 2; ion row nIe + k holds n0 - k SPT items
 // (n0 = nS - nSe) and starts at E + k n0 - SPT k (k - 1) / 2, E the items of
@@ -91,7 +100,7 @@ __device__ __forceinline__ void n3_sub(const N3Geom &a, int S, int &start, int &
 // S = nS.
 template <int TILE>
 __device__ __forceinline__ void n3_decode(const N3Geom &a, long long it, int &I, int &S) {
-    constexpr int SPT = TILE / kN3Sub;
+    constexpr int SPT = TILE / kN3Unit;
     const long long E = (long long)a.nIe * a.nS - (long long)SPT * a.nIe * (a.nIe - 1) / 2;
     const bool ion = it >= E;
     const long long x = ion ? it - E : it;
@@ -112,7 +121,7 @@ __device__ __forceinline__ void n3_decode(const N3Geom &a, long long it, int &I,
     S = (ion ? a.nSe : 0) + k * SPT + (int)(x - start(k));
 }
 
-// global item -> replica (0 for a single system), row and subtile
+// global unit -> replica (0 for a single system), row and j-unit
 template <int TILE, bool BATCH>
 __device__ __forceinline__ void n3_locate(const N3Args &a, long long it, int &rep, int &I, int &S) {
     rep = 0;
@@ -142,9 +151,9 @@ __device__ __forceinline__ const PairConsts &n3_consts(const N3Args &a, int rep)
 // Tile geometry of a system of nel + nion particles for i-tiles of `tile`.
 N3Geom n3_geometry(int off, int nel, int nion, int tile, long long item0, long long *items);
 
-// Chunk boundaries of guided self-scheduling over `total` items for up to
-// `ctas` CTAs: chunk sizes ceil(rest / (2 ctas)), at least one item, so the
-// first chunks are long runs of one row and the last ones single items.
+// Chunk boundaries of guided self-scheduling over `total` units for up to
+// `ctas` CTAs: chunk sizes ceil(rest / (2 ctas)), at least one unit, so the
+// first chunks are long runs of one row and the last ones single units.
 void n3_chunk_table(long long total, int ctas, std::vector<long long> &starts);
 
 }  // namespace tcp
