@@ -199,24 +199,33 @@ __device__ __forceinline__ float2 erfc_poly2(float2 t) {
 }
 
 // RDF: +2 per unique pair inside rc in bin INT(r/dx) <= kNdist of this pair
-// type (the ordered-pair kernels add 1 from each side), in a CTA histogram.
-// Branch-free on the common path: a pair that does not count adds to its
-// lane's spare slot (kRdfSpare + lane, never flushed), so every lane issues
-// the same atomic (a predicated atomic, skipping the ~half of the pairs past
-// rc = L/2, made the RDF step 10 % slower).  Measured at N = 65,536: the
-// binning with its atomics costs 0.5 ms of a 2.6 ms step, the exact test of
-// the pairs near a bin edge (taken in ~2 % of the steps) 2.6 ms when inlined
-// behind a per-lane branch, 1.7 ms behind a warp vote, 1.1 ms out of line.  Pairs whose FP32 r/dx or r^2 lies
-// near a bin edge or rc take the exact test of the fixed-point separation
-// (rdf_exact_bin), so the counts equal those of exact arithmetic on the
-// fixed-point positions.
-constexpr int kRdfSpare = 3 * kNbin;
+// type (the ordered-pair kernels add 1 from each side), counted in a CTA
+// histogram and doubled when it is flushed.
+//
+// The bin is read from the mantissa: r/dx + 1536, rounded down, has 13 fraction
+// bits (r/dx < 512 here), so that bits 13.. of the float are the bin and the
+// low 13 bits the distance from its lower edge in 1/8192.  An offset of two
+// such units, kRdfEdge, puts the pairs within kRdfEdge of an edge where the low
+// bits are 0 .. 3.  rc (or bin kNbin where that is nearer) is a threshold on
+// the same integer.  Pairs near an edge or near that threshold take the exact
+// test of the fixed-point separation (rdf_exact_bin), so the counts equal
+// those of exact arithmetic on the fixed-point positions.
+//
+// What bounds it: issue slots.  With separate floor, fraction, r^2 and bin
+// tests, and a warp vote and a call for the exact test in every step, a pair
+// took 59 issued instructions against 31 without the binning, and waits for
+// instructions and branches; this form takes 45: 754 -> 516 us at N = 24,001,
+// 4,100 -> 3,406 at 65,536.
+constexpr float kRdfBase = 1536.0f + kRdfEdge;
+constexpr int kRdfFrac = 13, kRdfNear = 0x1ffc;    // low bits 0 .. 3: near an edge
+constexpr int kRdfBin0 = 0x44c00000 >> kRdfFrac;   // the bits of 1536
 struct N3Rdf {
-    unsigned *hist;
-    int hoff;                  // pair type * kNbin
+    unsigned *hist;            // of this pair type
+    unsigned base;             // its address in shared memory less that of code 0
+    int spare;                 // code of the lane's spare slot, not near an edge
     int pt;                    // pair type
     float inv_dx;              // u / dx of this pair type
-    float rc2;                 // cut-off^2 in u^2
+    int lo, hi;                // PairConsts::u_rdf_lo, u_rdf_hi
     const RdfEdges *E;
 };
 
@@ -224,80 +233,91 @@ __device__ __forceinline__ int idiff_i(int a, int b) { return (int)((unsigned)a 
 
 // The exact bin test of one pair, out of line: inlined, its 64-bit integer
 // arithmetic and table loops weighed on the register allocation and
-// scheduling of every rotation step although a step takes it rarely.  bin:
-// the FP32 estimate, or -1 when the pair lies past rc in FP32 (the estimate is
-// then taken from r2).  Returns bin << 1 | (r < rc exactly).
-__device__ __noinline__ int rdf_exact_call(int d0, int d1, int d2, const RdfEdges *E, int t, int bin, float r2,
-                                           float inv_dx) {
-    if (bin < 0) bin = (int)(sqrtf(r2) * inv_dx);
+// scheduling of every rotation step although a step takes it rarely.  The
+// code, computed as in the step, says where the step counted the pair.
+__device__ __noinline__ void rdf_exact_add(int d0, int d1, int d2, const N3Rdf h) {
+    const float x = (float)d0, y = (float)d1, z = (float)d2;
+    const float r2 = __fmaf_rn(x, x, __fmaf_rn(y, y, __fmul_rn(z, z)));
+    const int code = __float_as_int(__fmaf_rz(__fmul_rn(r2, rsqrt_approx(r2)), h.inv_dx, kRdfBase));
     bool ok;
-    bin = rdf_exact_bin<true>(d0, d1, d2, E, t, nullptr, bin, ok);
-    return (bin << 1) | (ok ? 1 : 0);
+    const int bin = rdf_exact_bin<true>(d0, d1, d2, h.E, h.pt, nullptr, (code >> kRdfFrac) - kRdfBin0, ok);
+    if (code < h.lo) atomicSub(&h.hist[(code >> kRdfFrac) - kRdfBin0], 1u);
+    if (ok && bin <= kNdist) atomicAdd(&h.hist[bin], 1u);
 }
 
-// The bins of the two pairs of a packed step.  r: FP32 distances (meaningless
-// where the caller replaced r^2 by 1); r2: the pairs' FP32 r^2; ok: the FP32
-// cut-off and index masks; v: the index masks.  floor(r/dx) comes from packed
-// FP32 arithmetic without a float->int conversion: (tb - 1/2) + 1.5 2^23
-// rounds tb - 1/2 to an integer held in the low mantissa bits, which is
-// floor(tb) unless tb lies within rounding of an integer; there, and within
-// 2^-12 of any bin edge or of rc, the exact test of the fixed-point separation
-// decides (two conversions per pair on the slow pipe had cost more than the
-// pair's own arithmetic).
-constexpr float kRdfRound = 12582912.0f;   // 1.5 * 2^23
-constexpr int kRdfRoundBits = 0x4B400000;  // the bit pattern of kRdfRound
-template <bool RDF>
-__device__ __forceinline__ void rdf_add2(const N3Rdf &h, float2 r, float2 r2, bool ok0, bool ok1, bool v0, bool v1,
-                                         const int4 &xa, const int4 &xb, const int4 &xj) {
-    if (RDF) {
-        const float2 tb = __fmul2_rn(r, make_float2(h.inv_dx, h.inv_dx));
-        const float2 m = __fadd2_rn(__fadd2_rn(tb, make_float2(-0.5f, -0.5f)), make_float2(kRdfRound, kRdfRound));
-        const float2 binf = __fadd2_rn(m, make_float2(-kRdfRound, -kRdfRound));
-        const float2 fr = __ffma2_rn(binf, make_float2(-1.0f, -1.0f), tb);   // tb - floor estimate, exact
-        int bin0 = __float_as_int(m.x) - kRdfRoundBits, bin1 = __float_as_int(m.y) - kRdfRoundBits;
-        // the exact test where the estimate may be wrong: a bin edge within
-        // 2^-12 of a pair inside rc, or rc itself within 2^-12; a pair clearly
-        // past rc counts nothing whatever its bin
-        // (one warp vote per step: a per-lane branch in every rotation step,
-        // rarely taken, had cost as much as the pair arithmetic by breaking
-        // the step's straight-line code)
-        const float nrc = kRdfEdge * h.rc2;
-        const bool x0 = v0 && (fabsf(r2.x - h.rc2) < nrc || (ok0 && fabsf(fr.x - 0.5f) > 0.5f - kRdfEdge));
-        const bool x1 = v1 && (fabsf(r2.y - h.rc2) < nrc || (ok1 && fabsf(fr.y - 0.5f) > 0.5f - kRdfEdge));
-        if (__any_sync(0xffffffffu, x0 || x1)) {
-            if (x0) {
-                const int pk = rdf_exact_call(idiff_i(xa.x, xj.x), idiff_i(xa.y, xj.y), idiff_i(xa.z, xj.z), h.E,
-                                              h.pt, ok0 ? bin0 : -1, r2.x, h.inv_dx);
-                bin0 = pk >> 1;
-                ok0 = (pk & 1) != 0;
-            }
-            if (x1) {
-                const int pk = rdf_exact_call(idiff_i(xb.x, xj.x), idiff_i(xb.y, xj.y), idiff_i(xb.z, xj.z), h.E,
-                                              h.pt, ok1 ? bin1 : -1, r2.y, h.inv_dx);
-                bin1 = pk >> 1;
-                ok1 = (pk & 1) != 0;
-            }
+// The codes of two pairs from their FP32 distances; v: the index masks of a
+// MASKED step.
+template <bool MASKED>
+__device__ __forceinline__ void rdf_codes(const N3Rdf &h, float2 r, bool v0, bool v1, int &c0, int &c1) {
+    const float2 m = __ffma2_rz(r, f2(h.inv_dx), f2(kRdfBase));
+    c0 = __float_as_int(m.x);
+    c1 = __float_as_int(m.y);
+    if (MASKED) {
+        c0 = v0 ? c0 : 0x7fffffff;
+        c1 = v1 ? c1 : 0x7fffffff;
+    }
+}
+
+// Counts the R pairs of a rotation step and marks those that need the exact
+// test in `bit` of near[r]; they are counted after the 32 steps of a chunk
+// (rdf_near_pairs).  Straight-line code, 9 instructions a pair: a pair that
+// does not count adds to its lane's spare slot, as a branch around each atomic
+// cost 10 % of the pair sum, and in C++ the compiler made branches of the tests.
+template <int R>
+__device__ __forceinline__ void rdf_add(const N3Rdf &h, const int (&code)[R], unsigned bit, unsigned (&near)[R]) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        asm volatile(
+            "{\n\t"
+            ".reg .pred in, nr, hi;\n\t"
+            ".reg .b32 at, lo;\n\t"
+            "setp.lt.s32 in, %1, %2;\n\t"
+            "selp.b32 at, %1, %4, in;\n\t"
+            "setp.lt.and.s32 hi, %1, %3, !in;\n\t"
+            "and.b32 lo, at, %7;\n\t"
+            "setp.eq.or.b32 nr, lo, 0, hi;\n\t"
+            "@nr or.b32 %0, %0, %5;\n\t"
+            "shr.u32 at, at, %8;\n\t"
+            "mad.lo.u32 at, at, 4, %6;\n\t"
+            "red.shared.add.u32 [at], 1;\n\t"
+            "}"
+            : "+r"(near[r])
+            : "r"(code[r]), "r"(h.lo), "r"(h.hi), "r"(h.spare), "r"(bit), "r"(h.base), "n"(kRdfNear), "n"(kRdfFrac));
+}
+
+// The exact tests of the pairs marked during the 32 steps of a chunk: at step
+// s lane l met the chunk's j-particle (l + s) mod 32.
+template <int R>
+__device__ __forceinline__ void rdf_near_pairs(const N3Rdf &h, unsigned (&near)[R], const int4 (&xi)[R],
+                                               const int4 *__restrict__ tj) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        while (near[r]) {
+            const int s = __ffs(near[r]) - 1;
+            near[r] &= near[r] - 1;
+            const int4 xj = tj[(lane + s) & 31];
+            rdf_exact_add(idiff_i(xi[r].x, xj.x), idiff_i(xi[r].y, xj.y), idiff_i(xi[r].z, xj.z), h);
         }
-        const int spare = kRdfSpare + (int)(threadIdx.x & 31);
-        atomicAdd(&h.hist[(ok0 && bin0 <= kNdist) ? h.hoff + bin0 : spare], 2u);
-        atomicAdd(&h.hist[(ok1 && bin1 <= kNdist) ? h.hoff + bin1 : spare], 2u);
     }
 }
 
 // PD: degree of the Ewald erfc polynomial (kErfcH6, or kErfcH5 when
 // alpha rc <= kErfc5Xmax); the Kelbg erfc(r/lambda) always uses kErfcH6.
-// RDF: h, the index masks v0, v1 and the positions xa, xb (i-particles) and
-// xj of the two pairs.
+// RDF: h and the index masks v0, v1 give the codes c0, c1 of the two pairs.
 template <int KIND, bool ENERGY, bool MASKED, bool RDF = false, int PD = kErfcH6>
 __device__ __forceinline__ float2 n3_pair_x2(const PairConsts &c, float2 r2, bool ok0, bool ok1, bool near_any,
                                              float2 &pe, const N3Rdf *h = nullptr, bool v0 = true, bool v1 = true,
-                                             const int4 *xa = nullptr, const int4 *xb = nullptr,
-                                             const int4 *xj = nullptr) {
+                                             int *c0 = nullptr, int *c1 = nullptr) {
     const float2 r2s = MASKED ? make_float2(ok0 ? r2.x : 1.0f, ok1 ? r2.y : 1.0f) : r2;
     const float2 rinv = make_float2(rsqrt_approx(r2s.x), rsqrt_approx(r2s.y));
     const float2 rinv_m = make_float2(ok0 ? rinv.x : 0.0f, ok1 ? rinv.y : 0.0f);
     const float2 r = __fmul2_rn(r2s, rinv);
-    if (RDF) rdf_add2<RDF>(*h, r, r2, ok0, ok1, v0, v1, *xa, *xb, *xj);
+    if (RDF) {
+        // where MASKED replaced the r^2 of a pair past rc, its own distance
+        const float2 rt = MASKED ? __fmul2_rn(r2, make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y))) : r;
+        rdf_codes<MASKED>(*h, rt, v0, v1, *c0, *c1);
+    }
     const float2 ta = __ffma2_rn(f2(PD == kErfcH6 ? c.u_p_alpha : c.u_p_alpha5), r, f2(1.0f));
     const float2 t = make_float2(rcp_approx(ta.x), rcp_approx(ta.y));
     const float2 ea = __fmul2_rn(f2(c.u_c_exp), r2s);
@@ -371,11 +391,13 @@ __device__ __forceinline__ void n3_item_x2(const PairConsts &c, const int4 *__re
             __syncwarp();
         }
         float2 jx = f2(0.0f), jy = f2(0.0f), jz = f2(0.0f);
+        unsigned near[RDF ? R : 1] = {};
 #pragma unroll UNROLL
         for (int s = 0; s < 32; ++s) {
             if (LDSJ) xj = jb[lane + s];
             float2 d[G][3], r2[G];
             bool ok[R], valid[R];
+            int code[R];
             float r2min = 3.0e38f;
 #pragma unroll
             for (int g = 0; g < G; ++g) {
@@ -399,8 +421,8 @@ __device__ __forceinline__ void n3_item_x2(const PairConsts &c, const int4 *__re
 #pragma unroll
             for (int g = 0; g < G; ++g) {
                 const float2 w = n3_pair_x2<KIND, ENERGY, MASKED, RDF, PD>(
-                    c, r2[g], ok[2 * g], ok[2 * g + 1], near_any, pe2, rh, valid[2 * g], valid[2 * g + 1], &xi[2 * g],
-                    &xi[2 * g + 1], &xj);
+                    c, r2[g], ok[2 * g], ok[2 * g + 1], near_any, pe2, rh, valid[2 * g], valid[2 * g + 1],
+                    &code[2 * g], &code[2 * g + 1]);
                 pg[g][0] = __ffma2_rn(w, d[g][0], pg[g][0]);
                 pg[g][1] = __ffma2_rn(w, d[g][1], pg[g][1]);
                 pg[g][2] = __ffma2_rn(w, d[g][2], pg[g][2]);
@@ -408,6 +430,7 @@ __device__ __forceinline__ void n3_item_x2(const PairConsts &c, const int4 *__re
                 jy = __ffma2_rn(w, d[g][1], jy);
                 jz = __ffma2_rn(w, d[g][2], jz);
             }
+            if constexpr (RDF) rdf_add<R>(*rh, code, 1u << s, near);
             // rotate j (position and both halves of the reaction) to the next lane
             if (!LDSJ) {
                 xj.x = __shfl_sync(0xffffffffu, xj.x, src);
@@ -421,6 +444,7 @@ __device__ __forceinline__ void n3_item_x2(const PairConsts &c, const int4 *__re
             jz.x = __shfl_sync(0xffffffffu, jz.x, src);
             jz.y = __shfl_sync(0xffffffffu, jz.y, src);
         }
+        if constexpr (RDF) rdf_near_pairs<R>(*rh, near, xi, tj + ch * 32);
         float *q = sjacc[ch * 32 + lane];
         atomicAdd(q + 0, jx.x + jx.y);
         atomicAdd(q + 1, jy.x + jy.y);
@@ -459,7 +483,7 @@ __global__ void __launch_bounds__(32 * W, MINB) pair_n3_kernel(const N3Args a) {
     __shared__ double red[32];
     // the item of each ring slot, decoded once by thread 0 (s_I < 0: no item)
     __shared__ int s_rep[kN3Stages], s_I[kN3Stages], s_S[kN3Stages], s_run[kN3Stages];
-    __shared__ unsigned hist[RDF ? kRdfSpare + 32 : 1];
+    __shared__ unsigned hist[RDF ? 3 * kNbin + 32 : 1];
     // per-thread TwoSum (hi, lo) i-force accumulators, touched once per item:
     // in shared memory ([slot][thread], conflict-free) for the packed forms,
     // whose constant pairs need the registers
@@ -470,7 +494,7 @@ __global__ void __launch_bounds__(32 * W, MINB) pair_n3_kernel(const N3Args a) {
 
     for (int k = tid; k < kN3Sub * 3; k += NT) (&sjacc[0][0])[k] = 0.f;
     if (RDF)
-        for (int k = tid; k < kRdfSpare + 32; k += NT) hist[k] = 0u;
+        for (int k = tid; k < 3 * kNbin + 32; k += NT) hist[k] = 0u;
     if (tid == 0) {
         for (int s = 0; s < kN3Stages; ++s) mbar_init(&bars[s], 1);
         fence_mbar_init();
@@ -595,7 +619,13 @@ __global__ void __launch_bounds__(32 * W, MINB) pair_n3_kernel(const N3Args a) {
         for (int r = 0; r < R; ++r) p[r][0] = p[r][1] = p[r][2] = 0.f;
         const int kind = pt == 1 ? (c.ei_model == TCP_EI_DEUTSCH ? 1 : (c.ei_model == TCP_EI_KELBG ? 2 : 0)) : 0;
         N3Rdf rh;
-        if (RDF) rh = N3Rdf{hist, pt * kNbin, pt, c.u_inv_dx[pt], c.u_rc2, a.rdf_edges};
+        if (RDF) {
+            rh = N3Rdf{hist + pt * kNbin, smem_u32(hist + pt * kNbin) - 4u * kRdfBin0,
+                       ((kRdfBin0 + (3 - pt) * kNbin + lane) << kRdfFrac) + 4096, pt, c.u_inv_dx[pt], c.u_rdf_lo[pt],
+                       c.u_rdf_hi[pt], a.rdf_edges};
+            // opaque, or the compiler loads them again from the constant bank in every step
+            asm volatile("" : "+r"(rh.base), "+r"(rh.spare), "+f"(rh.inv_dx), "+r"(rh.lo), "+r"(rh.hi));
+        }
 #define TCP_N3_ITEM(KIND, MASKED)                                                                      \
     do {                                                                                                \
         if (X2)                                                                                         \
@@ -674,7 +704,7 @@ __global__ void __launch_bounds__(32 * W, MINB) pair_n3_kernel(const N3Args a) {
     if (RDF) {
         __syncthreads();
         for (int q = tid; q < 3 * kNbin; q += NT)
-            if (hist[q]) atomicAdd(&a.rdf[q], (unsigned long long)hist[q]);
+            if (hist[q]) atomicAdd(&a.rdf[q], 2ull * hist[q]);
     }
 }
 
@@ -737,18 +767,20 @@ static const N3Variant kVariants[] = {
 constexpr int kN3Variants = sizeof(kVariants) / sizeof(kVariants[0]);
 
 // Forms that also accumulate the RDF histograms (steps with TCP_FLAG_RDF,
-// which the reference accumulates in every force call): the 2-warp form of
-// the variants above with the degree-5 (0, the default where alpha rc allows
-// it) or degree-6 (1, the default otherwise) erfc, and two 8-warp forms: RDF
-// steps of 4.25 / 4.30 / 4.59 / 4.52 ms at N = 65,536; TCP_RDF_VARIANT=k picks
-// one.
+// which the reference accumulates in every force call): 2 warps a CTA and a
+// rolled step with the degree-5 (0, the default where alpha rc allows it) or
+// degree-6 (1, the default otherwise) erfc, and forms of 4 and 8 warps;
+// TCP_RDF_VARIANT=k picks one.  Pair sums of 0 / 0 unrolled twice / 2 / 3:
+// 32 / 33 / 39 / 41 us at N = 3,000, 516 / 543 / 535 / 561 at 24,001 (754 with
+// the earlier binning), 3,406 / 3,400 / 3,405 / 3,535 at 65,536 (4,100):
+// unrolled, half a warp waits for the instruction cache at any time.
 static const N3Variant kRdfVariants[] = {
-    {pair_n3_kernel<true, 4, 2, 8, false, 1, 2, true, kErfcH5>,
-     pair_n3_kernel<false, 4, 2, 8, false, 1, 2, true, kErfcH5>, 4, 2, "n3_r4_u2_w2b8_x2_p5_rdf", true},
-    {pair_n3_kernel<true, 4, 2, 8, false, 1, 2, true>, pair_n3_kernel<false, 4, 2, 8, false, 1, 2, true>, 4, 2,
-     "n3_r4_u2_w2b8_x2_rdf"},
-    {pair_n3_kernel<true, 4, 1, 3, false, 2, 8, true>, pair_n3_kernel<false, 4, 1, 3, false, 2, 8, true>, 4, 8,
-     "n3_r4_u1_b3_x2l_rdf"},
+    {pair_n3_kernel<true, 4, 1, 8, false, 1, 2, true, kErfcH5>,
+     pair_n3_kernel<false, 4, 1, 8, false, 1, 2, true, kErfcH5>, 4, 2, "n3_r4_u1_w2b8_x2_p5_rdf", true},
+    {pair_n3_kernel<true, 4, 1, 8, false, 1, 2, true>, pair_n3_kernel<false, 4, 1, 8, false, 1, 2, true>, 4, 2,
+     "n3_r4_u1_w2b8_x2_rdf"},
+    {pair_n3_kernel<true, 4, 1, 5, false, 2, 4, true, kErfcH5>,
+     pair_n3_kernel<false, 4, 1, 5, false, 2, 4, true, kErfcH5>, 4, 4, "n3_r4_u1_w4b5_x2l_p5_rdf", true},
     {pair_n3_kernel<true, 4, 1, 2, false, 1, 8, true>, pair_n3_kernel<false, 4, 1, 2, false, 1, 8, true>, 4, 8,
      "n3_r4_u1_b2_x2_rdf"},
 };
