@@ -24,22 +24,28 @@
 //  * the segment index, the terms in FP32 and the cut-off test use the bits of
 //    r^2; the RDF bin comes from FP32 and takes the FP64 square root only next
 //    to a bin edge.
-// That leaves 19 FP64 operations per Coulomb pair (r^2 3, h 1, the two
-// polynomials 8, energy 1, the six force components 6), 59 with the
-// table-driven exp, rsqrt and erfcx of pair_math.cuh (N = 65,536, Kelbg: 217.9 ms a
-// force call with those, 70.5 ms with the tables; N = 3,001: 1,495 against 202 us), which stay for the pairs
-// below the tables (ar < 1/8, or r < lambda/8 or rs/8: about one in 10^5) and
-// for the ordered-pair kernel.
+// That leaves 20 FP64 operations per Coulomb pair (r^2 3, h 1, the two
+// polynomials 8, energy 1, forces 7), 59 with the table-driven exp, rsqrt and
+// erfcx of pair_math.cuh, which stay for the pairs below the tables (ar < 1/8,
+// or r < lambda/8 or rs/8: about one in 10^5) and for the ordered-pair kernel.
+//
+// And only the pairs inside rc, 52 % of all at rc = L/2, are evaluated: a warp
+// finds them with FP32 arithmetic as a bit mask per lane (pair_f64.cuh), each
+// lane then takes the next pair of its own i-particle, and when the first lane
+// has none left the rest are dealt out over the warp.  A reaction goes to the
+// global FP64 force with an atomic per component (91 G/s at the FP64 rate; L2
+// takes 200 and more), without an operation on the FP64 pipe.
+// Force sums, Kelbg, in us: with exp, rsqrt and erfcx per pair; all pairs from
+// the tables; the near pairs alone:
+//   N = 65,536   217,900  70,500  41,400 (38,700 at the FP64 rate)
+//   N =  3,001     1,495     202     136 (    81)
 //
 // Work: a warp takes items from an atomic counter: 32 i-particles (a chunk,
-// one per lane) against up to `group` j-chunks of 32; j's position and
-// reaction rotate through the warp with shuffles.  Small systems, whose items
-// would leave SM quarters idle, split the 32 rotation steps of a tile over
-// `split` items.  Forces and energies are summed in FP64 per item and added to
-// the global FP64 force with one atomic per particle and component.  The order
-// of those atomics varies from run to run, so results vary in the last bits;
-// TCP_FLAG_DETERMINISTIC selects the ordered-pair kernel with its fixed-order
-// reduction instead.
+// one per lane) against up to `group` j-chunks of 32, in the ring order of
+// f64_ring; small systems, whose items would leave SM quarters idle, split the
+// j-particles of a tile over `split` items.  The order of the atomics varies
+// from run to run, so results vary in the last bits; TCP_FLAG_DETERMINISTIC
+// selects the ordered-pair kernel with its fixed-order reduction instead.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -266,64 +272,76 @@ __device__ __forceinline__ void rdf_add_f64(const F64Fast &p, const PairConsts &
     if (ok && bin < kNbin) atomicAdd(&hist[bin], 2u);
 }
 
-// One tile: the warp's 32 i-particles against chunk b, rotation steps [s0, s1).
-template <int KIND, bool ENERGY, bool MASKED, bool RDF, bool CUBIC>
-__device__ __forceinline__ void f64_tile(const F64Fast &p, const N3Args &a, const F64Shared &sh, int pt, bool diag,
-                                         int icnt, long long xi0, long long xi1, long long xi2, int jstart, int jcnt,
-                                         int s0, int s1, double (&fi)[3], double &pe) {
-    const int lane = threadIdx.x & 31, src = (lane + 1) & 31;
-    const int j0 = (lane + s0) & 31;
-    const longlong4_32a t = a.xl[jstart + min(j0, jcnt - 1)];
-    long long xj0 = t.x, xj1 = t.y, xj2 = t.z;
-    double jx = 0.0, jy = 0.0, jz = 0.0;
-#pragma unroll 1
-    for (int s = s0; s < s1; ++s) {
-        const long long d0 = (long long)((unsigned long long)xi0 - (unsigned long long)xj0);
-        const long long d1 = (long long)((unsigned long long)xi1 - (unsigned long long)xj1);
-        const long long d2 = (long long)((unsigned long long)xi2 - (unsigned long long)xj2);
-        bool small = false;
-        double dx = box_diff(d0, small), dy = box_diff(d1, small), dz = box_diff(d2, small);
-        if (__any_sync(0xffffffffu, small)) {   // a component below 2^-32 of the box, zero among them
-            constexpr double k = 5.421010862427522e-20;   // 2^-64
-            dx = (double)d0 * k;
-            dy = (double)d1 * k;
-            dz = (double)d2 * k;
-        }
-        if (!CUBIC) {
-            dx *= a.c.box[0];
-            dy *= a.c.box[1];
-            dz *= a.c.box[2];
-        }
-        const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-        // 0 < r2 < rc^2 on the bit patterns (r2 >= 0: they order as the values)
-        const long long rb = __double_as_longlong(r2);
-        bool ok = rb > 0 && rb < __double_as_longlong(p.rc2);
-        if (MASKED) {   // diagonal tiles: lane l with l + s, s = 1 .. 16, meets every pair once
-            ok = ok && lane < icnt && ((lane + s) & 31) < jcnt;
-            if (diag) ok = ok && s >= 1 && (s < 16 || (s == 16 && lane < 16));
-        }
-        if (RDF) rdf_add_f64(p, a.c, r2, ok, pt, sh.hist);
-        const double w = n3_pair_f64<KIND, ENERGY>(p, a.c, r2, ok, pe, sh);
-        fi[0] = fma(w, dx, fi[0]);
-        fi[1] = fma(w, dy, fi[1]);
-        fi[2] = fma(w, dz, fi[2]);
-        jx = fma(w, dx, jx);
-        jy = fma(w, dy, jy);
-        jz = fma(w, dz, jz);
-        xj0 = __shfl_sync(0xffffffffu, xj0, src);
-        xj1 = __shfl_sync(0xffffffffu, xj1, src);
-        xj2 = __shfl_sync(0xffffffffu, xj2, src);
-        jx = __shfl_sync(0xffffffffu, jx, src);
-        jy = __shfl_sync(0xffffffffu, jy, src);
-        jz = __shfl_sync(0xffffffffu, jz, src);
+// One pair: separation, weight (units of a^3, zero where !ok) and energy.  All
+// lanes of the warp call it.
+struct F64Pair {
+    double w, dx, dy, dz;
+    bool ok;
+};
+template <int KIND, bool ENERGY, bool RDF, bool CUBIC>
+__device__ __forceinline__ F64Pair f64_pair(const F64Fast &p, const N3Args &a, const F64Shared &sh, int pt,
+                                            const F64Pos &xi, int j, bool live, double &pe) {
+    const longlong4_32a xj = a.xl[j];
+    const long long d0 = f64_sub(xi.x, xj.x), d1 = f64_sub(xi.y, xj.y), d2 = f64_sub(xi.z, xj.z);
+    F64Pair q;
+    bool small = false;
+    q.dx = box_diff(d0, small);
+    q.dy = box_diff(d1, small);
+    q.dz = box_diff(d2, small);
+    if (__any_sync(0xffffffffu, small)) {   // a component below 2^-32 of the box, zero among them
+        constexpr double k = 5.421010862427522e-20;   // 2^-64
+        q.dx = (double)d0 * k;
+        q.dy = (double)d1 * k;
+        q.dz = (double)d2 * k;
     }
-    const int jl = (lane + s1) & 31;   // the particle whose reaction this lane holds now
-    if (jl < jcnt) {
-        const double q = -p.qf[pt];
-        double *f = a.facc + jstart + jl;
-        atomicAdd(f, q * jx);
-        atomicAdd(f + a.ntot, q * jy);
-        atomicAdd(f + 2 * (size_t)a.ntot, q * jz);
+    if (!CUBIC) {
+        q.dx *= a.c.box[0];
+        q.dy *= a.c.box[1];
+        q.dz *= a.c.box[2];
+    }
+    const double r2 = fma(q.dx, q.dx, fma(q.dy, q.dy, q.dz * q.dz));
+    // 0 < r2 < rc^2 on the bit patterns (r2 >= 0: they order as the values)
+    const long long rb = __double_as_longlong(r2);
+    q.ok = live && rb > 0 && rb < __double_as_longlong(p.rc2);
+    if (RDF) rdf_add_f64(p, a.c, r2, q.ok, pt, sh.hist);
+    q.w = n3_pair_f64<KIND, ENERGY>(p, a.c, r2, q.ok, pe, sh);
+    return q;
+}
+
+// The near pairs of the warp's 32 i-particles (from i0 on, one per lane) with
+// up to 128 j-particles of one species (from j0 on).  As long as every lane
+// has one left, each takes its own next; the rest, a few per lane, are dealt
+// out evenly.
+template <int KIND, bool ENERGY, bool RDF, bool CUBIC>
+__device__ __forceinline__ void f64_near(const F64Fast &p, const N3Args &a, const F64Shared &sh, int pt, int i0,
+                                         const F64Pos &xi, int j0, F64Mask m, double (&fi)[3], double &pe) {
+    const double qf = p.qf[pt];
+    const size_t n = a.ntot;
+#pragma unroll 1
+    while (__all_sync(0xffffffffu, (m.lo | m.hi) != 0)) {
+        const int j = j0 + mask_pop(m);
+        const F64Pair q = f64_pair<KIND, ENERGY, RDF, CUBIC>(p, a, sh, pt, xi, j, true, pe);
+        const double w = qf * q.w;
+        fi[0] = fma(w, q.dx, fi[0]);
+        fi[1] = fma(w, q.dy, fi[1]);
+        fi[2] = fma(w, q.dz, fi[2]);
+        if (q.ok) add_force(a.facc + j, n, -w * q.dx, -w * q.dy, -w * q.dz);
+    }
+    const F64Deal deal = mask_deal(m);
+#pragma unroll 1
+    for (int t0 = 0; t0 < deal.total; t0 += 32) {
+        const F64Dealt t = mask_dealt(m, deal, t0);
+        F64Pos x;
+        x.x = __shfl_sync(0xffffffffu, xi.x, t.lane);
+        x.y = __shfl_sync(0xffffffffu, xi.y, t.lane);
+        x.z = __shfl_sync(0xffffffffu, xi.z, t.lane);
+        const int j = j0 + t.bit;
+        const F64Pair q = f64_pair<KIND, ENERGY, RDF, CUBIC>(p, a, sh, pt, x, j, t.live, pe);
+        if (q.ok) {
+            const double w = qf * q.w, fx = w * q.dx, fy = w * q.dy, fz = w * q.dz;
+            add_force(a.facc + i0 + t.lane, n, fx, fy, fz);
+            add_force(a.facc + j, n, -fx, -fy, -fz);
+        }
     }
 }
 
@@ -364,41 +382,28 @@ __global__ void __launch_bounds__(kF64Threads, 1) pair_n3_f64_kernel(const N3Arg
         unsigned nx = 0;
         if (lane == 0) nx = atomicAdd(a.counter, 1u);
         const long long it = __shfl_sync(0xffffffffu, nx, 0);
-        if (it >= p.total) break;
-        int ca, grp, part, istart, icnt, isp;
-        f64_item(p, it, ca, grp, part);
-        if (ca >= p.nc) continue;                         // the last block of rows may be short
+        if (it >= p.items) break;
+        int ca, d0, nd, part, istart, icnt, isp;
+        f64_ring(p, it, ca, d0, nd, part);
         f64_chunk(p, a.g, ca, istart, icnt, isp);
-        const int s0 = part * 32 / p.split, s1 = (part + 1) * 32 / p.split;
         const longlong4_32a t = a.xl[istart + min(lane, icnt - 1)];
+        const F64Pos xi{t.x, t.y, t.z};
         double fi[3] = {0.0, 0.0, 0.0};
-        const int b1 = min(p.nc, (grp + 1) * p.group);
-        for (int b = max(ca, grp * p.group); b < b1; ++b) {
-            int jstart, jcnt, jsp;
-            f64_chunk(p, a.g, b, jstart, jcnt, jsp);
-            const int pt = isp + jsp;
-            const bool diag = b == ca, masked = diag || icnt < 32 || jcnt < 32;
-            double pe = 0.0, ft[3] = {0.0, 0.0, 0.0};
+        for (int d = d0; d < d0 + nd;) {                  // runs of chunks of one species
+            const int b = ca + d < p.nc ? ca + d : ca + d - p.nc, jsp = b < p.nce ? 0 : 1;
+            const int run = min(min(d0 + nd - d, (jsp ? p.nc : p.nce) - b), kMaskChunks);
+            const int pt = isp + jsp, j0 = jsp ? a.g.nel + (b - p.nce) * 32 : b * 32;
+            const F64Mask m = f64_mask(p, a.xl, xi, lane < icnt, j0, min(run * 32, (jsp ? a.g.n : a.g.nel) - j0), d == 0, part);
+            d += run;
+            double pe = 0.0;
             if (RDF) sh.hist = hist + pt * kNbin;
-#define TCP_F64_TILE(KIND, MASKED) \
-    f64_tile<KIND, ENERGY, MASKED, RDF, CUBIC>(p, a, sh, pt, diag, icnt, t.x, t.y, t.z, jstart, jcnt, s0, s1, ft, pe)
-            if (EI != 0 && pt == 1) {
-                if (masked) TCP_F64_TILE(EI, true);
-                else TCP_F64_TILE(EI, false);
-            } else {
-                if (masked) TCP_F64_TILE(0, true);
-                else TCP_F64_TILE(0, false);
-            }
-#undef TCP_F64_TILE
-            for (int k = 0; k < 3; ++k) fi[k] = fma(p.qf[pt], ft[k], fi[k]);
+            if (EI != 0 && pt == 1)
+                f64_near<EI, ENERGY, RDF, CUBIC>(p, a, sh, pt, istart, xi, j0, m, fi, pe);
+            else
+                f64_near<0, ENERGY, RDF, CUBIC>(p, a, sh, pt, istart, xi, j0, m, fi, pe);
             if (ENERGY) etot = fma(p.qe[pt], pe, etot);
         }
-        if (lane < icnt) {
-            double *f = a.facc + istart + lane;
-            atomicAdd(f, fi[0]);
-            atomicAdd(f + a.ntot, fi[1]);
-            atomicAdd(f + 2 * (size_t)a.ntot, fi[2]);
-        }
+        if (lane < icnt) add_force(a.facc + istart + lane, a.ntot, fi[0], fi[1], fi[2]);
     }
     if (ENERGY) {
         const double tot = block_sum(etot, red);
@@ -487,6 +492,16 @@ F64Fast f64_args(const tcp_ctx *c, int ew_seg, int ei_seg) {
     p.rc2 = pc.rc2 / p.to_a2;
     while (p.rc2 * p.to_a2 < pc.rc2) p.rc2 = std::nextafter(p.rc2, HUGE_VAL);
     for (double t; (t = std::nextafter(p.rc2, 0.0)) * p.to_a2 >= pc.rc2;) p.rc2 = t;
+    // the FP32 test of f64_mask: the upper words of two coordinates are less
+    // than a unit of 2^-32 of the box off, and FP32 rounding 1e-6
+    const double rcl = std::sqrt(p.rc2), u32 = 1.0 / 4294967296.0;
+    double bmax = 0.0;
+    for (int d = 0; d < 3; ++d) {
+        const double box = pc.cubic ? 1.0 : pc.box[d];
+        p.boxf[d] = (float)(box * u32);
+        bmax = std::max(bmax, box);
+    }
+    p.near2 = (float)((rcl + 4.0 * bmax * u32) * (rcl + 4.0 * bmax * u32) * 1.00001);
     p.ia3 = 1.0 / a3;
     p.ia = 1.0 / al;
     if (p.ei_seg) {
@@ -500,15 +515,22 @@ F64Fast f64_args(const tcp_ctx *c, int ew_seg, int ei_seg) {
         p.qe[t] = pc.qq[t] * al;
         p.rinv_dx[t] = (float)(L * pc.inv_dxd[t]);
     }
-    // Items of four tiles once there are enough of them that the last ones,
-    // about 0.3 ms each, are a small part of the launch; single tiles below,
-    // and halves or quarters of a tile's rotation where even those are too few
-    // to fill the SM quarters evenly.
+    // Items of four tiles (their near pairs deal out to full warps, and the
+    // last ones are a small part of the launch), smaller ones where fewer items
+    // would leave SM quarters idle at the end, down to eighths of a tile where
+    // there is not one for every warp.  Measured (us) at group/split 4/1, 2/1,
+    // 1/1, 1/2, 1/4, 1/8: N = 24,000 5,768 5,817 5,946; 9,000 935 900 910;
+    // 5,000 354 335 316 321 343; 3,001 230 183 145 136 142 157;
+    // 1,500 230 125 75 60 53 56; 512 204 121 73 45 31 26.
     p.nce = (c->nel + 31) / 32;
     p.nc = p.nce + (c->nion + 31) / 32;
     const long long tiles = (long long)p.nc * (p.nc + 1) / 2, quarters = 4LL * c->num_sms;
-    p.group = tiles >= 512 * quarters ? 4 : 1;
-    p.split = tiles >= 16 * quarters ? 1 : (tiles >= 8 * quarters ? 2 : 4);
+    p.group = tiles >= 150 * quarters ? 4 : (tiles >= 50 * quarters ? 2 : 1);
+    p.split = tiles >= 14 * quarters ? 1 : (tiles >= 5 * quarters ? 2 : (2 * tiles >= 3 * quarters ? 4 : 8));
+    p.nd = p.nc / 2 + 1;
+    auto items = [&p] { return (long long)p.nc * ((p.nd + p.group - 1) / p.group) * p.split; };
+    while (items() > 0x7fffffff) p.group *= 2;   // the counter and f64_ring are 32-bit
+    p.items = items();
     p.ng = (p.nc + p.group - 1) / p.group;
     p.total = (long long)p.group * p.ng * (p.ng + 1) / 2 * p.split;
     return p;
@@ -531,7 +553,7 @@ int launch_pair_n3_f64(tcp_ctx *c, bool energy, bool rdf, bool cleared) {
     a.rdf = c->rdf;
     F64Fast p = f64_args(c, c->f64_ew_seg, c->f64_ei_seg);
     p.tab = reinterpret_cast<const uint4 *>(c->f64tab);
-    const int grid = (int)std::min<long long>(n3_f64_grid(c), (p.total + kF64Warps - 1) / kF64Warps);
+    const int grid = (int)std::min<long long>(n3_f64_grid(c), (p.items + kF64Warps - 1) / kF64Warps);
     if (grid > c->n_upart) return set_error(TCP_ERR_STATE, "energy partial buffer smaller than the Newton-3 grid");
     c->n_upart_used = grid;
     if (!cleared) {
