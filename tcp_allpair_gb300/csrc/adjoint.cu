@@ -21,9 +21,10 @@
 // gl = -y/(rs^3 r), y = exp(-r/rs).
 //
 // The default real-space kernels visit every unique pair once and add +t to
-// row i and -t to row j: adj_f64_kernel on the tiles and tables of the FP64
-// force kernel, adj_n3_kernel (FP32C) on the Newton-3 item schedule.  With TCP_FLAG_DETERMINISTIC the ordered-pair kernel visits
-// every ordered pair (i, j) once: thread i sums
+// row i and -t to row j: adj_f64_kernel on the items and tables of the FP64
+// force kernel, adj_n3_kernel (FP32C) on the Newton-3 item schedule.  With
+// TCP_FLAG_DETERMINISTIC the ordered-pair kernel visits every ordered pair
+// (i, j) once: thread i sums
 // (H w)_i = sum_j qq (-G1 dw + G2 (u.dw) u), dw = w_i - w_j, and the scalars
 // dE/dlambda = 1/2 sum qq dl and dF/dlambda . w = sum qq gl (u.w_i).  The
 // j-range is split over gridDim.y; rows are added to hw with FP64 atomics.
@@ -431,13 +432,13 @@ __global__ void __launch_bounds__(kAdjN3Threads) adj_n3_kernel(const AdjArgs a, 
 }
 
 // ---- FP64 tile form --------------------------------------------------------------
-// The unique-pair sums in FP64 on the tiles and radial tables of the FP64 force
-// kernel (pair_f64.cuh; bound: the FP64 pipe).  Per pair of a Hessian-vector
-// product 32 FP64 operations (r^2 3, table argument 1, G1 and G2 4 each, dw 3,
-// u.dw 3, weight 2, the six components of +t and -t 12), about 100 with the
-// radial functions of radial_f64: N = 4,096 Kelbg takes 617 us for the real-space part (2,150 us then).  dE/dlambda
-// (hw null) needs the e-i chunks only, and of those the pairs within the e-i
-// table.
+// The unique-pair sums in FP64 on the items, near-pair masks and radial tables
+// of the FP64 force kernel (pair_f64.cuh; bound: the FP64 pipe).  Per near pair
+// of a Hessian-vector product 31 FP64 operations (r^2 3, table argument 1, G1
+// and G2 4 each, dw 3, u.dw 3, weights 4, t 6, its sum 3), about 100 with the
+// radial functions of radial_f64.  Real-space part at N = 4,096, Kelbg: 2,150 us
+// with those, 617 with the tables for all pairs, about 390 for the near pairs
+// alone.  dE/dlambda (hw null) takes the e-i pairs within the e-i table.
 struct AdjFast {
     F64Fast p;
     const double *w;      // [3][n] or null
@@ -453,112 +454,111 @@ __device__ __noinline__ void radial_general(const AdjArgs &a, const F64Tab &tb, 
     radial_f64<KIND>(a, tb, r2, g[0], g[1], g[2], g[3]);
 }
 
-// minimum-image separation of two particles in units of the box (A where it is not cubic)
-template <bool CUBIC>
-__device__ __forceinline__ void f64_separation(const PairConsts &c, const long long (&xi)[3], const long long (&xj)[3],
-                                               double (&u)[3]) {
-    long long d[3];
-    bool small = false;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        d[k] = (long long)((unsigned long long)xi[k] - (unsigned long long)xj[k]);
-        u[k] = box_diff(d[k], small);
-    }
-    if (__any_sync(0xffffffffu, small))
-#pragma unroll
-        for (int k = 0; k < 3; ++k) u[k] = (double)d[k] * 5.421010862427522e-20;   // 2^-64
-    if (!CUBIC)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) u[k] *= c.box[k];
-}
-
-template <int KIND, bool HVP, bool MASKED, bool CUBIC>
-__device__ __forceinline__ void adj_tile_f64(const AdjArgs &a, const AdjFast &f, const uint4 *ew, const uint4 *ei,
-                                             const F64Tab &tb, int pt, bool diag, int icnt, const long long (&xi)[3],
-                                             const double (&wi)[3], int jstart, int jcnt, int s0, int s1,
-                                             double (&ti)[3], double &sum) {
+// One pair: t, the part of H.w of particle i (-t: of j); its term of the lambda
+// derivative is added to sum.  All lanes of the warp call it.
+struct AdjPair {
+    double t[3];
+    bool ok;
+};
+template <int KIND, bool HVP, bool CUBIC>
+__device__ __forceinline__ AdjPair adj_pair_f64(const AdjArgs &a, const AdjFast &f, const uint4 *ew, const uint4 *ei,
+                                                const F64Tab &tb, double hq, const F64Pos &xi, const double (&wi)[3], int j,
+                                                bool live, double &sum) {
     constexpr int NEI = HVP ? 3 : 1;
     const F64Fast &p = f.p;
-    const int lane = threadIdx.x & 31, src = (lane + 1) & 31;
-    const int j0 = jstart + min((lane + s0) & 31, jcnt - 1);
-    const longlong4_32a t = a.xl[j0];
-    long long xj[3] = {t.x, t.y, t.z};
-    double wj[3] = {0.0, 0.0, 0.0}, hj[3] = {0.0, 0.0, 0.0};
+    const longlong4_32a xj = a.xl[j];
+    double wj[3] = {0.0, 0.0, 0.0}, u[3];
     if (HVP)
 #pragma unroll
-        for (int k = 0; k < 3; ++k) wj[k] = f.w[(size_t)k * a.n + j0];
-#pragma unroll 1
-    for (int s = s0; s < s1; ++s) {
-        double u[3];
-        f64_separation<CUBIC>(a.c, xi, xj, u);
-        const double r2 = fma(u[0], u[0], fma(u[1], u[1], u[2] * u[2]));
-        const long long rb = __double_as_longlong(r2);
-        bool ok = rb > 0 && rb < __double_as_longlong(p.rc2);
-        if (MASKED) {
-            ok = ok && lane < icnt && ((lane + s) & 31) < jcnt;
-            if (diag) ok = ok && s >= 1 && (s < 16 || (s == 16 && lane < 16));
-        }
-        const float r2f = narrow(r2);
-        const unsigned xb = __float_as_uint(r2f * p.kxf), yb = __float_as_uint(r2f * p.kyf);
-        const bool near = KIND != 0 && ok && yb < p.ei_hi;
-        const bool any_near = KIND != 0 && __any_sync(0xffffffffu, near);
-        bool need = (HVP && ok && xb < kTabLowBits) || (near && yb < kTabLowBits);
-        double g1 = 0.0, g2 = 0.0, gl = 0.0;     // units of a^3, a^5; gl (HVP) or dl
-        F64At y;
-        if (any_near) y = f64_at<kEiBits>(ei, yb, p.ei_hi, r2, p.ky, r2f, p.kyf);
-        if (HVP) {
-            const bool in = ok && xb < p.ew_hi;
-            const F64At x = f64_at<kEwBits>(ew, xb, p.ew_hi, r2, p.kx, r2f, p.kxf);
-            g1 = ew_poly(x, p.ew_seg, 0);
-            g2 = ew_poly(x, p.ew_seg, 1);
-            g1 = in ? g1 : 0.0;
-            g2 = in ? g2 : 0.0;
-            if (any_near) {
-                g1 = fma(near ? p.cf : 0.0, ei_poly<true>(y, p.ei_seg, 0, NEI), g1);
-                g2 = fma(near ? f.c2 : 0.0, ei_poly<true>(y, p.ei_seg, 1, NEI), g2);
-            }
-        }
+        for (int k = 0; k < 3; ++k) wj[k] = f.w[(size_t)k * a.n + j];
+    f64_separation<CUBIC>(a.c, xi, xj, u);
+    const double r2 = fma(u[0], u[0], fma(u[1], u[1], u[2] * u[2]));
+    const long long rb = __double_as_longlong(r2);
+    AdjPair q;
+    q.ok = live && rb > 0 && rb < __double_as_longlong(p.rc2);
+    const float r2f = narrow(r2);
+    const unsigned xb = __float_as_uint(r2f * p.kxf), yb = __float_as_uint(r2f * p.kyf);
+    const bool near = KIND != 0 && q.ok && yb < p.ei_hi;
+    const bool any_near = KIND != 0 && __any_sync(0xffffffffu, near);
+    const bool need = (HVP && q.ok && xb < kTabLowBits) || (near && yb < kTabLowBits);
+    double g1 = 0.0, g2 = 0.0, gl = 0.0;     // units of a^3, a^5; gl (HVP) or dl
+    F64At y;
+    if (any_near) y = f64_at<kEiBits>(ei, yb, p.ei_hi, r2, p.ky, r2f, p.kyf);
+    if (HVP) {
+        const bool in = q.ok && xb < p.ew_hi;
+        const F64At x = f64_at<kEwBits>(ew, xb, p.ew_hi, r2, p.kx, r2f, p.kxf);
+        g1 = ew_poly(x, p.ew_seg, 0);
+        g2 = ew_poly(x, p.ew_seg, 1);
+        g1 = in ? g1 : 0.0;
+        g2 = in ? g2 : 0.0;
         if (any_near) {
-            gl = ei_poly<true>(y, p.ei_seg, NEI - 1, NEI);
-            gl = near ? gl : 0.0;
-        }
-        if (__any_sync(0xffffffffu, need)) {
-            if (need) {
-                double g[4];
-                radial_general<KIND>(a, tb, r2 * p.to_a2, g);
-                g1 = g[0] * p.ia3;
-                g2 = g[1] * f.ia5;
-                gl = KIND == 0 ? 0.0 : (HVP ? g[3] / f.kgl : g[2] / f.kdl);
-            }
-        }
-        if (HVP) {
-            double dw[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) dw[k] = wi[k] - wj[k];
-            const double ud = fma(u[0], dw[0], fma(u[1], dw[1], u[2] * dw[2]));
-            const double a2 = (p.kx * g2) * ud;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                ti[k] = fma(a2, u[k], fma(-g1, dw[k], ti[k]));
-                hj[k] = fma(-a2, u[k], fma(g1, dw[k], hj[k]));
-            }
-            if (any_near) sum = fma(gl, ud, sum);
-        } else if (any_near) {
-            sum += gl;
-        }
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            xj[k] = __shfl_sync(0xffffffffu, xj[k], src);
-            if (HVP) {
-                wj[k] = __shfl_sync(0xffffffffu, wj[k], src);
-                hj[k] = __shfl_sync(0xffffffffu, hj[k], src);
-            }
+            g1 = fma(near ? p.cf : 0.0, ei_poly<true>(y, p.ei_seg, 0, NEI), g1);
+            g2 = fma(near ? f.c2 : 0.0, ei_poly<true>(y, p.ei_seg, 1, NEI), g2);
         }
     }
-    const int jl = (lane + s1) & 31;
-    if (HVP && jl < jcnt)
+    if (any_near) {
+        gl = ei_poly<true>(y, p.ei_seg, NEI - 1, NEI);
+        gl = near ? gl : 0.0;
+    }
+    if (__any_sync(0xffffffffu, need)) {
+        if (need) {
+            double g[4];
+            radial_general<KIND>(a, tb, r2 * p.to_a2, g);
+            g1 = g[0] * p.ia3;
+            g2 = g[1] * f.ia5;
+            gl = KIND == 0 ? 0.0 : (HVP ? g[3] / f.kgl : g[2] / f.kdl);
+        }
+    }
+    q.t[0] = q.t[1] = q.t[2] = 0.0;
+    if (HVP) {
+        double dw[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) atomicAdd(f.hw + (size_t)k * a.n + jstart + jl, f.hq[pt] * hj[k]);
+        for (int k = 0; k < 3; ++k) dw[k] = wi[k] - wj[k];
+        const double ud = fma(u[0], dw[0], fma(u[1], dw[1], u[2] * dw[2]));
+        const double a2 = (p.kx * g2) * ud * hq, a1 = hq * g1;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) q.t[k] = fma(a2, u[k], -a1 * dw[k]);
+        if (any_near) sum = fma(gl, ud, sum);
+    } else if (any_near) {
+        sum += gl;
+    }
+    return q;
+}
+
+// The near pairs of 32 i-particles with up to 128 j-particles, as f64_near takes them.
+template <int KIND, bool HVP, bool CUBIC>
+__device__ __forceinline__ void adj_near_f64(const AdjArgs &a, const AdjFast &f, const uint4 *ew, const uint4 *ei,
+                                             const F64Tab &tb, double hq, int i0, const F64Pos &xi, const double (&wi)[3],
+                                             int j0, F64Mask m, double (&hi)[3], double &sum) {
+#pragma unroll 1
+    while (__all_sync(0xffffffffu, (m.lo | m.hi) != 0)) {
+        const int j = j0 + mask_pop(m);
+        const AdjPair q = adj_pair_f64<KIND, HVP, CUBIC>(a, f, ew, ei, tb, hq, xi, wi, j, true, sum);
+        if (HVP) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) hi[k] += q.t[k];
+            if (q.ok) add_force(f.hw + j, a.n, -q.t[0], -q.t[1], -q.t[2]);
+        }
+    }
+    const F64Deal deal = mask_deal(m);
+#pragma unroll 1
+    for (int t0 = 0; t0 < deal.total; t0 += 32) {
+        const F64Dealt t = mask_dealt(m, deal, t0);
+        F64Pos x;
+        x.x = __shfl_sync(0xffffffffu, xi.x, t.lane);
+        x.y = __shfl_sync(0xffffffffu, xi.y, t.lane);
+        x.z = __shfl_sync(0xffffffffu, xi.z, t.lane);
+        double w[3] = {0.0, 0.0, 0.0};
+        if (HVP)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) w[k] = __shfl_sync(0xffffffffu, wi[k], t.lane);
+        const int j = j0 + t.bit;
+        const AdjPair q = adj_pair_f64<KIND, HVP, CUBIC>(a, f, ew, ei, tb, hq, x, w, j, t.live, sum);
+        if (HVP && q.ok) {
+            add_force(f.hw + i0 + t.lane, a.n, q.t[0], q.t[1], q.t[2]);
+            add_force(f.hw + j, a.n, -q.t[0], -q.t[1], -q.t[2]);
+        }
+    }
 }
 
 template <int EI, bool HVP, bool CUBIC>
@@ -595,46 +595,25 @@ __global__ void __launch_bounds__(kF64Threads, 1) adj_f64_kernel(const AdjArgs a
         unsigned nx = 0;
         if (lane == 0) nx = atomicAdd(counter, 1u);
         const long long it = __shfl_sync(0xffffffffu, nx, 0);
-        if (it >= p.total) break;
-        int ca, grp, part, istart, icnt, isp;
-        f64_item(p, it, ca, grp, part);
-        if (ca >= p.nc) continue;
-        const int b1c = min(p.nc, (grp + 1) * p.group);
-        int b = max(ca, grp * p.group);
-        if (!HVP) {                              // e-i chunks only
-            if (ca >= p.nce) continue;
-            b = max(b, p.nce);
-            if (b >= b1c) continue;
-        }
+        if (it >= p.items) break;
+        int ca, d0, nd, part, istart, icnt, isp;
+        f64_ring(p, it, ca, d0, nd, part);
         f64_chunk(p, g, ca, istart, icnt, isp);
-        const int s0 = part * 32 / p.split, s1 = (part + 1) * 32 / p.split, i = istart + min(lane, icnt - 1);
+        const int i = istart + min(lane, icnt - 1);
         const longlong4_32a t = a.xl[i];
-        const long long xi[3] = {t.x, t.y, t.z};
+        const F64Pos xi{t.x, t.y, t.z};
         double wi[3] = {0.0, 0.0, 0.0}, hi[3] = {0.0, 0.0, 0.0};
         if (HVP)
             for (int k = 0; k < 3; ++k) wi[k] = f.w[(size_t)k * a.n + i];
-        for (; b < b1c; ++b) {
-            int jstart, jcnt, jsp;
-            f64_chunk(p, g, b, jstart, jcnt, jsp);
-            const int pt = isp + jsp;
-            const bool diag = b == ca, masked = diag || icnt < 32 || jcnt < 32;
-            double ti[3] = {0.0, 0.0, 0.0}, sum = 0.0;
-#define TCP_ADJ_TILE(KIND, MASKED) \
-    adj_tile_f64<KIND, HVP, MASKED, CUBIC>(a, f, ew, ei, tab, pt, diag, icnt, xi, wi, jstart, jcnt, s0, s1, ti, sum)
-            if (EI != 0 && pt == 1) {
-                if (masked) TCP_ADJ_TILE(EI, true);
-                else TCP_ADJ_TILE(EI, false);
-            } else if (HVP) {
-                if (masked) TCP_ADJ_TILE(0, true);
-                else TCP_ADJ_TILE(0, false);
-            }
-#undef TCP_ADJ_TILE
-            if (HVP)
-                for (int k = 0; k < 3; ++k) hi[k] = fma(f.hq[pt], ti[k], hi[k]);
-            total += sum;
+        for (F64Run r{d0, d0 + nd}; f64_run(p, g, ca, isp, r);) {
+            if (!HVP && r.pt != 1) continue;     // the e-i chunks only
+            const F64Mask m = f64_mask(p, a.xl, xi, lane < icnt, r.j0, r.nj, r.diag, part);
+            if (EI != 0 && r.pt == 1)
+                adj_near_f64<EI, HVP, CUBIC>(a, f, ew, ei, tab, f.hq[1], istart, xi, wi, r.j0, m, hi, total);
+            else if (HVP)
+                adj_near_f64<0, HVP, CUBIC>(a, f, ew, ei, tab, f.hq[r.pt], istart, xi, wi, r.j0, m, hi, total);
         }
-        if (HVP && lane < icnt)
-            for (int k = 0; k < 3; ++k) atomicAdd(f.hw + (size_t)k * a.n + istart + lane, hi[k]);
+        if (HVP && lane < icnt) add_force(f.hw + istart + lane, a.n, hi[0], hi[1], hi[2]);
     }
     total = block_sum(total, red);
     if (tid == 0) atomicAdd(a.scal + (HVP ? kAdjDFdl : kAdjDEdl), total * (HVP ? f.qgl : f.qdl));
@@ -858,7 +837,8 @@ static int launch_adj_f64(tcp_ctx *c, const AdjArgs &a, const double *w, double 
     for (int t = 0; t < 3; ++t) f.hq[t] = kEps * pc.qq[t] * al * al * al;
     f.qgl = kEps * pc.qq[1] * f.kgl * L;
     f.qdl = kEps * pc.qq[1] * f.kdl;
-    const int grid = (int)std::min<long long>(c->num_sms, (f.p.total + kF64Warps - 1) / kF64Warps);
+    if (!hvp) f.p.near2 = std::min(f.p.near2, f64_near2(pc, std::sqrt(std::ldexp(1.0, (T.ei >> kEiBits) + kTabLow) / f.p.ky)));   // of the e-i table's end
+    const int grid = (int)std::min<long long>(c->num_sms, (f.p.items + kF64Warps - 1) / kF64Warps);
     TCP_CUDA(cudaMemsetAsync(c->counter, 0, sizeof(unsigned), c->stream));
     fn<<<grid, kF64Threads, T.bytes, c->stream>>>(a, f, c->counter, c->status);
     c->launches++;

@@ -73,11 +73,10 @@ struct F64Fast {
     int group, split;        // j-chunks per item; items per tile
     int nce, nc, nd;         // electron chunks, chunks, distances in their ring (f64_ring)
     long long items;
-    int ng;                  // groups and items of the triangle (f64_item)
-    long long total;
 };
 
 F64Fast f64_args(const tcp_ctx *c, int ew_seg, int ei_seg);   // tab: the caller's
+float f64_near2(const PairConsts &pc, double r);   // F64Fast::near2 for a distance r (units of F64Fast)
 
 // ---- pair arithmetic --------------------------------------------------------------
 // (double)d 2^-64 for a 64-bit integer d without the FP64 pipe: the magnitude
@@ -160,24 +159,6 @@ __device__ __forceinline__ void f64_chunk(const F64Fast &p, const N3Geom &g, int
     cnt = min(32, (sp ? g.n : g.nel) - start);
 }
 
-// Item -> (chunk a, group of j-chunks, part of the rotation).  Rows come in
-// blocks of `group` chunks: the rows of block A hold the groups A .. ng-1, so
-// block A starts at group (A ng - A (A - 1)/2).
-__device__ __forceinline__ void f64_item(const F64Fast &p, long long it, int &a, int &grp, int &part) {
-    part = (int)(it % p.split);
-    const long long t = it / p.split;
-    auto start = [&](int A) { return (long long)p.group * ((long long)A * p.ng - (long long)A * (A - 1) / 2); };
-    const float b = (float)p.ng + 0.5f;
-    int A = (int)(b - sqrtf(fmaxf(b * b - 2.0f * (float)t / (float)p.group, 0.0f)));
-    A = max(0, min(A, p.ng - 1));
-    while (A > 0 && start(A) > t) --A;
-    while (A + 1 < p.ng && start(A + 1) <= t) ++A;
-    const int o = (int)(t - start(A)), w = p.ng - A;
-    a = A * p.group + o / w;
-    grp = A + o % w;
-}
-
-
 // The chunks form a ring: chunk a meets the chunks a, a + 1, .., a + nc/2
 // behind it, at the distance nc/2 of an even ring in its first half only, so
 // that every pair of chunks meets once.  Item -> (a, first distance d0 of up to
@@ -194,6 +175,26 @@ __device__ __forceinline__ void f64_ring(const F64Fast &p, long long it, int &a,
     if (2 * (d0 + nd - 1) == p.nc && 2 * a >= p.nc) --nd;
 }
 
+// The next run of an item: up to kMaskChunks chunks of one species among its
+// distances [d, end); false after the last.
+constexpr int kMaskChunks = 4;
+struct F64Run {
+    int d, end;
+    int pt, j0, nj;          // pair type, particles
+    bool diag;               // starts with the i-particles' own chunk
+};
+__device__ __forceinline__ bool f64_run(const F64Fast &p, const N3Geom &g, int a, int isp, F64Run &r) {
+    if (r.d >= r.end) return false;
+    const int b = a + r.d < p.nc ? a + r.d : a + r.d - p.nc, jsp = b < p.nce ? 0 : 1;
+    const int run = min(min(r.end - r.d, (jsp ? p.nc : p.nce) - b), kMaskChunks);
+    r.pt = isp + jsp;
+    r.j0 = jsp ? g.nel + (b - p.nce) * 32 : b * 32;
+    r.nj = min(run * 32, (jsp ? g.n : g.nel) - r.j0);
+    r.diag = r.d == 0;
+    r.d += run;
+    return true;
+}
+
 // ---- near pairs ---------------------------------------------------------------------
 // Half of all pairs lie past rc = L/2, and a warp instruction on the FP64 pipe
 // takes as long whether its lanes need it or not.  So a warp first finds the
@@ -202,13 +203,28 @@ __device__ __forceinline__ void f64_ring(const F64Fast &p, long long it, int &a,
 struct F64Pos {
     long long x, y, z;       // 64-bit fixed point
 };
-constexpr int kMaskChunks = 4;
 struct F64Mask {
     unsigned long long lo, hi;   // j-particles 0 .. 127 of a lane's i-particle
 };
 
 __device__ __forceinline__ long long f64_sub(long long a, long long b) {
     return (long long)((unsigned long long)a - (unsigned long long)b);
+}
+
+// minimum-image separation of two particles in units of the box (A where it is not cubic)
+template <bool CUBIC>
+__device__ __forceinline__ void f64_separation(const PairConsts &c, const F64Pos &xi, const longlong4_32a &xj,
+                                               double (&u)[3]) {
+    const long long d[3] = {f64_sub(xi.x, xj.x), f64_sub(xi.y, xj.y), f64_sub(xi.z, xj.z)};
+    bool small = false;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) u[k] = box_diff(d[k], small);
+    if (__any_sync(0xffffffffu, small))   // a component below 2^-32 of the box, zero among them
+#pragma unroll
+        for (int k = 0; k < 3; ++k) u[k] = (double)d[k] * 5.421010862427522e-20;   // 2^-64
+    if (!CUBIC)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) u[k] *= c.box[k];
 }
 
 // The pairs of the lane's i-particle with the nj (up to 128) j-particles from

@@ -275,31 +275,15 @@ __device__ __forceinline__ void rdf_add_f64(const F64Fast &p, const PairConsts &
 // One pair: separation, weight (units of a^3, zero where !ok) and energy.  All
 // lanes of the warp call it.
 struct F64Pair {
-    double w, dx, dy, dz;
+    double w, u[3];
     bool ok;
 };
 template <int KIND, bool ENERGY, bool RDF, bool CUBIC>
 __device__ __forceinline__ F64Pair f64_pair(const F64Fast &p, const N3Args &a, const F64Shared &sh, int pt,
                                             const F64Pos &xi, int j, bool live, double &pe) {
-    const longlong4_32a xj = a.xl[j];
-    const long long d0 = f64_sub(xi.x, xj.x), d1 = f64_sub(xi.y, xj.y), d2 = f64_sub(xi.z, xj.z);
     F64Pair q;
-    bool small = false;
-    q.dx = box_diff(d0, small);
-    q.dy = box_diff(d1, small);
-    q.dz = box_diff(d2, small);
-    if (__any_sync(0xffffffffu, small)) {   // a component below 2^-32 of the box, zero among them
-        constexpr double k = 5.421010862427522e-20;   // 2^-64
-        q.dx = (double)d0 * k;
-        q.dy = (double)d1 * k;
-        q.dz = (double)d2 * k;
-    }
-    if (!CUBIC) {
-        q.dx *= a.c.box[0];
-        q.dy *= a.c.box[1];
-        q.dz *= a.c.box[2];
-    }
-    const double r2 = fma(q.dx, q.dx, fma(q.dy, q.dy, q.dz * q.dz));
+    f64_separation<CUBIC>(a.c, xi, a.xl[j], q.u);
+    const double r2 = fma(q.u[0], q.u[0], fma(q.u[1], q.u[1], q.u[2] * q.u[2]));
     // 0 < r2 < rc^2 on the bit patterns (r2 >= 0: they order as the values)
     const long long rb = __double_as_longlong(r2);
     q.ok = live && rb > 0 && rb < __double_as_longlong(p.rc2);
@@ -322,10 +306,10 @@ __device__ __forceinline__ void f64_near(const F64Fast &p, const N3Args &a, cons
         const int j = j0 + mask_pop(m);
         const F64Pair q = f64_pair<KIND, ENERGY, RDF, CUBIC>(p, a, sh, pt, xi, j, true, pe);
         const double w = qf * q.w;
-        fi[0] = fma(w, q.dx, fi[0]);
-        fi[1] = fma(w, q.dy, fi[1]);
-        fi[2] = fma(w, q.dz, fi[2]);
-        if (q.ok) add_force(a.facc + j, n, -w * q.dx, -w * q.dy, -w * q.dz);
+        fi[0] = fma(w, q.u[0], fi[0]);
+        fi[1] = fma(w, q.u[1], fi[1]);
+        fi[2] = fma(w, q.u[2], fi[2]);
+        if (q.ok) add_force(a.facc + j, n, -w * q.u[0], -w * q.u[1], -w * q.u[2]);
     }
     const F64Deal deal = mask_deal(m);
 #pragma unroll 1
@@ -338,7 +322,7 @@ __device__ __forceinline__ void f64_near(const F64Fast &p, const N3Args &a, cons
         const int j = j0 + t.bit;
         const F64Pair q = f64_pair<KIND, ENERGY, RDF, CUBIC>(p, a, sh, pt, x, j, t.live, pe);
         if (q.ok) {
-            const double w = qf * q.w, fx = w * q.dx, fy = w * q.dy, fz = w * q.dz;
+            const double w = qf * q.w, fx = w * q.u[0], fy = w * q.u[1], fz = w * q.u[2];
             add_force(a.facc + i0 + t.lane, n, fx, fy, fz);
             add_force(a.facc + j, n, -fx, -fy, -fz);
         }
@@ -389,19 +373,15 @@ __global__ void __launch_bounds__(kF64Threads, 1) pair_n3_f64_kernel(const N3Arg
         const longlong4_32a t = a.xl[istart + min(lane, icnt - 1)];
         const F64Pos xi{t.x, t.y, t.z};
         double fi[3] = {0.0, 0.0, 0.0};
-        for (int d = d0; d < d0 + nd;) {                  // runs of chunks of one species
-            const int b = ca + d < p.nc ? ca + d : ca + d - p.nc, jsp = b < p.nce ? 0 : 1;
-            const int run = min(min(d0 + nd - d, (jsp ? p.nc : p.nce) - b), kMaskChunks);
-            const int pt = isp + jsp, j0 = jsp ? a.g.nel + (b - p.nce) * 32 : b * 32;
-            const F64Mask m = f64_mask(p, a.xl, xi, lane < icnt, j0, min(run * 32, (jsp ? a.g.n : a.g.nel) - j0), d == 0, part);
-            d += run;
+        for (F64Run r{d0, d0 + nd}; f64_run(p, a.g, ca, isp, r);) {
+            const F64Mask m = f64_mask(p, a.xl, xi, lane < icnt, r.j0, r.nj, r.diag, part);
             double pe = 0.0;
-            if (RDF) sh.hist = hist + pt * kNbin;
-            if (EI != 0 && pt == 1)
-                f64_near<EI, ENERGY, RDF, CUBIC>(p, a, sh, pt, istart, xi, j0, m, fi, pe);
+            if (RDF) sh.hist = hist + r.pt * kNbin;
+            if (EI != 0 && r.pt == 1)
+                f64_near<EI, ENERGY, RDF, CUBIC>(p, a, sh, r.pt, istart, xi, r.j0, m, fi, pe);
             else
-                f64_near<0, ENERGY, RDF, CUBIC>(p, a, sh, pt, istart, xi, j0, m, fi, pe);
-            if (ENERGY) etot = fma(p.qe[pt], pe, etot);
+                f64_near<0, ENERGY, RDF, CUBIC>(p, a, sh, r.pt, istart, xi, r.j0, m, fi, pe);
+            if (ENERGY) etot = fma(p.qe[r.pt], pe, etot);
         }
         if (lane < icnt) add_force(a.facc + istart + lane, a.ntot, fi[0], fi[1], fi[2]);
     }
@@ -472,6 +452,14 @@ int n3_f64_prepare(tcp_ctx *c) {
     return TCP_OK;
 }
 
+// The upper words of two coordinates are less than a unit of 2^-32 of the box
+// off, and the FP32 arithmetic of f64_mask 1e-6.
+float f64_near2(const PairConsts &pc, double r) {
+    const double box = pc.cubic ? 1.0 : std::max(pc.box[0], std::max(pc.box[1], pc.box[2]));
+    const double b = r + 4.0 * box / 4294967296.0;
+    return (float)(b * b * 1.00001);
+}
+
 // Constants and items for tables of ew_seg and ei_seg segments.
 F64Fast f64_args(const tcp_ctx *c, int ew_seg, int ei_seg) {
     const PairConsts &pc = c->pc;
@@ -492,16 +480,8 @@ F64Fast f64_args(const tcp_ctx *c, int ew_seg, int ei_seg) {
     p.rc2 = pc.rc2 / p.to_a2;
     while (p.rc2 * p.to_a2 < pc.rc2) p.rc2 = std::nextafter(p.rc2, HUGE_VAL);
     for (double t; (t = std::nextafter(p.rc2, 0.0)) * p.to_a2 >= pc.rc2;) p.rc2 = t;
-    // the FP32 test of f64_mask: the upper words of two coordinates are less
-    // than a unit of 2^-32 of the box off, and FP32 rounding 1e-6
-    const double rcl = std::sqrt(p.rc2), u32 = 1.0 / 4294967296.0;
-    double bmax = 0.0;
-    for (int d = 0; d < 3; ++d) {
-        const double box = pc.cubic ? 1.0 : pc.box[d];
-        p.boxf[d] = (float)(box * u32);
-        bmax = std::max(bmax, box);
-    }
-    p.near2 = (float)((rcl + 4.0 * bmax * u32) * (rcl + 4.0 * bmax * u32) * 1.00001);
+    for (int d = 0; d < 3; ++d) p.boxf[d] = (float)((pc.cubic ? 1.0 : pc.box[d]) / 4294967296.0);
+    p.near2 = f64_near2(pc, std::sqrt(p.rc2));
     p.ia3 = 1.0 / a3;
     p.ia = 1.0 / al;
     if (p.ei_seg) {
@@ -531,8 +511,6 @@ F64Fast f64_args(const tcp_ctx *c, int ew_seg, int ei_seg) {
     auto items = [&p] { return (long long)p.nc * ((p.nd + p.group - 1) / p.group) * p.split; };
     while (items() > 0x7fffffff) p.group *= 2;   // the counter and f64_ring are 32-bit
     p.items = items();
-    p.ng = (p.nc + p.group - 1) / p.group;
-    p.total = (long long)p.group * p.ng * (p.ng + 1) / 2 * p.split;
     return p;
 }
 
