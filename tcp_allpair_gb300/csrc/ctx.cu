@@ -99,6 +99,13 @@ static int ensure_stage(tcp_ctx *c, size_t bytes) {
     return TCP_OK;
 }
 
+bool host_direct(int device) {
+    int pageable = 0;
+    cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device);
+    const char *env = getenv("TCP_HOST_DIRECT");
+    return pageable == 1 && !(env && env[0] == '0');
+}
+
 static bool energy_on(const tcp_ctx *c) { return (c->flags & TCP_FLAG_ENERGY) != 0; }
 
 static int recip_launch(tcp_ctx *c) {
@@ -314,12 +321,7 @@ int tcp_create(const tcp_params *p_in, int nel, int nion, int device, tcp_ctx **
     c->n = nel + nion;
     c->device = device;
     c->num_sms = prop.multiProcessorCount;
-    {
-        int pageable = 0;
-        cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device);
-        const char *env = getenv("TCP_HOST_DIRECT");
-        c->host_direct = pageable == 1 && !(env && env[0] == '0');
-    }
+    c->host_direct = host_direct(device);
     const size_t n = c->n;
     auto fail = [&](int code) {
         tcp_destroy(c);

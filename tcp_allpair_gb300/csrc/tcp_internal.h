@@ -365,6 +365,7 @@ int launch_spme_sum(tcp_ctx *c);
 int launch_fsum(tcp_ctx *c);
 int launch_remove_rigid(tcp_ctx *c);
 int launch_kick2(tcp_ctx *c, double dt, bool remove_net, bool apply_thermo, bool vdf);
+bool host_direct(int device);   // kernels may address pageable host memory (TCP_HOST_DIRECT=0: told not to)
 int launch_extract(tcp_ctx *c, const unsigned char *src, int first, int count, long stride, long off_x, long off_v,
                    long off_f, cudaStream_t st = nullptr);   // st: c->stream when null
 int launch_scatter(tcp_ctx *c, unsigned char *dst, int first, int count, long stride, long off_x, long off_v,
