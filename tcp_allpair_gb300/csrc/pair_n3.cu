@@ -838,12 +838,28 @@ void n3_chunk_table(long long total, int ctas, std::vector<long long> &starts) {
     }
 }
 
+// The SPME chain's mesh kernels need up to 140 KB of shared memory (a plane of
+// the mesh).  An SM takes a CTA of another kernel only if its split between L1
+// and shared memory has room, and changes the split only when it is empty: with
+// the split that the pair kernel's own 70 KB ask for, the chain beside it
+// waited for its end.
+static int max_carveout(const void *fn) {
+    TCP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    return TCP_OK;
+}
+
 // Chunk tables of every i-tile size the variants use, in one device array
 // (c->n3_chunks; c->n3_chunk_meta holds tile, items, offset, chunks per
 // table).  Built on the host when the pair constants change, outside any
 // stream capture, each for the largest persistent grid among the variants of
 // that i-tile.
 int n3_prepare_chunks(tcp_ctx *c) {
+    for (const N3Variant &v : kVariants)
+        for (const N3Kernel k : {v.energy, v.plain})
+            if (int rc = max_carveout(reinterpret_cast<const void *>(k))) return rc;
+    for (const N3Variant &v : kRdfVariants)
+        for (const N3Kernel k : {v.energy, v.plain})
+            if (int rc = max_carveout(reinterpret_cast<const void *>(k))) return rc;
     std::vector<int> tiles;
     for (const N3Variant &v : kVariants) tiles.push_back(32 * v.R * v.W);
     for (const N3Variant &v : kRdfVariants) tiles.push_back(32 * v.R * v.W);
