@@ -141,15 +141,18 @@ static int recip_join(tcp_ctx *c) {
 // Mean time of the real-space launch with the reciprocal chain beside it on
 // stream2, as inside a step (the autotuner's measure for the grid reserve).
 int time_pair_with_recip(tcp_ctx *c, int reps, double *ms) {
-    // The fork, the pair launch and the join are captured as one graph and
-    // replayed, as they run inside the step graph: both branches become ready
-    // together.  Launched one by one, the chain's kernels would run ahead on
-    // an idle GPU while the host is still issuing the rest.
+    // The preparation, the fork, the pair launch and the join are captured as
+    // one graph and replayed, as they run inside the step graph: both branches
+    // become ready together.  Launched one by one, the chain's kernels would
+    // run ahead on an idle GPU while the host is still issuing the rest; with
+    // the chain's own binning before it, the pair kernel fills every SM first.
     cudaGraph_t g = nullptr;
     cudaGraphExec_t ge = nullptr;
     TCP_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = recip_fork(c);
+    int rc = launch_prepare(c);
+    if (!rc) rc = recip_fork(c);
     if (!rc) rc = launch_pair(c, energy_on(c), false);
+    c->cleared = c->binned = false;
     const int jrc = recip_join(c);
     const cudaError_t ce = cudaStreamEndCapture(c->stream, &g);
     if (!rc) rc = jrc;

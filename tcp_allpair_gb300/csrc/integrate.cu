@@ -98,7 +98,8 @@ struct StepPrep {
 // A thread per component: the FP64 chain of a particle (its three components
 // one after the other took 45 dependent operations of 34 ns) is a third as
 // long and a small system spreads over three times the warps.
-template <bool BIN>
+// Without KICK the preparation alone (the autotuner's replays).
+template <bool BIN, bool KICK>
 __global__ void __launch_bounds__(kPartThreads) vverlet1_kernel(const IntArgs a, double dt, double hdm0, double hdm1,
                                                                 double alpha_lgv, int stoch, const StepPrep s) {
     __shared__ int sb[BIN ? 3 : 1][kPartBlock];
@@ -107,16 +108,19 @@ __global__ void __launch_bounds__(kPartThreads) vverlet1_kernel(const IntArgs a,
     const bool live = i < a.n;
     if (live) {
         const double L = d == 0 ? a.L0 : (d == 1 ? a.L1 : a.L2), iL = d == 0 ? a.iL0 : (d == 1 ? a.iL1 : a.iL2);
-        const double hdm = i < a.nel ? hdm0 : hdm1;    // dt/(2m), divided on the host
         const size_t o = (size_t)d * a.n + i;
-        double v = a.v[o];
-        if (stoch)
-            v = v * (1.0 - alpha_lgv * hdm) + hdm * a.f[o];   // vverlet.f90:37-38
-        else
-            v = v + hdm * a.f[o];                      // vverlet.f90:151
-        a.v[o] = v;
-        const double y = wrap_fast(a.x[o] + dt * v, L, iL);   // vverlet.f90:152-153
-        store_comp(a, d, i, y, iL);
+        double y = a.x[o];
+        if (KICK) {
+            const double hdm = i < a.nel ? hdm0 : hdm1;    // dt/(2m), divided on the host
+            double v = a.v[o];
+            if (stoch)
+                v = v * (1.0 - alpha_lgv * hdm) + hdm * a.f[o];   // vverlet.f90:37-38
+            else
+                v = v + hdm * a.f[o];                      // vverlet.f90:151
+            a.v[o] = v;
+            y = wrap_fast(y + dt * v, L, iL);              // vverlet.f90:152-153
+            store_comp(a, d, i, y, iL);
+        }
         if (s.fpart) s.fpart[o] = 0.0;
         if (BIN) {
             const SpmeGeom &g = s.chain.one;
@@ -563,28 +567,45 @@ int launch_shift(tcp_ctx *c, double sdt) {
     return TCP_OK;
 }
 
+static StepPrep step_prep(tcp_ctx *c) {
+    StepPrep s;
+    s.fpart = c->fpart;
+    s.upart = c->upart;
+    s.nupart = c->n_upart;
+    s.counter = c->counter;
+    s.bin = c->p.reciprocal == TCP_RECIP_SPME;
+    if (s.bin) {
+        s.chain = spme_chain_args(c);
+        s.chain.ticket = c->tickets + kTickStep;
+    }
+    return s;
+}
+
 int launch_vverlet1(tcp_ctx *c, double dt, bool prepare) {
     StepPrep s;
     s.fpart = nullptr;
     s.bin = 0;
-    if (prepare) {
-        s.fpart = c->fpart;
-        s.upart = c->upart;
-        s.nupart = c->n_upart;
-        s.counter = c->counter;
-        s.bin = c->p.reciprocal == TCP_RECIP_SPME;
-        if (s.bin) {
-            s.chain = spme_chain_args(c);
-            s.chain.ticket = c->tickets + kTickStep;
-        }
-    }
+    if (prepare) s = step_prep(c);
     const double h0 = 0.5 * dt / c->p.xm[0], h1 = 0.5 * dt / c->p.xm[1];
     const int stoch = c->p.thermo == TCP_THERMO_STOCH, nb = part_blocks(c->n);
     if (s.bin)
-        vverlet1_kernel<true><<<nb, kPartThreads, 0, c->stream>>>(int_args(c), dt, h0, h1, c->p.alpha_lgv, stoch, s);
+        vverlet1_kernel<true, true><<<nb, kPartThreads, 0, c->stream>>>(int_args(c), dt, h0, h1, c->p.alpha_lgv, stoch, s);
     else
-        vverlet1_kernel<false><<<nb, kPartThreads, 0, c->stream>>>(int_args(c), dt, h0, h1, c->p.alpha_lgv, stoch, s);
+        vverlet1_kernel<false, true><<<nb, kPartThreads, 0, c->stream>>>(int_args(c), dt, h0, h1, c->p.alpha_lgv, stoch, s);
     c->cleared = prepare;
+    c->binned = s.bin != 0;
+    c->launches++;
+    TCP_CUDA(cudaGetLastError());
+    return TCP_OK;
+}
+
+int launch_prepare(tcp_ctx *c) {
+    const StepPrep s = step_prep(c);
+    if (s.bin)
+        vverlet1_kernel<true, false><<<part_blocks(c->n), kPartThreads, 0, c->stream>>>(int_args(c), 0.0, 0.0, 0.0, 0.0, 0, s);
+    else
+        vverlet1_kernel<false, false><<<part_blocks(c->n), kPartThreads, 0, c->stream>>>(int_args(c), 0.0, 0.0, 0.0, 0.0, 0, s);
+    c->cleared = true;
     c->binned = s.bin != 0;
     c->launches++;
     TCP_CUDA(cudaGetLastError());

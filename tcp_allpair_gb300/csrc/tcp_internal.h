@@ -361,6 +361,7 @@ int part_blocks(int n);
 int launch_refresh_positions(tcp_ctx *c, const double *x = nullptr);   // from x [3][n] (null: the positions as they are)
 int launch_shift(tcp_ctx *c, double sdt);
 int launch_vverlet1(tcp_ctx *c, double dt, bool prepare);   // prepare: also clear and bin for the forces of this step
+int launch_prepare(tcp_ctx *c);   // that preparation alone
 int launch_spme_sum(tcp_ctx *c);
 int launch_fsum(tcp_ctx *c);
 int launch_remove_rigid(tcp_ctx *c);
