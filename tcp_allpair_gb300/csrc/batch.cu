@@ -1,6 +1,6 @@
 // batch.cu -- many independent systems (replicas) in one context: one
 // persistent Newton-3 pair launch over the items of all replicas, SPME with
-// one batched cuFFT plan per distinct mesh, and replica-aware integrator and
+// one group of transforms per distinct mesh, and replica-aware integrator and
 // reduction kernels, captured together as one CUDA graph per MD step.
 //
 // Each replica is a complete system of the reference (its own box, charges,

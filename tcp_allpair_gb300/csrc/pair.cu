@@ -1008,7 +1008,7 @@ static int choose_variant(tcp_ctx *c, const char *cache, const std::string &key)
 
 // CTAs left out of the persistent Newton-3 grid.  In a step the reciprocal
 // chain runs on a second stream beside the pair kernel; with every SM holding
-// its full share of pair CTAs, the chain's kernels (cuFFT's among them) find no
+// its full share of pair CTAs, the chain's kernels find no
 // registers free and wait for the pair kernel's tail.  The reserved CTAs
 // rejoin the pair launch once the chain is done (launch_pair_n3_rejoin), so a
 // large reserve costs the pair kernel only while the chain runs: where the
