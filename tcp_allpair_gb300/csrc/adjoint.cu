@@ -816,8 +816,7 @@ static int launch_adj_f64(tcp_ctx *c, const AdjArgs &a, const double *w, double 
         TCP_CUDA(cudaMalloc(&T.dev, T.bytes));
         TCP_CUDA(cudaMemcpy(T.dev, t.data(), T.bytes, cudaMemcpyHostToDevice));
         if (T.fits)
-            TCP_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void *>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)T.bytes));
+            if (int rc = allow_shared(reinterpret_cast<const void *>(fn), T.bytes)) return rc;
     }
     *done = T.fits;
     if (!T.fits) return TCP_OK;

@@ -34,6 +34,24 @@ int cuda_check(cudaError_t e, const char *what) {
     return e == cudaErrorMemoryAllocation ? TCP_ERR_NOMEM : TCP_ERR_CUDA;
 }
 
+// The limit of a kernel's dynamic shared memory belongs to the kernel on its
+// device, not to a context: set to what the last prepared context needs, it made
+// the launches of an earlier one that needs more fail.  It is therefore always
+// the most that the device gives a CTA, whoever asks.
+int allow_shared(const void *fn, size_t bytes) {
+    cudaFuncAttributes at;
+    int device = 0, most = 0;
+    TCP_CUDA(cudaFuncGetAttributes(&at, fn));
+    TCP_CUDA(cudaGetDevice(&device));
+    TCP_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    most -= (int)at.sharedSizeBytes;
+    if (bytes > (size_t)most)
+        return set_error(TCP_ERR_CUDA, "a kernel needs " + std::to_string(bytes) + " bytes of shared memory, the device has " +
+                                           std::to_string(most));
+    TCP_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    return TCP_OK;
+}
+
 static int validate(const tcp_params *p, int nel, int nion) {
     if (!p) return set_error(TCP_ERR_BAD_PARAM, "params is NULL");
     if (nel < 0 || nion < 0 || nel + nion < 2) return set_error(TCP_ERR_BAD_PARAM, "need nel, nion >= 0 and nel+nion >= 2");

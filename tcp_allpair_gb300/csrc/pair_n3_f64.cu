@@ -447,8 +447,8 @@ int n3_f64_prepare(tcp_ctx *c) {
     c->f64_ew_seg = ew;
     c->f64_ei_seg = ei;
     for (int k = 0; k < 4; ++k)
-        TCP_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void *>(f64_kernel(c, k & 1, (k & 2) != 0)),
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f64_smem(ew, ei)));
+        if (int rc = allow_shared(reinterpret_cast<const void *>(f64_kernel(c, k & 1, (k & 2) != 0)), f64_smem(ew, ei)))
+            return rc;
     return TCP_OK;
 }
 

@@ -562,9 +562,6 @@ int ewald_setup(tcp_ctx *c) {
         return set_error(TCP_ERR_NOMEM, "Ewald sum: device allocation failed");
     TCP_CUDA(cudaMemcpyAsync(c->ew_item, items.data(), sizeof(int4) * (size_t)ni, cudaMemcpyHostToDevice, c->stream));
     TCP_CUDA(cudaMemcpyAsync(c->ew_th, th.data(), sizeof(double) * th.size(), cudaMemcpyHostToDevice, c->stream));
-    const int smem = (int)(sizeof(double2) * 3 * (size_t)(nm + 1) * std::max(kEwPart, kEwThreads / 32));
-    TCP_CUDA(cudaFuncSetAttribute(ewald_sfac_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    TCP_CUDA(cudaFuncSetAttribute(ewald_force_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     TCP_CUDA(cudaStreamSynchronize(c->stream));
     return TCP_OK;
 }
@@ -591,6 +588,7 @@ int launch_ewald(tcp_ctx *c, bool energy) {
     a.epart = recip_epart(c);
     a.nblk = c->ew_nblk;
     a.per = c->ew_per;
+    // at most 10 KB: ewald_setup takes no more than 73,728 vectors, indexes up to 26
     const size_t phases = sizeof(double2) * 3 * (size_t)(a.nm + 1);
     const dim3 sgrid(a.nblk, (a.nitem + kEwThreads - 1) / kEwThreads);
     const int nsum = (kEwN1 * a.nitem + 31) / 32, wpb = kEwThreads / 32;

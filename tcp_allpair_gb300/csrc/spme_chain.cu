@@ -410,8 +410,10 @@ int chain_gather_hvp(const ChainArgs &c, const double *phi, const double *dphi, 
 
 // shared-memory limit of the spread for this mesh (once, outside any capture)
 int chain_prepare(const ChainArgs &c) {
-    const int bytes = (int)chain_spread_bytes(c.P, c.k1max);
-#define TCP_LIMIT(K) TCP_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes))
+    const size_t bytes = chain_spread_bytes(c.P, c.k1max);
+    int rc = TCP_OK;
+#define TCP_LIMIT(K) \
+    if (!rc) rc = allow_shared(reinterpret_cast<const void *>(K), bytes)
 #define TCP_CALL(P)                                    \
     do {                                               \
         TCP_LIMIT((chain_spread_kernel<P, float, true>));    \
@@ -422,7 +424,7 @@ int chain_prepare(const ChainArgs &c) {
     TCP_CHAIN_ORDER(TCP_CALL)
 #undef TCP_CALL
 #undef TCP_LIMIT
-    return TCP_OK;
+    return rc;
 }
 
 // bins of a system of n particles and nbins mesh columns (T at most double)

@@ -492,11 +492,10 @@ static int convolve_n(const ChainArgs &c, const FftArgs &f, int systems, cudaStr
 template <int N, typename T, bool BATCH>
 static int prepare_n(int P) {
     constexpr bool D = !BATCH && sizeof(T) == 8;
-    TCP_CUDA(cudaFuncSetAttribute(fft_forward_kernel<N, T, BATCH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_bytes<N, T>(P)));
-    if (D)
-        TCP_CUDA(cudaFuncSetAttribute(fft_forward_kernel<N, T, BATCH, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_bytes<N, T>(P, true)));
-    TCP_CUDA(cudaFuncSetAttribute(fft_inverse_kernel<N, T, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_bytes<N, T>(0)));
-    return TCP_OK;
+    int rc = allow_shared(reinterpret_cast<const void *>(fft_forward_kernel<N, T, BATCH, false>), plane_bytes<N, T>(P));
+    if (!rc && D) rc = allow_shared(reinterpret_cast<const void *>(fft_forward_kernel<N, T, BATCH, D>), plane_bytes<N, T>(P, true));
+    if (!rc) rc = allow_shared(reinterpret_cast<const void *>(fft_inverse_kernel<N, T, BATCH>), plane_bytes<N, T>(0));
+    return rc;
 }
 
 #define TCP_FFT_SIZE(N, CALL)          \

@@ -299,6 +299,7 @@ struct TraceRange {
 // sets the timeout status and returns, and the call reports TCP_ERR_TIMEOUT.
 bool inject_fault(const char *site);
 int cuda_check(cudaError_t e, const char *what);
+int allow_shared(const void *fn, size_t bytes);   // launches of fn may use that much dynamic shared memory
 #define TCP_CUDA(call)                                        \
     do {                                                      \
         cudaError_t _e = (call);                              \
