@@ -191,8 +191,8 @@ __global__ void __launch_bounds__(kGatherThreads) chain_gather_kernel(const Chai
     const int t = t0 + min(p, np - 1);           // idle groups repeat the last particle
     const int m = c.b.order[t];
     const SpmeGeom &g = BATCH ? c.many[c.sys_of[m]] : c.one;
-    const int pk = c.b.base[t], K1 = g.K[0], K2 = g.K[1], K3 = g.K[2];
-    const int bx = pk & 1023, by = (pk >> 10) & 1023, bz = pk >> 20;
+    const int4 base = c.b.base[t];
+    const int K1 = g.K[0], K2 = g.K[1], K3 = g.K[2], bx = base.x, by = base.y, bz = base.z;
     const T *w = sw + (size_t)min(p, np - 1) * 6 * P;
     const T *mesh = static_cast<const T *>(c.mesh) + g.mesh_off;
     int xs[P];
@@ -269,8 +269,9 @@ __global__ void __launch_bounds__(kGatherThreads) chain_gather_hvp_kernel(const 
         }
     }
     __syncthreads();
-    const int pk = c.b.base[t0 + p], K1 = g.K[0], K2 = g.K[1], K3 = g.K[2];
-    const int bx = pk & 1023, by = (pk >> 10) & 1023, bz = pk >> 20;
+    const int4 base = c.b.base[t0 + p];
+    const int K1 = g.K[0], K2 = g.K[1], K3 = g.K[2];
+    const int bx = base.x, by = base.y, bz = base.z;
     const double *sx = sw[p][0], *sy = sw[p][1], *sz = sw[p][2];
     const double w0 = w[m], w1 = w[(size_t)c.n + m], w2 = w[2 * (size_t)c.n + m];
     double h[3] = {0.0, 0.0, 0.0};
@@ -434,8 +435,8 @@ int chain_alloc(SpreadBins &b, int n, int nbins, int order) {
         {(void **)&b.count, sizeof(int) * rounds}, {(void **)&b.start, sizeof(int) * ((size_t)nbins + 1)},
         {(void **)&b.bsum, sizeof(int) * ((size_t)nbins / kScanBlock + 1)}, {(void **)&b.rank, sizeof(int) * (size_t)n},
         {(void **)&b.list, sizeof(int) * (size_t)n}, {(void **)&b.order, sizeof(int) * (size_t)n},
-        {(void **)&b.bin, sizeof(int) * (size_t)n}, {(void **)&b.base_m, sizeof(int) * (size_t)n},
-        {(void **)&b.base, sizeof(int) * (size_t)n}, {&b.arg, sizeof(double) * 3 * (size_t)n},
+        {(void **)&b.bin, sizeof(int) * (size_t)n}, {(void **)&b.base_m, sizeof(int4) * (size_t)n},
+        {(void **)&b.base, sizeof(int4) * (size_t)n}, {&b.arg, sizeof(double) * 3 * (size_t)n},
         {&b.q_m, sizeof(double) * (size_t)n}, {&b.q, sizeof(double) * (size_t)n},
         {&b.ew, sizeof(double) * 6 * (size_t)order * (size_t)n}};
     for (auto &w : want)

@@ -39,8 +39,6 @@ __device__ __forceinline__ int bin_axis(double x, double hL, double KL, int K, i
     return wrapi(iu - (P - 3), K);
 }
 
-__device__ __forceinline__ int pack_base(int bx, int by, int bz) { return bx | (by << 10) | (bz << 20); }
-
 // Exclusive prefix sum of count[0..nbins) into start[0..nbins] by one CTA;
 // the counts are left at zero for the next binning.  Sixteen bins per thread
 // and round (count is padded to whole rounds).
@@ -90,7 +88,7 @@ __device__ __forceinline__ void bin_store(const SpreadBins &b, int m, int n, con
     const int bin = bin_off + by + K2 * bz;
     b.rank[m] = atomicAdd(&b.count[bin], 1);
     b.bin[m] = bin;
-    b.base_m[m] = pack_base(bx, by, bz);
+    b.base_m[m] = make_int4(bx, by, bz, 0);
     T *a = static_cast<T *>(b.arg);
     for (int d = 0; d < 3; ++d) a[(size_t)d * n + m] = (T)arg[d];
     static_cast<T *>(b.q_m)[m] = (T)q;
@@ -116,7 +114,7 @@ constexpr int kStageBins = 136;          // bins that reach one CTA's rows: at m
 template <typename T>
 struct StageBuf {
     T *w;                // [kStage][2 P]: W_x, then q W_z W_y (dipoles: [kStage][4 P], W_x, W_x', then their factors)
-    int *bx;             // [kStage] base x and y
+    int *bx;             // [kStage] base x, and base y as the number of its bin among those of run (bits 24 and up)
     int2 *run;           // [kStageBins] list range of each bin
 };
 template <typename T>
@@ -186,7 +184,9 @@ __device__ __forceinline__ void chain_rows(const ChainArgs &c, const SpmeGeom &g
                             o[P + j] = qz * w[2 * P + j];
                         }
                     }
-                    st.bx[e] = c.b.base[c0 + e];
+                    const int4 base = c.b.base[c0 + e];
+                    const int ybin = base.y - blo >= K2 ? base.y - blo - K2 : base.y - blo;
+                    st.bx[e] = (int)((unsigned)ybin << 24) | base.x;
                 }
                 group_sync(bar, NG);
                 if (grp < RG)
@@ -204,9 +204,9 @@ __device__ __forceinline__ void chain_rows(const ChainArgs &c, const SpmeGeom &g
 #pragma unroll 1
                             for (int e = e0; e < e1; ++e) {
                                 const int nx = st.bx[min(e + 1, e1 - 1)];
-                                int jy = y - ((pk >> 10) & 1023);
+                                int jy = y - blo - (int)((unsigned)pk >> 24);
                                 jy += jy < 0 ? K2 : 0;
-                                int x = (pk & 1023) + l;
+                                int x = (pk & 0xffffff) + l;
                                 x -= x >= K1 ? K1 : 0;
                                 const T *w = st.w + e * (DIP ? 4 : 2) * P;
                                 const T v = w[(DIP ? 2 : 1) * P + jy], wx = w[l];

@@ -124,8 +124,9 @@ namespace tcp {
 // are by particle, the others by place in the sorted order.
 struct SpreadBins {
     int *count, *start, *bsum;   // per bin; count is zero between binnings
-    int *rank, *bin, *base_m;    // slot in the bin, bin, packed base indexes (10 bits each)
-    int *list, *order, *base;    // particles by bin, the same in particle order inside each bin
+    int *rank, *bin;             // slot in the bin, bin
+    int *list, *order;           // particles by bin, the same in particle order inside each bin
+    int4 *base_m, *base;         // base indexes x, y, z
     void *arg, *q_m, *q, *ew;    // [3][n] spline arguments, charges, [n][3][2 P] weights and derivatives
 };
 // One system's mesh and charges as the chain kernels need them.
