@@ -421,9 +421,11 @@ bool n3_f64_applicable(const tcp_ctx *c) {
 
 int n3_f64_grid(const tcp_ctx *c) { return std::max(1, c->num_sms); }   // the tables: one CTA per SM
 
+// The table ends past the cut-off by more than the rounding of the FP32
+// argument: pairs at its end get no Ewald term.
 int ewald_octaves(const tcp_ctx *c) {
     int top = kTabLow + 1;
-    while (top < kEwTopMax && std::ldexp(1.0, top) < c->pc.alpha2 * c->rc2) ++top;
+    while (top < kEwTopMax && std::ldexp(1.0, top) < c->pc.alpha2 * c->rc2 * (1.0 + 1e-6)) ++top;
     return top - kTabLow;
 }
 
