@@ -462,7 +462,7 @@ struct AdjPair {
 };
 template <int KIND, bool HVP, bool CUBIC>
 __device__ __forceinline__ AdjPair adj_pair_f64(const AdjArgs &a, const AdjFast &f, const uint4 *ew, const uint4 *ei,
-                                                const F64Tab &tb, double hq, const F64Pos &xi, const double (&wi)[3], int j,
+                                                const int *oct, const F64Tab &tb, double hq, const F64Pos &xi, const double (&wi)[3], int j,
                                                 bool live, double &sum) {
     constexpr int NEI = HVP ? 3 : 1;
     const F64Fast &p = f.p;
@@ -480,17 +480,16 @@ __device__ __forceinline__ AdjPair adj_pair_f64(const AdjArgs &a, const AdjFast 
     const unsigned xb = __float_as_uint(r2f * p.kxf), yb = __float_as_uint(r2f * p.kyf);
     const bool near = KIND != 0 && q.ok && yb < p.ei_hi;
     const bool any_near = KIND != 0 && __any_sync(0xffffffffu, near);
-    const bool need = (HVP && q.ok && xb < kTabLowBits) || (near && yb < kTabLowBits);
+    const bool need = (HVP && q.ok && (xb < kEwLowBits || xb >= p.ew_hi)) || (near && yb < kEiLowBits);
     double g1 = 0.0, g2 = 0.0, gl = 0.0;     // units of a^3, a^5; gl (HVP) or dl
     F64At y;
-    if (any_near) y = f64_at<kEiBits>(ei, yb, p.ei_hi, r2, p.ky, r2f, p.kyf);
+    if (any_near) y = ei_at(ei, oct, yb, p.ei_hi, r2, p.ky);
     if (HVP) {
-        const bool in = q.ok && xb < p.ew_hi;
-        const F64At x = f64_at<kEwBits>(ew, xb, p.ew_hi, r2, p.kx, r2f, p.kxf);
+        const F64At x = ew_at(ew, xb, p.ew_hi, r2, p.kx);
         g1 = ew_poly(x, p.ew_seg, 0);
         g2 = ew_poly(x, p.ew_seg, 1);
-        g1 = in ? g1 : 0.0;
-        g2 = in ? g2 : 0.0;
+        g1 = q.ok ? g1 : 0.0;
+        g2 = q.ok ? g2 : 0.0;
         if (any_near) {
             g1 = fma(near ? p.cf : 0.0, ei_poly<true>(y, p.ei_seg, 0, NEI), g1);
             g2 = fma(near ? f.c2 : 0.0, ei_poly<true>(y, p.ei_seg, 1, NEI), g2);
@@ -528,12 +527,12 @@ __device__ __forceinline__ AdjPair adj_pair_f64(const AdjArgs &a, const AdjFast 
 // The near pairs of 32 i-particles with up to 128 j-particles, as f64_near takes them.
 template <int KIND, bool HVP, bool CUBIC>
 __device__ __forceinline__ void adj_near_f64(const AdjArgs &a, const AdjFast &f, const uint4 *ew, const uint4 *ei,
-                                             const F64Tab &tb, double hq, int i0, const F64Pos &xi, const double (&wi)[3],
+                                             const int *oct, const F64Tab &tb, double hq, int i0, const F64Pos &xi, const double (&wi)[3],
                                              int j0, F64Mask m, double (&hi)[3], double &sum) {
 #pragma unroll 1
     while (__all_sync(0xffffffffu, (m.lo | m.hi) != 0)) {
         const int j = j0 + mask_pop(m);
-        const AdjPair q = adj_pair_f64<KIND, HVP, CUBIC>(a, f, ew, ei, tb, hq, xi, wi, j, true, sum);
+        const AdjPair q = adj_pair_f64<KIND, HVP, CUBIC>(a, f, ew, ei, oct, tb, hq, xi, wi, j, true, sum);
         if (HVP) {
 #pragma unroll
             for (int k = 0; k < 3; ++k) hi[k] += q.t[k];
@@ -553,7 +552,7 @@ __device__ __forceinline__ void adj_near_f64(const AdjArgs &a, const AdjFast &f,
 #pragma unroll
             for (int k = 0; k < 3; ++k) w[k] = __shfl_sync(0xffffffffu, wi[k], t.lane);
         const int j = j0 + t.bit;
-        const AdjPair q = adj_pair_f64<KIND, HVP, CUBIC>(a, f, ew, ei, tb, hq, x, w, j, t.live, sum);
+        const AdjPair q = adj_pair_f64<KIND, HVP, CUBIC>(a, f, ew, ei, oct, tb, hq, x, w, j, t.live, sum);
         if (HVP && q.ok) {
             add_force(f.hw + i0 + t.lane, a.n, q.t[0], q.t[1], q.t[2]);
             add_force(f.hw + j, a.n, -q.t[0], -q.t[1], -q.t[2]);
@@ -568,9 +567,11 @@ __global__ void __launch_bounds__(kF64Threads, 1) adj_f64_kernel(const AdjArgs a
     __shared__ __align__(8) uint64_t bar;
     __shared__ double red[32];
     __shared__ F64Tab tab;
+    __shared__ int oct[kEiOct];
     constexpr int NEI = HVP ? 3 : 1;
     const F64Fast &p = f.p;
     const int tid = threadIdx.x, lane = tid & 31;
+    if (tid < kEiOct) oct[tid] = p.ei_oct[tid];
     const uint32_t b0 = (uint32_t)p.ew_seg * ew_vec(2) * 16u, b1 = (uint32_t)p.ei_seg * ei_vec(NEI) * 16u;
     if (tid == 0) {
         mbar_init(&bar, 1);
@@ -609,9 +610,9 @@ __global__ void __launch_bounds__(kF64Threads, 1) adj_f64_kernel(const AdjArgs a
             if (!HVP && r.pt != 1) continue;     // the e-i chunks only
             const F64Mask m = f64_mask(p, a.xl, xi, lane < icnt, r.j0, r.nj, r.diag, part);
             if (EI != 0 && r.pt == 1)
-                adj_near_f64<EI, HVP, CUBIC>(a, f, ew, ei, tab, f.hq[1], istart, xi, wi, r.j0, m, hi, total);
+                adj_near_f64<EI, HVP, CUBIC>(a, f, ew, ei, oct, tab, f.hq[1], istart, xi, wi, r.j0, m, hi, total);
             else if (HVP)
-                adj_near_f64<0, HVP, CUBIC>(a, f, ew, ei, tab, f.hq[r.pt], istart, xi, wi, r.j0, m, hi, total);
+                adj_near_f64<0, HVP, CUBIC>(a, f, ew, ei, oct, tab, f.hq[r.pt], istart, xi, wi, r.j0, m, hi, total);
         }
         if (HVP && lane < icnt) add_force(f.hw + istart + lane, a.n, hi[0], hi[1], hi[2]);
     }
@@ -794,7 +795,7 @@ static AdjF64Kernel adj_f64_of(bool hvp, bool cubic) {
 }
 
 // The FP64 tile form; *done = 0 where its tables do not fit in shared memory
-// (Deutsch with alpha rc > 4: the item form below takes it).
+// (an e-i model with alpha rc > 4.2: the item form below takes it).
 static int launch_adj_f64(tcp_ctx *c, const AdjArgs &a, const double *w, double *hw, int *done) {
     const bool hvp = w != nullptr;
     const int k = hvp ? 0 : 1, eim = c->p.ei_model;
@@ -806,7 +807,7 @@ static int launch_adj_f64(tcp_ctx *c, const AdjArgs &a, const double *w, double 
     if (!T.dev) {
         std::vector<F64Vec> t;
         T.ew = T.ei = 0;
-        if (hvp) t = f64_table(TCP_EI_COULOMB, kHvpEw, 2, ewald_octaves(c), &T.ew);
+        if (hvp) t = f64_table(TCP_EI_COULOMB, kHvpEw, 2, ewald_segments(c), &T.ew);
         if (eim != TCP_EI_COULOMB) {
             const std::vector<F64Vec> m = f64_table(eim, hvp ? kHvpEi : kDlEi, hvp ? 3 : 1, 0, &T.ei);
             t.insert(t.end(), m.begin(), m.end());
@@ -836,7 +837,7 @@ static int launch_adj_f64(tcp_ctx *c, const AdjArgs &a, const double *w, double 
     for (int t = 0; t < 3; ++t) f.hq[t] = kEps * pc.qq[t] * al * al * al;
     f.qgl = kEps * pc.qq[1] * f.kgl * L;
     f.qdl = kEps * pc.qq[1] * f.kdl;
-    if (!hvp) f.p.near2 = std::min(f.p.near2, f64_near2(pc, std::sqrt(std::ldexp(1.0, (T.ei >> kEiBits) + kTabLow) / f.p.ky)));   // of the e-i table's end
+    if (!hvp) f.p.near2 = std::min(f.p.near2, f64_near2(pc, std::sqrt(f64_segment_end(eim, T.ei - 1) / f.p.ky)));   // of the e-i table's end
     const int grid = (int)std::min<long long>(c->num_sms, (f.p.items + kF64Warps - 1) / kF64Warps);
     TCP_CUDA(cudaMemsetAsync(c->counter, 0, sizeof(unsigned), c->stream));
     fn<<<grid, kF64Threads, T.bytes, c->stream>>>(a, f, c->counter, c->status);

@@ -17,21 +17,37 @@ constexpr int kF64Threads = 384;
 constexpr int kF64Warps = kF64Threads / 32;
 
 // ---- tables ---------------------------------------------------------------------
-// Segments of an argument x in [2^-6, 2^top): the leading kEwBits (kEiBits)
-// mantissa bits of x.  Per segment and function the Taylor coefficients c0..c3
-// (Ewald) or c0..c4 (e-i) in FP64 and the magnitudes of the four next ones in
-// FP32, in 16-byte vectors [vector][segment] so that lanes on different
-// segments use different banks.  A table holds several functions:
+// Segments of the argument, a power of two of them per octave (the leading
+// mantissa bits select one).  Per segment and function the Taylor coefficients
+// c0..c3 (Ewald) or c0..c4 (e-i) in FP64 and the four next ones in FP32, in
+// 16-byte vectors [vector][segment] so that lanes on different segments use
+// different banks.  A table holds several functions:
 //   Ewald   c0 c1 | c2 c3 | t4 .. t7           per function
 //   e-i     c0 c1 | c2 c3 | c4 t5 t6           per function, then t7 t8 of two functions per vector
-constexpr int kEwBits = 7, kEiBits = 5;
+//
+// Where the functions fall as e^{-x} the terms do so with the segment's width,
+// not with its width over x: the octaves from there on have more segments, so
+// that the FP32 terms stay below 2^-24 of the sum.  Largest relative errors of
+// all the functions (100 to 150 random arguments an octave, against 45 digits),
+// and with the first octave's number of segments in every octave:
+//   Ewald    x < 4 3e-16, < 8 5e-16, < 16 4e-16 (1.5e-14), < 32 5e-15 (3e-13)
+//   Kelbg    y < 4 1.5e-15, < 16 1.1e-15 (2.7e-13), < 32 9e-16 (3e-11), < 64 6e-14 (1e-8)
+//   Deutsch  s < 8 5e-15, < 23 1.1e-15 (4e-13), < 32 3e-12, < 45 3e-11
+// An argument rounded to FP64 alone makes them uncertain by x 2^-53.  The last
+// octaves are coarser than that, for shared memory: there the functions are
+// below e^{-32} (Kelbg) and e^{-22} (Deutsch), so that a pair's force and
+// energy do not feel it; the derivatives with respect to lambda of a system
+// with no nearer e-i pair do.
+constexpr int kEwLow = -6, kEwMid = 3, kEwTop = 5;   // 2^kEwBits segments an octave, twice that from 2^kEwMid on
+constexpr int kEwBits = 7;
+constexpr unsigned kEwLowBits = (127 + kEwLow) << 23, kEwMidBits = (127 + kEwMid) << 23;
+constexpr int kEiLow = -1, kEiOct = 12;              // octaves of the longer one; F64Fast::ei_oct
+constexpr unsigned kEiLowBits = (127 + kEiLow) << 23;
 __host__ __device__ constexpr int ew_vec(int nf) { return 3 * nf; }
 __host__ __device__ constexpr int ei_vec(int nf) { return 3 * nf + (nf + 1) / 2; }
-constexpr int kTabLow = -6;              // the tables start at 2^-6
-constexpr unsigned kTabLowBits = (127 + kTabLow) << 23;
-constexpr int kEwTopMax = 6;             // Ewald: erfc(ar) is 0 beyond ar = 8 (1e-29 of the pair's 1/r)
-constexpr int kKelbgTop = 6;             // Kelbg: e^{-64} = 1.6e-28
-constexpr int kDeutschTop = 11;          // Deutsch: e^{-45} = 2.6e-20 of the pair's Coulomb term
+// Below the tables, and past the end of the Ewald one (a^2 r^2 = 32), the
+// general form takes the pair.  The e-i functions are 0 from the end of theirs
+// on: e^{-64} = 1.6e-28 (Kelbg), e^{-45} = 2.6e-20 (Deutsch) of the Coulomb term.
 
 // The functions.  Ewald (x = a^2 r^2): the Taylor families of B_n, B_0 =
 // erfc(sqrt x)/sqrt x; Deutsch (z = r^2/rs^2): A_n, A_0 = e^{-s}/s, s = sqrt z;
@@ -45,15 +61,16 @@ enum F64Func {
 };
 
 // Host side (pair_n3_f64.cu): the vectors of one table for the functions
-// given, the first `octaves` of it (0: all); *nseg: its segments.
+// given, the first `segments` of it (0: all); *nseg: its segments.
 struct F64Vec {
     union {
         double d[2];
         float f[4];
     };
 };
-std::vector<F64Vec> f64_table(int model, const int *funcs, int nf, int octaves, int *nseg);
-int ewald_octaves(const tcp_ctx *c);   // octaves of the Ewald table that the cut-off reaches
+std::vector<F64Vec> f64_table(int model, const int *funcs, int nf, int segments, int *nseg);
+double f64_segment_end(int model, int k);   // upper end of segment k
+int ewald_segments(const tcp_ctx *c);       // segments of the Ewald table that the cut-off reaches
 
 // What the kernel needs besides PairConsts.  Lengths in units of the box where
 // it is cubic (the fixed-point differences unscaled), in A otherwise.
@@ -61,6 +78,7 @@ struct F64Fast {
     const uint4 *tab;        // Ewald vectors, then e-i vectors
     int ew_seg, ei_seg;      // segments per vector
     unsigned ew_hi, ei_hi;   // float bits of the table ends
+    int ei_oct[kEiOct];      // per octave of the e-i table: shift of the segment's bits | 32 x offset
     double kx, ky;           // r^2 -> a^2 r^2, r^2/lambda^2 (or /rs^2)
     float kxf, kyf;
     double rc2;              // cut-off^2 (r^2 < rc2)
@@ -111,23 +129,40 @@ __device__ __forceinline__ float narrow(double x) {
 __device__ __forceinline__ double2 lds2(const uint4 *p) { return *reinterpret_cast<const double2 *>(p); }
 __device__ __forceinline__ float4 lds4(const uint4 *p) { return *reinterpret_cast<const float4 *>(p); }
 
-// Where an argument lies in a table: vector offset of its segment, distance to
-// the centre in FP64 and FP32.  xb: the bits of the FP32 argument.
+// the same for either sign
+__device__ __forceinline__ float narrow_signed(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), mag = hi & 0x7fffffffu;
+    const unsigned b = __funnelshift_l((unsigned)__double2loint(x), mag, 3) + 0x40000000u;
+    return __uint_as_float((mag < 0x38100000u ? 0u : b) | (hi & 0x80000000u));
+}
+
+// Where an argument lies in a table: vector offset of its segment, distance h
+// to the centre in FP64, and in FP32 from that (a difference in FP32 would be
+// off by 2^-23 x).  xb: the bits of the FP32 argument; sh, base: the segment is
+// (xb >> sh) + base.
 struct F64At {
     const uint4 *t;
     double h;
     float hf;
 };
-template <int BITS>
-__device__ __forceinline__ F64At f64_at(const uint4 *tab, unsigned xb, unsigned hi, double r2, double k, float r2f,
-                                        float kf) {
-    const unsigned xi = min(max(xb, kTabLowBits), hi - 1u);
-    const unsigned cb = (xi & ~((1u << (23 - BITS)) - 1u)) | (1u << (22 - BITS));   // segment centre
+__device__ __forceinline__ F64At f64_at(const uint4 *tab, unsigned xi, int sh, int base, double r2, double k) {
+    const unsigned q = xi >> sh;
     F64At a;
-    a.t = tab + ((xi - kTabLowBits) >> (23 - BITS));
-    a.h = fma(r2, k, -widen(__uint_as_float(cb)));
-    a.hf = fmaf(r2f, kf, -__uint_as_float(cb));
+    a.t = tab + ((int)q + base);
+    a.h = fma(r2, k, -widen(__uint_as_float((2u * q + 1u) << (sh - 1))));
+    a.hf = narrow_signed(a.h);
     return a;
+}
+__device__ __forceinline__ F64At ew_at(const uint4 *tab, unsigned xb, unsigned hi, double r2, double k) {
+    constexpr int SH = 23 - kEwBits, MID = (kEwMid - kEwLow) << kEwBits;
+    const unsigned xi = min(max(xb, kEwLowBits), hi - 1u);
+    const bool low = xi < kEwMidBits;
+    return f64_at(tab, xi, low ? SH : SH - 1, low ? -(int)(kEwLowBits >> SH) : MID - (int)(kEwMidBits >> (SH - 1)), r2, k);
+}
+__device__ __forceinline__ F64At ei_at(const uint4 *tab, const int *oct, unsigned yb, unsigned hi, double r2, double k) {
+    const unsigned yi = min(max(yb, kEiLowBits), hi - 1u);
+    const int o = oct[(yi - kEiLowBits) >> 23];
+    return f64_at(tab, yi, o & 31, o >> 5, r2, k);
 }
 
 // function f of an Ewald table of n segments

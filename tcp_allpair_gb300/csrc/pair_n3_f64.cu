@@ -7,13 +7,14 @@
 // and SM quarter (596e9 FMA/s measured; conversions to or from FP64 cost the
 // same slot), while the other pipes have 64 issue slots in that time, and one
 // warp's dependent chain already reaches 94 % of the rate.  So everything that
-// can leave the FP64 pipe without losing a bit of the result does:
+// can leave the FP64 pipe without a loss in the result does:
 //  * the radial functions of force.f90:104-106, 135-139 are Taylor
 //    polynomials in x = a^2 r^2 around the centre of the segment that the
-//    leading bits of x select (128 segments per octave, tables in shared
-//    memory): F(x) = (erfc(ar) + 2ar/sqrt(pi) e^{-x}) / (ar)^3 and
-//    U(x) = erfc(ar)/(ar).  With |h| <= 2^-8 x the terms from h^4 on are
-//    below 2^-31 of the sum and are evaluated in FP32 without loss; the
+//    leading bits of x select (128 segments per octave, 256 above x = 8; tables
+//    in shared memory): F(x) = (erfc(ar) + 2ar/sqrt(pi) e^{-x}) / (ar)^3 and
+//    U(x) = erfc(ar)/(ar).  The terms from h^4 on are below 2^-24 of the sum
+//    and are evaluated in FP32, whose rounding then weighs less than that of x
+//    (the errors stand in pair_f64.cuh); the
 //    others are four FMAs.  No square root, reciprocal, exponential or
 //    erfc per pair.  The e-i terms (Kelbg: e^{-y} y^{-3/2} and
 //    sqrt(pi) erfc(sqrt y) - e^{-y} y^{-1/2}, y = r^2/lambda^2; Deutsch:
@@ -26,8 +27,8 @@
 //    to a bin edge.
 // That leaves 20 FP64 operations per Coulomb pair (r^2 3, h 1, the two
 // polynomials 8, energy 1, forces 7), 59 with the table-driven exp, rsqrt and
-// erfcx of pair_math.cuh, which stay for the pairs below the tables (ar < 1/8,
-// or r < lambda/8 or rs/8: about one in 10^5) and for the ordered-pair kernel.
+// erfcx of pair_math.cuh, which stay for the pairs outside the tables (ar < 1/8
+// or > 5.6, r < 0.7 lambda or rs) and for the ordered-pair kernel.
 //
 // And only the pairs inside rc, 52 % of all at rc = L/2, are evaluated: a warp
 // finds them with FP32 arithmetic as a bit mask per lane (pair_f64.cuh), each
@@ -128,22 +129,43 @@ static void taylor_of(int model, int func, long double xc, long double *out) {
     }
 }
 
-static long double segment_centre(int k, int bits) {
-    const int oct = kTabLow + (k >> bits), m = k & ((1 << bits) - 1);
-    return ldexpl(1.0L + (m + 0.5L) / (1 << bits), oct);
+// Octaves of the tables: the lowest, and how many bits select the segments of each.
+struct F64Octaves {
+    int low, n, bits[kEiOct];
+};
+static const F64Octaves &octaves_of(int model) {
+    static const F64Octaves ew = {kEwLow, kEwTop - kEwLow, {7, 7, 7, 7, 7, 7, 7, 7, 7, 8, 8}};
+    static const F64Octaves kelbg = {kEiLow, 7, {5, 5, 5, 6, 6, 7, 7}};
+    static const F64Octaves deutsch = {kEiLow, 12, {5, 5, 5, 5, 5, 5, 5, 6, 6, 6, 5, 5}};
+    return model == TCP_EI_COULOMB ? ew : (model == TCP_EI_KELBG ? kelbg : deutsch);
 }
+
+static int segments_of(int model) {
+    const F64Octaves &o = octaves_of(model);
+    int n = 0;
+    for (int k = 0; k < o.n; ++k) n += 1 << o.bits[k];
+    return n;
+}
+
+// the point at fraction f of segment k
+static double segment_at(int model, int k, double f) {
+    const F64Octaves &o = octaves_of(model);
+    int q = 0;
+    while (q + 1 < o.n && k >= 1 << o.bits[q]) k -= 1 << o.bits[q++];
+    return std::ldexp(1.0 + (k + f) / (1 << o.bits[q]), o.low + q);
+}
+
+double f64_segment_end(int model, int k) { return segment_at(model, k, 1.0); }
 
 // One function over all its octaves, [vector][segment]: three vectors, and for
 // the e-i families a fourth with t7, t8.  Written once per process.
 static std::vector<F64Vec> build_function(int model, int func) {
     const bool ew = model == TCP_EI_COULOMB;
-    const int bits = ew ? kEwBits : kEiBits;
-    const int top = ew ? kEwTopMax : (model == TCP_EI_KELBG ? kKelbgTop : kDeutschTop);
-    const int n = (top - kTabLow) << bits;
+    const int n = segments_of(model);
     std::vector<F64Vec> t((size_t)4 * n);
     for (int s = 0; s < n; ++s) {
         long double c[kTaylor];
-        taylor_of(model, func, segment_centre(s, bits), c);
+        taylor_of(model, func, segment_at(model, s, 0.5), c);
         t[s].d[0] = (double)c[0];
         t[s].d[1] = (double)c[1];
         t[n + s].d[0] = (double)c[2];
@@ -170,10 +192,10 @@ static const std::vector<F64Vec> &function_of(int model, int func) {
     return tab[m][func];
 }
 
-std::vector<F64Vec> f64_table(int model, const int *funcs, int nf, int octaves, int *nseg) {
+std::vector<F64Vec> f64_table(int model, const int *funcs, int nf, int segments, int *nseg) {
     const bool ew = model == TCP_EI_COULOMB;
     const int full = (int)function_of(model, funcs[0]).size() / 4;
-    const int n = octaves > 0 ? std::min(full, octaves << (ew ? kEwBits : kEiBits)) : full;
+    const int n = segments > 0 ? std::min(full, segments) : full;
     std::vector<F64Vec> t((size_t)(ew ? ew_vec(nf) : ei_vec(nf)) * n);
     for (int f = 0; f < nf; ++f) {
         const std::vector<F64Vec> &q = function_of(model, funcs[f]);
@@ -214,6 +236,7 @@ __device__ __noinline__ void n3_pair_general(const PairConsts &c, double r2, dou
 
 struct F64Shared {
     const uint4 *ew, *ei;
+    const int *oct;          // F64Fast::ei_oct
     const F64Tab *tb;
     unsigned *hist;          // RDF: this pair type's bins
 };
@@ -225,21 +248,20 @@ __device__ __forceinline__ double n3_pair_f64(const F64Fast &p, const PairConsts
                                               const F64Shared &sh) {
     const float r2f = narrow(r2);
     const unsigned xb = __float_as_uint(r2f * p.kxf);
-    bool need = ok && xb < kTabLowBits;                   // below the tables
-    const bool in = ok && xb < p.ew_hi;
-    const F64At x = f64_at<kEwBits>(sh.ew, xb, p.ew_hi, r2, p.kx, r2f, p.kxf);
+    bool need = ok && (xb < kEwLowBits || xb >= p.ew_hi);   // outside the Ewald table
+    const F64At x = ew_at(sh.ew, xb, p.ew_hi, r2, p.kx);
     double w = ew_poly(x, p.ew_seg, 0), u = 0.0;
-    w = in ? w : 0.0;
+    w = ok ? w : 0.0;
     if (ENERGY) {
         u = ew_poly(x, p.ew_seg, 1);
-        u = in ? u : 0.0;
+        u = ok ? u : 0.0;
     }
     if (KIND != 0) {
         const unsigned yb = __float_as_uint(r2f * p.kyf);
         const bool near = ok && yb < p.ei_hi;
         if (__any_sync(0xffffffffu, near)) {
-            need = need || (near && yb < kTabLowBits);
-            const F64At y = f64_at<kEiBits>(sh.ei, yb, p.ei_hi, r2, p.ky, r2f, p.kyf);
+            need = need || (near && yb < kEiLowBits);
+            const F64At y = ei_at(sh.ei, sh.oct, yb, p.ei_hi, r2, p.ky);
             w = fma(near ? p.cf : 0.0, ei_poly<true>(y, p.ei_seg, 0, 2), w);
             if (ENERGY) u = fma(near ? p.cu : 0.0, ei_poly<KIND == 1>(y, p.ei_seg, 1, 2), u);
         }
@@ -336,7 +358,9 @@ __global__ void __launch_bounds__(kF64Threads, 1) pair_n3_f64_kernel(const N3Arg
     __shared__ double red[32];
     __shared__ unsigned hist[RDF ? 3 * kNbin : 1];
     __shared__ F64Tab tab;
+    __shared__ int oct[kEiOct];
     const int tid = threadIdx.x, lane = tid & 31;
+    if (tid < kEiOct) oct[tid] = p.ei_oct[tid];
     if (RDF)
         for (int k = tid; k < 3 * kNbin; k += kF64Threads) hist[k] = 0u;
     if (tid == 0) {
@@ -359,6 +383,7 @@ __global__ void __launch_bounds__(kF64Threads, 1) pair_n3_f64_kernel(const N3Arg
     F64Shared sh;
     sh.ew = tabs;
     sh.ei = tabs + p.ew_seg * ew_vec(2);
+    sh.oct = oct;
     sh.tb = &tab;
     sh.hist = nullptr;
     double etot = 0.0;
@@ -422,11 +447,16 @@ bool n3_f64_applicable(const tcp_ctx *c) {
 int n3_f64_grid(const tcp_ctx *c) { return std::max(1, c->num_sms); }   // the tables: one CTA per SM
 
 // The table ends past the cut-off by more than the rounding of the FP32
-// argument: pairs at its end get no Ewald term.
-int ewald_octaves(const tcp_ctx *c) {
-    int top = kTabLow + 1;
-    while (top < kEwTopMax && std::ldexp(1.0, top) < c->pc.alpha2 * c->rc2 * (1.0 + 1e-6)) ++top;
-    return top - kTabLow;
+// argument: pairs at its end would take the general form.
+int ewald_segments(const tcp_ctx *c) {
+    const F64Octaves &o = octaves_of(TCP_EI_COULOMB);
+    const double x = c->pc.alpha2 * c->rc2 * (1.0 + 1e-6);
+    int n = 0;
+    for (int q = 0; q < o.n; ++q) {
+        const double low = std::ldexp(1.0, o.low + q), part = std::min(std::max(x / low - 1.0, 0.0), 1.0);
+        n += (int)std::ceil(part * (1 << o.bits[q]));
+    }
+    return std::max(n, 1 << kEwBits);
 }
 
 static const int kPairFuncs[] = {kFuncF, kFuncU};
@@ -436,7 +466,7 @@ static size_t f64_smem(int ew_seg, int ei_seg) { return 16 * ((size_t)ew_seg * e
 // the pair constants, outside any stream capture).
 int n3_f64_prepare(tcp_ctx *c) {
     int ew = 0, ei = 0;
-    std::vector<F64Vec> t = f64_table(TCP_EI_COULOMB, kPairFuncs, 2, ewald_octaves(c), &ew);
+    std::vector<F64Vec> t = f64_table(TCP_EI_COULOMB, kPairFuncs, 2, ewald_segments(c), &ew);
     if (c->p.ei_model != TCP_EI_COULOMB) {
         const std::vector<F64Vec> m = f64_table(c->p.ei_model, kPairFuncs, 2, 0, &ei);
         t.insert(t.end(), m.begin(), m.end());
@@ -471,8 +501,21 @@ F64Fast f64_args(const tcp_ctx *c, int ew_seg, int ei_seg) {
     std::memset(&p, 0, sizeof p);
     p.ew_seg = ew_seg;
     p.ei_seg = ei_seg;
-    p.ew_hi = kTabLowBits + ((unsigned)(p.ew_seg >> kEwBits) << 23);
-    p.ei_hi = kTabLowBits + ((unsigned)(p.ei_seg >> kEiBits) << 23);
+    auto end_bits = [](int model, int segments) {
+        const float e = (float)f64_segment_end(model, segments - 1);
+        unsigned b;
+        std::memcpy(&b, &e, sizeof b);
+        return b;
+    };
+    p.ew_hi = ew_seg ? end_bits(TCP_EI_COULOMB, ew_seg) : kEwLowBits + 1;
+    if (ei_seg) {
+        p.ei_hi = end_bits(c->p.ei_model, ei_seg);
+        const F64Octaves &o = octaves_of(c->p.ei_model);
+        for (int q = 0, n = 0; q < o.n; n += 1 << o.bits[q++]) {
+            const int sh = 23 - o.bits[q];
+            p.ei_oct[q] = sh + 32 * (n - (int)((unsigned)(127 + o.low + q) << o.bits[q]));
+        }
+    }
     p.kx = pc.alpha2 * (L * L);
     p.kxf = (float)p.kx;
     p.to_a2 = L * L;
