@@ -850,6 +850,7 @@ static int launch_adj_f64(tcp_ctx *c, const AdjArgs &a, const double *w, double 
 // Newton-3 form unless TCP_FLAG_DETERMINISTIC asks for the ordered-pair sums
 // (which add their rows in a fixed pattern).
 static int launch_adj_pair(tcp_ctx *c, const double *w, double *hw) {
+    if (inject_fault("adj_pair")) return set_error(TCP_ERR_NOMEM, "injected: derivative tables failed");
     AdjArgs a = adj_args(c, w, hw);
     if (!(c->flags & TCP_FLAG_DETERMINISTIC)) {
         const bool f32 = c->p.precision == TCP_PREC_FP32C;

@@ -658,8 +658,11 @@ int launch_spme_hvp(tcp_ctx *c, const double *w, double *hw, const std::function
     c->launches += chain_bin(chain, c->x, c->stream2);
     c->launches += chain_sort(chain, c->stream2);
     TCP_CUDA(cudaEventRecord(c->ev_pair_ready, c->stream2));
-    int rc = real();
-    for (int pass = 0; pass < 2 && !rc; ++pass) {
+    if (int rc = real()) {
+        TCP_CUDA(cudaStreamWaitEvent(c->stream, c->ev_pair_ready, 0));   // the sort: later calls sort into the same arrays
+        return rc;
+    }
+    for (int pass = 0; pass < 2; ++pass) {
         chain.mesh = mesh[pass];
         chain.dipole = pass ? w : nullptr;
         if (c->own_fft) {
@@ -682,8 +685,7 @@ int launch_spme_hvp(tcp_ctx *c, const double *w, double *hw, const std::function
         if (cufftExecZ2D(c->hplan_b, c->hQk, mesh[pass]) != CUFFT_SUCCESS) return set_error(TCP_ERR_CUFFT, "cufftExecZ2D failed");
         c->launches++;
     }
-    TCP_CUDA(cudaStreamWaitEvent(c->stream, c->ev_join, 0));   // also after a failed real-space part
-    if (rc) return rc;
+    TCP_CUDA(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
     c->launches += chain_gather_hvp(chain, c->hQ, c->hdQ, w, hw, c->stream);
     TCP_CUDA(cudaGetLastError());
     return TCP_OK;
