@@ -4,8 +4,8 @@
 //
 // All state is FP64 SoA [3][n].  Every kernel that moves positions also
 // refreshes the two pair-kernel copies: 32-bit fixed point (int4) and
-// double4_32a.  Reductions write one partial per CTA; a single-CTA kernel sums
-// them in a fixed order, so results do not depend on scheduling.
+// double4_32a.  Reductions write one partial per CTA; the last CTA of the same
+// launch sums them in a fixed order, so results do not depend on scheduling.
 #include <cmath>
 
 #include "device_util.cuh"

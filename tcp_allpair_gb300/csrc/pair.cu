@@ -537,7 +537,7 @@ void make_pair_consts(tcp_ctx *c) {
     k.u_alpha = (float)(c->alpha * u);
     for (int t = 0; t < 3; ++t) {
         k.u_inv_dx[t] = dxs[t] > 0 ? (float)(u / dxs[t]) : 0.f;
-        // r/dx of rc, in the codes of rdf_add2; 4 of them are 5e-4 in r/dx, over
+        // r/dx of rc, in the codes of rdf_codes (pair_n3.cu); 4 of them are 5e-4 in r/dx, over
         // three times the FP32 error at r/dx = 500
         const double tlim = dxs[t] > 0 ? std::min(std::sqrt(c->rc2) / dxs[t], (double)kNbin) : (double)kNbin;
         const int code = (int)((tlim + kRdfEdge) * 8192.0) + 0x44c00000;

@@ -11,8 +11,9 @@
 
 namespace tcp {
 
-// Three warps per SM quarter hide the latency of the FP32 and integer work and
-// leave registers and shared memory for the reciprocal chain beside the launch.
+// Three warps per SM quarter hide the latency of the FP32 and integer work.  The
+// tables take 64 to 210 KB of shared memory: one CTA per SM, and no room for
+// the plane kernels of a reciprocal chain beside it, which run before or after.
 constexpr int kF64Threads = 384;
 constexpr int kF64Warps = kF64Threads / 32;
 

@@ -13,9 +13,12 @@
 //
 // cuFFT takes three launches each way for these sizes, and spread and
 // influence multiply one each; on small meshes every launch is a few
-// microseconds of latency.  The whole chain at N = 4,096, 32^3: 81 us with cuFFT,
-// 47 here; N = 16,384, 64^3: 97 and 69; N = 65,536, 128^3: 182 and 160; FP64 at
-// N = 4,096, 32^3: 127 and 75.
+// microseconds of latency.  The whole chain in us, cuFFT and here:
+//   N = 4,096, 32^3, order 4     FP32C 80  45   FP64 125  73
+//   N = 9,000, 48^3, order 6          112  76        166 135
+//   N = 16,384, 64^3, order 4          93  68        179 141
+//   N = 40,000, 96^3, order 5         145 125        381 339
+//   N = 65,536, 128^3, order 5        182 161        710 538
 //
 // A line of N = R1 R2 points is transformed in place in two passes of small
 // DFTs held in registers: over the R1 points R2 a + b of each b, times the
@@ -436,6 +439,13 @@ __global__ void __launch_bounds__(plane_threads<N, T>()) fft_inverse_kernel(cons
 }
 
 // ---------------------------------------------------------------------------
+// The lengths of the workloads in system.py, and 96 between the last two.  Others
+// are not built, each being a set of kernels: 72 or 144 would take the radices
+// that are there, 40, 56, 80 or 100 one of 5 or 7, and beyond about 150 points
+// a plane of 8-byte points (FP64, or two-float FP32) and its stage do not fit
+// in the shared memory of an SM.  With cuFFT the FP32C chain takes 78 us at N =
+// 4,096, 40^3, order 4, 126 at 24,000, 80^3, order 5, 137 at 40,000, 100^3,
+// order 5, where 32^3, 64^3 and 96^3 take 45, 105 and 125 here.
 bool fft_own(int K1, int K2, int K3) {
     return K1 == K2 && K2 == K3 && (K1 == 32 || K1 == 48 || K1 == 64 || K1 == 96 || K1 == 128);
 }

@@ -70,7 +70,7 @@ struct PairConsts {
     float u_p_alpha5;          // kErfc5P alpha u: the degree-5 erfc of the Newton-3 kernels
     int erfc5_ok;              // alpha rc <= kErfc5Xmax: the degree-5 fit covers the Ewald term
     float u_inv_dx[3], u_qq_force[3], u_qq_energy[3];
-    int u_rdf_lo[3], u_rdf_hi[3];   // RDF of the Newton-3 kernels: codes (rdf_add2) below lo lie inside rc and bin kNbin, from hi on outside
+    int u_rdf_lo[3], u_rdf_hi[3];   // RDF of the Newton-3 kernels: codes (rdf_codes) below lo lie inside rc and bin kNbin, from hi on outside
     // FP64 path
     double box[3];
     double rc2, alpha, rs, lambda;
